@@ -408,8 +408,8 @@ int prodm_batch_set_launch(prodm_batch* h, int threads_per_cta, int ctas_per_sm)
 int prodm_batch_set_stage_launch(prodm_batch* h, int stage, int threads_per_cta, int ctas_per_sm);
 /* tile shape of the fused finest levels: about this many values per unit of
  * consecutive fine rows (256..8192; default 2112 = 8 rows of 264); rows per
- * unit are a multiple of 8, at most 64, and a unit whose planes no longer fit
- * a TMA box takes the cp.async kernel */
+ * unit are a multiple of 8, at most 64, and fewer where that many no longer
+ * fit a TMA box (long rows: 4, 2 or 1) */
 int prodm_batch_set_fused_unit(prodm_batch* h, int values_per_unit);
 int prodm_batch_refactor(prodm_batch* h, void* stream);
 int prodm_batch_set_tolerances(prodm_batch* h, const double* h_tolerances, void* stream);

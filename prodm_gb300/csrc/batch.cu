@@ -51,8 +51,8 @@ struct RowSeg {
     uint32_t* key_l;        // decompose: level |max| key
     uint32_t* key_c;        // decompose at level 1: level-0 |max| key
     uint32_t patch;         // work items are patch items (decompose_ / recompose_patch_item), not rows:
-                            // every 2^k + 1 level of a batch (all fields' levels share one launch,
-                            // so the single-field path's minimum item count does not apply)
+                            // every level of a batch with rows of three values or more (all fields' levels
+                            // share one launch, so the single-field path's minimum item count does not apply)
 };
 
 // segment of global row g: binary search over the segments' first rows,
@@ -92,11 +92,9 @@ __global__ void __launch_bounds__(256, 3) k_decompose_multi(const RowSeg* __rest
         const RowSeg& q = segs[s];
         if (q.patch)
             decompose_patch_item<float>(q.in, q.s0, q.s1, q.F, q.C, q.coef, q.out, g - q.row_begin, lane, mk, mc);
-        else if (q.F.n[2] & 1u)
-            decompose_row_odd_any<float>(q.in, q.s0, q.s1, q.F, q.C, q.coef, q.out, nullptr, g - q.row_begin, lane,
-                                         mk, mc);
         else
-            decompose_row<float>(q.in, q.s0, q.s1, q.F, q.C, q.coef, q.out, nullptr, g - q.row_begin, lane, mk, mc);
+            decompose_row_any<float>(q.in, q.s0, q.s1, q.F, q.C, q.coef, q.out, nullptr, g - q.row_begin, lane, mk,
+                                     mc);
     }
     flush();
 }
@@ -110,10 +108,8 @@ __global__ void __launch_bounds__(256) k_recompose_multi(const RowSeg* __restric
         const RowSeg& q = segs[s];
         if (q.patch)
             recompose_patch_item<float>(q.in, q.coef, q.F, q.C, q.out, q.s0, q.s1, g - q.row_begin, lane);
-        else if (q.F.n[2] & 1u)
-            recompose_row_odd_any<float>(q.in, q.coef, q.F, q.C, q.out, q.s0, q.s1, g - q.row_begin, lane);
         else
-            recompose_row<float>(q.in, q.coef, q.F, q.C, q.out, q.s0, q.s1, g - q.row_begin, lane);
+            recompose_row_any<float>(q.in, q.coef, q.F, q.C, q.out, q.s0, q.s1, g - q.row_begin, lane);
     }
 }
 
@@ -188,15 +184,14 @@ struct prodm_batch {
     uint64_t echunks = 0, dchunks = 0;
     // finest levels decoded inside their recomposition: fields whose plane
     // runs fit a TMA box of at most 96 words (fseg[0]) or 160 words (fseg[1])
-    // (tensor maps in fmaps, one per field), fields with longer rows
-    // (fseg[2]: cp.async staging), and fields with rows of 257 values and up
-    // whose 11-row units fit a 96-word tall box (fseg[3]: the
+    // (tensor maps in fmaps, one per field), and fields with rows of 257
+    // values and up whose 11-row units fit a 96-word tall box (fseg[2]: the
     // warp-specialised batched kernel; before the other classes)
-    FusedSeg* fseg[4] = {nullptr, nullptr, nullptr, nullptr};
-    int fn[4] = {0, 0, 0, 0};
-    uint64_t funits[4] = {0, 0, 0, 0};
-    uint32_t ftld[4] = {0, 0, 0, 0};
-    uint32_t fbw[4] = {0, 0, 0, 0};                // widest TMA box of each class
+    FusedSeg* fseg[3] = {nullptr, nullptr, nullptr};
+    int fn[3] = {0, 0, 0};
+    uint64_t funits[3] = {0, 0, 0};
+    uint32_t ftld[3] = {0, 0, 0};
+    uint32_t fbw[3] = {0, 0, 0};                // widest TMA box of each class
     uint8_t* fmaps = nullptr;                      // [nf][128] tensor maps
     int* kstatus = nullptr;                        // status word of the fused kernels
     std::vector<char> fused;                       // per field
@@ -223,19 +218,81 @@ struct prodm_batch {
 namespace prodm {
 namespace {
 
-// a field's finest level is fused when its rows have odd length and an
-// 8-row unit's tiles fit the fused kernel's shared memory
-bool batch_field_fused(const LevelGeom& g) {
-    if (g.L < 1) return false;
-    const Box& F = g.box[g.L];
-    return (F.n[2] & 1u) && fused_multi_smem(fused_unit_blocks(F)) <= 200 * 1024;
-}
-
 int batch_build_segments(prodm_batch* h) {
     const int nf = h->nf, B = h->B;
     int rc;
+    // Fused finest levels: fields whose units fit a TMA box; longer rows (above
+    // about 4850 values) decode with the other levels and recompose in patch
+    // form. 64-field batch (2-D fields of 1025 and 2049 values a row among
+    // them): 2.01 ms with a cp.async kernel for rows above 600 values, 1.96 ms
+    // with those rows in patch form, 1.81 ms with units of 4, 2 and 1 rows.
     h->fused.assign(nf, 0);
-    for (int f = 0; f < nf; f++) h->fused[f] = batch_field_fused(h->g[f]) ? 1 : 0;
+    for (uint32_t& b : h->fbw) b = 0;
+    {
+        std::vector<FusedSeg> fs[3];
+        uint64_t units[3] = {0, 0, 0};
+        uint32_t tld[3] = {0, 0, 0};
+        std::vector<uint8_t> maps((size_t)nf * 128, 0);
+        if (!h->fmaps && (rc = h->alloc((void**)&h->fmaps, (size_t)nf * 128))) return rc;
+        for (int f = 0; f < nf; f++) {
+            const LevelGeom& g = h->g[f];
+            const int L = g.L;
+            if (L < 1) continue;
+            FusedSeg s{};
+            s.F = g.box[L];
+            s.C = g.box[L - 1];
+            const uint64_t nbk = (g.elems[L] + 31) / 32;
+            s.base = (const uint32_t*)(h->streams + h->lvl_stream_off[f][L]);
+            s.stride = (nbk + 3) / 4 * 4;
+            s.key = h->keys + f * kMaxL + L;
+            s.dnum = h->index + f * kMaxL + L;
+            float* rb0 = h->rbuf + h->cb_off[f];
+            float* rb1 = rb0 + h->cb_len[f];
+            s.coarse = (L == 1) ? h->rcoef + h->rcoef_off[f] + h->roff[f][0] : ((L - 1) & 1 ? rb1 : rb0);
+            s.out = h->outs[f];
+            s.s0 = (uint64_t)s.F.n[1] * s.F.n[2];
+            s.s1 = s.F.n[2];
+            s.rpu = fused_unit_rows(s.F, h->unit_values);
+            s.bw = fused_tma_box(s.F, s.rpu);
+            int k;
+            uint32_t t;
+            void* m = maps.data() + (size_t)f * 128;
+            const uint32_t wr = fused_ws_unit_rows();
+            const uint32_t wbw = (fused_unit_blocks_rows(s.F, wr) + 3 + 3) & ~3u;
+            if (batch_ws() && s.F.n[2] >= batch_ws_min_row() && B <= 32 && wbw <= kWsMultiStride &&
+                encode_plane_map(m, s.base, nbk, B, s.stride, kWsMultiStride, 32) == PRODM_OK) {
+                k = 2;
+                s.tall = 1;
+                s.bw = wbw;
+                s.rpu = wr;
+                t = fused_unit_blocks_rows(s.F, wr);
+            } else if ((s.tall = s.bw && fused_tma_tall() && B <= 32 &&
+                                 encode_plane_map(m, s.base, nbk, B, s.stride, fused_tma_stride(s.bw), 32) ==
+                                     PRODM_OK) ||
+                       (s.bw && encode_plane_map(m, s.base, nbk, B, s.stride, s.bw) == PRODM_OK)) {
+                k = s.bw <= 96 ? 0 : 1;
+                t = fused_unit_blocks_rows(s.F, s.rpu);
+            } else {
+                continue;
+            }
+            h->fused[f] = 1;
+            s.map = h->fmaps + (size_t)f * 128;
+            s.unit_begin = units[k];
+            units[k] += ((uint64_t)s.F.n[0] * s.F.n[1] + s.rpu - 1) / s.rpu;
+            tld[k] = std::max(tld[k], t);
+            fs[k].push_back(s);
+            h->fbw[k] = std::max(h->fbw[k], s.bw);
+        }
+        PRODM_CUDA(cudaMemcpy(h->fmaps, maps.data(), maps.size(), cudaMemcpyHostToDevice));
+        for (int k = 0; k < 3; k++) {
+            h->fn[k] = (int)fs[k].size();
+            h->funits[k] = units[k];
+            h->ftld[k] = tld[k];
+            if (fs[k].empty()) continue;
+            if (!h->fseg[k] && (rc = h->alloc((void**)&h->fseg[k], nf * sizeof(FusedSeg)))) return rc;
+            PRODM_CUDA(cudaMemcpy(h->fseg[k], fs[k].data(), fs[k].size() * sizeof(FusedSeg), cudaMemcpyHostToDevice));
+        }
+    }
     // decompose depths: depth d processes level L_f - d of every field with L_f - d >= 1
     h->dseg.assign(h->maxL, nullptr);
     h->rseg.assign(h->maxL, nullptr);
@@ -268,8 +325,8 @@ int batch_build_segments(prodm_batch* h) {
                 s.row_begin = drow;
                 s.key_l = h->keys + f * kMaxL + l;
                 s.key_c = l == 1 ? h->keys + f * kMaxL : nullptr;
-                s.patch = patch_grid(s.F, s.C) ? 1u : 0u;
-                drow += s.patch ? (uint32_t)patch_items(s.C) : s.F.n[0] * s.F.n[1];
+                s.patch = s.F.n[2] >= 3 ? 1u : 0u;
+                drow += s.patch ? (uint32_t)patch_items(s.F, s.C) : s.F.n[0] * s.F.n[1];
                 ds.push_back(s);
             }
             const int lr = d + 1;                 // recompose level at this depth
@@ -283,8 +340,8 @@ int batch_build_segments(prodm_batch* h) {
                 s.s0 = (uint64_t)s.F.n[1] * s.F.n[2];
                 s.s1 = s.F.n[2];
                 s.row_begin = rrow;
-                s.patch = patch_grid(s.F, s.C) ? 1u : 0u;
-                rrow += s.patch ? (uint32_t)patch_items(s.C) : s.F.n[0] * s.F.n[1];
+                s.patch = s.F.n[2] >= 3 ? 1u : 0u;
+                rrow += s.patch ? (uint32_t)patch_items(s.F, s.C) : s.F.n[0] * s.F.n[1];
                 rs.push_back(s);
             }
         }
@@ -299,74 +356,6 @@ int batch_build_segments(prodm_batch* h) {
         if (!rs.empty()) {
             if (!h->rseg[d] && (rc = h->alloc((void**)&h->rseg[d], nf * sizeof(RowSeg)))) return rc;
             PRODM_CUDA(cudaMemcpy(h->rseg[d], rs.data(), rs.size() * sizeof(RowSeg), cudaMemcpyHostToDevice));
-        }
-    }
-    // fused finest levels
-    {
-        std::vector<FusedSeg> fs[4];
-        uint64_t units[4] = {0, 0, 0, 0};
-        uint32_t tld[4] = {0, 0, 0, 0};
-        std::vector<uint8_t> maps((size_t)nf * 128, 0);
-        if (!h->fmaps && (rc = h->alloc((void**)&h->fmaps, (size_t)nf * 128))) return rc;
-        for (int f = 0; f < nf; f++) {
-            if (!h->fused[f]) continue;
-            const LevelGeom& g = h->g[f];
-            const int L = g.L;
-            FusedSeg s{};
-            s.F = g.box[L];
-            s.C = g.box[L - 1];
-            const uint64_t nbk = (g.elems[L] + 31) / 32;
-            s.base = (const uint32_t*)(h->streams + h->lvl_stream_off[f][L]);
-            s.stride = (nbk + 3) / 4 * 4;
-            s.key = h->keys + f * kMaxL + L;
-            s.dnum = h->index + f * kMaxL + L;
-            float* rb0 = h->rbuf + h->cb_off[f];
-            float* rb1 = rb0 + h->cb_len[f];
-            s.coarse = (L == 1) ? h->rcoef + h->rcoef_off[f] + h->roff[f][0] : ((L - 1) & 1 ? rb1 : rb0);
-            s.out = h->outs[f];
-            s.s0 = (uint64_t)s.F.n[1] * s.F.n[2];
-            s.s1 = s.F.n[2];
-            uint32_t t = fused_unit_blocks(s.F);
-            s.rpu = fused_unit_rows(s.F, h->unit_values);
-            s.bw = fused_tma_box(s.F, s.rpu);
-            int k = 2;
-            void* m = maps.data() + (size_t)f * 128;
-            const uint32_t wr = fused_ws_unit_rows();
-            const uint32_t wbw = (fused_unit_blocks_rows(s.F, wr) + 3 + 3) & ~3u;
-            if (batch_ws() && s.F.n[2] >= batch_ws_min_row() && B <= 32 && wbw <= kWsMultiStride &&
-                encode_plane_map(m, s.base, nbk, B, s.stride, kWsMultiStride, 32) == PRODM_OK) {
-                k = 3;
-                s.tall = 1;
-                s.bw = wbw;
-                s.rpu = wr;
-                s.map = h->fmaps + (size_t)f * 128;
-                t = fused_unit_blocks_rows(s.F, wr);
-            } else if ((s.tall = s.bw && fused_tma_tall() && B <= 32 &&
-                                 encode_plane_map(m, s.base, nbk, B, s.stride, fused_tma_stride(s.bw), 32) ==
-                                     PRODM_OK) ||
-                       (s.bw && encode_plane_map(m, s.base, nbk, B, s.stride, s.bw) == PRODM_OK)) {
-                k = s.bw <= 96 ? 0 : 1;
-                s.map = h->fmaps + (size_t)f * 128;
-                t = fused_unit_blocks_rows(s.F, s.rpu);
-            } else {
-                s.bw = 0;
-                s.map = nullptr;
-                s.rpu = 8;
-            }
-            s.unit_begin = units[k];
-            units[k] += ((uint64_t)s.F.n[0] * s.F.n[1] + s.rpu - 1) / s.rpu;
-            tld[k] = std::max(tld[k], t);
-            fs[k].push_back(s);
-            h->fbw[k] = std::max(h->fbw[k], s.bw);
-        }
-        PRODM_CUDA(cudaMemcpy(h->fmaps, maps.data(), maps.size(), cudaMemcpyHostToDevice));
-        for (int k = 0; k < 4; k++) {
-            h->fn[k] = (int)fs[k].size();
-            h->funits[k] = units[k];
-            h->ftld[k] = tld[k];
-            if (fs[k].empty()) continue;
-            if (!h->fseg[k] && (rc = h->alloc((void**)&h->fseg[k], nf * sizeof(FusedSeg)))) return rc;
-            PRODM_CUDA(cudaMemcpy(h->fseg[k], fs[k].data(), fs[k].size() * sizeof(FusedSeg), cudaMemcpyHostToDevice));
         }
     }
     // encode / decode: every (field, level); the decode skips fused finest levels
@@ -460,9 +449,7 @@ int batch_retrieve(prodm_batch* h, int interp, int est, double s, cudaStream_t s
         if (h->fn[k] && (rc = launch_decode_recompose_nb32_tma_multi(h->fseg[k], h->fn[k], h->funits[k], h->ftld[k],
                                                                     h->fbw[k], fc, h->kstatus, st)))
             return rc;
-    if (h->fn[2] && (rc = launch_decode_recompose_nb32_multi(h->fseg[2], h->fn[2], h->funits[2], h->ftld[2], fc, st)))
-        return rc;
-    if (h->fn[3] && (rc = launch_decode_recompose_nb32_ws_multi(h->fseg[3], h->fn[3], h->funits[3], h->ftld[3],
+    if (h->fn[2] && (rc = launch_decode_recompose_nb32_ws_multi(h->fseg[2], h->fn[2], h->funits[2], h->ftld[2],
                                                                  h->kstatus, st)))
         return rc;
     return PRODM_OK;

@@ -77,137 +77,36 @@ __device__ __forceinline__ uint32_t natural_of(uint32_t r, uint32_t n, uint32_t 
     return r < nc ? fine_of_coarse(r, n, nc) : 2 * (r - nc) + 1;
 }
 
-// CTA = 8 warps = 8 consecutive rows in the reordered (interleaved-rank)
-// order, so the CTA's coefficients form one contiguous rank range: the CTA
-// stages the retrieved planes of that range in shared memory with coalesced
-// loads, decodes them (one transpose per 32-value block) into a shared
-// coefficient buffer, then each warp writes its natural-order output row.
-__global__ void __launch_bounds__(256) k_decode_recompose_nb32(const uint32_t* __restrict__ base, uint64_t stride,
-                                                              const uint32_t* __restrict__ maxkey,
-                                                              const uint8_t* __restrict__ dnum,
-                                                              const float* __restrict__ coarse, Box F, Box C,
-                                                              float* __restrict__ out, uint64_t s0, uint64_t s1,
-                                                              uint32_t max_blocks) {
-    extern __shared__ uint32_t smem[];
-    uint32_t* tile = smem;                                   // [plane][max_blocks]
-    const uint32_t pad = max_blocks | 1u;                    // odd row length: conflict-free
-    float* cbuf = (float*)(smem + 32 * max_blocks);          // [32][pad]
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int num = dnum[0];
-    const int exp = frexp_exp(__uint_as_float(*maxkey)) + 2;
-    const int e = num;
-    const bool neg = num != 0 && (e & 1);
-    const bool dfast = (exp - e) >= -126 && (exp - e) <= 127;
-    const float dscale = dfast ? pow2f_(exp - e) : 1.f;
-    const uint32_t rows = F.n[0] * F.n[1];
-    const uint32_t n2 = F.n[2], c2n = C.n[2];
-    const uint64_t cs0 = (uint64_t)C.n[1] * C.n[2], cs1 = C.n[2];
-    auto row_info = [&](uint32_t rho, uint32_t& r0, uint32_t& r1, bool& cc, uint64_t& rbase, uint32_t& len) {
-        r0 = rho / F.n[1];
-        r1 = rho - r0 * F.n[1];
-        cc = r0 < C.n[0] && r1 < C.n[1];
-        rbase = level_rank(r0, r1, cc ? c2n : 0u, F, C);
-        len = cc ? n2 - c2n : n2;
-    };
-    for (uint32_t rho0 = blockIdx.x * 8; rho0 < rows; rho0 += gridDim.x * 8) {
-        const uint32_t rho_last = min(rho0 + 7, rows - 1);
-        uint32_t a0, a1, z0, z1, alen, zlen;
-        bool acc_, zcc;
-        uint64_t abase, zbase;
-        row_info(rho0, a0, a1, acc_, abase, alen);
-        row_info(rho_last, z0, z1, zcc, zbase, zlen);
-        const uint64_t fb = abase >> 5, lb = (zbase + zlen - 1) >> 5;
-        const uint32_t nbk = (uint32_t)(lb - fb + 1);
-        // stage the planes of blocks [fb, lb]
-        for (int p = warp; p < num; p += 8) {
-            const uint32_t* src = base + (uint64_t)p * stride + fb;
-            uint32_t* row = tile + p * max_blocks;
-            for (uint32_t j = lane; j < nbk; j += 32) row[j] = __ldcs(src + j);
-        }
-        __syncthreads();
-        // one thread per 32-value block: register transpose of the block's
-        // plane words; value e of block t goes to cbuf[e * pad + t]
-        for (uint32_t t = threadIdx.x; t < nbk; t += blockDim.x) {
-            uint32_t a[32];
-#pragma unroll
-            for (int p = 0; p < 32; p++) a[p] = p < num ? tile[p * max_blocks + t] : 0u;
-            transpose32_regs(a);
-#pragma unroll
-            for (int v = 0; v < 32; v++) {
-                const uint32_t acc = num ? (__brev(a[v]) >> (32 - num)) : 0u;
-                float val = num ? (dfast ? (float)nb_to_bin(acc) * dscale : ldexpf((float)nb_to_bin(acc), exp - e)) : 0.f;
-                cbuf[v * pad + t] = neg ? -val : val;
-            }
-        }
-        __syncthreads();
-        const uint32_t rho = rho0 + warp;
-        if (rho < rows) {
-            uint32_t r0, r1, len;
-            bool cc;
-            uint64_t rbase;
-            row_info(rho, r0, r1, cc, rbase, len);
-            const uint32_t x0 = natural_of(r0, F.n[0], C.n[0]), x1 = natural_of(r1, F.n[1], C.n[1]);
-            const int m01 = (is_coarse(x0, F.n[0]) ? 0 : 1) | (is_coarse(x1, F.n[1]) ? 0 : 2);
-            const uint32_t c0 = (m01 & 1) ? (x0 >> 1) : r0;
-            const uint32_t c1 = (m01 & 2) ? (x1 >> 1) : r1;
-            const float* cb0 = coarse + c0 * cs0 + c1 * cs1;
-            int64_t co[4];
-            if (m01 == 0) { co[0] = 0; }
-            else if (m01 == 1) { co[0] = 0; co[1] = (int64_t)cs0; }
-            else if (m01 == 2) { co[0] = 0; co[1] = (int64_t)cs1; }
-            else { co[0] = 0; co[1] = (int64_t)cs1; co[2] = (int64_t)cs0; co[3] = (int64_t)(cs0 + cs1); }
-            const int nq = corner_count(m01);
-            float* orow = out + x0 * s0 + x1 * s1;
-            const uint32_t rb0 = (uint32_t)(rbase - fb * 32);
-            auto coefat = [&](uint32_t off) { const uint32_t r = rb0 + off; return cbuf[(r & 31) * pad + (r >> 5)]; };
-            for (uint32_t cbase = 0; cbase < c2n; cbase += 32) {
-                const uint32_t c2 = cbase + lane;
-                const bool act = c2 < c2n;
-                const bool odd = act && c2 + 1 < c2n && fine_of_coarse(c2 + 1, n2, c2n) == 2 * c2 + 2;
-                float q[4] = {0.f, 0.f, 0.f, 0.f}, qn[4];
-#pragma unroll
-                for (int i = 0; i < 4; i++)
-                    if (i < nq && act) q[i] = __ldg(cb0 + c2 + co[i]);
-#pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    qn[i] = __shfl_down_sync(FULL, q[i], 1);
-                    if (i < nq && lane == 31 && odd) qn[i] = __ldg(cb0 + c2 + 1 + co[i]);
-                }
-                if (act) {
-                    const uint32_t xe = fine_of_coarse(c2, n2, c2n);
-                    orow[xe] = m01 == 0 ? q[0] : __fadd_rn(coefat(cc ? c2 - c2n : c2), corner_tree(m01, q));
-                    if (odd) orow[2 * c2 + 1] = __fadd_rn(coefat(cc ? c2 : c2n + c2), corner_tree_mid(m01, q, qn));
-                }
-            }
-        }
-        __syncthreads();
-    }
-}
-
 // ---------------------------------------------------------------------------
-// Odd row length (n = 2^k + 1 and every other odd n): fine node 2c of a row is
-// coarse node c and the odd node 2c+1 lies between coarse nodes c and c+1, so
-// the row walk needs no index remapping. The planes of the next 8 rows are
-// fetched with cp.async into a second tile while the current rows are decoded
-// and recomposed; the coefficient buffer is value-major ([block][33]).
+// Rows: coarse column c of a row of n values sits at node 2c, except the last
+// one at node n - 1, and the odd node 2c + 1 of the column pairs c < P = n -
+// c2n lies between coarse columns c and c + 1 (odd n: P = c2n - 1 pairs and
+// one lone column; even n: P = c2n - 2 and two). The CTA's rows are
+// consecutive in the reordered (interleaved-rank) order, so its coefficients
+// form one contiguous rank range; the coefficient buffer is value-major.
 // ---------------------------------------------------------------------------
 constexpr int CB_LD = 36;   // value-major coefficient rows: conflict-free both ways
 
 __device__ __forceinline__ float cb_at(const float* cb, uint32_t r) { return cb[(r >> 5) * CB_LD + (r & 31)]; }
 
-// one fine row of odd length n = 2 c2n - 1; M01 = odd-dim mask over dims
-// 0/1 (0: both coarse -> only odd nodes carry coefficients, ranks c;
-// otherwise even node 2c has rank c and odd node 2c+1 rank c2n + c). The row
-// is c2n - 1 column pairs (nodes 2c, 2c+1) and a last node 2(c2n - 1). Lane l
-// handles the pairs 32k + l; the corner values of D column groups are in
-// flight at once (a ring of D groups in registers, refilled as each group is
-// used), so a row waits for the L2 latency about once instead of once per
-// group. Groups in which every lane has a pair run without bounds checks, on
-// pointers advanced once per D groups; the last node is written by lane 0.
-template <int M01, bool DEEP = false>
-__device__ __forceinline__ void recompose_row_odd(const float* __restrict__ cb0, uint64_t cs0, uint64_t cs1,
-                                                  uint32_t c2n, const float* __restrict__ cb, uint32_t rb0,
-                                                  float* __restrict__ orow, int lane) {
+// one fine row of n2 values; M01 = odd-dim mask over dims 0/1 (0: both coarse
+// -> only odd nodes carry coefficients, ranks c; otherwise the node of coarse
+// column c has rank c and odd node 2c+1 rank c2n + c). Lane l handles the
+// pairs 32k + l; the corner values of D column groups are in flight at once
+// (a ring of D groups in registers, refilled as each group is used), so a row
+// waits for the L2 latency about once instead of once per group. Groups in
+// which every lane has a pair run without bounds checks, on pointers advanced
+// once per D groups; the lone columns are written by lanes 0 (and 1).
+// Measured on even rows, 100 x 500 x 500 fp32: the finest level's retrieval
+// 106 us with one thread per block and remapped indices per column, 51 us
+// through these rows in the warp-specialised kernel. SPLIT: the warp takes
+// part `part` of `parts` of the row's column groups (long rows, several warps
+// per row).
+template <int M01, bool DEEP, bool SPLIT>
+__device__ __forceinline__ void recompose_row(const float* __restrict__ cb0, uint64_t cs0, uint64_t cs1, uint32_t n2,
+                                              uint32_t c2n, const float* __restrict__ cb, uint32_t rb0,
+                                              float* __restrict__ orow, int lane, uint32_t part = 0,
+                                              uint32_t parts = 1) {
     constexpr int NQ = M01 == 0 ? 1 : (M01 == 3 ? 4 : 2);
     constexpr int D = DEEP ? (M01 == 3 ? 4 : 6) : (M01 == 3 ? 3 : 4);   // column groups in flight
     int64_t co[NQ];   // corner row offsets, in corner_tree order
@@ -218,30 +117,32 @@ __device__ __forceinline__ void recompose_row_odd(const float* __restrict__ cb0,
         co[2] = (int64_t)cs0;
         co[3] = (int64_t)(cs0 + cs1);
     }
-    const uint32_t P = c2n - 1;
-    if (lane == 0) {   // the last node: coarse column P
+    const uint32_t P = n2 - c2n;
+    if ((!SPLIT || part == 0) && P + lane < c2n) {   // a lone column
+        const uint32_t c = P + lane, x = min(2 * c, n2 - 1);
         float q[NQ];
 #pragma unroll
-        for (int i = 0; i < NQ; i++) q[i] = __ldg(cb0 + P + co[i]);
-        if constexpr (M01 == 0) orow[2 * (uint64_t)P] = q[0];
-        else orow[2 * (uint64_t)P] = __fadd_rn(cb_at(cb, rb0 + P), corner_tree(M01, q));
+        for (int i = 0; i < NQ; i++) q[i] = __ldg(cb0 + c + co[i]);
+        if constexpr (M01 == 0) orow[x] = q[0];
+        else orow[x] = __fadd_rn(cb_at(cb, rb0 + c), corner_tree(M01, q));
     }
     if (P == 0) return;
+    const uint32_t all = (P + 31) >> 5;
+    const uint32_t g0 = SPLIT ? part * all / parts : 0u, groups = SPLIT ? (part + 1) * all / parts : all;
+    const uint32_t full = SPLIT ? min(P >> 5, groups) : P >> 5;
     const float* pc[NQ];
 #pragma unroll
-    for (int i = 0; i < NQ; i++) pc[i] = cb0 + co[i] + lane;
-    // coefficient of rank r at cb[r + (r >> 5)]: 33 floats further per 32 ranks
+    for (int i = 0; i < NQ; i++) pc[i] = cb0 + co[i] + lane + 32 * g0;
     const uint32_t re = rb0 + lane, ro = rb0 + (M01 == 0 ? 0u : c2n) + lane;
-    const float* pe = cb + (re >> 5) * CB_LD + (re & 31);
-    const float* po = cb + (ro >> 5) * CB_LD + (ro & 31);
-    float* o = orow + 2 * lane;
+    const float* pe = cb + ((re >> 5) + g0) * CB_LD + (re & 31);
+    const float* po = cb + ((ro >> 5) + g0) * CB_LD + (ro & 31);
+    float* o = orow + 2 * lane + 64 * g0;
     const int lim = (int)c2n - lane;   // column 32k + lane exists <=> 32k < lim
-    const uint32_t groups = (P + 31) >> 5, full = P >> 5;
     float ring[D][NQ];
 #pragma unroll
     for (int d = 0; d < D; d++)
 #pragma unroll
-        for (int i = 0; i < NQ; i++) ring[d][i] = 32 * d < lim ? __ldg(pc[i] + 32 * d) : 0.f;
+        for (int i = 0; i < NQ; i++) ring[d][i] = (int)(32 * (g0 + d)) < lim ? __ldg(pc[i] + 32 * d) : 0.f;
     const int src = (lane + 1) & 31;
     auto pair = [&](const float (&q)[NQ], const float (&qn)[NQ], const float* e, const float* od, float* out) {
         if constexpr (M01 == 0) {
@@ -256,7 +157,7 @@ __device__ __forceinline__ void recompose_row_odd(const float* __restrict__ cb0,
             out[1] = __fadd_rn(*od, avg_rn(avg_rn(q[0], qn[0]), avg_rn(q[1], qn[1])));
         }
     };
-    uint32_t k0 = 0;
+    uint32_t k0 = g0;
     for (; k0 + D <= full; k0 += D) {
 #pragma unroll
         for (int d = 0; d < D; d++) {
@@ -313,7 +214,7 @@ __device__ __forceinline__ void fused_row_rank(uint32_t rho, const Box& F, const
 
 // block range [fb, fb + nbk) of the coefficients of rows [rho0, rho0 + nr)
 __device__ __forceinline__ void fused_block_range(uint32_t rho0, uint32_t rows, const Box& F, const Box& C,
-                                                  uint64_t& fb, uint32_t& nbk, uint32_t nr = 8) {
+                                                  uint64_t& fb, uint32_t& nbk, uint32_t nr) {
     const uint32_t rho_last = min(rho0 + nr - 1, rows - 1);
     uint32_t a0, a1, z0, z1, alen, zlen;
     bool acc_, zcc;
@@ -350,205 +251,33 @@ __device__ __forceinline__ FusedRow fused_row(uint32_t rho, const Box& F, const 
     return r;
 }
 
-// one warp: a fine row (odd length) from the coarse box and the decoded
+// one warp: a fine row of n2 values from the coarse box and the decoded
 // coefficients in cb (value v of block t at cb[t * CB_LD + v], block fb first)
-template <bool DEEP = false>
-__device__ __forceinline__ void recompose_fine_row(const FusedRow& r, const Box& C, const float* __restrict__ coarse,
-                                                   float* __restrict__ out, const float* __restrict__ cb, int lane) {
+template <bool DEEP, bool SPLIT = false>
+__device__ __forceinline__ void recompose_fine_row(const FusedRow& r, uint32_t n2, const Box& C,
+                                                   const float* __restrict__ coarse, float* __restrict__ out,
+                                                   const float* __restrict__ cb, int lane, uint32_t part = 0,
+                                                   uint32_t parts = 1) {
     const uint32_t c2n = C.n[2];
     const uint64_t cs0 = (uint64_t)C.n[1] * C.n[2], cs1 = C.n[2];
     const float* cb0 = coarse + r.coarse_off;
     float* orow = out + r.out_off;
     const uint32_t rb0 = r.rb;
     switch (r.m01) {
-        case 0: recompose_row_odd<0, DEEP>(cb0, cs0, cs1, c2n, cb, rb0, orow, lane); break;
-        case 1: recompose_row_odd<1, DEEP>(cb0, cs0, cs1, c2n, cb, rb0, orow, lane); break;
-        case 2: recompose_row_odd<2, DEEP>(cb0, cs0, cs1, c2n, cb, rb0, orow, lane); break;
-        default: recompose_row_odd<3, DEEP>(cb0, cs0, cs1, c2n, cb, rb0, orow, lane); break;
+        case 0: recompose_row<0, DEEP, SPLIT>(cb0, cs0, cs1, n2, c2n, cb, rb0, orow, lane, part, parts); break;
+        case 1: recompose_row<1, DEEP, SPLIT>(cb0, cs0, cs1, n2, c2n, cb, rb0, orow, lane, part, parts); break;
+        case 2: recompose_row<2, DEEP, SPLIT>(cb0, cs0, cs1, n2, c2n, cb, rb0, orow, lane, part, parts); break;
+        default: recompose_row<3, DEEP, SPLIT>(cb0, cs0, cs1, n2, c2n, cb, rb0, orow, lane, part, parts); break;
     }
-}
-
-// decode of a staged tile: two threads per 32-value block, each transposing
-// one half; rows are taken in reverse tile order, so that value v's word has
-// plane p at bit num - 1 - p, its negabinary digits in place
-// (NegaBinaryBPEncoder.hpp:132-192); value v of block t -> cb[t * CB_LD + v].
-// FAST: 2^(exp - num) is a normal float (one exact multiplication).
-template <bool FAST>
-__device__ __forceinline__ void decode_tile(const uint32_t* __restrict__ tile, float* __restrict__ cb, uint32_t nbk,
-                                            int num, int exp, bool neg, float dscale) {
-    for (uint32_t i = threadIdx.x; i < 2 * nbk; i += blockDim.x) {
-        const uint32_t t = i >> 1;
-        const int half = i & 1;
-        float* dst = cb + t * CB_LD + 16 * half;
-        // row r of the transpose is tile word 31 - r: words 4q.. (rows
-        // 31-4q..28-4q) meet words 16+4q.. (rows 15-4q..12-4q) in the first
-        // stage, so each pair of 16-byte reads is consumed at once
-        const uint4* src = reinterpret_cast<const uint4*>(tile + t * TB_LD);
-        const uint32_t sel16 = half ? 0x7632u : 0x5410u;
-        uint32_t a[16];
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const uint4 hi = src[q], lo = src[q + 4];
-            a[15 - 4 * q] = __byte_perm(lo.x, hi.x, sel16);
-            a[14 - 4 * q] = __byte_perm(lo.y, hi.y, sel16);
-            a[13 - 4 * q] = __byte_perm(lo.z, hi.z, sel16);
-            a[12 - 4 * q] = __byte_perm(lo.w, hi.w, sel16);
-        }
-        transpose32_half_tail(a);
-        float f[16];
-#pragma unroll
-        for (int v = 0; v < 16; v++) {
-            const int32_t iv = nb_to_bin(a[v]);
-            if constexpr (FAST) f[v] = (float)iv * dscale;
-            else f[v] = neg ? -ldexpf((float)iv, exp - num) : ldexpf((float)iv, exp - num);
-        }
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-            reinterpret_cast<float4*>(dst)[q] = make_float4(f[4 * q], f[4 * q + 1], f[4 * q + 2], f[4 * q + 3]);
-    }
-}
-
-
-__global__ void __launch_bounds__(256, 5) k_decode_recompose_nb32_odd(const uint32_t* __restrict__ base, uint64_t stride,
-                                                                  const uint32_t* __restrict__ maxkey,
-                                                                  const uint8_t* __restrict__ dnum,
-                                                                  const float* __restrict__ coarse, Box F, Box C,
-                                                                  float* __restrict__ out, uint64_t s0, uint64_t s1,
-                                                                  uint32_t tld) {
-    extern __shared__ __align__(16) uint32_t smem[];
-    uint32_t* tiles = smem;                                  // [block][TB_LD]
-    float* cb = (float*)(smem + TB_LD * tld);                // [block][CB_LD]
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int num = dnum[0];
-    const int exp = frexp_exp(__uint_as_float(*maxkey)) + 2;
-    const bool neg = num != 0 && (num & 1);                  // NegaBinaryBPEncoder.hpp:153, :177
-    const bool dfast = (exp - num) >= -126 && (exp - num) <= 127;
-    const float dscale = dfast ? (neg ? -pow2f_(exp - num) : pow2f_(exp - num)) : 1.f;
-    const uint32_t rows = F.n[0] * F.n[1];
-    auto block_range = [&](uint32_t r, uint64_t& fb, uint32_t& nbk) { fused_block_range(r, rows, F, C, fb, nbk); };
-    // plane p of block j -> tile[j * TB_LD + 32 - num + p] (so that the
-    // transposed words hold plane p at bit num - 1 - p); warp w copies planes
-    // w, w+8, ..
-    const int poff = 32 - num;
-    auto fetch = [&](uint64_t fb, uint32_t nbk, uint32_t* tile) {
-        for (int p = warp; p < num; p += 8) {
-            const uint32_t* src = base + (uint64_t)p * stride + fb;
-            for (uint32_t j = lane; j < nbk; j += 32) cp_async4(tile + j * TB_LD + poff + p, src + j);
-        }
-        cp_async_commit();
-    };
-    uint32_t rho0 = blockIdx.x * 8;
-    if (rho0 >= rows) return;
-    // block ranges of the CTA's iterations, computed by one thread two
-    // iterations ahead: slot k % 3 holds iteration k's range
-    __shared__ uint64_t s_fb[3];
-    __shared__ uint32_t s_nbk[3];
-    const uint32_t step = gridDim.x * 8;
-    if (threadIdx.x == 0) {
-        block_range(rho0, s_fb[0], s_nbk[0]);
-        if (rho0 + step < rows) block_range(rho0 + step, s_fb[1], s_nbk[1]);
-    }
-    // the tile words of the planes not retrieved stay zero
-    for (uint32_t i = threadIdx.x; i < tld * poff; i += blockDim.x) {
-        const uint32_t row = i / poff, p = i - row * poff;
-        tiles[row * TB_LD + p] = 0u;
-    }
-    __syncthreads();
-    fetch(s_fb[0], s_nbk[0], tiles);
-    for (int it = 0; rho0 < rows; it++, rho0 += step) {
-        const uint32_t* tile = tiles;
-        cp_async_wait_all();
-        __syncthreads();
-        const uint64_t fb = s_fb[it % 3];
-        const uint32_t nbk = s_nbk[it % 3];
-        if (threadIdx.x == 0 && rho0 + 2 * step < rows) block_range(rho0 + 2 * step, s_fb[(it + 2) % 3], s_nbk[(it + 2) % 3]);
-        if (dfast) decode_tile<true>(tile, cb, nbk, num, exp, neg, dscale);
-        else decode_tile<false>(tile, cb, nbk, num, exp, neg, dscale);
-        __syncthreads();
-        // the tile is free again: fetch the next rows' planes during the recomposition
-        if (rho0 + step < rows) fetch(s_fb[(it + 1) % 3], s_nbk[(it + 1) % 3], tiles);
-        const uint32_t rho = rho0 + warp;
-        if (rho < rows) recompose_fine_row(fused_row(rho, F, C, s0, s1, fb), C, coarse, out, cb, lane);
-    }
-    cp_async_wait_all();
-}
-
-// The finest levels of many fields in one persistent launch (the batched
-// retrieval): the global 8-row units of all segments are walked as in
-// k_decode_recompose_nb32_odd, with each unit's field looked up in the segment
-// table (one segment per field, odd row lengths). The plane count, exponent
-// and decode scale are the unit's field's; a fetch zeroes the tile words of
-// the planes its field did not retrieve. Staging, decode and recomposition
-// are those of the single-field kernel, so the results are bit-identical.
-__global__ void __launch_bounds__(256, 4) k_decode_recompose_nb32_multi(const FusedSeg* __restrict__ segs, int nseg,
-                                                                       uint64_t total, uint32_t tld) {
-    extern __shared__ __align__(16) uint32_t smem[];
-    uint32_t* tiles = smem;                                  // [block][TB_LD]
-    float* cb = (float*)(smem + TB_LD * tld);                // [block][CB_LD]
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    __shared__ int s_seg[3];
-    __shared__ uint64_t s_fb[3];
-    __shared__ uint32_t s_nbk[3];
-    const uint64_t step = gridDim.x;
-    uint64_t u = blockIdx.x;
-    if (u >= total) return;
-    // thread 0: the field and block range of unit g into slot k
-    auto plan = [&](uint64_t g, int k) {
-        const int s = find_seg(segs, nseg, g, &FusedSeg::unit_begin);
-        const FusedSeg& q = segs[s];
-        s_seg[k] = s;
-        fused_block_range((uint32_t)(g - q.unit_begin) * 8, q.F.n[0] * q.F.n[1], q.F, q.C, s_fb[k], s_nbk[k]);
-    };
-    auto fetch = [&](int k) {
-        const FusedSeg& q = segs[s_seg[k]];
-        const int num = *q.dnum;
-        const int poff = 32 - num;
-        const uint64_t fb = s_fb[k];
-        const uint32_t nbk = s_nbk[k];
-        for (uint32_t i = threadIdx.x; i < nbk * (uint32_t)poff; i += blockDim.x) {
-            const uint32_t row = i / poff, p = i - row * poff;
-            tiles[row * TB_LD + p] = 0u;
-        }
-        for (int p = warp; p < num; p += 8) {
-            const uint32_t* src = q.base + (uint64_t)p * q.stride + fb;
-            for (uint32_t j = lane; j < nbk; j += 32) cp_async4(tiles + j * TB_LD + poff + p, src + j);
-        }
-        cp_async_commit();
-    };
-    if (threadIdx.x == 0) {
-        plan(u, 0);
-        if (u + step < total) plan(u + step, 1);
-    }
-    __syncthreads();
-    fetch(0);
-    for (int it = 0; u < total; it++, u += step) {
-        cp_async_wait_all();
-        __syncthreads();
-        const int k = it % 3;
-        const FusedSeg& q = segs[s_seg[k]];
-        const uint64_t fb = s_fb[k];
-        const uint32_t nbk = s_nbk[k];
-        if (threadIdx.x == 0 && u + 2 * step < total) plan(u + 2 * step, (it + 2) % 3);
-        const int num = *q.dnum;
-        const int exp = frexp_exp(__uint_as_float(*q.key)) + 2;
-        const bool neg = num != 0 && (num & 1);              // NegaBinaryBPEncoder.hpp:153, :177
-        const bool dfast = (exp - num) >= -126 && (exp - num) <= 127;
-        const float dscale = dfast ? (neg ? -pow2f_(exp - num) : pow2f_(exp - num)) : 1.f;
-        if (dfast) decode_tile<true>(tiles, cb, nbk, num, exp, neg, dscale);
-        else decode_tile<false>(tiles, cb, nbk, num, exp, neg, dscale);
-        __syncthreads();
-        // the tile is free again: fetch the next unit's planes during the recomposition
-        if (u + step < total) fetch((it + 1) % 3);
-        const uint32_t rows = q.F.n[0] * q.F.n[1];
-        const uint32_t rho = (uint32_t)(u - q.unit_begin) * 8 + warp;
-        if (rho < rows) recompose_fine_row(fused_row(rho, q.F, q.C, q.s0, q.s1, fb), q.C, q.coarse, q.out, cb, lane);
-    }
-    cp_async_wait_all();
 }
 
 // decode of a plane-major tile (row 32 - num + p = plane p, rows below zero;
-// block t of the range at column t): the same half transposes, each thread
-// reading its block's 32 rows and combining rows 31-k and 15-k at once
+// block t of the range at column t): two threads per 32-value block, each
+// transposing one half; rows are taken in reverse tile order, so that value
+// v's word has plane p at bit num - 1 - p, its negabinary digits in place
+// (NegaBinaryBPEncoder.hpp:132-192); value v of block t -> cb[t * CB_LD + v].
+// Each thread reads its block's 32 rows and combines rows 31-k and 15-k at
+// once. FAST: 2^(exp - num) is a normal float (one exact multiplication).
 template <bool FAST, int RS>
 __device__ __forceinline__ void decode_tile_pm(const uint32_t* __restrict__ tile, float* __restrict__ cb,
                                                uint32_t nbk, int num, int exp, bool neg, float dscale,
@@ -576,7 +305,8 @@ __device__ __forceinline__ void decode_tile_pm(const uint32_t* __restrict__ tile
     }
 }
 
-// Odd row length, planes staged by TMA: per CTA iteration (8 rows) one
+// Planes staged by TMA: per CTA iteration (nr = 8, 4, 2 or 1 rows, 8 / nr
+// warps per row: SPLIT unless nr is 8) one
 // elected warp issues one 2-D tensor copy per retrieved plane (box: `bw`
 // words of that plane's row, from the 16-byte aligned block fb & ~3) into the
 // plane-major tile, completing on an mbarrier; the copy for the next
@@ -586,11 +316,12 @@ __device__ __forceinline__ void decode_tile_pm(const uint32_t* __restrict__ tile
 // (bounded again) for its copies in flight and returns. `tx_extra` raises the
 // expected byte count (0 in normal use; a positive value makes every wait run
 // out, which is how the timeout path is tested).
-template <int RS>
+template <int RS, bool SPLIT>
 __global__ void __launch_bounds__(256, 5) k_decode_recompose_nb32_tma(
     const __grid_constant__ CUtensorMap tmap, uint32_t bw, const uint32_t* __restrict__ maxkey,
     const uint8_t* __restrict__ dnum, const float* __restrict__ coarse, Box F, Box C, float* __restrict__ out,
-    uint64_t s0, uint64_t s1, int* __restrict__ status, long long wait_limit, uint32_t tx_extra, int tall) {
+    uint64_t s0, uint64_t s1, uint32_t nr, int* __restrict__ status, long long wait_limit, uint32_t tx_extra,
+    int tall) {
     extern __shared__ __align__(128) uint32_t tma_smem[];
     uint32_t* tile = tma_smem;                               // [32][RS] plane-major
     float* cb = (float*)(tma_smem + 32 * RS);                // [block][CB_LD]
@@ -598,7 +329,7 @@ __global__ void __launch_bounds__(256, 5) k_decode_recompose_nb32_tma(
     __shared__ uint64_t s_fb[3];
     __shared__ uint32_t s_nbk[3];
     __shared__ FusedRow s_row[2][8];   // the rows of iterations it (slot it & 1) and it + 1
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int num = dnum[0];
     const int exp = frexp_exp(__uint_as_float(*maxkey)) + 2;
     const bool neg = num != 0 && (num & 1);                  // NegaBinaryBPEncoder.hpp:153, :177
@@ -606,21 +337,21 @@ __global__ void __launch_bounds__(256, 5) k_decode_recompose_nb32_tma(
     const float dscale = dfast ? (neg ? -pow2f_(exp - num) : pow2f_(exp - num)) : 1.f;
     const uint32_t rows = F.n[0] * F.n[1];
     const int poff = 32 - num;
-    // lanes 0..7 of warp 0: the rows of the iteration starting at r, block range fb
+    // lanes of warp 0: the rows of the iteration starting at r, block range fb
     auto rows_of = [&](uint32_t r, uint64_t fb, FusedRow* slot) {
-        if (lane < 8 && r + lane < rows) slot[lane] = fused_row(r + lane, F, C, s0, s1, fb);
+        if (lane < nr && r + lane < rows) slot[lane] = fused_row(r + lane, F, C, s0, s1, fb);
     };
-    uint32_t rho0 = blockIdx.x * 8;
+    uint32_t rho0 = blockIdx.x * nr;
     if (rho0 >= rows) return;
     if ((smem_addr(tile) & 127u) != 0) {   // TMA destinations need 128-byte alignment
         if (threadIdx.x == 0) atomicExch(status, PRODM_ECUDA);
         return;
     }
-    const uint32_t step = gridDim.x * 8;
+    const uint32_t step = gridDim.x * nr;
     if (threadIdx.x == 0) {
         mbar_init(&bar, 1);
-        fused_block_range(rho0, rows, F, C, s_fb[0], s_nbk[0]);
-        if (rho0 + step < rows) fused_block_range(rho0 + step, rows, F, C, s_fb[1], s_nbk[1]);
+        fused_block_range(rho0, rows, F, C, s_fb[0], s_nbk[0], nr);
+        if (rho0 + step < rows) fused_block_range(rho0 + step, rows, F, C, s_fb[1], s_nbk[1], nr);
     }
     if (!tall)
         for (uint32_t i = threadIdx.x; i < (uint32_t)poff * RS; i += blockDim.x) tile[i] = 0u;   // planes not retrieved
@@ -654,7 +385,7 @@ __global__ void __launch_bounds__(256, 5) k_decode_recompose_nb32_tma(
         const uint64_t fb = s_fb[it % 3];
         const uint32_t nbk = s_nbk[it % 3];
         if (threadIdx.x == 0 && rho0 + 2 * step < rows)
-            fused_block_range(rho0 + 2 * step, rows, F, C, s_fb[(it + 2) % 3], s_nbk[(it + 2) % 3]);
+            fused_block_range(rho0 + 2 * step, rows, F, C, s_fb[(it + 2) % 3], s_nbk[(it + 2) % 3], nr);
         const uint32_t* t0 = tile + (fb & 3u);
         if (dfast) decode_tile_pm<true, RS>(t0, cb, nbk, num, exp, neg, dscale);
         else decode_tile_pm<false, RS>(t0, cb, nbk, num, exp, neg, dscale);
@@ -665,7 +396,9 @@ __global__ void __launch_bounds__(256, 5) k_decode_recompose_nb32_tma(
             issue(s_fb[(it + 1) % 3]);
             rows_of(rho0 + step, s_fb[(it + 1) % 3], s_row[(it + 1) & 1]);
         }
-        if (rho0 + warp < rows) recompose_fine_row(s_row[it & 1][warp], C, coarse, out, cb, lane);
+        const uint32_t parts = SPLIT ? 8u / nr : 1u, r = SPLIT ? warp / parts : warp;
+        if (rho0 + r < rows)
+            recompose_fine_row<false, SPLIT>(s_row[it & 1][r], F.n[2], C, coarse, out, cb, lane, warp % parts, parts);
     }
 }
 
@@ -780,8 +513,15 @@ __global__ void __launch_bounds__(256, 5) k_decode_recompose_nb32_tma_multi(cons
         }
         const uint32_t rows = q.F.n[0] * q.F.n[1];
         const uint32_t rho0 = (uint32_t)(u - q.unit_begin) * q.rpu;
-        for (uint32_t r = warp; r < q.rpu && rho0 + r < rows; r += 8)
-            recompose_fine_row(s_row[it & 1][r], q.C, q.coarse, q.out, cb, lane);
+        if (q.rpu < 8) {   // long rows: 8 / rpu warps per row
+            const uint32_t parts = 8u / q.rpu, r = warp / parts;
+            if (rho0 + r < rows)
+                recompose_fine_row<false, true>(s_row[it & 1][r], q.F.n[2], q.C, q.coarse, q.out, cb, lane,
+                                                warp % parts, parts);
+        } else {
+            for (uint32_t r = warp; r < q.rpu && rho0 + r < rows; r += 8)
+                recompose_fine_row<false>(s_row[it & 1][r], q.F.n[2], q.C, q.coarse, q.out, cb, lane);
+        }
     }
 }
 
@@ -915,7 +655,7 @@ __global__ void __launch_bounds__(512, 2) k_decode_recompose_nb32_ws(
                 return;
             }
             const FusedRow r = s_row[b][rw];
-            if (r.m01 >= 0) recompose_fine_row<true>(r, C, coarse, out, cbs + (size_t)b * tld * CB_LD, lane);
+            if (r.m01 >= 0) recompose_fine_row<true>(r, F.n[2], C, coarse, out, cbs + (size_t)b * tld * CB_LD, lane);
             mbar_arrive(&bar_empty[b]);
         }
     }
@@ -1038,7 +778,7 @@ __global__ void __launch_bounds__(512, 2) k_decode_recompose_nb32_ws_multi(const
             }
             const FusedRow r = s_row[b][rw];
             const FusedSeg& q = segs[s_rseg[b]];
-            if (r.m01 >= 0) recompose_fine_row<true>(r, q.C, q.coarse, q.out, cbs + (size_t)b * tld * CB_LD, lane);
+            if (r.m01 >= 0) recompose_fine_row<true>(r, q.F.n[2], q.C, q.coarse, q.out, cbs + (size_t)b * tld * CB_LD, lane);
             mbar_arrive(&bar_empty[b]);
         }
     }
@@ -1046,16 +786,18 @@ __global__ void __launch_bounds__(512, 2) k_decode_recompose_nb32_ws_multi(const
 
 }  // namespace
 
-static uint32_t fused_max_blocks(const Box& F) { return (8 * F.n[2] + 31) / 32 + 2; }
-static size_t fused_smem(const Box& F) {
-    const uint32_t mb = fused_max_blocks(F);
-    if (F.n[2] & 1u) return (size_t)mb * TB_LD * 4 + (size_t)mb * CB_LD * 4;
-    return (size_t)mb * 32 * 4 + (size_t)(mb | 1u) * 32 * 4;
-}
-
-bool decode_recompose_nb32_ok(const Box& F) {
-    const uint64_t rows = (uint64_t)F.n[0] * F.n[1];
-    return rows >= 1024 && fused_smem(F) <= 200 * 1024;
+// blocks that nr consecutive rows' coefficients touch at most, and the box
+// width in words: plus up to 3 words of alignment, a multiple of 4
+uint32_t fused_unit_blocks_rows(const Box& F, uint32_t nr) { return (uint32_t)(((uint64_t)nr * F.n[2] + 31) / 32 + 2); }
+static uint32_t box_words(uint32_t blocks) { return (blocks + 3 + 3) & ~3u; }
+// Rows per unit of the 8-warp kernel: 8 where their box fits 256 words, else 4,
+// 2 or 1 in a box of 160 words (rows of up to about 4850 values, 8 / nr warps
+// per row); 0 for longer rows.
+static uint32_t fused_rows(const Box& F) {
+    if (box_words(fused_unit_blocks_rows(F, 8)) <= 256) return 8;
+    for (uint32_t nr = 4; nr; nr /= 2)
+        if (box_words(fused_unit_blocks_rows(F, nr)) <= 160) return nr;
+    return 0;
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link
@@ -1073,6 +815,14 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     return fn;
 }
 
+// A level is fused when it has rows enough and its rows fit a unit; longer
+// rows decode first and recompose in patch form. Against those two launches
+// (fp32, decode + recompose of the finest level): 2049 x 2049 25 us fused and
+// 33 us apart, 1800 x 3600 30 and 45 us, 129 x 129 x 1025 52 and 75 us.
+bool decode_recompose_nb32_ok(const Box& F) {
+    return (uint64_t)F.n[0] * F.n[1] >= 1024 && fused_rows(F) && tensor_map_encoder() != nullptr;
+}
+
 static int g_tma_tx_extra = 0;                 // test hook: extra expected bytes per tile
 static long long g_tma_wait_cycles = 4000000000ll;   // about two seconds at 2 GHz
 
@@ -1081,7 +831,7 @@ void fused_tma_test_hook(int tx_extra, long long wait_cycles) {
     g_tma_wait_cycles = wait_cycles > 0 ? wait_cycles : 4000000000ll;
 }
 
-// The TMA kernel for odd rows whose 8-row block range fits one box (at most
+// The TMA kernel for rows whose 8-row block range fits one box (at most
 // 256 words): box width and tile row stride (a multiple of 32 words, so that
 // every tile row starts on a 128-byte boundary).
 // Which TMA kernel a fused level takes: the warp-specialised form, with
@@ -1101,7 +851,7 @@ static int fused_ws() {
 
 // rows per unit of the warp-specialised kernel with nd decode warps (one per recomposition warp)
 static uint32_t ws_unit_rows(int nd) { return 16u - (uint32_t)nd; }
-static uint32_t ws_tile_blocks(const Box& F, int nd) { return (ws_unit_rows(nd) * F.n[2] + 31) / 32 + 2; }
+static uint32_t ws_tile_blocks(const Box& F, int nd) { return fused_unit_blocks_rows(F, ws_unit_rows(nd)); }
 // Decode warps of the warp-specialised kernel (the other 16 - nd warps
 // recompose, one unit row each). Measured at 513^3 (level 7, CUDA events):
 // 8 decode warps (8-row units) 263 us, 7: 245 us, 6: 237 us, 5: 237 us
@@ -1136,18 +886,20 @@ template <int RS>
 static int launch_fused_tma(const CUtensorMap& map, uint32_t bw, const void* maxkey, const uint8_t* dnum,
                             const float* coarse, const Box& F, const Box& C, float* out, uint64_t s0, uint64_t s1,
                             int* status, cudaStream_t st, bool pdl, int tall) {
-    if (fused_ws() == 1 || (fused_ws() == 2 && RS >= 160))
+    const uint32_t nr = fused_rows(F);
+    if (nr == 8 && (fused_ws() == 1 || (fused_ws() == 2 && RS >= 160)))
         return launch_fused_ws<RS, 8>(map, bw, maxkey, dnum, coarse, F, C, out, s0, s1, status, st, pdl, tall);
-    const size_t smem = (size_t)32 * RS * 4 + (size_t)fused_max_blocks(F) * CB_LD * 4;
-    const void* kern = (const void*)k_decode_recompose_nb32_tma<RS>;
+    const size_t smem = (size_t)32 * RS * 4 + (size_t)fused_unit_blocks_rows(F, nr) * CB_LD * 4;
+    const auto kernel = nr == 8 ? k_decode_recompose_nb32_tma<RS, false> : k_decode_recompose_nb32_tma<RS, true>;
+    const void* kern = (const void*)kernel;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute");
     const uint64_t rows = (uint64_t)F.n[0] * F.n[1];
-    const uint64_t need = (rows + 7) / 8;
+    const uint64_t need = (rows + nr - 1) / nr;
     const unsigned grid = persistent_grid_for(kern, 256, smem, need, need);
     count_launch();
-    e = launch_chain(pdl, k_decode_recompose_nb32_tma<RS>, dim3(grid), dim3(256), smem, st, map, bw,
-                     (const uint32_t*)maxkey, dnum, coarse, F, C, out, s0, s1, status, g_tma_wait_cycles,
+    e = launch_chain(pdl, kernel, dim3(grid), dim3(256), smem, st, map, bw,
+                     (const uint32_t*)maxkey, dnum, coarse, F, C, out, s0, s1, nr, status, g_tma_wait_cycles,
                      (uint32_t)g_tma_tx_extra, tall);
     if (e != cudaSuccess) return cuda_status(e, "k_decode_recompose_nb32_tma");
     return PRODM_OK;
@@ -1161,88 +913,59 @@ static int tma_tall() {
 bool fused_tma_tall() { return tma_tall() != 0; }
 uint32_t fused_tma_stride(uint32_t bw) { return bw <= 96 ? 96u : (bw <= 160 ? 160u : 256u); }
 
-// Returns PRODM_EUNSUPPORTED when the shape does not suit the row mapping
-// (the caller then runs the unfused kernels). Odd rows take the TMA kernel
-// when the planes' tensor map can be built (base and row stride 16-byte
-// aligned, box of at most 256 words), else the cp.async kernel.
+// base: plane rows on 16-byte boundaries, stride words apart (a multiple of 4)
 int launch_decode_recompose_nb32(const void* base, uint64_t stride, int planes, uint64_t nblocks, const void* maxkey,
                                  const uint8_t* dnum, const float* coarse, const Box& F, const Box& C, float* out,
                                  uint64_t s0, uint64_t s1, int* status, cudaStream_t st, bool pdl) {
-    if (!decode_recompose_nb32_ok(F)) return PRODM_EUNSUPPORTED;
-    const size_t smem = fused_smem(F);
-    const bool odd = (F.n[2] & 1u) != 0;
-    if (odd && status && (uintptr_t)base % 16 == 0 && stride % 4 == 0) {
-        const uint32_t bw = (fused_max_blocks(F) + 3 + 3) & ~3u;   // block range + up to 3 words of alignment
-        const int nd = ws_decode_warps();
-        const uint32_t bwn = (ws_tile_blocks(F, nd) + 3 + 3) & ~3u;
-        // rows of 257 values and up take the warp-specialised form with
-        // 16 - nd rows per unit where its tile rows fit 192 words (two CTAs
-        // per SM; level 6 at 513^3: 46.4 us against 48.9 us for the 8-warp
-        // kernel); longer rows keep 8-row units
-        if (nd != 8 && ((fused_ws() == 2 && F.n[2] >= 257) || fused_ws() == 1) && bwn <= 192) {
-            const uint32_t rs = bwn <= 96 ? 96 : (bwn <= 160 ? 160 : 192);
-            alignas(64) CUtensorMap map;
-            const int tall =
-                tma_tall() && planes <= 32 && encode_plane_map(&map, base, nblocks, planes, stride, rs, 32) == PRODM_OK;
-            if (tall || encode_plane_map(&map, base, nblocks, planes, stride, bwn, 1) == PRODM_OK) {
+    if (!decode_recompose_nb32_ok(F)) return fail(PRODM_EUNSUPPORTED, "fused level: rows too few or too long");
+    const uint32_t bw = box_words(fused_unit_blocks_rows(F, fused_rows(F)));
+    const int nd = ws_decode_warps();
+    const uint32_t bwn = box_words(ws_tile_blocks(F, nd));
+    // rows of 257 values and up take the
+    // warp-specialised form with 16 - nd rows per unit where its tile rows fit
+    // 192 words (two CTAs per SM; level 6 at 513^3: 46.4 us against 48.9 us
+    // for the 8-warp kernel); longer rows keep 8-row units
+    if (nd != 8 && ((fused_ws() == 2 && F.n[2] >= 257) || fused_ws() == 1) && bwn <= 192) {
+        const uint32_t rs = bwn <= 96 ? 96 : (bwn <= 160 ? 160 : 192);
+        alignas(64) CUtensorMap map;
+        const int tall =
+            tma_tall() && planes <= 32 && encode_plane_map(&map, base, nblocks, planes, stride, rs, 32) == PRODM_OK;
+        if (tall || encode_plane_map(&map, base, nblocks, planes, stride, bwn, 1) == PRODM_OK) {
 #define PRODM_WS_CASE(R, N)                                                                                   \
     if (rs == R && nd == N)                                                                                   \
         return launch_fused_ws<R, N>(map, bwn, maxkey, dnum, coarse, F, C, out, s0, s1, status, st, pdl, tall);
-                PRODM_WS_CASE(96, 5) PRODM_WS_CASE(160, 5) PRODM_WS_CASE(192, 5)
-                PRODM_WS_CASE(96, 6) PRODM_WS_CASE(160, 6) PRODM_WS_CASE(192, 6)
+            PRODM_WS_CASE(96, 5) PRODM_WS_CASE(160, 5) PRODM_WS_CASE(192, 5)
+            PRODM_WS_CASE(96, 6) PRODM_WS_CASE(160, 6) PRODM_WS_CASE(192, 6)
 #undef PRODM_WS_CASE
-            }
-        }
-        if (bw <= 256) {
-            const uint32_t rs = fused_tma_stride(bw);
-            // tall: one box of rs words x 32 plane rows per unit (planes above
-            // the retrieved ones at negative coordinates, zero filled); else one
-            // box of bw words per retrieved plane
-            alignas(64) CUtensorMap map;
-            const int tall =
-                tma_tall() && planes <= 32 && encode_plane_map(&map, base, nblocks, planes, stride, rs, 32) == PRODM_OK;
-            if (tall || encode_plane_map(&map, base, nblocks, planes, stride, bw, 1) == PRODM_OK) {
-                if (rs == 96)
-                    return launch_fused_tma<96>(map, bw, maxkey, dnum, coarse, F, C, out, s0, s1, status, st, pdl, tall);
-                if (rs == 160)
-                    return launch_fused_tma<160>(map, bw, maxkey, dnum, coarse, F, C, out, s0, s1, status, st, pdl, tall);
-                return launch_fused_tma<256>(map, bw, maxkey, dnum, coarse, F, C, out, s0, s1, status, st, pdl, tall);
-            }
         }
     }
-    const void* kern = odd ? (const void*)k_decode_recompose_nb32_odd : (const void*)k_decode_recompose_nb32;
-    if (smem > 48 * 1024) {   // per device; cheap to repeat
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute");
-    }
-    const uint64_t rows = (uint64_t)F.n[0] * F.n[1];
-    const uint64_t need = (rows + 7) / 8;
-    if (odd) {
-        const unsigned grid = persistent_grid_for(kern, 256, smem, need, need);
-        k_decode_recompose_nb32_odd<<<grid, 256, smem, st>>>((const uint32_t*)base, stride, (const uint32_t*)maxkey,
-                                                             dnum, coarse, F, C, out, s0, s1, fused_max_blocks(F));
-        PRODM_CHECK_LAUNCH("k_decode_recompose_nb32_odd");
-        return PRODM_OK;
-    }
-    const unsigned grid = persistent_grid_for((const void*)k_decode_recompose_nb32, 256, smem, need, need);
-    k_decode_recompose_nb32<<<grid, 256, smem, st>>>((const uint32_t*)base, stride, (const uint32_t*)maxkey, dnum,
-                                                     coarse, F, C, out, s0, s1, fused_max_blocks(F));
-    PRODM_CHECK_LAUNCH("k_decode_recompose_nb32");
-    return PRODM_OK;
+    const uint32_t rs = fused_tma_stride(bw);
+    // tall: one box of rs words x 32 plane rows per unit (planes above
+    // the retrieved ones at negative coordinates, zero filled); else one
+    // box of bw words per retrieved plane
+    alignas(64) CUtensorMap map;
+    const int tall =
+        tma_tall() && planes <= 32 && encode_plane_map(&map, base, nblocks, planes, stride, rs, 32) == PRODM_OK;
+    if (!tall && encode_plane_map(&map, base, nblocks, planes, stride, bw, 1) != PRODM_OK)
+        return fail(PRODM_ECUDA, "fused level: cuTensorMapEncodeTiled refused the planes' tensor map");
+    if (rs == 96) return launch_fused_tma<96>(map, bw, maxkey, dnum, coarse, F, C, out, s0, s1, status, st, pdl, tall);
+    if (rs == 160)
+        return launch_fused_tma<160>(map, bw, maxkey, dnum, coarse, F, C, out, s0, s1, status, st, pdl, tall);
+    return launch_fused_tma<256>(map, bw, maxkey, dnum, coarse, F, C, out, s0, s1, status, st, pdl, tall);
 }
-
-uint32_t fused_unit_blocks(const Box& F) { return fused_max_blocks(F); }
 
 uint32_t fused_unit_rows(const Box& F, uint32_t values) {
     const uint32_t m = values / 8 / (F.n[2] ? F.n[2] : 1);
     return 8 * (m < 1 ? 1 : (m > kMaxUnitRows / 8 ? kMaxUnitRows / 8 : m));
 }
-uint32_t fused_unit_blocks_rows(const Box& F, uint32_t nr) { return (uint32_t)(((uint64_t)nr * F.n[2] + 31) / 32 + 2); }
 
-uint32_t fused_tma_box(const Box& F, uint32_t nr) {
-    if (!(F.n[2] & 1u)) return 0;
-    const uint32_t bw = (fused_unit_blocks_rows(F, nr) + 3 + 3) & ~3u;   // block range + up to 3 words of alignment
-    return bw <= 160 ? bw : 0;
+// 8 rows or more, else 4, 2 or 1, in a box of 160 words
+uint32_t fused_tma_box(const Box& F, uint32_t& nr) {
+    for (; nr; nr = nr > 8 ? nr - 8 : nr / 2) {
+        const uint32_t bw = box_words(fused_unit_blocks_rows(F, nr));
+        if (bw <= 160) return bw;
+    }
+    return 0;
 }
 
 int encode_plane_map(void* map, const void* base, uint64_t nblocks, int planes, uint64_t stride, uint32_t bw,
@@ -1297,24 +1020,6 @@ int launch_decode_recompose_nb32_ws_multi(const FusedSeg* segs, int nseg, uint64
     k_decode_recompose_nb32_ws_multi<RS, 5><<<grid, 512, smem, st>>>(segs, nseg, total_units, tld, status,
                                                                     g_tma_wait_cycles, (uint32_t)g_tma_tx_extra);
     PRODM_CHECK_LAUNCH("k_decode_recompose_nb32_ws_multi");
-    return PRODM_OK;
-}
-size_t fused_multi_smem(uint32_t tld) { return (size_t)tld * TB_LD * 4 + (size_t)tld * CB_LD * 4; }
-
-// ctas_per_sm == 0: as many as fit
-int launch_decode_recompose_nb32_multi(const FusedSeg* segs, int nseg, uint64_t total_units, uint32_t tld,
-                                       unsigned ctas_per_sm, cudaStream_t st) {
-    if (!total_units) return PRODM_OK;
-    const size_t smem = fused_multi_smem(tld);
-    if (smem > 200 * 1024) return fail(PRODM_EUNSUPPORTED, "batched fused level: rows too long");
-    const void* kern = (const void*)k_decode_recompose_nb32_multi;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute");
-    uint64_t cap = persistent_grid_for(kern, 256, smem, total_units, total_units);
-    if (ctas_per_sm) cap = std::min<uint64_t>(cap, (uint64_t)device_sms() * ctas_per_sm);
-    const unsigned grid = (unsigned)std::max<uint64_t>(cap, 1);
-    k_decode_recompose_nb32_multi<<<grid, 256, smem, st>>>(segs, nseg, total_units, tld);
-    PRODM_CHECK_LAUNCH("k_decode_recompose_nb32_multi");
     return PRODM_OK;
 }
 

@@ -177,11 +177,8 @@ __global__ void __launch_bounds__(256) k_decompose_rows(const T* __restrict__ in
     K mk = 0, mc = 0;
     const uint32_t rows = F.n[0] * F.n[1];
     const uint32_t lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-    const bool odd = (F.n[2] & 1u) != 0;
-    for (uint32_t row = blockIdx.x * wpb + (threadIdx.x >> 5); row < rows; row += gridDim.x * wpb) {
-        if (odd) decompose_row_odd_any<T>(in, s0, s1, F, C, coef, coarse, fnat, row, lane, mk, mc);
-        else decompose_row<T>(in, s0, s1, F, C, coef, coarse, fnat, row, lane, mk, mc);
-    }
+    for (uint32_t row = blockIdx.x * wpb + (threadIdx.x >> 5); row < rows; row += gridDim.x * wpb)
+        decompose_row_any<T>(in, s0, s1, F, C, coef, coarse, fnat, row, lane, mk, mc);
     if (maxkey_level) {
         mk = warp_max_key(mk);
         if ((threadIdx.x & 31) == 0 && mk) atomicMax(maxkey_level, mk);
@@ -192,7 +189,7 @@ __global__ void __launch_bounds__(256) k_decompose_rows(const T* __restrict__ in
     }
 }
 
-// patch form (grids whose every dim is 2 C - 1, no natural-order copy): one
+// patch form (no natural-order copy): one
 // warp item = coarse columns 32g .. 32g + 31 of a 2 x 2 kPatchSteps strip of
 // fine rows (decompose_patch_item)
 template <class T>
@@ -202,7 +199,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_decompose_patch
                                                          typename KeyOf<T>::type* maxkey_coarse) {
     using K = typename KeyOf<T>::type;
     K mk = 0, mc = 0;
-    const uint64_t items = patch_items(C);
+    const uint64_t items = patch_items(F, C);
     const uint32_t lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
     for (uint64_t w = (uint64_t)blockIdx.x * wpb + (threadIdx.x >> 5); w < items; w += (uint64_t)gridDim.x * wpb)
         decompose_patch_item<T>(in, s0, s1, F, C, coef, coarse, w, lane, mk, mc);
@@ -224,7 +221,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_recompose_patch
                                                                                   uint64_t s0, uint64_t s1) {
     pdl_wait();   // the coarse box and the coefficients come from the previous launches
     pdl_release();
-    const uint64_t items = patch_items(C);
+    const uint64_t items = patch_items(F, C);
     const uint32_t lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
     for (uint64_t w = (uint64_t)blockIdx.x * wpb + (threadIdx.x >> 5); w < items; w += (uint64_t)gridDim.x * wpb)
         recompose_patch_item<T>(coarse, coef, F, C, out, s0, s1, w, lane);
@@ -237,11 +234,8 @@ __global__ void __launch_bounds__(256) k_recompose_rows(const T* __restrict__ co
     pdl_release();
     const uint32_t rows = F.n[0] * F.n[1];
     const uint32_t lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-    const bool odd = (F.n[2] & 1u) != 0;
-    for (uint32_t row = blockIdx.x * wpb + (threadIdx.x >> 5); row < rows; row += gridDim.x * wpb) {
-        if (odd) recompose_row_odd_any<T>(coarse, coef, F, C, out, s0, s1, row, lane);
-        else recompose_row<T>(coarse, coef, F, C, out, s0, s1, row, lane);
-    }
+    for (uint32_t row = blockIdx.x * wpb + (threadIdx.x >> 5); row < rows; row += gridDim.x * wpb)
+        recompose_row_any<T>(coarse, coef, F, C, out, s0, s1, row, lane);
 }
 
 // copy a box between strided arrays
@@ -563,7 +557,7 @@ int launch_decompose_level_packed(const T* in, uint64_t s0, uint64_t s1, const B
     using K = typename KeyOf<T>::type;
     const unsigned th = row_threads(F.n[2]);
     if (!fnat && patch_level(F, C) && decompose_patch_enabled()) {
-        k_decompose_patch<T><<<row_grid(patch_items(C), th), th, 0, st>>>(in, s0, s1, F, C, coef, coarse,
+        k_decompose_patch<T><<<row_grid(patch_items(F, C), th), th, 0, st>>>(in, s0, s1, F, C, coef, coarse,
                                                                           (K*)maxkey_level, (K*)maxkey_coarse);
         PRODM_CHECK_LAUNCH("k_decompose_patch");
         return PRODM_OK;
@@ -590,7 +584,7 @@ int launch_recompose_level_packed(const T* coarse, const T* coef, const Box& F, 
     const unsigned th = row_threads(F.n[2]);
     count_launch();
     if (patch_level(F, C) && decompose_patch_enabled()) {
-        const cudaError_t e = launch_chain(pdl, k_recompose_patch<T>, dim3(row_grid(patch_items(C), th)), dim3(th), 0,
+        const cudaError_t e = launch_chain(pdl, k_recompose_patch<T>, dim3(row_grid(patch_items(F, C), th)), dim3(th), 0,
                                            st, coarse, coef, F, C, out, s0, s1);
         if (e != cudaSuccess) return cuda_status(e, "k_recompose_patch");
         return PRODM_OK;

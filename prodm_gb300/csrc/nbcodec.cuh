@@ -38,12 +38,7 @@ __device__ __forceinline__ float scale2(float v, int e, bool fast, float sc) { r
 __device__ __forceinline__ constexpr float nbw(int i) { return (i & 1) ? -(float)(1u << i) : (float)(1u << i); }
 
 
-// asynchronous 4-byte global -> shared copies (cp.async), one group per call
-__device__ __forceinline__ void cp_async4(uint32_t* dst, const uint32_t* src) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
-}
-// 16-byte copy, both addresses 16-byte aligned (L2 only)
+// asynchronous 16-byte global -> shared copy (cp.async), both addresses 16-byte aligned (L2 only)
 __device__ __forceinline__ void cp_async16(uint32_t* dst, const uint32_t* src) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
@@ -84,8 +79,6 @@ __device__ __forceinline__ void transpose32_half(const uint32_t (&R)[32], int ha
     for (int k = 0; k < 16; k++) a[k] = __byte_perm(R[k], R[k + 16], sel16);
     transpose32_half_tail(a);
 }
-
-constexpr int TB_LD = 36;   // block-major plane tile row: 32 planes + pad, 16-byte aligned rows
 
 constexpr int NB_G = 8;              // blocks per warp iteration
 constexpr int NB_CHUNK = 256;        // blocks per CTA chunk
