@@ -445,20 +445,22 @@ int pb_progressive_decode(prodm_decoder* h, const uint8_t* blob, const uint32_t*
         PRODM_CUDA(cudaMemcpyAsync(tmp, blob, total, cudaMemcpyDeviceToDevice, st));
         base = tmp;
     }
-    std::vector<uint64_t> hv(2 * num);
+    PbParseJob job;
     uint64_t o = 0;
     for (int i = 0; i < num; i++) {
-        hv[i] = (uint64_t)(uintptr_t)(base + o);
-        hv[num + i] = hs[i] / 8;
+        job.planes.push_back((const uint64_t*)(base + o));
+        job.nwords.push_back(hs[i] / 8);
         o += hs[i];
     }
-    uint64_t* dv;   // plane pointers, word counts, then the parse pipeline's scratch
-    const size_t head = (hv.size() * 8 + 255) / 256 * 256;
-    PRODM_CUDA(cudaMallocAsync((void**)&dv, head + pb_parse_scratch_bytes(num), st));
-    PRODM_CUDA(cudaMemcpyAsync(dv, hv.data(), hv.size() * 8, cudaMemcpyHostToDevice, st));
+    job.a = s;
+    job.n = n;
+    job.rows = rows;
+    job.stride = rw;
+    job.unseen = rows + (uint64_t)(B + 1) * rw;
+    job.signs = rows + (uint64_t)B * rw;
+    job.status = status;
     PRODM_CUDA(cudaMemsetAsync(status, 0, 4, st));
-    int rc = launch_pb_parse((const uint64_t* const*)dv, dv + num, s, num, n, rows, rw, rows + (uint64_t)(B + 1) * rw,
-                             rows + (uint64_t)B * rw, (uint8_t*)dv + head, status, st);
+    int rc = launch_pb_parse({job}, st);
     if (!rc)
         rc = launch_pb_decode<T>(rows, rw, n, nullptr, exp, B, s, s + num, nullptr, rows + (uint64_t)B * rw,
                                  rows + (uint64_t)(B + 1) * rw, out, st);
@@ -468,7 +470,6 @@ int pb_progressive_decode(prodm_decoder* h, const uint8_t* blob, const uint32_t*
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) rc = cuda_status(e, "per-bit decode");
     }
-    cudaFreeAsync(dv, st);
     if (tmp) cudaFreeAsync(tmp, st);
     // a failed parse leaves the level's state behind the data: the next call
     // for this level starts again at plane 0
@@ -612,7 +613,7 @@ struct prodm_mdr {
     std::vector<uint32_t> hsz;                     // host copy of `sizes` (export), valid while hsz_valid
     bool hsz_valid = false;
     uint32_t* pbcounts = nullptr;                  // per-bit: first-one counts, 64 per level
-    int* pbstatus = nullptr;                       // per-bit: parse status of loaded streams
+    int* pbstatus = nullptr;                       // per-bit: parse status of each level's loaded streams
     int* kstatus = nullptr;                        // bounded device waits of retrievals (0 or a PRODM_E* code)
     uint8_t* hmap = nullptr;                       // mapped pinned host memory: plane counts [0, 64), status [64, 68)
     bool after_reconstruct = false;                // the last call on the handle was a reconstruction
@@ -837,7 +838,7 @@ int mdr_alloc_all(prodm_mdr* h) {
         PRODM_CUDA(cudaMemcpy(h->sizes, sz.data(), sz.size() * 4, cudaMemcpyHostToDevice));
     } else if (h->pb) {
         if ((rc = h->alloc((void**)&h->pbcounts, (L + 1) * 64 * 4))) return rc;
-        if ((rc = h->alloc((void**)&h->pbstatus, 16))) return rc;
+        if ((rc = h->alloc((void**)&h->pbstatus, (L + 1) * 4))) return rc;
     } else {
         if ((rc = h->alloc((void**)&h->rbs, h->rb_off[L + 1]))) return rc;
         if ((rc = h->alloc((void**)&h->chunk_words, maxch * B * 4))) return rc;
@@ -1049,70 +1050,76 @@ int mdr_interpret(prodm_mdr* h, double tol, int interp, int est, double s, cudaS
                                h->index, 0, h->rsz, st, true, early);
 }
 
-// grouped levels loaded from files: header -> rb + chunk offsets, then the
-// planes completely inside the loaded prefix -> aligned layout
 // per-bit levels loaded from files: parse the planes that lie completely
-// inside the loaded prefix and are not parsed yet into the level's rows
-int pb_parse_loaded(prodm_mdr* h, int l, cudaStream_t st) {
-    const int B = h->B;
-    const uint64_t n = h->g.elems[l], rw = h->plane_cap[l];
-    uint32_t* rows = (uint32_t*)(h->streams + h->lvl_byte_off[l]);
+// inside the loaded prefixes and are not parsed yet into the levels' rows, the
+// finest level's CTAs first and all levels together
+int pb_parse_loaded(prodm_mdr* h, cudaStream_t st) {
+    const int L = h->g.L, B = h->B;
     int rc;
-    if (!h->header_done[l]) {
-        if ((rc = launch_pb_init_unseen(rows + (uint64_t)(B + 1) * rw, rows + (uint64_t)B * rw, n, st))) return rc;
-        h->header_done[l] = 1;
+    std::vector<PbParseJob> jobs;
+    std::vector<std::pair<int, int>> upto;   // level, planes complete
+    for (int l = L; l >= 0; l--) {
+        if (!h->lfile[l]) continue;
+        const uint64_t n = h->g.elems[l], rw = h->plane_cap[l];
+        uint32_t* rows = (uint32_t*)(h->streams + h->lvl_byte_off[l]);
+        if (!h->header_done[l]) {
+            if ((rc = launch_pb_init_unseen(rows + (uint64_t)(B + 1) * rw, rows + (uint64_t)B * rw, n, st))) return rc;
+            h->header_done[l] = 1;
+        }
+        uint64_t off = 0;
+        int complete = 0;
+        for (int p = 0; p < B; p++) {
+            off += h->hsizes[l * B + p];
+            if (off <= h->loaded[l]) complete = p + 1;
+            else break;
+        }
+        const int first = (int)h->unpacked[l];
+        if (complete <= first) continue;
+        PbParseJob job;
+        uint64_t o = 0;
+        for (int p = 0; p < first; p++) o += h->hsizes[l * B + p];
+        for (int p = first; p < complete; p++) {
+            const uint64_t sz = h->hsizes[l * B + p];
+            if (sz == 0 || sz % 8) return fail(PRODM_ECORRUPT, "load: per-bit stream size not a positive multiple of 8");
+            job.planes.push_back((const uint64_t*)(h->lfile[l] + o));
+            job.nwords.push_back(sz / 8);
+            o += sz;
+        }
+        job.a = first;
+        job.n = n;
+        job.rows = rows;
+        job.stride = rw;
+        job.unseen = rows + (uint64_t)(B + 1) * rw;
+        job.signs = rows + (uint64_t)B * rw;
+        job.status = h->pbstatus + l;
+        jobs.push_back(job);
+        upto.push_back({l, complete});
     }
-    uint64_t off = 0;
-    int complete = 0;
-    for (int p = 0; p < B; p++) {
-        off += h->hsizes[l * B + p];
-        if (off <= h->loaded[l]) complete = p + 1;
-        else break;
+    if (jobs.empty()) return PRODM_OK;
+    PRODM_CUDA(cudaMemsetAsync(h->pbstatus, 0, (L + 1) * 4, st));
+    if ((rc = launch_pb_parse(jobs, st))) return rc;
+    std::vector<int> hstat(L + 1);
+    PRODM_CUDA(cudaMemcpyAsync(hstat.data(), h->pbstatus, (L + 1) * 4, cudaMemcpyDeviceToHost, st));
+    PRODM_CUDA(cudaStreamSynchronize(st));
+    for (const auto& u : upto) {
+        const int e = hstat[u.first];
+        if (!e) h->unpacked[u.first] = u.second;
+        else rc = rc == PRODM_ETIMEOUT ? rc : e;
     }
-    const int first = (int)h->unpacked[l];
-    if (complete <= first) return PRODM_OK;
-    const int num = complete - first;
-    std::vector<uint64_t> hv(2 * num);
-    uint64_t o = 0;
-    for (int p = 0; p < first; p++) o += h->hsizes[l * B + p];
-    for (int i = 0; i < num; i++) {
-        const uint64_t sz = h->hsizes[l * B + first + i];
-        if (sz == 0 || sz % 8) return fail(PRODM_ECORRUPT, "load: per-bit stream size not a positive multiple of 8");
-        hv[i] = (uint64_t)(uintptr_t)(h->lfile[l] + o);
-        hv[num + i] = sz / 8;
-        o += sz;
-    }
-    uint64_t* dv;   // plane pointers, word counts, then the parse pipeline's scratch
-    const size_t head = (hv.size() * 8 + 255) / 256 * 256;
-    PRODM_CUDA(cudaMallocAsync((void**)&dv, head + pb_parse_scratch_bytes(num), st));
-    PRODM_CUDA(cudaMemcpyAsync(dv, hv.data(), hv.size() * 8, cudaMemcpyHostToDevice, st));
-    PRODM_CUDA(cudaMemsetAsync(h->pbstatus, 0, 4, st));
-    rc = launch_pb_parse((const uint64_t* const*)dv, dv + num, first, num, n, rows, rw, rows + (uint64_t)(B + 1) * rw,
-                         rows + (uint64_t)B * rw, (uint8_t*)dv + head, h->pbstatus, st);
-    int hstat = 0;
-    if (!rc) {
-        cudaError_t e = cudaMemcpyAsync(&hstat, h->pbstatus, 4, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        if (e != cudaSuccess) rc = cuda_status(e, "per-bit load");
-    }
-    cudaFreeAsync(dv, st);
-    if (rc) return rc;
-    if (hstat == PRODM_ETIMEOUT) return fail(PRODM_ETIMEOUT, "load: the per-bit parse pipeline stalled");
-    if (hstat) return fail(PRODM_ECORRUPT, "load: a per-bit stream does not end where its size says");
-    h->unpacked[l] = complete;
+    if (rc == PRODM_ETIMEOUT) return fail(PRODM_ETIMEOUT, "load: the per-bit parse pipeline stalled");
+    if (rc) return fail(PRODM_ECORRUPT, "load: a per-bit stream does not end where its size says");
     return PRODM_OK;
 }
 
+// grouped levels loaded from files: header -> rb + chunk offsets, then the
+// planes completely inside the loaded prefix -> aligned layout
 int mdr_unpack_loaded(prodm_mdr* h, cudaStream_t st) {
     const int L = h->g.L, B = h->B;
     const int wb = (int)h->es;
     int rc;
+    if (h->pb) return pb_parse_loaded(h, st);
     for (int l = 0; l <= L; l++) {
         if (!h->lfile[l]) continue;
-        if (h->pb) {
-            if ((rc = pb_parse_loaded(h, l, st))) return rc;
-            continue;
-        }
         const uint64_t nbk = h->nblocks[l];
         const uint64_t hdr = 4 + nbk;
         if (!h->header_done[l]) {

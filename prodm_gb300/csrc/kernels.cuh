@@ -1,6 +1,7 @@
 // Host-side launchers of the CUDA kernels (declarations).
 #pragma once
 #include <functional>
+#include <vector>
 
 #include "common.cuh"
 
@@ -167,9 +168,40 @@ size_t pb_pack_scratch_bytes(uint64_t n, int B);
 int launch_pb_pack(const uint32_t* rows, uint64_t stride, uint64_t n, int B, const uint32_t* sizes, uint64_t total,
                    uint8_t* dst, void* scratch, cudaStream_t st);
 int launch_pb_init_unseen(uint32_t* unseen, uint32_t* signs, uint64_t n, cudaStream_t st);
-size_t pb_parse_scratch_bytes(int np);
-int launch_pb_parse(const uint64_t* const* planes, const uint64_t* nwords, int a, int np, uint64_t n, uint32_t* rows,
-                    uint64_t stride, uint32_t* unseen, uint32_t* signs, void* scratch, int* status, cudaStream_t st);
+// planes [a, a + planes.size()) of one level, read from the reference's streams
+// (nwords 64-bit words each) into the level's rows; status: a device word, 0 or
+// the PRODM_E* code of a failed parse
+struct PbParseJob {
+    std::vector<const uint64_t*> planes;
+    std::vector<uint64_t> nwords;
+    int a;
+    uint64_t n;
+    uint32_t* rows;
+    uint64_t stride;
+    uint32_t* unseen;
+    uint32_t* signs;
+    int* status;
+};
+// the same for the kernel: ring and flags of its planes, its first CTA
+struct PbParse {
+    const uint64_t* const* planes;
+    const uint64_t* nwords;
+    uint32_t* rows;
+    uint64_t stride;
+    uint32_t* unseen;
+    uint32_t* signs;
+    uint32_t* ring;
+    int* flags;
+    int* status;
+    uint64_t n;
+    int a, np, cta0;
+};
+constexpr int kPbParseLevels = 17;
+struct PbParseSet {
+    int n;
+    PbParse seg[kPbParseLevels];
+};
+int launch_pb_parse(const std::vector<PbParseJob>& jobs, cudaStream_t st);
 
 // lossless.cu: ZCB codec, one descriptor per stream; chunk0 = the stream's
 // first chunk in the flattened chunk index (sorted), clen = compressed length

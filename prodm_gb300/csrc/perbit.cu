@@ -313,21 +313,49 @@ __global__ void __launch_bounds__(PK_T) k_pb_pack_write(const uint32_t* __restri
 }
 
 // ---------------------------------------------------------------------------
-// parse: reference streams of planes [a, a+np) -> rows a..a+np-1, with the
-// unseen / sign rows carried from the planes before a and updated.
+// parse: reference streams of planes [a, a+np) of one or more levels -> rows
+// a..a+np-1, with the unseen / sign rows carried from the planes before a and
+// updated.
 //
-// One single-warp CTA per plane, all co-resident (cooperative launch). The
-// chain over planes is a software pipeline over chunks of 32 groups: CTA k
-// receives each chunk's unseen / sign masks from CTA k-1 through a ring in
-// global memory (release / acquire flags) and hands them on after its plane.
-// Within a chunk, only groups with unseen elements can hold sign bits: they
-// are parsed in order, one step per sign bit (pz_group); the other groups
-// hold exactly one bit per element, so once the sign bits before them are
-// counted, every lane reads its group's word directly. Every wait is bounded: past the limit the CTA
-// records PRODM_ETIMEOUT in *status and returns.
+// One CTA per (level, plane), all co-resident (cooperative launch). The chain
+// over a level's planes is a software pipeline over chunks of PZ_G groups: a
+// plane's CTA receives each chunk's unseen / sign masks from the plane before
+// through a ring in global memory (release / acquire flags) and hands them on
+// after its plane. Every wait is bounded: past the limit the CTA records
+// PRODM_ETIMEOUT in the level's status and returns.
+//
+// Within a chunk the start of a group depends on the number of sign bits
+// before it, and only groups with unseen elements hold sign bits. Those
+// groups are taken in steps of up to 32 pairs: for each pair the threads
+// parse every start in a window around the expected one, a pair per start and
+// thread, and note which slot of the next pair their end leads to (the
+// window's middle is the sign count expected from the rate of the groups just
+// parsed; the widths, which grow with the root of the distance from the
+// step's first group, are laid out over the threads once per chunk); then one
+// warp follows the chain of true starts through the slots, and two others
+// parse their words while the next step's windows are tried. A true start outside its window ends the step there, and the first
+// pair of a step has its exact start, so every step goes on. The groups
+// without unseen elements hold one bit per element at offsets known once the
+// signs before them are counted. One warp of the CTA moves the masks: it
+// fetches the next chunk's and hands on the last one's while the other warps
+// parse the current one.
+// What bounds it is this chain, not memory: one warp taking a plane's groups
+// one after the other, a step per sign bit, ran at 570 SM cycles per group in
+// the planes where most elements become significant (129^3 fp64, 60 planes:
+// all levels' parse 20.0 ms, 4.8 ms this way; with 320 and 416 starts per step
+// 5.0 and 5.3 ms).
 // ---------------------------------------------------------------------------
 constexpr int PZ_R = 8;                      // ring depth (chunks)
 constexpr long long kPzSpin = 1ll << 24;     // x >= 256 ns per wait
+constexpr int PZ_N = 224;                    // parsing threads: starts tried per step
+constexpr int PZ_S = PZ_N + 64;              // and the warps that keep the true starts' words
+constexpr int PZ_T = PZ_S + 32;              // and the warp that moves the masks
+constexpr int PZ_G = 128;                    // groups per chunk
+constexpr int PZ_E = 2 * PZ_G;               // ring entry: a chunk's unseen + sign words
+// staged stream words (64-bit): a chunk takes at most 2 PZ_G bits x 32, and its
+// start lies at most PZ_G / 2 + 1 words behind the first staged one
+constexpr int PZ_W = 3 * PZ_G / 2 + 8;
+constexpr uint32_t PZ_END = 0xffffu;
 
 __device__ __forceinline__ int ld_acquire(const int* p) {
     int v;
@@ -337,239 +365,381 @@ __device__ __forceinline__ int ld_acquire(const int* p) {
 __device__ __forceinline__ void st_release(int* p, int v) {
     asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
+// one lane polls *p until it is above `above`, at most kPzSpin times
+__device__ __forceinline__ bool pz_wait(const int* p, int above, int& seen) {
+    for (long long spins = 0; (seen = ld_acquire(p)) <= above; spins++) {
+        if (spins > kPzSpin) return false;
+        __nanosleep(32);
+    }
+    return true;
+}
+__device__ __forceinline__ void pz_sync() { asm volatile("bar.sync 1, %0;" ::"n"(PZ_S) : "memory"); }
 
-// a plane's stream: the chunk's 64 64-bit words are staged in shared memory;
-// the next chunk's are prefetched into registers n0 / n1 (lane i: words
-// npb + i and npb + 32 + i)
-struct PlaneReader {
-    const uint64_t* w;
-    uint64_t nw, pos, pb, npb;
-    uint64_t n0, n1;
-    __device__ __forceinline__ uint64_t load(uint64_t k) const { return k < nw ? __ldcs(w + k) : 0ull; }
+struct PzMasks {                 // one chunk's masks, updated by the parse
+    uint32_t U[PZ_G], S[PZ_G];   // unseen / sign words of its groups
+    uint32_t seq[PZ_G + 1];      // groups with unseen elements, in order
+    uint32_t PU[PZ_G + 2];       // unseen elements of the groups seq[0..k)
+    int nseq;
+};
+// the smallest start tried of a window of w starts, d unseen elements into the
+// step (one value wherever it is computed: no contraction is left open)
+__device__ __forceinline__ uint32_t pz_low(float rate, uint32_t d, uint32_t w) {
+    return (uint32_t)fmaxf(__fmaf_rn(rate, (float)d, __fmaf_rn(-0.5f, (float)w, 0.5f)), 0.f);
+}
+
+struct PzShared {
+    uint8_t used[4096];          // four elements: (unseen bits << 8 | stream bits) -> stream bits used
+    uint16_t tab[4096];          // and -> magnitude | sign << 4 | bits used << 8
+    uint32_t ws[2 * PZ_W];       // the chunk's stream, 32-bit words from word 2 * pb on
+    PzMasks m[3];                // chunks c - 1 (handed on), c (parsed), c + 1 (fetched)
+    uint32_t M[PZ_G];            // the plane's words of the groups with unseen elements
+    uint32_t cnt[PZ_G];          // their sign bits
+    uint16_t before[PZ_N];       // per start tried: the step's sign bits before it,
+    uint8_t first[PZ_N], both[PZ_N];   // the first group's and the pair's,
+    uint16_t next[PZ_N];         // and the slot of the next pair that its end starts, or PZ_END
+    uint32_t base[34];           // per pair of a step: its starts' first slot
+    uint32_t start[64];          // the true starts of the last step's groups: the sign bits before each
+    int npairs;                  // pairs of a full step
+    int k0, run;                 // the step: its first group, the sign bits before it,
+    float rate;                  // and sign bits expected per unseen element
+    int kept, kept_k0, kept_run; // the last step: groups with a true start, ..
 };
 
-__device__ __forceinline__ uint32_t bits_below(int k) { return k >= 32 ? FULL : ((1u << k) - 1u); }
-
-// One group of one plane from the 64 stream bits W at its start. With d sign
-// bits before them, the remaining elements' bits are the frame W >> d (bit i
-// = element i); the next element to carry a sign is the lowest unseen one
-// whose bit is set there, and its sign is bit i of the next frame W >> (d+1).
-// One step per sign.
-__device__ __forceinline__ void pz_group(uint64_t W, uint32_t U, int nv, uint32_t& M, uint32_t& SG, uint32_t& cnt) {
-    const uint32_t lo32 = (uint32_t)W, hi32 = (uint32_t)(W >> 32);
-    const uint32_t vm = bits_below(nv);
-    uint32_t rest = U & vm, m = 0, sg = 0, below = 0, d = 0;
-    uint32_t Wd = lo32;
-    for (int it = 0; it < 33; it++) {
-        const uint32_t T = rest & Wd;
-        if (!T) break;
-        const uint32_t bit = T & (0u - T);          // element i
-        const uint32_t upto = (bit << 1) - 1u;      // elements 0..i
-        m |= Wd & upto & ~below;
-        below = upto;
-        rest &= ~upto;
-        d++;
-        Wd = __funnelshift_rc(lo32, hi32, d);
-        sg |= Wd & bit;
-    }
-    M = m | (Wd & vm & ~below);
-    SG = sg;
-    cnt = d;
-}
-
-// A group whose values are all unseen is a stream of the tokens "0" and
-// "1 s": a 1 at a token start escapes the next bit. Runs of 1s start at token
-// starts; inside a run the odd offsets are escaped, and the bit after a run
-// of odd length is escaped too (the run-start parities split by adding the
-// run starts: the carry clears a run and marks its end).
-__device__ __forceinline__ uint64_t pz_escaped(uint64_t W) {
-    constexpr uint64_t EVEN = 0x5555555555555555ull, ODD = 0xaaaaaaaaaaaaaaaaull;
-    const uint64_t starts = W & ~(W << 1);
-    const uint64_t es = W + (starts & EVEN), os = W + (starts & ODD);
-    const uint64_t inside = ((W & ~es) & ODD) | ((W & ~os) & EVEN);
-    const uint64_t after = ((es & ~W) & ODD) | ((os & ~W) & EVEN);
-    return inside | after;
-}
-// position of zero number e (from 0) of E: binary search on popcounts
-__device__ __forceinline__ int pz_select_zero(uint64_t E, int e) {
-    const uint64_t Z = ~E;
-    int pos = 0, rem = e;
+// One group from the 64 stream bits W at its start: magnitude bits M and signs
+// SG of its unseen elements U, by table steps of four elements
+__device__ __forceinline__ void pz_group(const uint16_t* tab, uint64_t W, uint32_t U, uint32_t& M, uint32_t& SG) {
+    uint32_t m = 0, sg = 0;
 #pragma unroll
-    for (int step = 32; step > 0; step >>= 1) {
-        const int c = __popcll((Z >> pos) & ((1ull << step) - 1ull));
-        if (c <= rem) {
-            rem -= c;
-            pos += step;
-        }
+    for (int i = 0; i < 8; i++) {
+        const uint32_t u = i < 2 ? U << (8 - 4 * i) : U >> (4 * i - 8);
+        const uint32_t e = tab[(u & 0xf00u) | ((uint32_t)W & 255u)];
+        m |= (e & 15u) << (4 * i);
+        sg |= ((e >> 4) & 15u) << (4 * i);
+        W >>= e >> 8;
     }
-    return pos;
+    M = m;
+    SG = sg;
+}
+// its sign bits alone
+__device__ __forceinline__ uint32_t pz_count(const uint8_t* used, uint64_t W, uint32_t U) {
+    uint32_t lo = (uint32_t)W, hi = (uint32_t)(W >> 32), total = 0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const uint32_t u = i < 2 ? U << (8 - 4 * i) : U >> (4 * i - 8);
+        const uint32_t e = used[(u & 0xf00u) | (lo & 255u)];
+        total += e;
+        lo = __funnelshift_r(lo, hi, e);
+        hi >>= e;
+    }
+    return total - 32u;
+}
+// and by one step per sign bit, for planes with few of them: with d sign bits
+// taken, the remaining elements' bits are the frame W >> d (bit i = element
+// i); the next element to carry a sign is the lowest unseen one whose bit is
+// set there
+__device__ __forceinline__ uint32_t pz_count_few(uint64_t W, uint32_t U) {
+    const uint32_t lo = (uint32_t)W, hi = (uint32_t)(W >> 32);
+    uint32_t d = 0;
+    for (uint32_t T = U & lo; T && d < 32; T = U & __funnelshift_rc(lo, hi, d)) {
+        U &= T ^ (0u - T);   // the elements behind the lowest set one
+        d++;
+    }
+    return d;
+}
+__device__ __forceinline__ uint64_t pz_window(const uint32_t* ws, uint32_t at) {
+    const uint32_t k = at >> 5, sh = at & 31;
+    const uint32_t x0 = ws[k], x1 = ws[k + 1], x2 = ws[k + 2];
+    return ((uint64_t)__funnelshift_r(x1, x2, sh) << 32) | __funnelshift_r(x0, x1, sh);
 }
 
-// one chunk (32 groups, lane g = group g0 + g) of one plane; U / S: the
-// lane's group's unseen and sign masks, updated; returns the group's word.
-// ws: the chunk's stream as 128 32-bit words (word 2*pb + i at ws[i])
-__device__ __forceinline__ uint32_t pz_chunk(PlaneReader& r, bool first, uint64_t g0, uint64_t ng, uint64_t n,
-                                             uint32_t& U, uint32_t& S, int lane, uint32_t* ws, uint32_t* us,
-                                             int* nvs) {
-    // the chunk reads words [pos/64, pos/64 + 33); its successor starts 16..32
-    // 64-bit words on (a full group takes 32..64 bits)
-    const uint64_t wb = r.pos >> 6;
-    __syncwarp();
-    uint64_t a, b;
-    if (first) {
-        r.pb = wb;
-        a = r.load(wb + lane);
-        b = r.load(wb + 32 + lane);
-    } else {
-        r.pb = r.npb;
-        a = r.n0;
-        b = r.n1;
-    }
-    ws[2 * lane] = (uint32_t)a;
-    ws[2 * lane + 1] = (uint32_t)(a >> 32);
-    ws[64 + 2 * lane] = (uint32_t)b;
-    ws[64 + 2 * lane + 1] = (uint32_t)(b >> 32);
-    r.npb = wb + 16;
-    r.n0 = r.load(r.npb + lane);
-    r.n1 = r.load(r.npb + 32 + lane);
-    const uint64_t g = g0 + lane;
-    const int nv = pk_nvalid(g, ng, n);
-    us[lane] = U;
-    nvs[lane] = nv;
-    __syncwarp();
-    const uint32_t p0 = (uint32_t)(r.pos - 64 * r.pb);   // chunk start within the staged words (< 1088)
-    uint32_t M = 0, extra = 0;
-    // groups with unseen elements, in order (every lane computes the same):
-    // the sign bits before group j are those of the earlier groups of this kind
-    const uint32_t seq = __ballot_sync(FULL, nv > 0 && U != 0);
-    uint32_t todo = seq, run = 0;
-    while (todo) {
-        const int j = __ffs(todo) - 1;
-        todo &= todo - 1;
-        const uint32_t Uj = us[j];
-        const int nvj = nvs[j];
-        const uint32_t at = p0 + 32u * j + run;
-        const uint32_t k = at >> 5, sh = at & 31;
-        const uint32_t x0 = ws[k], x1 = ws[k + 1], x2 = ws[k + 2];
-        const uint64_t W = ((uint64_t)__funnelshift_r(x1, x2, sh) << 32) | __funnelshift_r(x0, x1, sh);
-        uint32_t Mj, SG, cnt;
-        if (Uj == bits_below(nvj)) {   // all unseen: bit-parallel, one value per lane
-            const int q = pz_select_zero(pz_escaped(W), lane);
-            const bool b = lane < nvj && ((W >> q) & 1ull);
-            Mj = __ballot_sync(FULL, b);
-            SG = __ballot_sync(FULL, b && ((W >> (q + 1)) & 1ull));
-            cnt = __popc(Mj);
-        } else {
-            pz_group(W, Uj, nvj, Mj, SG, cnt);
-        }
-        const bool mine = lane == j;
-        M = mine ? Mj : M;
-        extra = mine ? cnt : extra;
-        U = mine ? (Uj & ~Mj) : U;
-        S = mine ? (S | SG) : S;
-        run += cnt;
-    }
-    // groups without unseen elements: one bit per element at known offsets
-    uint32_t inc = extra;
+__device__ __forceinline__ uint32_t warp_scan(uint32_t v, int lane) {   // inclusive
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(FULL, inc, o);
-        if (lane >= o) inc += t;
+        const uint32_t t = __shfl_up_sync(FULL, v, o);
+        if (lane >= o) v += t;
     }
-    if (nv > 0 && !((seq >> lane) & 1u)) {
-        const uint32_t at = p0 + 32u * lane + (inc - extra);
-        M = __funnelshift_r(ws[at >> 5], ws[(at >> 5) + 1], at & 31) & valid_mask(nv);
-    }
-    uint32_t used = (uint32_t)nv;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) used += __shfl_xor_sync(FULL, used, o);
-    r.pos += used + run;
-    return M;
+    return v;
 }
 
-constexpr int PZ_SUB = 4;                    // 32-group sub-chunks per hand-off
-constexpr int PZ_E = 64 * PZ_SUB;            // ring entry: unseen + sign words of 32 * PZ_SUB groups
-// dynamic shared memory reserved (unused) so that no two planes' CTAs share an SM
-constexpr int PZ_SPREAD_SMEM = 116 * 1024;
-
-__global__ void __launch_bounds__(32) k_pb_parse(const uint64_t* const* __restrict__ planes,
-                                                 const uint64_t* __restrict__ nwords, int a, int np, uint64_t n,
-                                                 uint32_t* __restrict__ rows, uint64_t stride,
-                                                 uint32_t* __restrict__ unseen, uint32_t* __restrict__ signs,
-                                                 uint32_t* __restrict__ ring, int* __restrict__ flags,
-                                                 int* __restrict__ status) {
-    __shared__ uint32_t ws[130];
-    __shared__ uint32_t us[32];
-    __shared__ int nvs[32];
-    const int k = blockIdx.x, lane = threadIdx.x;
-    int* produced = flags;
-    int* consumed = flags + np;
-    const uint64_t ng = (n + 31) / 32, nch = (ng + 32 * PZ_SUB - 1) / (32 * PZ_SUB);
-    PlaneReader r{planes[k], nwords[k], 0, 0, 0, 0, 0};
-    uint32_t* row = rows + (uint64_t)(a + k) * stride;
-    const bool last = k == np - 1;
-    int seen_consumed = 0;   // the consumer's progress as last read
-    for (uint64_t c = 0; c < nch; c++) {
-        const int slot = (int)(c % PZ_R);
-        uint32_t U[PZ_SUB], S[PZ_SUB];
-        if (k == 0) {
+// one warp: chunk c's masks into m, with the list of its groups with unseen elements
+__device__ __forceinline__ void pz_fetch(const PbParse& q, int k, uint64_t c, uint64_t ng, PzMasks& m, int lane) {
+    const uint64_t g0 = c * PZ_G;
+    const uint32_t* src = q.ring + ((uint64_t)(k - 1) * PZ_R + c % PZ_R) * PZ_E;
+    uint32_t U[PZ_G / 32], S[PZ_G / 32];
 #pragma unroll
-            for (int t = 0; t < PZ_SUB; t++) {
-                const uint64_t g = c * 32 * PZ_SUB + t * 32 + lane;
-                U[t] = g < ng ? unseen[g] : 0u;
-                S[t] = g < ng ? signs[g] : 0u;
-            }
+    for (int t = 0; t < PZ_G / 32; t++) {
+        const int i = 32 * t + lane;
+        if (k) {
+            U[t] = __ldcg(src + i);
+            S[t] = __ldcg(src + PZ_G + i);
         } else {
-            long long spins = 0;
-            while (ld_acquire(produced + k - 1) <= (int)c) {
-                if (++spins > kPzSpin) { if (lane == 0) atomicExch(status, PRODM_ETIMEOUT); return; }
-                __nanosleep(128);
-            }
-            const uint32_t* src = ring + ((uint64_t)(k - 1) * PZ_R + slot) * PZ_E;
-#pragma unroll
-            for (int t = 0; t < PZ_SUB; t++) {
-                U[t] = __ldcg(src + t * 64 + lane);
-                S[t] = __ldcg(src + t * 64 + 32 + lane);
-            }
-            __syncwarp();
-            if (lane == 0) st_release(consumed + k - 1, (int)c + 1);
-        }
-#pragma unroll
-        for (int t = 0; t < PZ_SUB; t++) {
-            const uint64_t g0 = c * 32 * PZ_SUB + t * 32;
-            if (g0 >= ng) break;
-            const uint32_t M = pz_chunk(r, c == 0 && t == 0, g0, ng, n, U[t], S[t], lane, ws, us, nvs);
-            if (g0 + lane < ng) row[g0 + lane] = M;
-        }
-        if (last) {
-#pragma unroll
-            for (int t = 0; t < PZ_SUB; t++) {
-                const uint64_t g = c * 32 * PZ_SUB + t * 32 + lane;
-                if (g < ng) { unseen[g] = U[t]; signs[g] = S[t]; }
-            }
-        } else {
-            if ((int)c - seen_consumed >= PZ_R) {
-                long long spins = 0;
-                while ((int)c - (seen_consumed = ld_acquire(consumed + k)) >= PZ_R) {
-                    if (++spins > kPzSpin) { if (lane == 0) atomicExch(status, PRODM_ETIMEOUT); return; }
-                    __nanosleep(128);
-                }
-            }
-            uint32_t* dst = ring + ((uint64_t)k * PZ_R + slot) * PZ_E;
-#pragma unroll
-            for (int t = 0; t < PZ_SUB; t++) {
-                __stcg(dst + t * 64 + lane, U[t]);
-                __stcg(dst + t * 64 + 32 + lane, S[t]);
-            }
-            __syncwarp();
-            if (lane == 0) {
-                __threadfence();
-                st_release(produced + k, (int)c + 1);
-            }
+            U[t] = g0 + i < ng ? q.unseen[g0 + i] : 0u;
+            S[t] = g0 + i < ng ? q.signs[g0 + i] : 0u;
         }
     }
-    // a well-formed stream ends in its last word
-    if (lane == 0 && (r.pos + 63) / 64 != r.nw) atomicCAS(status, 0, PRODM_ECORRUPT);
+    uint32_t at = 0, u0 = 0;
+#pragma unroll
+    for (int t = 0; t < PZ_G / 32; t++) {
+        m.U[32 * t + lane] = U[t];
+        m.S[32 * t + lane] = S[t];
+        const uint32_t has = __ballot_sync(FULL, U[t] != 0), own = __popc(U[t]);
+        const uint32_t inc = warp_scan(own, lane);
+        if (U[t]) {
+            const uint32_t i = at + __popc(has & ((1u << lane) - 1u));
+            m.seq[i] = 32 * t + lane;
+            m.PU[i] = u0 + inc - own;
+        }
+        at += __popc(has);
+        u0 += __shfl_sync(FULL, inc, 31);
+    }
+    if (lane == 0) {
+        m.nseq = (int)at;
+        m.seq[at] = 0;
+        m.PU[at] = u0;
+        m.PU[at + 1] = u0;
+    }
+}
+
+__global__ void __launch_bounds__(PZ_T, 3) k_pb_parse(const __grid_constant__ PbParseSet set) {
+    extern __shared__ __align__(16) unsigned char pz_smem[];
+    PzShared& sh = *reinterpret_cast<PzShared*>(pz_smem);
+    int l = 0;   // the CTA's level and plane
+    while (l + 1 < set.n && (int)blockIdx.x >= set.seg[l + 1].cta0) l++;
+    const PbParse& q = set.seg[l];
+    const int k = (int)blockIdx.x - q.cta0;
+    const int np = q.np, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint64_t n = q.n;
+    int* produced = q.flags;
+    int* consumed = q.flags + np;
+    const uint64_t ng = (n + 31) / 32, nch = (ng + PZ_G - 1) / PZ_G;
+    const uint64_t* words = q.planes[k];
+    const uint64_t nw = q.nwords[k];
+    uint32_t* row = q.rows + (uint64_t)(q.a + k) * q.stride;
+    const bool last = k == np - 1, mover = tid >= PZ_S, keeper = tid >= PZ_N && !mover;
+    for (int i = tid; i < 4096; i += PZ_T) {
+        const uint32_t u = i >> 8;
+        uint32_t w = i & 255, m = 0, sg = 0, used = 0;
+        for (int j = 0; j < 4; j++) {
+            const uint32_t b = w & 1u;
+            w >>= 1;
+            used++;
+            m |= b << j;
+            if (b && ((u >> j) & 1u)) {
+                sg |= (w & 1u) << j;
+                w >>= 1;
+                used++;
+            }
+        }
+        sh.tab[i] = (uint16_t)(m | sg << 4 | used << 8);
+        sh.used[i] = (uint8_t)used;
+    }
+    int seen_produced = 0, seen_consumed = 0;   // mover lane 0: the neighbours' progress as last read
+    int gave_up = 0;                            // mover: a wait ran out
+    // the mover warp, while the others parse chunk c: chunk c - 1 to the next
+    // plane (or the last plane's masks to the level's rows), chunk c + 1 in
+    auto move = [&](uint64_t c, bool give, bool take) {
+        bool ok = true;
+        if (give) {
+            const uint64_t o = c - 1, g0 = o * PZ_G;
+            const PzMasks& m = sh.m[o % 3];
+            if (last) {
+                for (int i = lane; i < PZ_G; i += 32)
+                    if (g0 + i < ng) {
+                        q.unseen[g0 + i] = m.U[i];
+                        q.signs[g0 + i] = m.S[i];
+                    }
+            } else {
+                if (lane == 0 && (int)o - seen_consumed >= PZ_R)
+                    ok = pz_wait(consumed + k, (int)o - PZ_R, seen_consumed);
+                ok = __shfl_sync(FULL, ok, 0);
+                if (ok) {
+                    uint32_t* dst = q.ring + ((uint64_t)k * PZ_R + o % PZ_R) * PZ_E;
+                    for (int i = lane; i < PZ_G; i += 32) {
+                        __stcg(dst + i, m.U[i]);
+                        __stcg(dst + PZ_G + i, m.S[i]);
+                    }
+                    __syncwarp();
+                    if (lane == 0) {
+                        __threadfence();
+                        st_release(produced + k, (int)o + 1);
+                    }
+                }
+            }
+        }
+        if (take && ok) {
+            const uint64_t t = c + 1;
+            if (k) {
+                if (lane == 0 && seen_produced <= (int)t) ok = pz_wait(produced + k - 1, (int)t, seen_produced);
+                ok = __shfl_sync(FULL, ok, 0);
+            }
+            if (ok) {
+                pz_fetch(q, k, t, ng, sh.m[t % 3], lane);
+                __syncwarp();
+                if (k && lane == 0) st_release(consumed + k - 1, (int)t + 1);
+            }
+        }
+        if (!ok) gave_up = 1;
+    };
+    if (mover) move(~0ull, false, true);   // chunk 0
+    uint64_t pos = 0, pb = 0;          // the chunk's first bit; the first staged word
+    uint64_t ahead = tid < PZ_W && (uint64_t)tid < nw ? __ldcs(words + tid) : 0ull;   // words pb + tid
+    float rs = 0.f, ru = 0.f;          // warp 0: sign bits and unseen elements of the groups just parsed
+    for (uint64_t c = 0; c < nch; c++) {
+        const uint64_t g0 = c * PZ_G;
+        // stage the stream; the next chunk starts PZ_G / 2 words on or later
+        if (tid < PZ_W) {
+            sh.ws[2 * tid] = (uint32_t)ahead;
+            sh.ws[2 * tid + 1] = (uint32_t)(ahead >> 32);
+            const uint64_t w = (pos >> 6) + PZ_G / 2 + tid;
+            ahead = w < nw ? __ldcs(words + w) : 0ull;
+        }
+        if (tid < PZ_G) sh.cnt[tid] = 0;
+        const uint32_t p0 = (uint32_t)(pos - 64 * pb);
+        pb = (pos >> 6) + PZ_G / 2;
+        if (__syncthreads_or(gave_up)) {   // (also: the stream and the mover's chunk c are there)
+            if (tid == 0) atomicExch(q.status, PRODM_ETIMEOUT);
+            return;
+        }
+        PzMasks& m = sh.m[c % 3];
+        uint32_t run_all = 0;
+        if (mover) {
+            move(c, c > 0, c + 1 < nch);
+        } else {
+            const int nseq = m.nseq;
+            int k0 = 0;
+            uint32_t run = 0;
+            if (warp == 0) {   // the chunk's windows: 2.5 sigma on either side
+                const float p = __fdividef(rs + 0.5f, ru + 1.f);
+                const float v = ((p - p * p) + 0.002f) * 2.f * __fdividef((float)m.PU[nseq], (float)max(nseq, 1));
+                const float vi = v * (float)lane;
+                const uint32_t w = lane ? min(3u + (uint32_t)(5.f * vi * rsqrtf(vi)), 120u) : 1u;
+                const uint32_t inc = warp_scan(w, lane);
+                const uint32_t fit = __ballot_sync(FULL, inc <= PZ_N);
+                sh.base[lane + 1] = inc;
+                if (lane == 0) {
+                    sh.base[0] = 0;
+                    sh.base[33] = ~0u;
+                    sh.npairs = __popc(fit);
+                    sh.k0 = 0;
+                    sh.run = 0;
+                    sh.rate = p;
+                    sh.kept = 0;
+                }
+            }
+            pz_sync();
+            // this thread's pair and place in its window
+            const int npairs = sh.npairs;
+            int pi = 0;
+#pragma unroll
+            for (int step = 16; step > 0; step >>= 1)
+                if (pi + step < npairs && sh.base[pi + step] <= (uint32_t)tid) pi += step;
+            const uint32_t b0 = sh.base[pi], b1 = sh.base[pi + 1], b2 = sh.base[pi + 2];
+            const bool mine = !keeper && (uint32_t)tid < b1, more = pi + 1 < npairs;
+            for (;;) {
+                const int first = sh.k0;
+                if (keeper) {   // the last step's true starts: thread i parses group i's words
+                    const int i = tid - PZ_N;
+                    if (i < sh.kept) {
+                        const uint32_t g = m.seq[sh.kept_k0 + i], U = m.U[g];
+                        uint32_t M, SG;
+                        pz_group(sh.tab, pz_window(sh.ws, p0 + sh.kept_run + sh.start[i] + 32 * g), U, M, SG);
+                        sh.M[g] = M;
+                        sh.cnt[g] = __popc(M & U);
+                        m.U[g] = U & ~M;
+                        m.S[g] |= SG;
+                    }
+                } else if (mine && first + 2 * pi < nseq) {   // try one start of one pair
+                    const int kk = first + 2 * pi;
+                    const uint32_t ga = m.seq[kk], gb = m.seq[kk + 1];
+                    const uint32_t P0 = m.PU[first], Pa = m.PU[kk], Pb = m.PU[kk + 1], Pc = m.PU[kk + 2];
+                    const float rate = sh.rate;
+                    // sign bits before it in this step
+                    const uint32_t x = pi ? pz_low(rate, Pa - P0, b1 - b0) + (uint32_t)tid - b0 : 0u;
+                    const uint32_t at = p0 + sh.run + x;
+                    const uint32_t Ua = m.U[ga], Ub = Pc != Pb ? m.U[gb] : 0u;
+                    const uint64_t Wa = pz_window(sh.ws, at + 32 * ga);
+                    uint32_t cc;
+                    if (rate < 0.12f) {
+                        cc = pz_count_few(Wa, Ua);
+                        sh.first[tid] = (uint8_t)cc;
+                        cc += pz_count_few(pz_window(sh.ws, at + 32 * gb + cc), Ub);
+                    } else {
+                        cc = pz_count(sh.used, Wa, Ua);
+                        sh.first[tid] = (uint8_t)cc;
+                        cc += pz_count(sh.used, pz_window(sh.ws, at + 32 * gb + cc), Ub);
+                    }
+                    uint32_t nx = PZ_END;
+                    if (more && kk + 2 < nseq) {   // below the window the difference wraps
+                        const uint32_t y = x + cc - pz_low(rate, Pc - P0, b2 - b1);
+                        if (y < b2 - b1) nx = b1 + y;
+                    }
+                    sh.before[tid] = (uint16_t)x;
+                    sh.next[tid] = (uint16_t)nx;
+                    sh.both[tid] = (uint8_t)cc;
+                }
+                if (first >= nseq) break;   // every group with unseen elements is parsed
+                pz_sync();
+                if (warp == 0) {   // follow the true starts (lane i: pair i)
+                    uint32_t slot = 0, own = 0;
+                    int done = 0;
+                    for (;;) {
+                        const uint32_t nx = sh.next[slot];
+                        if (lane == done) own = slot;
+                        done++;
+                        if (nx == PZ_END) break;   // at the latest behind the step's last pair
+                        slot = nx;
+                    }
+                    const uint32_t r = sh.before[slot] + sh.both[slot];
+                    const int k1 = min(k0 + 2 * done, nseq);
+                    rs = 0.25f * rs + (float)r;
+                    ru = 0.25f * ru + (float)(m.PU[k1] - m.PU[k0]);
+                    const uint32_t x = sh.before[own];
+                    sh.start[2 * lane] = x;
+                    sh.start[2 * lane + 1] = x + sh.first[own];
+                    if (lane == 0) {
+                        sh.kept = k1 - k0;
+                        sh.kept_k0 = k0;
+                        sh.kept_run = (int)run;
+                        sh.k0 = k1;
+                        sh.run = (int)(run + r);
+                        sh.rate = __fdividef(rs + 0.5f, ru + 1.f);
+                    }
+                    k0 = k1;
+                    run += r;
+                }
+                pz_sync();
+            }
+            pz_sync();   // the last step's words
+            // words of all groups: thread t < PZ_G takes group t
+            if (tid < PZ_G) {
+                const int nv = pk_nvalid(g0 + tid, ng, n);
+                const uint32_t own = sh.cnt[tid];
+                uint32_t before = warp_scan(own, lane) - own;
+                for (int j = 0; j < warp; j++) before += __reduce_add_sync(FULL, sh.cnt[32 * j + lane]);
+                uint32_t M;
+                if (m.U[tid] != 0 || own != 0) {   // it had unseen elements: parsed above
+                    M = sh.M[tid];
+                } else {
+                    const uint32_t at = p0 + 32u * tid + before;
+                    M = __funnelshift_r(sh.ws[at >> 5], sh.ws[(at >> 5) + 1], at & 31);
+                }
+                if (nv > 0) row[g0 + tid] = M & valid_mask(nv);
+            }
+            run_all = (uint32_t)sh.run;
+        }
+        if (mover) run_all = 0;
+        __syncthreads();   // the chunk is parsed, and the mover is done with its neighbours
+        const uint64_t left = n - 32 * g0;
+        pos += (left < 32 * PZ_G ? left : 32 * PZ_G) + run_all;
+    }
+    // the last chunk's masks
+    if (mover && nch) move(nch, true, false);
+    gave_up = __syncthreads_or(gave_up);
+    if (tid == 0) {
+        if (gave_up) atomicExch(q.status, PRODM_ETIMEOUT);
+        // a well-formed stream ends in its last word
+        else if ((pos + 63) / 64 != nw) atomicCAS(q.status, 0, PRODM_ECORRUPT);
+    }
 }
 
 // unseen row of a fresh level: every element present
@@ -643,28 +813,60 @@ int launch_pb_init_unseen(uint32_t* unseen, uint32_t* signs, uint64_t n, cudaStr
     return PRODM_OK;
 }
 
-size_t pb_parse_scratch_bytes(int np) { return (size_t)np * PZ_R * PZ_E * 4 + (size_t)2 * np * 4 + 256; }
-
-int launch_pb_parse(const uint64_t* const* planes, const uint64_t* nwords, int a, int np, uint64_t n, uint32_t* rows,
-                    uint64_t stride, uint32_t* unseen, uint32_t* signs, void* scratch, int* status, cudaStream_t st) {
-    if (np < 1 || np > 64) return fail(PRODM_EINVAL, "perbit parse: 1..64 planes per call");
-    uint32_t* ring = (uint32_t*)scratch;
-    int* flags = (int*)(ring + (size_t)np * PZ_R * PZ_E);
-    PRODM_CUDA(cudaMemsetAsync(flags, 0, (size_t)2 * np * 4, st));
-    static thread_local int attr_dev = -1;
-    int dev = 0;
-    PRODM_CUDA(cudaGetDevice(&dev));
-    if (attr_dev != dev) {
-        PRODM_CUDA(cudaFuncSetAttribute((const void*)k_pb_parse, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        PZ_SPREAD_SMEM));
-        attr_dev = dev;
+// The parse of several levels' planes in as few launches as are co-resident
+// (the planes' CTAs wait on one another, so they are launched cooperatively).
+// Scratch: the plane pointers and word counts, a ring and two flags per plane.
+int launch_pb_parse(const std::vector<PbParseJob>& jobs, cudaStream_t st) {
+    size_t planes = 0;
+    for (const PbParseJob& j : jobs) {
+        const size_t np = j.planes.size();
+        if (np < 1 || np > 64 || j.nwords.size() != np) return fail(PRODM_EINVAL, "perbit parse: 1..64 planes per level");
+        planes += np;
     }
-    // the planes' CTAs wait on one another: launched cooperatively, so that
-    // all of them are resident together
-    void* args[] = {(void*)&planes, (void*)&nwords, &a, &np, &n, &rows, &stride, &unseen, &signs, &ring, &flags,
-                    &status};
-    PRODM_CUDA(cudaLaunchCooperativeKernel((const void*)k_pb_parse, dim3(np), dim3(32), args, PZ_SPREAD_SMEM, st));
-    PRODM_CHECK_LAUNCH("k_pb_parse");
+    if (!planes) return PRODM_OK;
+    const size_t head = (planes * 16 + 255) / 256 * 256, fl = (planes * 8 + 255) / 256 * 256;
+    std::vector<uint64_t> hv;
+    hv.reserve(2 * planes);
+    for (const PbParseJob& j : jobs) {
+        for (const uint64_t* p : j.planes) hv.push_back((uint64_t)(uintptr_t)p);
+        for (uint64_t w : j.nwords) hv.push_back(w);
+    }
+    uint8_t* scratch;
+    PRODM_CUDA(cudaMallocAsync((void**)&scratch, head + fl + planes * PZ_R * PZ_E * 4, st));
+    cudaError_t e = cudaMemcpyAsync(scratch, hv.data(), hv.size() * 8, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(scratch + head, 0, fl, st);
+    const unsigned resident = resident_ctas((const void*)k_pb_parse, PZ_T, sizeof(PzShared));
+    size_t at = 0, next = 0;
+    while (e == cudaSuccess && next < jobs.size()) {
+        PbParseSet set;
+        set.n = 0;
+        unsigned ctas = 0;
+        while (next < jobs.size() && set.n < kPbParseLevels &&
+               (ctas == 0 || ctas + jobs[next].planes.size() <= resident)) {
+            const PbParseJob& j = jobs[next++];
+            PbParse& q = set.seg[set.n++];
+            q.np = (int)j.planes.size();
+            q.planes = (const uint64_t* const*)((uint64_t*)scratch + 2 * at);
+            q.nwords = (const uint64_t*)scratch + 2 * at + q.np;
+            q.flags = (int*)(scratch + head) + 2 * at;
+            q.ring = (uint32_t*)(scratch + head + fl) + at * PZ_R * PZ_E;
+            q.rows = j.rows;
+            q.stride = j.stride;
+            q.unseen = j.unseen;
+            q.signs = j.signs;
+            q.status = j.status;
+            q.n = j.n;
+            q.a = j.a;
+            q.cta0 = (int)ctas;
+            ctas += (unsigned)q.np;
+            at += q.np;
+        }
+        count_launch();
+        void* args[] = {(void*)&set};
+        e = cudaLaunchCooperativeKernel((const void*)k_pb_parse, dim3(ctas), dim3(PZ_T), args, sizeof(PzShared), st);
+    }
+    cudaFreeAsync(scratch, st);
+    if (e != cudaSuccess) return cuda_status(e, "k_pb_parse");
     return PRODM_OK;
 }
 
