@@ -117,6 +117,8 @@ __global__ void __launch_bounds__(256) k_nb_encode32(const float* __restrict__ x
 __global__ void __launch_bounds__(256, 3) k_nb_encode32_levels(const ChunkSeg* __restrict__ segs, int nseg,
                                                                uint64_t total, int B) {
     __shared__ uint32_t tile[32 * NB_TILE_LD];
+    pdl_wait();
+    pdl_release();
     int cur = -1, se = 0;
     bool fast = true;
     float scale = 1.f;
@@ -636,15 +638,33 @@ __device__ __forceinline__ T gr_value(typename Traits<T>::FP acc, int s, bool ne
 // word counts contributed by a block with recording plane r to plane p
 __device__ __forceinline__ uint32_t gr_words(int r, int p) { return (r < p ? 1u : 0u) + (r == p ? 2u : 0u); }
 
+// Every kernel below takes the chunks of all levels of a field in one launch
+// (GrSet, one segment per level): a chain of one launch per level left a small
+// level's few CTAs alone on the chip for their latency (65^3 fp32, five
+// retrievals: decode 385 us in 25 launches, 91 us in 5; encode 157 and 24 us). The recording planes of a
+// warp's 32 blocks are fetched by one load and the next blocks' words loaded
+// a few blocks ahead, so a warp waits for memory once per group of blocks
+// instead of twice per block.
+template <class T>
+__device__ __forceinline__ const GrSeg<T>& gr_seg(const GrSet<T>& set, uint32_t& chunk) {
+    int l = 0;
+    while (l + 1 < set.n && blockIdx.x >= set.seg[l + 1].chunk0) l++;
+    chunk = blockIdx.x - set.seg[l].chunk0;
+    return set.seg[l];
+}
+
+// first pass: each block's recording bitplane and the chunk's word counts
 template <class T, bool ERR>
-__global__ void __launch_bounds__(256) k_gr_rb(const T* __restrict__ x, uint64_t n,
-                                               const typename KeyOf<T>::type* __restrict__ maxkey, int exp_arg, int B,
-                                               uint8_t* __restrict__ rbs, uint32_t* __restrict__ chunk_words,
+__global__ void __launch_bounds__(256) k_gr_rb(const __grid_constant__ GrSet<T> set, int B,
                                                double* __restrict__ partial) {
     using FP = typename Traits<T>::FP;
     using A = typename Acc<T>::type;
-    constexpr int BS = Traits<T>::kBlock;
-    const int exp = level_exp<T>(maxkey, exp_arg);
+    constexpr int BS = Traits<T>::kBlock, H = BS / 32;
+    constexpr int U = ERR ? 1 : 8 / H;   // blocks loaded ahead
+    uint32_t chunk;
+    const GrSeg<T>& q = gr_seg(set, chunk);
+    const T* __restrict__ x = q.x;
+    const uint64_t n = q.n;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t nblocks = (n + BS - 1) / BS;
     __shared__ uint32_t cnt[GR_WARPS][64];
@@ -654,217 +674,231 @@ __global__ void __launch_bounds__(256) k_gr_rb(const T* __restrict__ x, uint64_t
 #pragma unroll
         for (int k = 0; k < Acc<T>::N; k++) acc[k] = 0;
     }
-    const uint64_t b0 = (uint64_t)blockIdx.x * GR_CHUNK + (uint64_t)warp * GR_BPW;
-    for (int j = 0; j < GR_BPW; j++) {
-        uint64_t b = b0 + j;
-        if (b >= nblocks) break;
-        FP orv = 0;
+    pdl_wait();
+    pdl_release();
+    const int exp = level_exp<T>(q.key, q.exp);
+    const bool fast = pow2_normal(B - exp);
+    const float sc = fast ? pow2f(B - exp) : 1.f;
+    const uint64_t b0 = (uint64_t)chunk * GR_CHUNK + (uint64_t)warp * GR_BPW;
+    int rv = B;   // lane j: block j's recording plane
+    for (int j0 = 0; j0 < GR_BPW && b0 + j0 < nblocks; j0 += U) {
+        T v[U * H];
 #pragma unroll
-        for (int h = 0; h < BS / 32; h++) {
-            uint64_t i = b * BS + h * 32 + lane;
-            if (i < n) {
-                bool neg;
-                T sh;
-                FP q = gr_mag<T, ERR>(x[i], B, exp, neg, sh);
-                orv |= q;
-                if (ERR) gr_errors(acc, (A)fabs(sh), B);
+        for (int t = 0; t < U * H; t++) {
+            const uint64_t i = (b0 + j0) * BS + t * 32 + lane;
+            v[t] = i < n ? __ldg(x + i) : (T)0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            FP orv = 0;
+#pragma unroll
+            for (int h = 0; h < H; h++) {
+                if constexpr (std::is_same<T, float>::value) {
+                    const int64_t fix = (int64_t)scale2(v[u * H + h], B - exp, fast, sc);
+                    orv |= (FP)(fix < 0 ? -fix : fix);
+                } else {
+                    bool neg;
+                    T sh;
+                    orv |= gr_mag<T, ERR>(v[u * H + h], B, exp, neg, sh);
+                    if (ERR && (b0 + j0 + u) * BS + h * 32 + lane < n) gr_errors(acc, (A)fabs(sh), B);
+                }
+            }
+            int r;
+            if (BS == 32) {
+                const uint32_t o = __reduce_or_sync(FULL, (uint32_t)orv);
+                r = o ? B - 1 - (31 - __clz(o)) : B;
+            } else {
+                const uint32_t lo = __reduce_or_sync(FULL, (uint32_t)orv);
+                const uint32_t hi = __reduce_or_sync(FULL, (uint32_t)((uint64_t)orv >> 32));
+                r = hi ? B - 1 - (63 - __clz(hi)) : lo ? B - 1 - (31 - __clz(lo)) : B;
+            }
+            if (lane == j0 + u) rv = r;
+            if (b0 + j0 + u < nblocks) {
+                c0 += gr_words(r, lane);
+                c1 += gr_words(r, lane + 32);
             }
         }
-        int r;
-        if (BS == 32) {
-            uint32_t o = __reduce_or_sync(FULL, (uint32_t)orv);
-            r = o ? B - 1 - (31 - __clz(o)) : B;
-        } else {
-            uint32_t lo = __reduce_or_sync(FULL, (uint32_t)orv);
-            uint32_t hi = __reduce_or_sync(FULL, (uint32_t)((uint64_t)orv >> 32));
-            uint64_t o = ((uint64_t)hi << 32) | lo;
-            r = o ? B - 1 - (63 - __clzll((long long)o)) : B;
-        }
-        if (lane == 0) rbs[b] = (uint8_t)r;
-        c0 += gr_words(r, lane);
-        c1 += gr_words(r, lane + 32);
     }
+    if (b0 + lane < nblocks) q.rbs[b0 + lane] = (uint8_t)rv;
     cnt[warp][lane] = c0;
     cnt[warp][lane + 32] = c1;
     __syncthreads();
     if (threadIdx.x < 64 && (int)threadIdx.x < B) {
-        uint32_t s = 0;
-        for (int w = 0; w < GR_WARPS; w++) s += cnt[w][threadIdx.x];
-        chunk_words[(uint64_t)blockIdx.x * B + threadIdx.x] = s;
+        uint32_t t = 0;
+        for (int w = 0; w < GR_WARPS; w++) t += cnt[w][threadIdx.x];
+        q.cw[(uint64_t)chunk * B + threadIdx.x] = t;
     }
     if (ERR) flush_errors(acc, B, partial);
 }
 
-// exclusive scan of chunk_words over chunks, per plane; stream byte sizes.
-// One CTA per plane (the planes are independent).
-__global__ void k_gr_scan(const uint32_t* __restrict__ chunk_words, uint64_t nchunks, int B, uint64_t nblocks,
-                          int word_bytes, uint32_t* __restrict__ chunk_off, uint32_t* __restrict__ sizes) {
+// exclusive scan of the chunks' word counts, per plane (blockIdx.x) and level
+// (blockIdx.y); stream byte sizes
+template <class T>
+__global__ void k_gr_scan(const __grid_constant__ GrSet<T> set, int B) {
+    constexpr int BS = Traits<T>::kBlock;
     __shared__ uint32_t wsum[32];
     __shared__ uint32_t carry;
-    {
-        const int p = blockIdx.x;
-        if (p >= B) return;
-        if (threadIdx.x == 0) carry = 0;
+    const GrSeg<T>& q = set.seg[blockIdx.y];
+    const uint64_t nblocks = (q.n + BS - 1) / BS, nchunks = (nblocks + GR_CHUNK - 1) / GR_CHUNK;
+    const int p = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    pdl_wait();
+    pdl_release();
+    if (threadIdx.x == 0) carry = 0;
+    __syncthreads();
+    for (uint64_t base = 0; base < nchunks; base += blockDim.x) {
+        const uint64_t c = base + threadIdx.x;
+        const uint32_t v = c < nchunks ? q.cw[c * B + p] : 0;
+        uint32_t incl = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o) incl += t;
+        }
+        if (lane == 31) wsum[warp] = incl;
         __syncthreads();
-        for (uint64_t base = 0; base < nchunks; base += blockDim.x) {
-            uint64_t c = base + threadIdx.x;
-            uint32_t v = c < nchunks ? chunk_words[c * B + p] : 0;
-            uint32_t incl = v;
-            const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        if (warp == 0) {
+            const uint32_t ws = lane < (int)(blockDim.x >> 5) ? wsum[lane] : 0;
+            uint32_t wi = ws;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                uint32_t t = __shfl_up_sync(FULL, incl, o);
-                if (lane >= o) incl += t;
+                const uint32_t t = __shfl_up_sync(FULL, wi, o);
+                if (lane >= o) wi += t;
             }
-            if (lane == 31) wsum[warp] = incl;
-            __syncthreads();
-            if (warp == 0) {
-                uint32_t ws = lane < (int)(blockDim.x >> 5) ? wsum[lane] : 0;
-                uint32_t wi = ws;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    uint32_t t = __shfl_up_sync(FULL, wi, o);
-                    if (lane >= o) wi += t;
-                }
-                wsum[lane] = wi - ws;   // exclusive warp offsets
-            }
-            __syncthreads();
-            uint32_t excl = carry + wsum[warp] + incl - v;
-            if (c < nchunks) chunk_off[c * B + p] = excl;
-            __syncthreads();
-            if (threadIdx.x == blockDim.x - 1) carry = excl + v;
-            __syncthreads();
+            wsum[lane] = wi - ws;   // exclusive warp offsets
         }
-        if (threadIdx.x == 0) sizes[p] = carry * word_bytes + (p == 0 ? (uint32_t)(4 + nblocks) : 0u);
+        __syncthreads();
+        const uint32_t excl = carry + wsum[warp] + incl - v;
+        if (c < nchunks) q.co[c * B + p] = excl;
+        __syncthreads();
+        if (threadIdx.x == blockDim.x - 1) carry = excl + v;
         __syncthreads();
     }
+    if (threadIdx.x == 0)
+        q.sizes[p] = carry * (uint32_t)sizeof(typename Traits<T>::S) + (p == 0 ? (uint32_t)(4 + nblocks) : 0u);
 }
 
-// per-warp starting offsets (word index in each plane) for the warp's 32 blocks
-__device__ __forceinline__ void gr_warp_offsets(const uint8_t* __restrict__ rbs, uint64_t nblocks,
-                                                const uint32_t* __restrict__ chunk_off, int B, uint32_t& off0,
-                                                uint32_t& off1) {
+// A warp's blocks: its first one's word index in planes lane and lane + 32,
+// and the recording planes (lane j: block j; 255, which no plane reaches,
+// where there is no block)
+__device__ __forceinline__ int gr_warp_offsets(const uint8_t* __restrict__ rbs, uint64_t nblocks, uint64_t chunk,
+                                               const uint32_t* __restrict__ chunk_off, int B, uint32_t& off0,
+                                               uint32_t& off1) {
     __shared__ uint32_t cnt[GR_WARPS][64];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t b0 = (uint64_t)blockIdx.x * GR_CHUNK + (uint64_t)warp * GR_BPW;
+    const uint64_t b = chunk * GR_CHUNK + (uint64_t)warp * GR_BPW + lane;
+    const int rv = b < nblocks ? rbs[b] : 255;
+    off0 = lane < B ? chunk_off[chunk * B + lane] : 0;
+    off1 = lane + 32 < B ? chunk_off[chunk * B + lane + 32] : 0;
     uint32_t c0 = 0, c1 = 0;
+#pragma unroll 8
     for (int j = 0; j < GR_BPW; j++) {
-        uint64_t b = b0 + j;
-        if (b >= nblocks) break;
-        int r = rbs[b];
+        const int r = __shfl_sync(FULL, rv, j);
         c0 += gr_words(r, lane);
         c1 += gr_words(r, lane + 32);
     }
     cnt[warp][lane] = c0;
     cnt[warp][lane + 32] = c1;
     __syncthreads();
-    off0 = lane < B ? chunk_off[(uint64_t)blockIdx.x * B + lane] : 0;
-    off1 = lane + 32 < B ? chunk_off[(uint64_t)blockIdx.x * B + lane + 32] : 0;
     for (int w = 0; w < warp; w++) {
         off0 += cnt[w][lane];
         off1 += cnt[w][lane + 32];
     }
+    return rv;
 }
 
-template <class T>
-__global__ void __launch_bounds__(256, 4) k_gr_write(const T* __restrict__ x, uint64_t n,
-                                                  const typename KeyOf<T>::type* __restrict__ maxkey, int exp_arg,
-                                                  int B, const uint8_t* __restrict__ rbs,
-                                                  const uint32_t* __restrict__ chunk_off,
-                                                  typename Traits<T>::S* __restrict__ out, uint64_t cap) {
-    using S = typename Traits<T>::S;
-    using FP = typename Traits<T>::FP;
-    constexpr int BS = Traits<T>::kBlock;
-    const int exp = level_exp<T>(maxkey, exp_arg);
+// fp64 writer
+__global__ void __launch_bounds__(256, 4) k_gr_write64(const __grid_constant__ GrSet<double> set, int B) {
+    using S = uint64_t;
+    constexpr int U = 2;   // blocks loaded ahead
+    uint32_t chunk;
+    const GrSeg<double>& q = gr_seg(set, chunk);
+    const double* __restrict__ x = q.x;
+    const uint64_t n = q.n, cap = q.cap;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t nblocks = (n + BS - 1) / BS;
+    const uint64_t nblocks = (n + 63) / 64;
+    pdl_wait();
+    pdl_release();
+    const int exp = level_exp<double>(q.key, q.exp);
     uint32_t off0, off1;
-    gr_warp_offsets(rbs, nblocks, chunk_off, B, off0, off1);
-    const uint64_t b0 = (uint64_t)blockIdx.x * GR_CHUNK + (uint64_t)warp * GR_BPW;
-    for (int j = 0; j < GR_BPW; j++) {
-        uint64_t b = b0 + j;
-        if (b >= nblocks) break;
-        FP q[BS / 32];
-        S sign = 0;
+    const int rv = gr_warp_offsets(q.rbs, nblocks, chunk, q.co, B, off0, off1);
+    const uint64_t b0 = (uint64_t)chunk * GR_CHUNK + (uint64_t)warp * GR_BPW;
+    for (int j0 = 0; j0 < GR_BPW && b0 + j0 < nblocks; j0 += U) {
+        double v[2 * U];
 #pragma unroll
-        for (int h = 0; h < BS / 32; h++) {
-            uint64_t i = b * BS + h * 32 + lane;
-            bool neg = false;
-            q[h] = 0;
-            if (i < n) {
-                T sh;
-                q[h] = gr_mag<T, false>(x[i], B, exp, neg, sh);
-            }
-            sign |= (S)__ballot_sync(FULL, neg) << (h * 32);
+        for (int t = 0; t < 2 * U; t++) {
+            const uint64_t i = (b0 + j0) * 64 + t * 32 + lane;
+            v[t] = i < n ? __ldcs(x + i) : 0.0;
         }
-        const int r = rbs[b];
-        S mine0 = 0, mine1 = 0;
-        if constexpr (BS == 64) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int r = __shfl_sync(FULL, rv, j0 + u);
+            uint64_t m[2];
+            S sign = 0;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                bool neg;
+                double sh;
+                m[h] = gr_mag<double, false>(v[2 * u + h], B, exp, neg, sh);
+                sign |= (S)__ballot_sync(FULL, neg) << (h * 32);
+            }
             // encode_block :337-357 by four warp bit transposes: lane k gets the
             // words of magnitude bit k (low halves) and bit 32 + k (high halves)
             // of values 0..31 and 32..63; lane p then fetches plane p (bit
             // B-1-p) and plane p + 32 (bit B-33-p). Planes below r are not written.
-            const uint32_t lo0 = transpose32((uint32_t)q[0], lane), hi0 = transpose32((uint32_t)(q[0] >> 32), lane);
-            const uint32_t lo1 = transpose32((uint32_t)q[1], lane), hi1 = transpose32((uint32_t)(q[1] >> 32), lane);
+            const uint32_t lo0 = transpose32((uint32_t)m[0], lane), hi0 = transpose32((uint32_t)(m[0] >> 32), lane);
+            const uint32_t lo1 = transpose32((uint32_t)m[1], lane), hi1 = transpose32((uint32_t)(m[1] >> 32), lane);
             S w[2];
 #pragma unroll
             for (int t = 0; t < 2; t++) {   // plane lane + 32 t (a valid plane for the shuffles' sake)
                 const int p = lane + 32 * t < B ? lane + 32 * t : 0;
                 const int k = B - 1 - p, src = k & 31;
-                const uint32_t a0 = __shfl_sync(FULL, lo0, src), b0 = __shfl_sync(FULL, hi0, src);
-                const uint32_t a1 = __shfl_sync(FULL, lo1, src), b1 = __shfl_sync(FULL, hi1, src);
-                w[t] = k >= 32 ? ((S)b1 << 32 | b0) : ((S)a1 << 32 | a0);
+                const uint32_t a0 = __shfl_sync(FULL, lo0, src), c0 = __shfl_sync(FULL, hi0, src);
+                const uint32_t a1 = __shfl_sync(FULL, lo1, src), c1 = __shfl_sync(FULL, hi1, src);
+                w[t] = k >= 32 ? ((S)c1 << 32 | c0) : ((S)a1 << 32 | a0);
             }
-            mine0 = lane >= r ? w[0] : 0;
-            mine1 = lane + 32 >= r ? w[1] : 0;
-        } else {
-            for (int p = r; p < B; p++) {                      // encode_block :337-357
-                const int k = B - 1 - p;
-                S w = (S)__ballot_sync(FULL, (q[0] >> k) & 1u);
-                if ((p & 31) == lane) {
-                    if (p < 32) mine0 = w; else mine1 = w;
-                }
+            if (lane < B && lane >= r) {
+                S* dst = q.out + (uint64_t)lane * cap + off0;
+                if (lane == r) { dst[0] = sign; dst[1] = w[0]; }
+                else dst[0] = w[0];
             }
+            if (lane + 32 < B && lane + 32 >= r) {
+                S* dst = q.out + (uint64_t)(lane + 32) * cap + off1;
+                if (lane + 32 == r) { dst[0] = sign; dst[1] = w[1]; }
+                else dst[0] = w[1];
+            }
+            off0 += gr_words(r, lane);
+            off1 += gr_words(r, lane + 32);
         }
-        if (lane < B && lane >= r) {
-            S* dst = out + (uint64_t)lane * cap + off0;
-            if (lane == r) { dst[0] = sign; dst[1] = mine0; }
-            else dst[0] = mine0;
-        }
-        if (lane + 32 < B && lane + 32 >= r) {
-            S* dst = out + (uint64_t)(lane + 32) * cap + off1;
-            if (lane + 32 == r) { dst[0] = sign; dst[1] = mine1; }
-            else dst[0] = mine1;
-        }
-        off0 += gr_words(r, lane);
-        off1 += gr_words(r, lane + 32);
     }
 }
 
 // fp32 grouped writer: one transpose per block instead of B ballots. With
 // ERR, the exact squared-error tables (errtab.cuh, GroupedBPEncoder.hpp:76-145
 // with collect_level_errors :324-335) of the CTA's chunk go to its record
-// recs + blockIdx.x: four blocks per step, t = trunc(|x|), bit counts from the
-// transposed magnitude words.
+// recs + blockIdx.x (one level per launch): four blocks per step, t =
+// trunc(|x|), bit counts from the transposed magnitude words.
 constexpr size_t kErrSmemGR = 8 * sizeof(errtab::WarpQ) + errtab::kSlotsPad * sizeof(unsigned long long);
 
 template <bool ERR>
-__global__ void __launch_bounds__(256) k_gr_write32(const float* __restrict__ x, uint64_t n,
-                                                   const uint32_t* __restrict__ maxkey, int exp_arg, int B,
-                                                   const uint8_t* __restrict__ rbs,
-                                                   const uint32_t* __restrict__ chunk_off, uint32_t* __restrict__ out,
-                                                   uint64_t cap, unsigned long long* __restrict__ recs) {
+__global__ void __launch_bounds__(256) k_gr_write32(const __grid_constant__ GrSet<float> set, int B,
+                                                   unsigned long long* __restrict__ recs) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const int exp = maxkey ? frexp_exp(__uint_as_float(*maxkey)) : exp_arg;
+    uint32_t chunk;
+    const GrSeg<float>& q = gr_seg(set, chunk);
+    const float* __restrict__ x = q.x;
+    const uint64_t n = q.n, cap = q.cap;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t nblocks = (n + 31) / 32;
+    pdl_wait();
+    pdl_release();
+    const int exp = level_exp<float>(q.key, q.exp);
     uint32_t off0, off1;
-    gr_warp_offsets(rbs, nblocks, chunk_off, B, off0, off1);
+    const int rv = gr_warp_offsets(q.rbs, nblocks, chunk, q.co, B, off0, off1);
     const int plane = B - 1 - lane;                    // lane k owns bit k
     uint32_t off = __shfl_sync(FULL, off0, plane & 31);
     const bool fast = pow2_normal(B - exp);
     const float sc = fast ? pow2f(B - exp) : 1.f;
-    const uint64_t b0 = (uint64_t)blockIdx.x * GR_CHUNK + (uint64_t)warp * GR_BPW;
+    const uint64_t b0 = (uint64_t)chunk * GR_CHUNK + (uint64_t)warp * GR_BPW;
     errtab::WarpQ* wq = (errtab::WarpQ*)smem;
     unsigned long long* red = (unsigned long long*)(wq + 8);
     errtab::Lane acc;
@@ -874,9 +908,9 @@ __global__ void __launch_bounds__(256) k_gr_write32(const float* __restrict__ x,
         acc.zero();
         errtab::zero_q(wq[warp], lane);
     }
-    for (int j0 = 0; j0 < GR_BPW; j0 += 4) {
+    for (int j0 = 0; j0 < GR_BPW && (ERR || b0 + j0 < nblocks); j0 += 4) {
         float sh[4], mag[4];
-        uint32_t q[4], sign[4];
+        uint32_t m[4], sign[4];
         bool small[4];
 #pragma unroll
         for (int g = 0; g < 4; g++) {
@@ -886,7 +920,7 @@ __global__ void __launch_bounds__(256) k_gr_write32(const float* __restrict__ x,
             sh[g] = scale2(v, B - exp, fast, sc);
             const int64_t fix = (int64_t)sh[g];
             const bool neg = v < 0.f;
-            q[g] = (uint32_t)(neg ? -fix : fix);
+            m[g] = (uint32_t)(neg ? -fix : fix);
             sign[g] = __ballot_sync(FULL, neg);
             if (ERR) {
                 mag[g] = fabsf(sh[g]);
@@ -898,22 +932,19 @@ __global__ void __launch_bounds__(256) k_gr_write32(const float* __restrict__ x,
         if (ERR) {
             errtab::enqueue4(wq[warp], head, qn, small, mag, lane);
             errtab::drain_full<false>(wq[warp], head, qn, lane);
-            acc.add4(q[0], q[1], q[2], q[3]);
+            acc.add4(m[0], m[1], m[2], m[3]);
         }
 #pragma unroll
         for (int g = 0; g < 4; g++) {
-            const uint64_t b = b0 + j0 + g;
-            const uint32_t w = transpose32(q[g], lane);
+            const uint32_t w = transpose32(m[g], lane);
             if (ERR) acc.pc += __popc(w);
-            if (b < nblocks) {
-                const int r = rbs[b];
-                if (lane < B && plane >= r) {
-                    uint32_t* dst = out + (uint64_t)plane * cap + off;
-                    if (plane == r) { dst[0] = sign[g]; dst[1] = w; }
-                    else dst[0] = w;
-                }
-                off += gr_words(r, plane);
+            const int r = __shfl_sync(FULL, rv, j0 + g);
+            if (lane < B && plane >= r) {
+                uint32_t* dst = q.out + (uint64_t)plane * cap + off;
+                if (plane == r) { dst[0] = sign[g]; dst[1] = w; }
+                else dst[0] = w;
             }
+            off += gr_words(r, plane);
         }
     }
     if (ERR) {
@@ -928,172 +959,124 @@ __global__ void __launch_bounds__(256) k_gr_write32(const float* __restrict__ x,
     }
 }
 
-// fp32 grouped decoder, planes [s, e): lane p loads plane p's word of the block
-__global__ void __launch_bounds__(256) k_gr_decode32(const uint32_t* const* __restrict__ planes, uint64_t n,
-                                                    const uint32_t* __restrict__ maxkey, int exp_arg, int B, int s,
-                                                    int e, const uint8_t* __restrict__ dnum,
-                                                    const uint8_t* __restrict__ rbs,
-                                                    const uint32_t* __restrict__ chunk_off,
-                                                    uint32_t* __restrict__ signs, float* __restrict__ out) {
-    if (dnum) e = dnum[0];
-    const int exp = maxkey ? frexp_exp(__uint_as_float(*maxkey)) : exp_arg;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t nblocks = (n + 31) / 32;
-    uint32_t off0, off1;
-    gr_warp_offsets(rbs, nblocks, chunk_off, B, off0, off1);
-    const uint32_t* src = (lane < B && lane >= s && lane < e) ? planes[lane] : nullptr;
-    const bool fast = pow2_normal(exp - e);
-    const float sc = fast ? pow2f(exp - e) : 1.f;
-    const uint64_t b0 = (uint64_t)blockIdx.x * GR_CHUNK + (uint64_t)warp * GR_BPW;
-    for (int j = 0; j < GR_BPW; j++) {
-        const uint64_t b = b0 + j;
-        if (b >= nblocks) break;
-        const int r = rbs[b];
-        const uint64_t i = b * 32 + lane;
-        if (r < e) {
-            uint32_t w = 0, sg = 0;
-            if (src && lane >= r) {
-                if (lane == r) { sg = src[off0]; w = src[off0 + 1]; }
-                else w = src[off0];
-            }
-            uint32_t sign;
-            if (r >= s) {
-                sign = __shfl_sync(FULL, sg, r);
-                if (signs && lane == 0) signs[b] = sign;
-            } else {
-                sign = signs[b];
-            }
-            const uint32_t col = transpose32(w, lane);
-            const uint32_t acc = __brev(col) >> (32 - e);
-            const float v = scale2((float)acc, exp - e, fast, sc);
-            if (i < n) out[i] = ((sign >> lane) & 1u) ? -v : v;
-        } else {
-            if (i < n) out[i] = 0.f;
-        }
-        off0 += gr_words(r, lane);
-    }
-}
-
-// fp32 grouped pass 1: each block's recording bitplane and the chunk's word counts
-__global__ void __launch_bounds__(256) k_gr_rb32(const float* __restrict__ x, uint64_t n,
-                                                const uint32_t* __restrict__ maxkey, int exp_arg, int B,
-                                                uint8_t* __restrict__ rbs, uint32_t* __restrict__ chunk_words) {
-    const int exp = maxkey ? frexp_exp(__uint_as_float(*maxkey)) : exp_arg;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t nblocks = (n + 31) / 32;
-    __shared__ uint32_t cnt[GR_WARPS][32];
-    uint32_t c0 = 0;
-    const bool fast = pow2_normal(B - exp);
-    const float sc = fast ? pow2f(B - exp) : 1.f;
-    const uint64_t b0 = (uint64_t)blockIdx.x * GR_CHUNK + (uint64_t)warp * GR_BPW;
-    for (int j = 0; j < GR_BPW; j++) {
-        const uint64_t b = b0 + j;
-        if (b >= nblocks) break;
-        const uint64_t i = b * 32 + lane;
-        uint32_t q = 0;
-        if (i < n) {
-            const float sh = scale2(__ldg(x + i), B - exp, fast, sc);
-            const int64_t fix = (int64_t)sh;
-            q = (uint32_t)(fix < 0 ? -fix : fix);
-        }
-        const uint32_t o = __reduce_or_sync(FULL, q);
-        const int r = o ? B - 1 - (31 - __clz(o)) : B;
-        if (lane == 0) rbs[b] = (uint8_t)r;
-        c0 += gr_words(r, lane);
-    }
-    cnt[warp][lane] = c0;
-    __syncthreads();
-    if (threadIdx.x < 32 && (int)threadIdx.x < B) {
-        uint32_t t = 0;
-        for (int w = 0; w < GR_WARPS; w++) t += cnt[w][threadIdx.x];
-        chunk_words[(uint64_t)blockIdx.x * B + threadIdx.x] = t;
-    }
-}
-
 // GroupedBPEncoder::progressive_decode -- :210-297 (planes [s, e)); plane p's
 // words at planes[p] (absolute plane index). signs: per-block sign words kept
 // between calls (nullable when s == 0). A device count (dnum[0]) overrides e.
-template <class T>
-__global__ void __launch_bounds__(256) k_gr_decode(const typename Traits<T>::S* const* __restrict__ planes,
-                                                   uint64_t n, const typename KeyOf<T>::type* __restrict__ maxkey,
-                                                   int exp_arg, int B, int s, int e,
-                                                   const uint8_t* __restrict__ dnum, const uint8_t* __restrict__ rbs,
-                                                   const uint32_t* __restrict__ chunk_off,
-                                                   typename Traits<T>::S* __restrict__ signs, T* __restrict__ out) {
-    using S = typename Traits<T>::S;
-    using FP = typename Traits<T>::FP;
-    constexpr int BS = Traits<T>::kBlock;
-    if (dnum) e = dnum[0];
-    const int exp = level_exp<T>(maxkey, exp_arg);
+// fp32: lane p loads plane p's word of the block.
+__global__ void __launch_bounds__(256) k_gr_decode32(const __grid_constant__ GrSet<float> set, int B, int s, int e) {
+    constexpr int U = 8;   // blocks loaded ahead
+    uint32_t chunk;
+    const GrSeg<float>& q = gr_seg(set, chunk);
+    const uint64_t n = q.n;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t nblocks = (n + BS - 1) / BS;
-    uint32_t off0, off1;
-    gr_warp_offsets(rbs, nblocks, chunk_off, B, off0, off1);
-    const uint64_t b0 = (uint64_t)blockIdx.x * GR_CHUNK + (uint64_t)warp * GR_BPW;
-    for (int j = 0; j < GR_BPW; j++) {
-        uint64_t b = b0 + j;
-        if (b >= nblocks) break;
-        const int r = rbs[b];
-        if (r < e) {
-            S w0 = 0, w1 = 0, sg0 = 0, sg1 = 0;
-            int p0 = lane, p1 = lane + 32;
-            if (p0 < e && p0 >= s && p0 >= r) {
-                const S* src = planes[p0] + off0;
-                if (p0 == r) { sg0 = src[0]; w0 = src[1]; } else w0 = src[0];
-            }
-            if (p1 < e && p1 >= s && p1 >= r) {
-                const S* src = planes[p1] + off1;
-                if (p1 == r) { sg1 = src[0]; w1 = src[1]; } else w1 = src[0];
-            }
-            S sign;
-            if (r >= s) {
-                sign = __shfl_sync(FULL, r < 32 ? sg0 : sg1, r & 31);
-                if (signs && lane == 0) signs[b] = sign;
-            } else {
-                sign = signs[b];
-            }
-            FP acc[BS / 32];
+    const uint64_t nblocks = (n + 31) / 32;
+    pdl_wait();
+    pdl_release();
+    if (q.dnum) e = q.dnum[0];
+    const int exp = level_exp<float>(q.key, q.exp);
+    uint32_t off, unused;
+    const int rv = gr_warp_offsets(q.rbs, nblocks, chunk, q.co, B, off, unused);
+    const uint32_t* src = (lane < B && lane >= s && lane < e) ? q.planes[lane] : nullptr;
+    const bool fast = pow2_normal(exp - e);
+    const float sc = fast ? pow2f(exp - e) : 1.f;
+    const uint64_t b0 = (uint64_t)chunk * GR_CHUNK + (uint64_t)warp * GR_BPW;
+    for (int j0 = 0; j0 < GR_BPW && b0 + j0 < nblocks; j0 += U) {
+        uint32_t w[U], sg[U];
 #pragma unroll
-            for (int h = 0; h < BS / 32; h++) acc[h] = 0;
-            if constexpr (BS == 64) {
+        for (int u = 0; u < U; u++) {
+            const int r = __shfl_sync(FULL, rv, j0 + u);
+            w[u] = sg[u] = 0;
+            if (src && lane >= r) {
+                const bool head = lane == r;
+                w[u] = __ldcs(src + off + (head ? 1 : 0));
+                if (head) sg[u] = __ldcs(src + off);
+            }
+            if (r < s && lane == 0) sg[u] = q.signs[b0 + j0 + u];   // kept by an earlier call
+            off += gr_words(r, lane);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int r = __shfl_sync(FULL, rv, j0 + u);
+            const uint64_t b = b0 + j0 + u, i = b * 32 + lane;
+            if (r < e) {
+                const uint32_t sign = __shfl_sync(FULL, sg[u], r >= s ? r : 0);
+                if (r >= s && q.signs && lane == 0) q.signs[b] = sign;
+                const uint32_t col = transpose32(w[u], lane);
+                const uint32_t acc = __brev(col) >> (32 - e);
+                const float v = scale2((float)acc, exp - e, fast, sc);
+                if (i < n) q.y[i] = ((sign >> lane) & 1u) ? -v : v;
+            } else if (i < n) {
+                q.y[i] = 0.f;
+            }
+        }
+    }
+}
+
+// fp64
+__global__ void __launch_bounds__(256) k_gr_decode64(const __grid_constant__ GrSet<double> set, int B, int s, int e) {
+    using S = uint64_t;
+    constexpr int U = 4;   // blocks loaded ahead
+    uint32_t chunk;
+    const GrSeg<double>& q = gr_seg(set, chunk);
+    const uint64_t n = q.n;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t nblocks = (n + 63) / 64;
+    pdl_wait();
+    pdl_release();
+    if (q.dnum) e = q.dnum[0];
+    const int exp = level_exp<double>(q.key, q.exp);
+    uint32_t off0, off1;
+    const int rv = gr_warp_offsets(q.rbs, nblocks, chunk, q.co, B, off0, off1);
+    const S* src0 = (lane >= s && lane < e) ? q.planes[lane] : nullptr;
+    const S* src1 = (lane + 32 >= s && lane + 32 < e) ? q.planes[lane + 32] : nullptr;
+    const uint64_t b0 = (uint64_t)chunk * GR_CHUNK + (uint64_t)warp * GR_BPW;
+    for (int j0 = 0; j0 < GR_BPW && b0 + j0 < nblocks; j0 += U) {
+        S w0[U], w1[U], sg[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int r = __shfl_sync(FULL, rv, j0 + u);
+            w0[u] = w1[u] = sg[u] = 0;
+            if (src0 && lane >= r) {
+                w0[u] = __ldcs(src0 + off0 + (lane == r ? 1 : 0));
+                if (lane == r) sg[u] = __ldcs(src0 + off0);
+            }
+            if (src1 && lane + 32 >= r) {
+                w1[u] = __ldcs(src1 + off1 + (lane + 32 == r ? 1 : 0));
+                if (lane + 32 == r) sg[u] = __ldcs(src1 + off1);
+            }
+            if (r < s && lane == 0) sg[u] = q.signs[b0 + j0 + u];   // kept by an earlier call
+            off0 += gr_words(r, lane);
+            off1 += gr_words(r, lane + 32);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int r = __shfl_sync(FULL, rv, j0 + u);
+            const uint64_t b = b0 + j0 + u, i = b * 64 + lane;
+            if (r < e) {
+                const S sign = __shfl_sync(FULL, sg[u], r >= s ? r & 31 : 0);
+                if (r >= s && q.signs && lane == 0) q.signs[b] = sign;
                 // decode_block :359-368 by four warp bit transposes: lane p holds
                 // planes p and p + 32 (zero where not read); after the
                 // transposes lane v holds, per half h of the block, a word whose
                 // bit p is plane p's bit of value 32 h + v (planes 0..31) and one
                 // for planes 32..63. Plane p weighs 2^(e-1-p): the bit-reversed
                 // words, shifted into place.
-                const uint32_t pl0 = transpose32((uint32_t)w0, lane), ph0 = transpose32((uint32_t)(w0 >> 32), lane);
-                const uint32_t pl1 = transpose32((uint32_t)w1, lane), ph1 = transpose32((uint32_t)(w1 >> 32), lane);
-                const uint32_t lo[2] = {pl0, ph0}, hi[2] = {pl1, ph1};
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    // planes 0..31 -> bits e-1 .. e-32, planes 32..63 -> bits e-33 ..
-                    const uint64_t a = (uint64_t)__brev(lo[h]) << 32 | __brev(hi[h]);   // plane p at bit 63 - p
-                    acc[h] = (FP)(e > 0 ? a >> (64 - e) : 0ull);
+                const uint32_t pl0 = transpose32((uint32_t)w0[u], lane), ph0 = transpose32((uint32_t)(w0[u] >> 32), lane);
+                uint32_t pl1 = 0, ph1 = 0;
+                if (e > 32) {
+                    pl1 = transpose32((uint32_t)w1[u], lane);
+                    ph1 = transpose32((uint32_t)(w1[u] >> 32), lane);
                 }
+                // planes 0..31 -> bits e-1 .. e-32, planes 32..63 -> bits e-33 ..
+                const uint64_t a0 = (uint64_t)__brev(pl0) << 32 | __brev(pl1);   // plane p at bit 63 - p
+                const uint64_t a1 = (uint64_t)__brev(ph0) << 32 | __brev(ph1);
+                if (i < n) q.y[i] = gr_value<double>(a0 >> (64 - e), exp - e, (sign >> lane) & 1u);
+                if (i + 32 < n) q.y[i + 32] = gr_value<double>(a1 >> (64 - e), exp - e, (sign >> (lane + 32)) & 1u);
             } else {
-                const int first = r > s ? r : s;
-                for (int p = first; p < e; p++) {             // decode_block :359-368
-                    S w = __shfl_sync(FULL, p < 32 ? w0 : w1, p & 31);
-                    const int k = e - 1 - p;
-#pragma unroll
-                    for (int h = 0; h < BS / 32; h++) acc[h] |= (FP)((w >> (h * 32 + lane)) & 1u) << k;
-                }
-            }
-#pragma unroll
-            for (int h = 0; h < BS / 32; h++) {
-                uint64_t i = b * BS + h * 32 + lane;
-                if (i < n) out[i] = gr_value<T>(acc[h], -e + exp, (sign >> (h * 32 + lane)) & 1u);
-            }
-        } else {
-#pragma unroll
-            for (int h = 0; h < BS / 32; h++) {
-                uint64_t i = b * BS + h * 32 + lane;
-                if (i < n) out[i] = (T)0;
+                if (i < n) q.y[i] = 0.0;
+                if (i + 32 < n) q.y[i + 32] = 0.0;
             }
         }
-        off0 += gr_words(r, lane);
-        off1 += gr_words(r, lane + 32);
     }
 }
 
@@ -1166,31 +1149,21 @@ __global__ void k_reduce_partials(const double* __restrict__ partial, int nparts
     }
 }
 
-// MaxErrorCollector::collect_level_error -- MaxErrorCollector.hpp:14-25, for
-// all levels at once from the device bound array.
+// per-chunk word counts from the rb arrays (used when only the headers are known)
 template <class T>
-__global__ void k_max_collect(const T* __restrict__ bounds, int nl, int B, double* __restrict__ out) {
-    for (int l = blockIdx.x * blockDim.x + threadIdx.x; l < nl; l += gridDim.x * blockDim.x) {
-        T bound = bounds[l];
-        int e = frexp_exp(bound);
-        double* o = out + (size_t)l * (B + 1);
-        o[0] = (double)bound;
-        double err = ldexp(1.0, e - 1);
-        for (int i = 1; i <= B; i++) { o[i] = err; err /= 2; }
-    }
-}
-
-// per-chunk word counts from an rb array (used when only the header is known)
-__global__ void k_chunk_words_from_rb(const uint8_t* __restrict__ rbs, uint64_t nblocks, int B,
-                                      uint32_t* __restrict__ chunk_words) {
+__global__ void k_chunk_words_from_rb(const __grid_constant__ GrSet<T> set, int B) {
+    constexpr int BS = Traits<T>::kBlock;
+    uint32_t chunk;
+    const GrSeg<T>& q = gr_seg(set, chunk);
     __shared__ uint32_t cnt[GR_WARPS][64];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t b0 = (uint64_t)blockIdx.x * GR_CHUNK + (uint64_t)warp * GR_BPW;
+    const uint64_t nblocks = (q.n + BS - 1) / BS;
+    const uint64_t b = (uint64_t)chunk * GR_CHUNK + (uint64_t)warp * GR_BPW + lane;
+    const int rv = b < nblocks ? q.rbs[b] : 255;
     uint32_t c0 = 0, c1 = 0;
+#pragma unroll 8
     for (int j = 0; j < GR_BPW; j++) {
-        uint64_t b = b0 + j;
-        if (b >= nblocks) break;
-        int r = rbs[b];
+        const int r = __shfl_sync(FULL, rv, j);
         c0 += gr_words(r, lane);
         c1 += gr_words(r, lane + 32);
     }
@@ -1200,7 +1173,7 @@ __global__ void k_chunk_words_from_rb(const uint8_t* __restrict__ rbs, uint64_t 
     if (threadIdx.x < 64 && (int)threadIdx.x < B) {
         uint32_t s = 0;
         for (int w = 0; w < GR_WARPS; w++) s += cnt[w][threadIdx.x];
-        chunk_words[(uint64_t)blockIdx.x * B + threadIdx.x] = s;
+        q.cw[(uint64_t)chunk * B + threadIdx.x] = s;
     }
 }
 
@@ -1302,8 +1275,9 @@ int launch_nb_encode_levels(const ChunkSeg* segs, int nseg, uint64_t total_chunk
     (void)keys;   // each segment carries its level's key
     if (errs_out) return nb_err_launch(segs, ChunkSeg{}, nseg, total_chunks, B, 0, partial, errs_out, st);
     const unsigned grid = (unsigned)nb_encode_levels_grid(0);
-    k_nb_encode32_levels<<<grid, 256, 0, st>>>(segs, nseg, total_chunks, B);
-    PRODM_CHECK_LAUNCH("k_nb_encode32_levels");
+    count_launch();
+    const cudaError_t e = launch_chain(true, k_nb_encode32_levels, dim3(grid), dim3(256), 0, st, segs, nseg, total_chunks, B);
+    if (e != cudaSuccess) return cuda_status(e, "k_nb_encode32_levels");
     return PRODM_OK;
 }
 
@@ -1330,90 +1304,79 @@ int launch_nb_decode(const void* base, uint64_t stride, uint64_t n, const void* 
 
 uint64_t gr_nchunks(uint64_t nblocks) { return (nblocks + GR_CHUNK - 1) / GR_CHUNK; }
 
+// the segments' first chunks; the launch's chunks
 template <class T>
-int launch_gr_encode(const T* x, uint64_t n, const void* maxkey, int exp, int B, uint8_t* rbs, uint32_t* chunk_words,
-                     uint32_t* chunk_off, uint32_t* sizes, void* out, uint64_t cap, double* partial, double* errs_out,
-                     cudaStream_t st) {
-    using K = typename KeyOf<T>::type;
-    constexpr int BS = Traits<T>::kBlock;
-    const uint64_t nblocks = (n + BS - 1) / BS;
-    const uint64_t nch = gr_nchunks(nblocks);
-    if (std::is_same<T, float>::value) {
-        k_gr_rb32<<<(unsigned)nch, GR_WARPS * 32, 0, st>>>((const float*)x, n, (const uint32_t*)maxkey, exp, B, rbs,
-                                                          chunk_words);
-        PRODM_CHECK_LAUNCH("k_gr_rb32");
-        k_gr_scan<<<B, 1024, 0, st>>>(chunk_words, nch, B, nblocks, 4, chunk_off, sizes);
-        PRODM_CHECK_LAUNCH("k_gr_scan");
+static unsigned gr_number(GrSet<T>& set) {
+    uint64_t c = 0;
+    for (int l = 0; l < set.n; l++) {
+        set.seg[l].chunk0 = (uint32_t)c;
+        c += gr_nchunks((set.seg[l].n + Traits<T>::kBlock - 1) / Traits<T>::kBlock);
+    }
+    return (unsigned)c;
+}
+
+#define PRODM_CHAIN(name, ...)                                   \
+    do {                                                         \
+        count_launch();                                          \
+        const cudaError_t e_ = launch_chain(true, __VA_ARGS__);  \
+        if (e_ != cudaSuccess) return cuda_status(e_, name);     \
+    } while (0)
+
+template <class T>
+int launch_gr_encode(GrSet<T> set, int B, double* partial, double* errs_out, cudaStream_t st) {
+    constexpr bool f32 = std::is_same<T, float>::value;
+    const dim3 grid(gr_number(set)), block(GR_WARPS * 32);
+    if (errs_out && set.n != 1) return fail(PRODM_EINVAL, "grouped encode: error tables take one level per call");
+    if (!grid.x) return PRODM_OK;
+    if (!f32 && errs_out) {
+        if constexpr (!f32) {
+            PRODM_CHAIN("k_gr_rb", k_gr_rb<T, true>, grid, block, 0, st, set, B, partial);
+            k_reduce_partials<T><<<(B + 8) / 8, 256, 0, st>>>(partial, (int)grid.x, B, set.seg[0].key, set.seg[0].exp, 0,
+                                                             1, errs_out);
+            PRODM_CHECK_LAUNCH("k_reduce_partials");
+        }
+    } else {
+        PRODM_CHAIN("k_gr_rb", k_gr_rb<T, false>, grid, block, 0, st, set, B, (double*)nullptr);
+    }
+    PRODM_CHAIN("k_gr_scan", k_gr_scan<T>, dim3(B, set.n), dim3(1024), 0, st, set, B);
+    if constexpr (f32) {
         unsigned long long* recs = (unsigned long long*)partial;
         if (errs_out) {
-            k_gr_write32<true><<<(unsigned)nch, GR_WARPS * 32, kErrSmemGR, st>>>(
-                (const float*)x, n, (const uint32_t*)maxkey, exp, B, rbs, chunk_off, (uint32_t*)out, cap, recs);
-            PRODM_CHECK_LAUNCH("k_gr_write32");
+            PRODM_CHAIN("k_gr_write32", k_gr_write32<true>, grid, block, kErrSmemGR, st, set, B, recs);
             ChunkSeg one = {};
-            one.n = n;
-            one.key = (const uint32_t*)maxkey;
-            k_errtab_final<false><<<1, 1024, 0, st>>>(recs, (int)nch, B, nullptr, one, exp, 0, errs_out);
+            one.n = set.seg[0].n;
+            one.key = set.seg[0].key;
+            k_errtab_final<false><<<1, 1024, 0, st>>>(recs, (int)grid.x, B, nullptr, one, set.seg[0].exp, 0, errs_out);
             PRODM_CHECK_LAUNCH("k_errtab_final");
         } else {
-            k_gr_write32<false><<<(unsigned)nch, GR_WARPS * 32, 0, st>>>(
-                (const float*)x, n, (const uint32_t*)maxkey, exp, B, rbs, chunk_off, (uint32_t*)out, cap, nullptr);
-            PRODM_CHECK_LAUNCH("k_gr_write32");
+            PRODM_CHAIN("k_gr_write32", k_gr_write32<false>, grid, block, 0, st, set, B, (unsigned long long*)nullptr);
         }
-        return PRODM_OK;
-    }
-    if (errs_out) {
-        k_gr_rb<T, true><<<(unsigned)nch, GR_WARPS * 32, 0, st>>>(x, n, (const K*)maxkey, exp, B, rbs, chunk_words,
-                                                                  partial);
     } else {
-        k_gr_rb<T, false><<<(unsigned)nch, GR_WARPS * 32, 0, st>>>(x, n, (const K*)maxkey, exp, B, rbs, chunk_words,
-                                                                   nullptr);
+        PRODM_CHAIN("k_gr_write64", k_gr_write64, grid, block, 0, st, set, B);
     }
-    PRODM_CHECK_LAUNCH("k_gr_rb");
-    if (errs_out) {
-        k_reduce_partials<T><<<(B + 8) / 8, 256, 0, st>>>(partial, (int)nch, B, (const K*)maxkey, exp, 0, 1, errs_out);
-        PRODM_CHECK_LAUNCH("k_reduce_partials");
-    }
-    k_gr_scan<<<B, 1024, 0, st>>>(chunk_words, nch, B, nblocks, (int)sizeof(typename Traits<T>::S), chunk_off, sizes);
-    PRODM_CHECK_LAUNCH("k_gr_scan");
-    k_gr_write<T><<<(unsigned)nch, GR_WARPS * 32, 0, st>>>(x, n, (const K*)maxkey, exp, B, rbs, chunk_off,
-                                                           (typename Traits<T>::S*)out, cap);
-    PRODM_CHECK_LAUNCH("k_gr_write");
     return PRODM_OK;
 }
 
-int launch_chunk_words_from_rb(const uint8_t* rbs, uint64_t nblocks, int B, uint32_t* chunk_words, cudaStream_t st) {
-    const uint64_t nch = gr_nchunks(nblocks);
-    k_chunk_words_from_rb<<<(unsigned)nch, GR_WARPS * 32, 0, st>>>(rbs, nblocks, B, chunk_words);
+// chunk offsets and plane sizes of levels whose rb arrays are known
+template <class T>
+int launch_gr_offsets(GrSet<T> set, int B, cudaStream_t st) {
+    const unsigned grid = gr_number(set);
+    if (!grid) return PRODM_OK;
+    k_chunk_words_from_rb<T><<<grid, GR_WARPS * 32, 0, st>>>(set, B);
     PRODM_CHECK_LAUNCH("k_chunk_words_from_rb");
-    return PRODM_OK;
-}
-
-int launch_gr_scan_only(const uint32_t* chunk_words, uint64_t nchunks, int B, uint64_t nblocks, int word_bytes,
-                        uint32_t* chunk_off, uint32_t* sizes, cudaStream_t st) {
-    k_gr_scan<<<B, 1024, 0, st>>>(chunk_words, nchunks, B, nblocks, word_bytes, chunk_off, sizes);
+    k_gr_scan<T><<<dim3(B, set.n), 1024, 0, st>>>(set, B);
     PRODM_CHECK_LAUNCH("k_gr_scan");
     return PRODM_OK;
 }
 
 template <class T>
-int launch_gr_decode(const void* const* planes, uint64_t n, const void* maxkey, int exp, int B, int s, int e,
-                     const uint8_t* dnum, const uint8_t* rbs, const uint32_t* chunk_off, void* signs, T* out,
-                     cudaStream_t st) {
-    using K = typename KeyOf<T>::type;
-    using S = typename Traits<T>::S;
-    constexpr int BS = Traits<T>::kBlock;
-    const uint64_t nblocks = (n + BS - 1) / BS;
-    const uint64_t nch = gr_nchunks(nblocks);
-    if (std::is_same<T, float>::value) {
-        k_gr_decode32<<<(unsigned)nch, GR_WARPS * 32, 0, st>>>((const uint32_t* const*)planes, n,
-                                                              (const uint32_t*)maxkey, exp, B, s, e, dnum, rbs,
-                                                              chunk_off, (uint32_t*)signs, (float*)out);
-        PRODM_CHECK_LAUNCH("k_gr_decode32");
-        return PRODM_OK;
-    }
-    k_gr_decode<T><<<(unsigned)nch, GR_WARPS * 32, 0, st>>>((const S* const*)planes, n, (const K*)maxkey, exp, B, s, e,
-                                                            dnum, rbs, chunk_off, (S*)signs, out);
-    PRODM_CHECK_LAUNCH("k_gr_decode");
+int launch_gr_decode(GrSet<T> set, int B, int s, int e, cudaStream_t st) {
+    const dim3 grid(gr_number(set)), block(GR_WARPS * 32);
+    if (!grid.x) return PRODM_OK;
+    if constexpr (std::is_same<T, float>::value)
+        PRODM_CHAIN("k_gr_decode32", k_gr_decode32, grid, block, 0, st, set, B, s, e);
+    else
+        PRODM_CHAIN("k_gr_decode64", k_gr_decode64, grid, block, 0, st, set, B, s, e);
     return PRODM_OK;
 }
 
@@ -1428,24 +1391,15 @@ int launch_sq_collect(const T* x, uint64_t n, int B, T maxv, double* partial, do
     return PRODM_OK;
 }
 
-template <class T>
-int launch_max_collect(const T* bounds, int nl, int B, double* out, cudaStream_t st) {
-    k_max_collect<T><<<1, 32, 0, st>>>(bounds, nl, B, out);
-    PRODM_CHECK_LAUNCH("k_max_collect");
-    return PRODM_OK;
-}
-
 #define INST(T)                                                                                                       \
     template int launch_nb_encode<T>(const T*, uint64_t, const void*, int, int, void*, uint64_t, double*, double*,    \
                                      cudaStream_t);                                                                   \
     template int launch_nb_decode<T>(const void*, uint64_t, uint64_t, const void*, int, int, int, const uint8_t*, T*, \
                                      cudaStream_t);                                                                   \
-    template int launch_gr_encode<T>(const T*, uint64_t, const void*, int, int, uint8_t*, uint32_t*, uint32_t*,       \
-                                     uint32_t*, void*, uint64_t, double*, double*, cudaStream_t);                     \
-    template int launch_gr_decode<T>(const void* const*, uint64_t, const void*, int, int, int, int, const uint8_t*,   \
-                                     const uint8_t*, const uint32_t*, void*, T*, cudaStream_t);                       \
-    template int launch_sq_collect<T>(const T*, uint64_t, int, T, double*, double*, cudaStream_t);                   \
-    template int launch_max_collect<T>(const T*, int, int, double*, cudaStream_t);
+    template int launch_gr_encode<T>(GrSet<T>, int, double*, double*, cudaStream_t);                                  \
+    template int launch_gr_offsets<T>(GrSet<T>, int, cudaStream_t);                                                   \
+    template int launch_gr_decode<T>(GrSet<T>, int, int, int, cudaStream_t);                                          \
+    template int launch_sq_collect<T>(const T*, uint64_t, int, T, double*, double*, cudaStream_t);
 INST(float)
 INST(double)
 #undef INST

@@ -350,7 +350,15 @@ int encode_impl(int enc, const T* x, uint64_t n, int exp, int B, uint8_t* blob, 
         uint32_t* rows = (uint32_t*)ws.take((uint64_t)(B + 1) * rw * 4);
         uint32_t* counts = (uint32_t*)ws.take(64 * 4);
         void* scratch = ws.take(pb_pack_scratch_bytes(n, B));
-        if ((rc = launch_pb_encode<T>(x, n, nullptr, exp, B, rows, rw, counts, sizes, st))) return rc;
+        PbSet<T> set{1, {}};
+        set.seg[0].x = x;
+        set.seg[0].rows = rows;
+        set.seg[0].stride = rw;
+        set.seg[0].counts = counts;
+        set.seg[0].sizes = sizes;
+        set.seg[0].n = n;
+        set.seg[0].exp = exp;
+        if ((rc = launch_pb_encode<T>(set, B, st))) return rc;
         return launch_pb_pack(rows, rw, n, B, sizes, encode_bound(enc, dtype, n, B), blob, scratch, st);
     }
     if (enc == PRODM_ENC_NEGABINARY) {
@@ -363,8 +371,17 @@ int encode_impl(int enc, const T* x, uint64_t n, int exp, int B, uint8_t* blob, 
     uint32_t* cw = (uint32_t*)ws.take(nch * B * 4);
     uint32_t* co = (uint32_t*)ws.take(nch * B * 4);
     void** dptrs = (void**)ws.take(64 * sizeof(void*));
-    if ((rc = launch_gr_encode<T>(x, n, nullptr, exp, B, rbs, cw, co, sizes, staging, 2 * nb, partial, errs, st)))
-        return rc;
+    GrSet<T> set{1, {}};
+    set.seg[0].x = x;
+    set.seg[0].rbs = rbs;
+    set.seg[0].cw = cw;
+    set.seg[0].co = co;
+    set.seg[0].sizes = sizes;
+    set.seg[0].out = (typename Traits<T>::S*)staging;
+    set.seg[0].n = n;
+    set.seg[0].cap = 2 * nb;
+    set.seg[0].exp = exp;
+    if ((rc = launch_gr_encode<T>(set, B, partial, errs, st))) return rc;
     std::vector<void*> ptrs(B);
     for (int p = 0; p < B; p++) ptrs[p] = staging + (uint64_t)p * 2 * nb * sizeof(T);
     PRODM_CUDA(cudaMemcpyAsync(dptrs, ptrs.data(), B * sizeof(void*), cudaMemcpyHostToDevice, st));
@@ -461,9 +478,17 @@ int pb_progressive_decode(prodm_decoder* h, const uint8_t* blob, const uint32_t*
     job.status = status;
     PRODM_CUDA(cudaMemsetAsync(status, 0, 4, st));
     int rc = launch_pb_parse({job}, st);
-    if (!rc)
-        rc = launch_pb_decode<T>(rows, rw, n, nullptr, exp, B, s, s + num, nullptr, rows + (uint64_t)B * rw,
-                                 rows + (uint64_t)(B + 1) * rw, out, st);
+    if (!rc) {
+        PbSet<T> set{1, {}};
+        set.seg[0].y = out;
+        set.seg[0].rows = rows;
+        set.seg[0].stride = rw;
+        set.seg[0].srow = job.signs;
+        set.seg[0].unseen = job.unseen;
+        set.seg[0].n = n;
+        set.seg[0].exp = exp;
+        rc = launch_pb_decode<T>(set, B, s, s + num, st);
+    }
     int hstat = 0;
     if (!rc) {
         cudaError_t e = cudaMemcpyAsync(&hstat, status, 4, cudaMemcpyDeviceToHost, st);
@@ -524,11 +549,14 @@ int progressive_decode_impl(prodm_decoder* h, const uint8_t* blob, const uint32_
         PRODM_CUDA(cudaMalloc(&L.signs, nb * sizeof(T)));
         PRODM_CUDA(cudaMemcpyAsync(L.rbs, blob + 4, nb, cudaMemcpyDeviceToDevice, st));
         uint32_t* cw;
-        uint32_t* sz;
         PRODM_CUDA(cudaMallocAsync((void**)&cw, nch * B * 4 + 64 * 4, st));
-        sz = cw + nch * B;
-        if ((rc = launch_chunk_words_from_rb(L.rbs, nb, B, cw, st))) return rc;
-        if ((rc = launch_gr_scan_only(cw, nch, B, nb, ws_, L.chunk_off, sz, st))) return rc;
+        GrSet<T> set{1, {}};
+        set.seg[0].rbs = L.rbs;
+        set.seg[0].cw = cw;
+        set.seg[0].co = L.chunk_off;
+        set.seg[0].sizes = cw + nch * B;
+        set.seg[0].n = n;
+        if ((rc = launch_gr_offsets<T>(set, B, st))) return rc;
         cudaFreeAsync(cw, st);
         L.have = true;
         L.n = n;
@@ -574,8 +602,15 @@ int progressive_decode_impl(prodm_decoder* h, const uint8_t* blob, const uint32_
     PRODM_CUDA(cudaMemcpyAsync(uptr_d, uptr.data(), num * sizeof(void*), cudaMemcpyHostToDevice, st));
     PRODM_CUDA(cudaStreamSynchronize(st));
     if ((rc = launch_unpack_planes(blob, doff, dnw, num, ws_, uptr_d, maxw, st))) return rc;
-    rc = launch_gr_decode<T>((const void* const*)dptr, n, nullptr, exp, B, s, s + num, nullptr, L.rbs, L.chunk_off,
-                             L.signs, out, st);
+    GrSet<T> set{1, {}};
+    set.seg[0].y = out;
+    set.seg[0].rbs = L.rbs;
+    set.seg[0].co = L.chunk_off;
+    set.seg[0].planes = (const typename Traits<T>::S* const*)dptr;
+    set.seg[0].signs = (typename Traits<T>::S*)L.signs;
+    set.seg[0].n = n;
+    set.seg[0].exp = exp;
+    rc = launch_gr_decode<T>(set, B, s, s + num, st);
     cudaFreeAsync(uptr_d, st);
     cudaFreeAsync(tmp, st);
     return rc;
@@ -630,7 +665,6 @@ struct prodm_mdr {
     void* bounds = nullptr;
     uint32_t* sizes = nullptr;
     double* sqerr = nullptr;
-    double* maxerr = nullptr;
     double* partial = nullptr;
     uint8_t* rbs = nullptr;
     std::vector<uint64_t> rb_off, co_off;
@@ -816,7 +850,6 @@ int mdr_alloc_all(prodm_mdr* h) {
     if ((rc = h->alloc((void**)&h->sizes, (L + 1) * B * 4))) return rc;
     if ((rc = h->alloc((void**)&h->rsizes, (L + 1) * B * 4))) return rc;
     if ((rc = h->alloc((void**)&h->sqerr, (L + 1) * (B + 1) * 8))) return rc;
-    if ((rc = h->alloc((void**)&h->maxerr, (L + 1) * (B + 1) * 8))) return rc;
     uint64_t parts = maxch > (uint64_t)kPartialSlots ? maxch : (uint64_t)kPartialSlots;
     if ((rc = h->alloc((void**)&h->partial, partial_bytes(parts, B)))) return rc;
     if ((rc = h->alloc((void**)&h->index, L + 1 + 15))) return rc;
@@ -841,7 +874,7 @@ int mdr_alloc_all(prodm_mdr* h) {
         if ((rc = h->alloc((void**)&h->pbstatus, (L + 1) * 4))) return rc;
     } else {
         if ((rc = h->alloc((void**)&h->rbs, h->rb_off[L + 1]))) return rc;
-        if ((rc = h->alloc((void**)&h->chunk_words, maxch * B * 4))) return rc;
+        if ((rc = h->alloc((void**)&h->chunk_words, h->co_off[L + 1] * 4))) return rc;
         if ((rc = h->alloc((void**)&h->chunk_off, h->co_off[L + 1] * 4))) return rc;
         if ((rc = h->alloc((void**)&h->plane_ptrs, (L + 1) * B * sizeof(void*)))) return rc;
         std::vector<void*> ptrs((L + 1) * B);
@@ -904,6 +937,46 @@ const T* level_tabs(prodm_mdr* h, int l, int d) {
     return (const T*)h->tabs + h->tab_off[l * 3 + d];
 }
 
+// the levels' segments of the grouped and the per-bit launches, finest first
+template <class T>
+GrSet<T> mdr_gr_set(prodm_mdr* h, int from, int to) {
+    GrSet<T> set{0, {}};
+    for (int l = to; l >= from; l--) {
+        GrSeg<T>& q = set.seg[set.n++];
+        q.x = (const T*)h->coef + h->g.offset[l];
+        q.y = (T*)h->rcoef + h->roff[l];
+        q.key = (const typename KeyOf<T>::type*)h->keys + l;
+        q.rbs = h->rbs + h->rb_off[l];
+        q.cw = h->chunk_words + h->co_off[l];
+        q.co = h->chunk_off + h->co_off[l];
+        q.sizes = h->sizes + (uint64_t)l * h->B;
+        q.out = (typename Traits<T>::S*)(h->streams + h->lvl_byte_off[l]);
+        q.planes = (const typename Traits<T>::S* const*)(h->plane_ptrs + (uint64_t)l * h->B);
+        q.dnum = h->index + l;
+        q.n = h->g.elems[l];
+        q.cap = h->plane_cap[l];
+    }
+    return set;
+}
+template <class T>
+PbSet<T> mdr_pb_set(prodm_mdr* h) {
+    PbSet<T> set{0, {}};
+    for (int l = h->g.L; l >= 0; l--) {
+        PbSeg<T>& q = set.seg[set.n++];
+        q.x = (const T*)h->coef + h->g.offset[l];
+        q.y = (T*)h->rcoef + h->roff[l];
+        q.key = (const typename KeyOf<T>::type*)h->keys + l;
+        q.rows = (uint32_t*)(h->streams + h->lvl_byte_off[l]);
+        q.stride = h->plane_cap[l];
+        q.counts = h->pbcounts + l * 64;
+        q.sizes = h->sizes + (uint64_t)l * h->B;
+        q.dnum = h->index + l;
+        q.srow = q.rows + (uint64_t)h->B * q.stride;
+        q.n = h->g.elems[l];
+    }
+    return set;
+}
+
 template <class T>
 int mdr_refactor(prodm_mdr* h, const T* field, cudaStream_t st) {
     const LevelGeom& g = h->g;
@@ -944,21 +1017,24 @@ int mdr_refactor(prodm_mdr* h, const T* field, cudaStream_t st) {
         return launch_nb_encode_levels(h->eseg, L + 1, h->eseg_chunks, B, h->lpartial, (const uint32_t*)keys,
                                        h->sq ? h->sqerr : nullptr, st);
     }
+    // every level in one go (timed as the finest level), but for the fp64
+    // negabinary encoder and the error tables, which take a level per launch
+    if (h->pb) {
+        Stage sg(h, 1, L, st);
+        return launch_pb_encode<T>(mdr_pb_set<T>(h), B, st);
+    }
+    if (!h->nb && !h->sq) {
+        Stage sg(h, 1, L, st);
+        return launch_gr_encode<T>(mdr_gr_set<T>(h, 0, L), B, h->partial, nullptr, st);
+    }
     for (int l = 0; l <= L; l++) {
-        const uint64_t n = g.elems[l];
-        uint8_t* out = h->streams + h->lvl_byte_off[l];
         double* errs = h->sq ? h->sqerr + (uint64_t)l * (B + 1) : nullptr;
         Stage sg(h, 1, l, st);
-        if (h->pb) {
-            rc = launch_pb_encode<T>(coef + g.offset[l], n, keys + l, 0, B, (uint32_t*)out, h->plane_cap[l],
-                                     h->pbcounts + l * 64, h->sizes + (uint64_t)l * B, st);
-        } else if (h->nb) {
-            rc = launch_nb_encode<T>(coef + g.offset[l], n, keys + l, 0, B, out, h->plane_cap[l], h->partial, errs, st);
-        } else {
-            rc = launch_gr_encode<T>(coef + g.offset[l], n, keys + l, 0, B, h->rbs + h->rb_off[l], h->chunk_words,
-                                     h->chunk_off + h->co_off[l], h->sizes + (uint64_t)l * B, out, h->plane_cap[l],
-                                     h->partial, errs, st);
-        }
+        if (h->nb)
+            rc = launch_nb_encode<T>(coef + g.offset[l], g.elems[l], keys + l, 0, B, h->streams + h->lvl_byte_off[l],
+                                     h->plane_cap[l], h->partial, errs, st);
+        else
+            rc = launch_gr_encode<T>(mdr_gr_set<T>(h, l, l), B, h->partial, errs, st);
         if (rc) return rc;
     }
     return PRODM_OK;
@@ -979,23 +1055,17 @@ int mdr_decode_recompose(prodm_mdr* h, T* out, cudaStream_t st) {
         Stage sg(h, 3, 0, st);
         if ((rc = launch_nb_decode_levels(h->dseg, h->dseg_n, h->dseg_chunks, st, true))) return rc;
     }
-    for (int l = 0; l <= L; l++) {
-        if (l >= ffrom || (h->dseg && sizeof(T) == 4)) continue;
-        const uint64_t n = g.elems[l];
-        Stage sg(h, 3, l, st);
-        if (h->pb) {
-            const uint32_t* rows = (const uint32_t*)(h->streams + h->lvl_byte_off[l]);
-            rc = launch_pb_decode<T>(rows, h->plane_cap[l], n, keys + l, 0, B, 0, 0, h->index + l,
-                                     rows + (uint64_t)B * h->plane_cap[l], nullptr, rcoef + h->roff[l], st);
-        } else if (h->nb) {
-            rc = launch_nb_decode<T>(h->streams + h->lvl_byte_off[l], h->plane_cap[l], n, keys + l, 0, 0, 0,
-                                     h->index + l, rcoef + h->roff[l], st);
-        } else {
-            rc = launch_gr_decode<T>((const void* const*)(h->plane_ptrs + (uint64_t)l * B), n, keys + l, 0, B, 0, 0,
-                                     h->index + l, h->rbs + h->rb_off[l], h->chunk_off + h->co_off[l], nullptr,
-                                     rcoef + h->roff[l], st);
-        }
+    if (!h->nb) {   // every level in one launch (timed as level 0)
+        Stage sg(h, 3, 0, st);
+        rc = h->pb ? launch_pb_decode<T>(mdr_pb_set<T>(h), B, 0, 0, st)
+                   : launch_gr_decode<T>(mdr_gr_set<T>(h, 0, L), B, 0, 0, st);
         if (rc) return rc;
+    }
+    for (int l = 0; h->nb && sizeof(T) == 8 && l <= L; l++) {   // fp64 negabinary
+        Stage sg(h, 3, l, st);
+        if ((rc = launch_nb_decode<T>(h->streams + h->lvl_byte_off[l], h->plane_cap[l], g.elems[l], keys + l, 0, 0, 0,
+                                      h->index + l, rcoef + h->roff[l], st)))
+            return rc;
     }
     if (L == 0) {
         PRODM_CUDA(cudaMemcpyAsync(out, rcoef, g.total * sizeof(T), cudaMemcpyDeviceToDevice, st));
@@ -1031,23 +1101,18 @@ int mdr_decode_recompose(prodm_mdr* h, T* out, cudaStream_t st) {
 
 template <class T>
 int mdr_interpret(prodm_mdr* h, double tol, int interp, int est, double s, cudaStream_t st) {
-    const int L = h->g.L, B = h->B;
-    int rc;
-    const double* errs;
-    if (est == PRODM_EST_MAX_HB || est == PRODM_EST_MAX_OB) {
-        if ((rc = launch_max_collect<T>((const T*)h->bounds, L + 1, B, h->maxerr, st))) return rc;
-        errs = h->maxerr;
-    } else {
+    const int B = h->B;
+    const bool max_est = est == PRODM_EST_MAX_HB || est == PRODM_EST_MAX_OB;
+    if (!max_est) {
         if (!h->sq) return fail(PRODM_EINVAL, "squared-error estimators need collector == PRODM_COLLECT_SQUARED");
-        errs = h->sqerr;
     }
     Stage sg(h, 2, 0, st);
     // right after a reconstruction (whose kernels write none of the tables
     // and read the plane counts), the interpreter may tabulate before it waits
     const bool early = h->after_reconstruct;
     h->after_reconstruct = false;
-    return launch_interpret<T>(1, interp, est, h->ndims_d, h->levels_d, s, B, h->sizes, 0, errs, 0, nullptr, tol,
-                               h->index, 0, h->rsz, st, true, early);
+    return launch_interpret<T>(1, interp, est, h->ndims_d, h->levels_d, s, B, h->sizes, 0, h->sqerr, 0, nullptr, tol,
+                               h->index, 0, h->rsz, st, true, early, max_est ? (const T*)h->bounds : nullptr);
 }
 
 // per-bit levels loaded from files: parse the planes that lie completely
@@ -1111,6 +1176,14 @@ int pb_parse_loaded(prodm_mdr* h, cudaStream_t st) {
     return PRODM_OK;
 }
 
+// chunk offsets of a loaded level, from its header (its plane sizes are known)
+template <class T>
+int mdr_gr_offsets(prodm_mdr* h, int l, cudaStream_t st) {
+    GrSet<T> set = mdr_gr_set<T>(h, l, l);
+    set.seg[0].sizes = (uint32_t*)h->partial;
+    return launch_gr_offsets<T>(set, h->B, st);
+}
+
 // grouped levels loaded from files: header -> rb + chunk offsets, then the
 // planes completely inside the loaded prefix -> aligned layout
 int mdr_unpack_loaded(prodm_mdr* h, cudaStream_t st) {
@@ -1125,10 +1198,8 @@ int mdr_unpack_loaded(prodm_mdr* h, cudaStream_t st) {
         if (!h->header_done[l]) {
             if (h->loaded[l] < hdr) continue;
             PRODM_CUDA(cudaMemcpyAsync(h->rbs + h->rb_off[l], h->lfile[l] + 4, nbk, cudaMemcpyDeviceToDevice, st));
-            if ((rc = launch_chunk_words_from_rb(h->rbs + h->rb_off[l], nbk, B, h->chunk_words, st))) return rc;
-            if ((rc = launch_gr_scan_only(h->chunk_words, gr_nchunks(nbk), B, nbk, wb, h->chunk_off + h->co_off[l],
-                                          (uint32_t*)h->partial, st)))
-                return rc;
+            rc = h->es == 8 ? mdr_gr_offsets<double>(h, l, st) : mdr_gr_offsets<float>(h, l, st);
+            if (rc) return rc;
             h->header_done[l] = 1;
         }
         // planes fully loaded

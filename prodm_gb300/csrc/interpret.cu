@@ -685,6 +685,7 @@ __global__ void __launch_bounds__(256, 1) k_interpret(int nfields, int kind, int
                                                    const int* __restrict__ levels, double s, int B,
                                                    const uint32_t* __restrict__ sizes, uint64_t sz_stride,
                                                    const double* __restrict__ errs, uint64_t err_stride,
+                                                   const T* __restrict__ bounds,
                                                    const double* __restrict__ tols, double tol0,
                                                    uint8_t* __restrict__ index, uint64_t idx_stride,
                                                    uint32_t* __restrict__ rsz, bool early) {
@@ -708,7 +709,16 @@ __global__ void __launch_bounds__(256, 1) k_interpret(int nfields, int kind, int
     __shared__ int8_t s_nan[kMaxLevels * 64];
     __shared__ int8_t s_en[kMaxLevels * 64];
     for (int i = threadIdx.x; i < nl * B; i += blockDim.x) s_sizes[i] = sizes[f * sz_stride + i];
-    for (int i = threadIdx.x; i < nl * (B + 1); i += blockDim.x) s_errs[i] = errs[f * err_stride + i];
+    if (bounds) {   // MaxErrorCollector::collect_level_error (MaxErrorCollector.hpp:14-25): the level's
+                    // bound, then 2^(e-1) for its exponent e, halved per plane
+        for (int i = threadIdx.x; i < nl * (B + 1); i += blockDim.x) {
+            const int l = i / (B + 1), j = i - l * (B + 1);
+            const T b = bounds[l];
+            s_errs[i] = j ? ldexp(1.0, frexp_exp(b) - j) : (double)b;
+        }
+    } else {
+        for (int i = threadIdx.x; i < nl * (B + 1); i += blockDim.x) s_errs[i] = errs[f * err_stride + i];
+    }
     __shared__ T s_tab[kMaxLevels];
     __shared__ uint8_t s_idx[kMaxLevels];
     uint8_t* gi = index + f * idx_stride;
@@ -781,10 +791,10 @@ template <class T>
 int launch_interpret(int nfields, int kind, int est_kind, const int* d_ndims, const int* d_levels, double s, int B,
                      const uint32_t* d_sizes, uint64_t sz_stride, const double* d_errs, uint64_t err_stride,
                      const double* d_tols, double tol0, uint8_t* d_index, uint64_t idx_stride, uint32_t* d_rsz,
-                     cudaStream_t st, bool pdl, bool early) {
+                     cudaStream_t st, bool pdl, bool early, const T* d_bounds) {
     count_launch();
     const cudaError_t e = launch_chain(pdl, k_interpret<T>, dim3(nfields), dim3(256), 0, st, nfields, kind, est_kind,
-                                       d_ndims, d_levels, s, B, d_sizes, sz_stride, d_errs, err_stride, d_tols, tol0,
+                                       d_ndims, d_levels, s, B, d_sizes, sz_stride, d_errs, err_stride, d_bounds, d_tols, tol0,
                                        d_index, idx_stride, d_rsz, pdl && early);
     if (e != cudaSuccess) return cuda_status(e, "k_interpret");
     return PRODM_OK;
@@ -792,9 +802,9 @@ int launch_interpret(int nfields, int kind, int est_kind, const int* d_ndims, co
 
 template int launch_interpret<float>(int, int, int, const int*, const int*, double, int, const uint32_t*, uint64_t,
                                      const double*, uint64_t, const double*, double, uint8_t*, uint64_t,
-                                     uint32_t*, cudaStream_t, bool, bool);
+                                     uint32_t*, cudaStream_t, bool, bool, const float*);
 template int launch_interpret<double>(int, int, int, const int*, const int*, double, int, const uint32_t*, uint64_t,
                                       const double*, uint64_t, const double*, double, uint8_t*, uint64_t,
-                                      uint32_t*, cudaStream_t, bool, bool);
+                                      uint32_t*, cudaStream_t, bool, bool, const double*);
 
 }  // namespace prodm

@@ -58,18 +58,39 @@ template <class T>
 int launch_nb_decode(const void* base, uint64_t stride, uint64_t n, const void* maxkey, int exp, int s, int num,
                      const uint8_t* dnum, T* out, cudaStream_t st);
 uint64_t gr_nchunks(uint64_t nblocks);
+// grouped encoder: one segment per level of a launch; planes p of a level's
+// streams at out + p * cap (encode) or planes[p] (decode)
 template <class T>
-int launch_gr_encode(const T* x, uint64_t n, const void* maxkey, int exp, int B, uint8_t* rbs, uint32_t* chunk_words,
-                     uint32_t* chunk_off, uint32_t* sizes, void* out, uint64_t cap, double* partial, double* errs_out,
-                     cudaStream_t st);
+struct GrSeg {
+    const T* x;                                       // encode input
+    T* y;                                             // decode output
+    const typename KeyOf<T>::type* key;               // level |max| key, or NULL and the exponent exp
+    uint8_t* rbs;                                     // recording planes, one per block
+    uint32_t* cw;                                     // encode: word counts, [chunk][B]
+    uint32_t* co;                                     // word offsets, [chunk][B]
+    uint32_t* sizes;                                  // encode: stream bytes, B
+    typename Traits<T>::S* out;
+    const typename Traits<T>::S* const* planes;
+    typename Traits<T>::S* signs;                     // decode: sign words kept between calls, or NULL
+    const uint8_t* dnum;                              // decode: planes (overrides e), or NULL
+    uint64_t n, cap;
+    uint32_t chunk0;                                  // set by the launchers
+    int exp;
+};
+constexpr int kGrLevels = 17;
 template <class T>
-int launch_gr_decode(const void* const* planes, uint64_t n, const void* maxkey, int exp, int B, int s, int e,
-                     const uint8_t* dnum, const uint8_t* rbs, const uint32_t* chunk_off, void* signs, T* out,
-                     cudaStream_t st);
+struct GrSet {
+    int n;
+    GrSeg<T> seg[kGrLevels];
+};
+template <class T>
+int launch_gr_encode(GrSet<T> set, int B, double* partial, double* errs_out, cudaStream_t st);
+template <class T>
+int launch_gr_offsets(GrSet<T> set, int B, cudaStream_t st);
+template <class T>
+int launch_gr_decode(GrSet<T> set, int B, int s, int e, cudaStream_t st);
 template <class T>
 int launch_sq_collect(const T* x, uint64_t n, int B, T maxv, double* partial, double* out, cudaStream_t st);
-template <class T>
-int launch_max_collect(const T* bounds, int nl, int B, double* out, cudaStream_t st);
 constexpr int kPartialSlots = kSMs * 4;   // per-CTA partial error tables of the fused collectors
 // bytes of `parts` per-CTA partials: B + 1 doubles (fp64 tables, squared-error
 // collector) or one record of the exact fp32 tables (errtab.cuh)
@@ -78,12 +99,13 @@ inline uint64_t partial_bytes(uint64_t parts, int B) {
     return parts * (uint64_t)(kErrRecWords > B + 1 ? kErrRecWords : B + 1) * 8;
 }
 
-// interpret.cu
+// interpret.cu: with d_bounds (level bounds, nlevels values) the max-error
+// tables are formed in the kernel and d_errs is not read
 template <class T>
 int launch_interpret(int nfields, int kind, int est_kind, const int* d_ndims, const int* d_levels, double s, int B,
                      const uint32_t* d_sizes, uint64_t sz_stride, const double* d_errs, uint64_t err_stride,
                      const double* d_tols, double tol0, uint8_t* d_index, uint64_t idx_stride, uint32_t* d_rsz,
-                     cudaStream_t st, bool pdl = false, bool early = false);
+                     cudaStream_t st, bool pdl = false, bool early = false, const T* d_bounds = nullptr);
 
 // one segment per (field, level) of the multi-level fp32 negabinary encode /
 // decode launches; chunk_begin is the segment's first global chunk
@@ -158,12 +180,32 @@ int launch_decode_recompose_nb32_tma_multi(const FusedSeg* segs, int nseg, uint6
 // planes 0..B-1, sign row B, unseen row B+1), each row `stride` words
 uint64_t pb_groups(uint64_t n);
 uint64_t pb_row_words(uint64_t n);
+// one segment per level of a launch
 template <class T>
-int launch_pb_encode(const T* x, uint64_t n, const void* maxkey, int exp, int B, uint32_t* rows, uint64_t stride,
-                     uint32_t* counts, uint32_t* sizes, cudaStream_t st);
+struct PbSeg {
+    const T* x;                           // encode input
+    T* y;                                 // decode output
+    const typename KeyOf<T>::type* key;   // level |max| key, or NULL and the exponent exp
+    uint32_t* rows;
+    uint64_t stride;
+    uint32_t* counts;                     // encode: first-one counts, 64 words
+    uint32_t* sizes;                      // encode: stream bytes, B
+    const uint8_t* dnum;                  // decode: planes (overrides e), or NULL
+    const uint32_t* srow;                 // decode: sign row
+    const uint32_t* unseen;               // decode: elements without a 1 bit so far, or NULL (s == 0)
+    uint64_t n;
+    uint32_t chunk0;                      // set by the launchers
+    int exp;
+};
 template <class T>
-int launch_pb_decode(const uint32_t* rows, uint64_t stride, uint64_t n, const void* maxkey, int exp, int B, int s, int e,
-                     const uint8_t* dnum, const uint32_t* srow, const uint32_t* unseen, T* out, cudaStream_t st);
+struct PbSet {
+    int n;
+    PbSeg<T> seg[17];
+};
+template <class T>
+int launch_pb_encode(PbSet<T> set, int B, cudaStream_t st);
+template <class T>
+int launch_pb_decode(PbSet<T> set, int B, int s, int e, cudaStream_t st);
 size_t pb_pack_scratch_bytes(uint64_t n, int B);
 int launch_pb_pack(const uint32_t* rows, uint64_t stride, uint64_t n, int B, const uint32_t* sizes, uint64_t total,
                    uint8_t* dst, void* scratch, cudaStream_t st);
@@ -244,9 +286,6 @@ int launch_gr_pack(const void* const* planes, const uint32_t* sizes, int B, uint
                    int word_bytes, uint8_t* dst, cudaStream_t st);
 int launch_unpack_planes(const uint8_t* src, const uint64_t* src_off, const uint64_t* nwords, int nplanes,
                          int word_bytes, void* const* dst, uint64_t max_words, cudaStream_t st);
-int launch_chunk_words_from_rb(const uint8_t* rbs, uint64_t nblocks, int B, uint32_t* chunk_words, cudaStream_t st);
-int launch_gr_scan_only(const uint32_t* chunk_words, uint64_t nchunks, int B, uint64_t nblocks, int word_bytes,
-                        uint32_t* chunk_off, uint32_t* sizes, cudaStream_t st);
 template <class T>
 int launch_maxabs(const T* x, uint64_t n, void* maxkey, cudaStream_t st);
 template <class T>

@@ -174,6 +174,8 @@ __global__ void __launch_bounds__(256) k_decompose_rows(const T* __restrict__ in
                                                         T* __restrict__ fnat, typename KeyOf<T>::type* maxkey_level,
                                                         typename KeyOf<T>::type* maxkey_coarse) {
     using K = typename KeyOf<T>::type;
+    pdl_wait();   // the level's input comes from the previous launch
+    pdl_release();
     K mk = 0, mc = 0;
     const uint32_t rows = F.n[0] * F.n[1];
     const uint32_t lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
@@ -198,6 +200,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_decompose_patch
                                                          typename KeyOf<T>::type* maxkey_level,
                                                          typename KeyOf<T>::type* maxkey_coarse) {
     using K = typename KeyOf<T>::type;
+    pdl_wait();   // the level's input comes from the previous launch
+    pdl_release();
     K mk = 0, mc = 0;
     const uint64_t items = patch_items(F, C);
     const uint32_t lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
@@ -556,15 +560,16 @@ int launch_decompose_level_packed(const T* in, uint64_t s0, uint64_t s1, const B
                                   T* fnat, void* maxkey_level, void* maxkey_coarse, cudaStream_t st) {
     using K = typename KeyOf<T>::type;
     const unsigned th = row_threads(F.n[2]);
+    count_launch();
     if (!fnat && patch_level(F, C) && decompose_patch_enabled()) {
-        k_decompose_patch<T><<<row_grid(patch_items(F, C), th), th, 0, st>>>(in, s0, s1, F, C, coef, coarse,
-                                                                          (K*)maxkey_level, (K*)maxkey_coarse);
-        PRODM_CHECK_LAUNCH("k_decompose_patch");
+        const cudaError_t e = launch_chain(true, k_decompose_patch<T>, dim3(row_grid(patch_items(F, C), th)), dim3(th), 0,
+                                           st, in, s0, s1, F, C, coef, coarse, (K*)maxkey_level, (K*)maxkey_coarse);
+        if (e != cudaSuccess) return cuda_status(e, "k_decompose_patch");
         return PRODM_OK;
     }
-    k_decompose_rows<T><<<row_grid((uint64_t)F.n[0] * F.n[1], th), th, 0, st>>>(in, s0, s1, F, C, coef, coarse, fnat,
-                                                                                 (K*)maxkey_level, (K*)maxkey_coarse);
-    PRODM_CHECK_LAUNCH("k_decompose_rows");
+    const cudaError_t e = launch_chain(true, k_decompose_rows<T>, dim3(row_grid((uint64_t)F.n[0] * F.n[1], th)), dim3(th),
+                                       0, st, in, s0, s1, F, C, coef, coarse, fnat, (K*)maxkey_level, (K*)maxkey_coarse);
+    if (e != cudaSuccess) return cuda_status(e, "k_decompose_rows");
     return PRODM_OK;
 }
 

@@ -85,6 +85,8 @@ __global__ void k_maxabs(const T* __restrict__ x, uint64_t n, typename KeyOf<T>:
 // level error bound = max (x4 for negabinary, ComposedRefactor.hpp:111-112)
 template <class T>
 __global__ void k_bounds(const typename KeyOf<T>::type* __restrict__ keys, int nl, int negabinary, T* __restrict__ bounds) {
+    pdl_wait();
+    pdl_release();
     int l = blockIdx.x * blockDim.x + threadIdx.x;
     if (l < nl) {
         T m = key_to_val(keys[l], T());
@@ -127,8 +129,10 @@ int launch_maxabs(const T* x, uint64_t n, void* maxkey, cudaStream_t st) {
 
 template <class T>
 int launch_bounds_from_keys(const void* keys, int nl, int negabinary, T* bounds, cudaStream_t st) {
-    k_bounds<T><<<1, 32, 0, st>>>((const typename KeyOf<T>::type*)keys, nl, negabinary, bounds);
-    PRODM_CHECK_LAUNCH("k_bounds");
+    count_launch();
+    const cudaError_t e = launch_chain(true, k_bounds<T>, dim3(1), dim3(32), 0, st,
+                                       (const typename KeyOf<T>::type*)keys, nl, negabinary, bounds);
+    if (e != cudaSuccess) return cuda_status(e, "k_bounds");
     return PRODM_OK;
 }
 

@@ -67,29 +67,55 @@ __device__ __forceinline__ bool pb_value_fast(float*, int s) { return pow2_norma
 
 __device__ __forceinline__ uint32_t valid_mask(int nvalid) { return nvalid >= 32 ? FULL : ((1u << nvalid) - 1u); }
 
+// The encoder and the decoder take the chunks of all levels of a field in one
+// launch (PbSet, one segment per level), so that the small levels' few chunks
+// run beside the large one's instead of one launch after the other
+// (513 x 257 x 257 fp64, 60 planes: encode 331 us in 14 launches, 203 us in 2;
+// decode 184 us per retrieval in 7, 125 us in one).
+template <class T>
+__device__ __forceinline__ int pb_seg(const PbSet<T>& set, uint32_t c) {
+    int l = 0;
+    while (l + 1 < set.n && c >= set.seg[l + 1].chunk0) l++;
+    return l;
+}
+
 // ---------------------------------------------------------------------------
 // encode: values -> rows 0..B (magnitude planes + signs) and, per plane, the
 // number of elements whose first 1 bit is in that plane
 // ---------------------------------------------------------------------------
 template <class T>
-__global__ void __launch_bounds__(256) k_pb_encode(const T* __restrict__ x, uint64_t n,
-                                                   const typename KeyOf<T>::type* __restrict__ maxkey, int exp_arg,
-                                                   int B, uint32_t* __restrict__ rows, uint64_t stride,
-                                                   uint32_t* __restrict__ counts) {
+__global__ void __launch_bounds__(256) k_pb_encode(const __grid_constant__ PbSet<T> set, uint32_t total, int B) {
     using FP = typename Traits<T>::FP;
     extern __shared__ uint32_t tile[];   // (B + 1) rows x PB_LD
     __shared__ uint32_t cnt[64];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int exp = pb_exp<T>(maxkey, exp_arg);
-    const int ks = B - exp;
-    const bool fast = pow2_normal(ks);
-    const float sc = fast ? pow2f(ks) : 1.f;
-    const uint64_t ng = (n + 31) / 32;
-    const uint64_t nch = (ng + PB_CHUNK - 1) / PB_CHUNK;
+    pdl_wait();
+    pdl_release();
     for (int k = threadIdx.x; k < 64; k += blockDim.x) cnt[k] = 0;
-    __syncthreads();
-    for (uint64_t c = blockIdx.x; c < nch; c += gridDim.x) {
-        const uint64_t g0 = c * PB_CHUNK;
+    int cur = -1;
+    auto flush = [&]() {   // the level's counts; every thread calls it
+        __syncthreads();
+        if (cur >= 0)
+            for (int p = threadIdx.x; p < B; p += blockDim.x)
+                if (cnt[p]) {
+                    atomicAdd(&set.seg[cur].counts[p], cnt[p]);
+                    cnt[p] = 0;
+                }
+        __syncthreads();
+    };
+    for (uint32_t c = blockIdx.x; c < total; c += gridDim.x) {
+        const int l = pb_seg(set, c);
+        if (l != cur) {
+            flush();
+            cur = l;
+        }
+        const PbSeg<T>& q = set.seg[l];
+        const T* __restrict__ x = q.x;
+        const uint64_t n = q.n, ng = (n + 31) / 32, g0 = (uint64_t)(c - q.chunk0) * PB_CHUNK;
+        const int exp = pb_exp<T>(q.key, q.exp);
+        const int ks = B - exp;
+        const bool fast = pow2_normal(ks);
+        const float sc = fast ? pow2f(ks) : 1.f;
 #pragma unroll 2
         for (int j = 0; j < PB_GPW; j++) {
             const int gl = warp * PB_GPW + j;
@@ -112,21 +138,23 @@ __global__ void __launch_bounds__(256) k_pb_encode(const T* __restrict__ x, uint
         __syncthreads();
         const int nvalid = (int)((ng - g0) < (uint64_t)PB_CHUNK ? (ng - g0) : PB_CHUNK);
         for (int p = warp; p <= B; p += PB_WARPS) {
-            uint32_t* dst = rows + (uint64_t)p * stride + g0;
+            uint32_t* dst = q.rows + (uint64_t)p * q.stride + g0;
             const uint32_t* src = tile + p * PB_LD;
             for (int j = lane; j < nvalid; j += 32) dst[j] = src[j];
         }
         __syncthreads();
     }
-    __syncthreads();
-    for (int p = threadIdx.x; p < B; p += blockDim.x)
-        if (cnt[p]) atomicAdd(&counts[p], cnt[p]);
+    flush();
 }
 
-// reference stream sizes: BitEncoder words (n + first-one count bits) * 8
-__global__ void k_pb_sizes(const uint32_t* __restrict__ counts, int B, uint64_t n, uint32_t* __restrict__ sizes) {
+// reference stream sizes: BitEncoder words (n + first-one count bits) * 8, one CTA per level
+template <class T>
+__global__ void k_pb_sizes(const __grid_constant__ PbSet<T> set, int B) {
+    pdl_wait();
+    pdl_release();
+    const PbSeg<T>& q = set.seg[blockIdx.x];
     const int p = threadIdx.x;
-    if (p < B) sizes[p] = (uint32_t)((n + counts[p] + 63) / 64 * 8);
+    if (p < B) q.sizes[p] = (uint32_t)((q.n + q.counts[p] + 63) / 64 * 8);
 }
 
 // ---------------------------------------------------------------------------
@@ -162,34 +190,44 @@ __device__ __forceinline__ void pb_decode_groups(const uint32_t* tile, int num, 
 }
 
 template <class T>
-__global__ void __launch_bounds__(256) k_pb_decode(const uint32_t* __restrict__ rows, uint64_t stride, uint64_t n,
-                                                   const typename KeyOf<T>::type* __restrict__ maxkey, int exp_arg,
-                                                   int s, int e, const uint8_t* __restrict__ dnum,
-                                                   const uint32_t* __restrict__ srow,
-                                                   const uint32_t* __restrict__ unseen, T* __restrict__ out) {
+__global__ void __launch_bounds__(256) k_pb_decode(const __grid_constant__ PbSet<T> set, uint32_t total, int s, int e_arg) {
     extern __shared__ uint32_t tile[];   // num + 2 rows x PB_LD
-    if (dnum) e = dnum[0];
-    const int num = e - s;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int exp = pb_exp<T>(maxkey, exp_arg);
-    const int vs = exp - e;
-    const bool fast = pb_value_fast((T*)nullptr, vs);
-    const float sc = (sizeof(T) == 4 && fast) ? pow2f(vs) : 1.f;
-    const uint64_t ng = (n + 31) / 32;
-    const uint64_t nch = (ng + PB_CHUNK - 1) / PB_CHUNK;
-    const int extra = unseen ? 2 : 1;
-    for (uint64_t c = blockIdx.x; c < nch; c += gridDim.x) {
-        const uint64_t g0 = c * PB_CHUNK;
+    pdl_wait();
+    pdl_release();
+    for (uint32_t c = blockIdx.x; c < total; c += gridDim.x) {
+        const PbSeg<T>& q = set.seg[pb_seg(set, c)];
+        const int e = q.dnum ? q.dnum[0] : e_arg, num = e - s;
+        const int vs = pb_exp<T>(q.key, q.exp) - e;
+        const bool fast = pb_value_fast((T*)nullptr, vs);
+        const float sc = (sizeof(T) == 4 && fast) ? pow2f(vs) : 1.f;
+        const uint64_t n = q.n, ng = (n + 31) / 32, g0 = (uint64_t)(c - q.chunk0) * PB_CHUNK;
         const int nvalid = (int)((ng - g0) < (uint64_t)PB_CHUNK ? (ng - g0) : PB_CHUNK);
-        for (int r = warp; r < num + extra; r += PB_WARPS) {
-            const uint32_t* src = r < num ? rows + (uint64_t)(s + r) * stride + g0
-                                          : (r == num ? srow + g0 : unseen + g0);
-            uint32_t* dst = tile + r * PB_LD;
-            for (int j = lane; j < nvalid; j += 32) dst[j] = __ldcs(src + j);
+        const int nr = num + (q.unseen ? 2 : 1);
+        // a row's 128 words are one 16-byte load per lane (rows are padded to 16 bytes)
+        constexpr int U = 4;
+        for (int r0 = warp; r0 < nr; r0 += U * PB_WARPS) {
+            uint4 w[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int r = r0 + u * PB_WARPS;
+                const uint32_t* src = (r < num ? q.rows + (uint64_t)(s + r) * q.stride : (r == num ? q.srow : q.unseen)) + g0;
+                w[u] = r < nr && 4 * lane < nvalid ? __ldcs(reinterpret_cast<const uint4*>(src) + lane) : make_uint4(0, 0, 0, 0);
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int r = r0 + u * PB_WARPS;
+                if (r >= nr) break;
+                uint32_t* dst = tile + r * PB_LD + 4 * lane;
+                dst[0] = w[u].x;
+                dst[1] = w[u].y;
+                dst[2] = w[u].z;
+                dst[3] = w[u].w;
+            }
         }
         __syncthreads();
-        if (fast) pb_decode_groups<T, true>(tile, num, nvalid, g0, n, vs, sc, unseen != nullptr, out);
-        else pb_decode_groups<T, false>(tile, num, nvalid, g0, n, vs, sc, unseen != nullptr, out);
+        if (fast) pb_decode_groups<T, true>(tile, num, nvalid, g0, n, vs, sc, q.unseen != nullptr, q.y);
+        else pb_decode_groups<T, false>(tile, num, nvalid, g0, n, vs, sc, q.unseen != nullptr, q.y);
         __syncthreads();
     }
 }
@@ -757,30 +795,49 @@ uint64_t pb_groups(uint64_t n) { return (n + 31) / 32; }
 uint64_t pb_row_words(uint64_t n) { return (pb_groups(n) + 3) / 4 * 4; }
 
 template <class T>
-int launch_pb_encode(const T* x, uint64_t n, const void* maxkey, int exp, int B, uint32_t* rows, uint64_t stride,
-                     uint32_t* counts, uint32_t* sizes, cudaStream_t st) {
-    if (B < 1 || B > (sizeof(T) == 8 ? 63 : 32)) return fail(PRODM_EINVAL, "perbit: num_bitplanes out of range");
-    PRODM_CUDA(cudaMemsetAsync(counts, 0, B * sizeof(uint32_t), st));
-    const uint64_t nch = (pb_groups(n) + PB_CHUNK - 1) / PB_CHUNK;
-    const size_t smem = (size_t)(B + 1) * PB_LD * 4;
-    const unsigned grid = persistent_grid_for((const void*)k_pb_encode<T>, 256, smem, nch, 1u << 20);
-    k_pb_encode<T><<<grid, 256, smem, st>>>(x, n, (const typename KeyOf<T>::type*)maxkey, exp, B, rows, stride, counts);
-    PRODM_CHECK_LAUNCH("k_pb_encode");
-    k_pb_sizes<<<1, 64, 0, st>>>(counts, B, n, sizes);
-    PRODM_CHECK_LAUNCH("k_pb_sizes");
-    return PRODM_OK;
+static uint32_t pb_number(PbSet<T>& set) {
+    uint64_t c = 0;
+    for (int l = 0; l < set.n; l++) {
+        set.seg[l].chunk0 = (uint32_t)c;
+        c += (pb_groups(set.seg[l].n) + PB_CHUNK - 1) / PB_CHUNK;
+    }
+    return (uint32_t)c;
 }
 
 template <class T>
-int launch_pb_decode(const uint32_t* rows, uint64_t stride, uint64_t n, const void* maxkey, int exp, int B, int s, int e,
-                     const uint8_t* dnum, const uint32_t* srow, const uint32_t* unseen, T* out, cudaStream_t st) {
-    const int maxnum = dnum ? B : e - s;
-    const size_t smem = (size_t)(maxnum + 2) * PB_LD * 4;
-    const uint64_t nch = (pb_groups(n) + PB_CHUNK - 1) / PB_CHUNK;
-    const unsigned grid = persistent_grid_for((const void*)k_pb_decode<T>, 256, smem, nch, 1u << 20);
-    k_pb_decode<T><<<grid, 256, smem, st>>>(rows, stride, n, (const typename KeyOf<T>::type*)maxkey, exp, s, e, dnum,
-                                            srow, unseen, out);
-    PRODM_CHECK_LAUNCH("k_pb_decode");
+int launch_pb_encode(PbSet<T> set, int B, cudaStream_t st) {
+    if (B < 1 || B > (sizeof(T) == 8 ? 63 : 32)) return fail(PRODM_EINVAL, "perbit: num_bitplanes out of range");
+    for (int l = 0; l < set.n;) {   // counts of consecutive levels in one clear
+        int m = l + 1;
+        while (m < set.n && set.seg[m].counts + 64 == set.seg[m - 1].counts) m++;
+        PRODM_CUDA(cudaMemsetAsync(set.seg[m - 1].counts, 0, (size_t)(m - l) * 64 * sizeof(uint32_t), st));
+        l = m;
+    }
+    const uint32_t total = pb_number(set);
+    if (!total) return PRODM_OK;
+    const size_t smem = (size_t)(B + 1) * PB_LD * 4;
+    const unsigned grid = persistent_grid_for((const void*)k_pb_encode<T>, 256, smem, total, 1u << 20);
+    count_launch();
+    cudaError_t e = launch_chain(true, k_pb_encode<T>, dim3(grid), dim3(256), smem, st, set, total, B);
+    if (e != cudaSuccess) return cuda_status(e, "k_pb_encode");
+    count_launch();
+    e = launch_chain(true, k_pb_sizes<T>, dim3(set.n), dim3(64), 0, st, set, B);
+    if (e != cudaSuccess) return cuda_status(e, "k_pb_sizes");
+    return PRODM_OK;
+}
+
+// B: most planes a level may have (shared memory)
+template <class T>
+int launch_pb_decode(PbSet<T> set, int B, int s, int e, cudaStream_t st) {
+    const uint32_t total = pb_number(set);
+    if (!total) return PRODM_OK;
+    bool counts = false;
+    for (int l = 0; l < set.n; l++) counts |= set.seg[l].dnum != nullptr;
+    const size_t smem = (size_t)((counts ? B : e - s) + 2) * PB_LD * 4;
+    const unsigned grid = persistent_grid_for((const void*)k_pb_decode<T>, 256, smem, total, 1u << 20);
+    count_launch();
+    const cudaError_t err = launch_chain(true, k_pb_decode<T>, dim3(grid), dim3(256), smem, st, set, total, s, e);
+    if (err != cudaSuccess) return cuda_status(err, "k_pb_decode");
     return PRODM_OK;
 }
 
@@ -870,13 +927,9 @@ int launch_pb_parse(const std::vector<PbParseJob>& jobs, cudaStream_t st) {
     return PRODM_OK;
 }
 
-template int launch_pb_encode<float>(const float*, uint64_t, const void*, int, int, uint32_t*, uint64_t, uint32_t*,
-                                     uint32_t*, cudaStream_t);
-template int launch_pb_encode<double>(const double*, uint64_t, const void*, int, int, uint32_t*, uint64_t, uint32_t*,
-                                      uint32_t*, cudaStream_t);
-template int launch_pb_decode<float>(const uint32_t*, uint64_t, uint64_t, const void*, int, int, int, int,
-                                     const uint8_t*, const uint32_t*, const uint32_t*, float*, cudaStream_t);
-template int launch_pb_decode<double>(const uint32_t*, uint64_t, uint64_t, const void*, int, int, int, int,
-                                      const uint8_t*, const uint32_t*, const uint32_t*, double*, cudaStream_t);
+template int launch_pb_encode<float>(PbSet<float>, int, cudaStream_t);
+template int launch_pb_encode<double>(PbSet<double>, int, cudaStream_t);
+template int launch_pb_decode<float>(PbSet<float>, int, int, int, cudaStream_t);
+template int launch_pb_decode<double>(PbSet<double>, int, int, int, cudaStream_t);
 
 }  // namespace prodm
