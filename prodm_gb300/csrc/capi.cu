@@ -1592,7 +1592,7 @@ int packed_pair_impl(const T* in, int ndims, const uint32_t* dims, int L, T* out
                     return rc;
             }
             if ((rc = launch_recompose_level_packed<T>(cin, in + g.offset[l], F, C, o, (uint64_t)F.n[1] * F.n[2], F.n[2],
-                                                       st)))
+                                                       st, true)))
                 return rc;
         }
         return PRODM_OK;
