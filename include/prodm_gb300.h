@@ -61,6 +61,11 @@ extern "C" {
 
 const char* prodm_last_error_string(void);
 int prodm_version(void);
+/* Calls that need device scratch and are given none (workspace == NULL, the
+ * level-file and lossless calls, decoder handles) take it stream ordered from
+ * a pool of this library, which keeps up to 1 GiB per device between calls;
+ * this gives back what is not in use. */
+int prodm_trim_scratch(void);
 
 /* ---------------------------------------------------------------------------
  * Level geometry
@@ -284,7 +289,7 @@ int prodm_mdr_level_info(prodm_mdr* h, uint32_t* h_sizes, double* h_bounds, doub
  * extension carrying the squared-error tables; *len receives the size. */
 int prodm_mdr_metadata(prodm_mdr* h, uint8_t* h_buf, size_t capacity, size_t* len, void* stream);
 /* reference level-file bytes of one level into dst: dst_is_host 0 device
- * memory, 1 host memory (returns when the bytes are there), 2 pinned host
+ * memory filled in stream order, 1 host memory (returns when the bytes are there), 2 pinned host
  * memory filled asynchronously in stream order (synchronise the stream, or
  * wait on an event recorded after the call, before reading it). */
 int prodm_mdr_export_level(prodm_mdr* h, int level, void* dst, uint64_t capacity, int dst_is_host, uint64_t* len,

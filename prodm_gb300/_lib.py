@@ -40,6 +40,7 @@ _i = C.c_int
 _SIGS = {
     "prodm_last_error_string": (C.c_char_p, []),
     "prodm_version": (_i, []),
+    "prodm_trim_scratch": (_i, []),
     "prodm_max_level": (_i, [_i, _u32p, C.POINTER(_i)]),
     "prodm_level_dims": (_i, [_i, _u32p, _i, _u32p, _u64p]),
     "prodm_decompose_workspace": (_i, [_i, _i, _u32p, C.c_uint32, _i, C.POINTER(C.c_size_t)]),

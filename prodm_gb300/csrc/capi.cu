@@ -39,6 +39,36 @@ int cuda_status(cudaError_t e, const char* where) {
     return e == cudaErrorMemoryAllocation ? PRODM_ENOMEM : PRODM_ECUDA;
 }
 
+namespace {
+std::mutex g_pool_mu;
+std::vector<std::pair<int, cudaMemPool_t>> g_pools;   // per device, made at its first use
+}  // namespace
+cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    cudaMemPool_t pool = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mu);
+        for (const auto& q : g_pools)
+            if (q.first == dev) pool = q.second;
+        if (!pool) {
+            cudaMemPoolProps props = {};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            if ((e = cudaMemPoolCreate(&pool, &props)) != cudaSuccess) return e;
+            uint64_t kept = kScratchKept;
+            if ((e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &kept)) != cudaSuccess) {
+                cudaMemPoolDestroy(pool);
+                return e;
+            }
+            g_pools.push_back({dev, pool});
+        }
+    }
+    return cudaMallocFromPoolAsync(p, bytes, pool, st);
+}
+
 int device_sms() {
     static std::mutex mu;
     static std::vector<std::pair<int, int>> cache;
@@ -113,7 +143,7 @@ int make_geom(int ndims, const uint32_t* dims, int L, LevelGeom& g) {
     return PRODM_OK;
 }
 
-// stream-ordered scratch: caller-provided memory or cudaMallocAsync
+// stream-ordered scratch: caller-provided memory or scratch_alloc
 class Workspace {
   public:
     Workspace(void* base, size_t bytes, cudaStream_t st) : base_((uint8_t*)base), cap_(bytes), st_(st) {}
@@ -128,8 +158,8 @@ class Workspace {
             return PRODM_OK;
         }
         if (need_ == 0) return PRODM_OK;
-        cudaError_t e = cudaMallocAsync((void**)&base_, need_, st_);
-        if (e != cudaSuccess) return cuda_status(e, "cudaMallocAsync(workspace)");
+        cudaError_t e = scratch_alloc((void**)&base_, need_, st_);
+        if (e != cudaSuccess) return cuda_status(e, "workspace");
         owned_ = true;
         cap_ = need_;
         return PRODM_OK;
@@ -251,8 +281,8 @@ int decompose_impl(T* data, int ndims, const uint32_t* dims, int L, const uint32
         os = orth_take(ws, top, sizeof(T));
         std::vector<T> tab = build_tabs<T>(g, toff);
         dtab = (T*)ws.take(tab.size() * sizeof(T));
+        // (a pageable source is staged before the call returns)
         PRODM_CUDA(cudaMemcpyAsync(dtab, tab.data(), tab.size() * sizeof(T), cudaMemcpyHostToDevice, st));
-        PRODM_CUDA(cudaStreamSynchronize(st));   // host table lifetime
     }
     for (int step = 0; step < L; step++) {
         const int l = inverse ? step + 1 : L - step;
@@ -325,7 +355,6 @@ void encode_reserve(Workspace& ws, int enc, int dtype, uint64_t n, int B) {
         ws.reserve(nb);                                   // rb
         ws.reserve(nch * B * 4);                          // chunk words
         ws.reserve(nch * B * 4);                          // chunk offsets
-        ws.reserve(64 * sizeof(void*));                   // plane pointers
     }
 }
 
@@ -370,7 +399,6 @@ int encode_impl(int enc, const T* x, uint64_t n, int exp, int B, uint8_t* blob, 
     uint8_t* rbs = (uint8_t*)ws.take(nb);
     uint32_t* cw = (uint32_t*)ws.take(nch * B * 4);
     uint32_t* co = (uint32_t*)ws.take(nch * B * 4);
-    void** dptrs = (void**)ws.take(64 * sizeof(void*));
     GrSet<T> set{1, {}};
     set.seg[0].x = x;
     set.seg[0].rbs = rbs;
@@ -382,11 +410,7 @@ int encode_impl(int enc, const T* x, uint64_t n, int exp, int B, uint8_t* blob, 
     set.seg[0].cap = 2 * nb;
     set.seg[0].exp = exp;
     if ((rc = launch_gr_encode<T>(set, B, partial, errs, st))) return rc;
-    std::vector<void*> ptrs(B);
-    for (int p = 0; p < B; p++) ptrs[p] = staging + (uint64_t)p * 2 * nb * sizeof(T);
-    PRODM_CUDA(cudaMemcpyAsync(dptrs, ptrs.data(), B * sizeof(void*), cudaMemcpyHostToDevice, st));
-    PRODM_CUDA(cudaStreamSynchronize(st));
-    return launch_gr_pack(dptrs, sizes, B, nb, rbs, (int)sizeof(T), blob, st);
+    return launch_gr_pack(staging, 2 * nb, sizes, B, nb, rbs, (int)sizeof(T), blob, st);
 }
 
 }  // namespace prodm
@@ -403,19 +427,48 @@ struct prodm_decoder {
         bool have = false;
         uint64_t n = 0;
         int B = 0;
+        uint8_t* state = nullptr;     // grouped: rbs, chunk_off, signs; per-bit: pbrows
+        size_t bytes = 0;
+        cudaEvent_t used = nullptr;   // behind the last call's work on the state,
+        bool open = false;            // unless that call left before it was recorded
         uint8_t* rbs = nullptr;
         uint32_t* chunk_off = nullptr;
         void* signs = nullptr;
         uint32_t* pbrows = nullptr;   // per-bit: rows 0..B-1, sign row, unseen row, status word
         int parsed = 0;               // per-bit: planes decoded so far
+        // the state comes from the scratch pool: a decoder per field and pass
+        // is the reference's use, and cudaMalloc and cudaFree wait for the device
+        cudaError_t hold(size_t need, cudaStream_t st) {
+            if (state && bytes >= need && !open) {
+                open = true;
+                return used ? cudaStreamWaitEvent(st, used, 0) : cudaSuccess;
+            }
+            drop();
+            open = true;
+            const cudaError_t e = scratch_alloc((void**)&state, need, st);
+            bytes = e == cudaSuccess ? need : 0;
+            return e;
+        }
+        cudaError_t mark(cudaStream_t st) {
+            cudaError_t e = cudaSuccess;
+            if (!used) e = cudaEventCreateWithFlags(&used, cudaEventDisableTiming);
+            if (e == cudaSuccess) e = cudaEventRecord(used, st);
+            open = open && e != cudaSuccess;
+            return e;
+        }
+        void drop() {   // behind the last use, whatever became of its stream
+            if (!state) return;
+            if (open || !used) cudaDeviceSynchronize();
+            else cudaEventSynchronize(used);
+            cudaFree(state);
+            state = nullptr;
+        }
     };
     std::vector<Level> levels;
     ~prodm_decoder() {
         for (auto& l : levels) {
-            if (l.pbrows) cudaFree(l.pbrows);
-            if (l.rbs) cudaFree(l.rbs);
-            if (l.chunk_off) cudaFree(l.chunk_off);
-            if (l.signs) cudaFree(l.signs);
+            l.drop();
+            if (l.used) cudaEventDestroy(l.used);
         }
     }
 };
@@ -434,8 +487,8 @@ int pb_progressive_decode(prodm_decoder* h, const uint8_t* blob, const uint32_t*
     const uint64_t rw = pb_row_words(n);
     if (!L.have) {
         if (s != 0) return fail(PRODM_EINVAL, "decode: the first call for a level must start at plane 0");
-        if (L.pbrows && (L.n != n || L.B != B)) { cudaFree(L.pbrows); L.pbrows = nullptr; }
-        if (!L.pbrows) PRODM_CUDA(cudaMalloc((void**)&L.pbrows, (uint64_t)(B + 2) * rw * 4 + 16));
+        PRODM_CUDA(L.hold((uint64_t)(B + 2) * rw * 4 + 16, st));
+        L.pbrows = (uint32_t*)L.state;
         int rc = launch_pb_init_unseen(L.pbrows + (uint64_t)(B + 1) * rw, L.pbrows + (uint64_t)B * rw, n, st);
         if (rc) return rc;
         L.have = true;
@@ -458,7 +511,7 @@ int pb_progressive_decode(prodm_decoder* h, const uint8_t* blob, const uint32_t*
     uint8_t* tmp = nullptr;
     const uint8_t* base = blob;
     if ((uintptr_t)blob % 8) {   // streams are read as 64-bit words
-        PRODM_CUDA(cudaMallocAsync((void**)&tmp, total, st));
+        PRODM_CUDA(scratch_alloc((void**)&tmp, total, st));
         PRODM_CUDA(cudaMemcpyAsync(tmp, blob, total, cudaMemcpyDeviceToDevice, st));
         base = tmp;
     }
@@ -493,6 +546,7 @@ int pb_progressive_decode(prodm_decoder* h, const uint8_t* blob, const uint32_t*
     if (!rc) {
         cudaError_t e = cudaMemcpyAsync(&hstat, status, 4, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        if (e == cudaSuccess) e = L.mark(st);
         if (e != cudaSuccess) rc = cuda_status(e, "per-bit decode");
     }
     if (tmp) cudaFreeAsync(tmp, st);
@@ -527,7 +581,7 @@ int progressive_decode_impl(prodm_decoder* h, const uint8_t* blob, const uint32_
             return launch_nb_decode<T>(blob, nb, n, nullptr, exp, s, num, nullptr, out, st);
         // misaligned planes: copy to aligned scratch first
         void* tmp;
-        PRODM_CUDA(cudaMallocAsync(&tmp, (uint64_t)num * nb * sizeof(T), st));
+        PRODM_CUDA(scratch_alloc(&tmp, (uint64_t)num * nb * sizeof(T), st));
         PRODM_CUDA(cudaMemcpyAsync(tmp, blob, (uint64_t)num * nb * sizeof(T), cudaMemcpyDeviceToDevice, st));
         rc = launch_nb_decode<T>(tmp, nb, n, nullptr, exp, s, num, nullptr, out, st);
         cudaFreeAsync(tmp, st);
@@ -544,12 +598,14 @@ int progressive_decode_impl(prodm_decoder* h, const uint8_t* blob, const uint32_
         PRODM_CUDA(cudaMemcpyAsync(&cnt, blob, 4, cudaMemcpyDeviceToHost, st));
         PRODM_CUDA(cudaStreamSynchronize(st));
         if (cnt != nb) return fail(PRODM_ECORRUPT, "decode: block count in stream 0 does not match n");
-        PRODM_CUDA(cudaMalloc(&L.rbs, nb));
-        PRODM_CUDA(cudaMalloc(&L.chunk_off, nch * B * 4));
-        PRODM_CUDA(cudaMalloc(&L.signs, nb * sizeof(T)));
+        const size_t a0 = Workspace::align(nb * sizeof(T)), a1 = Workspace::align(nch * B * 4);
+        PRODM_CUDA(L.hold(a0 + a1 + nb, st));
+        L.signs = L.state;
+        L.chunk_off = (uint32_t*)(L.state + a0);
+        L.rbs = L.state + a0 + a1;
         PRODM_CUDA(cudaMemcpyAsync(L.rbs, blob + 4, nb, cudaMemcpyDeviceToDevice, st));
         uint32_t* cw;
-        PRODM_CUDA(cudaMallocAsync((void**)&cw, nch * B * 4 + 64 * 4, st));
+        PRODM_CUDA(scratch_alloc((void**)&cw, nch * B * 4 + 64 * 4, st));
         GrSet<T> set{1, {}};
         set.seg[0].rbs = L.rbs;
         set.seg[0].cw = cw;
@@ -577,31 +633,22 @@ int progressive_decode_impl(prodm_decoder* h, const uint8_t* blob, const uint32_
         maxw = nw[i] > maxw ? nw[i] : maxw;
         o += hs[i];
     }
-    uint8_t* tmp;
-    // staged planes first, then the (8-byte) offset / count / pointer arrays on a
-    // 256-byte boundary
-    const uint64_t plane_bytes = ((uint64_t)num * (maxw + 1) * sizeof(T) + 255) & ~(uint64_t)255;
-    size_t tbytes = plane_bytes + 2 * num * 8 + B * sizeof(void*) + 256;
-    PRODM_CUDA(cudaMallocAsync((void**)&tmp, tbytes, st));
-    uint8_t* planes = tmp;
-    uint64_t* doff = (uint64_t*)(tmp + plane_bytes);
-    uint64_t* dnw = doff + num;
-    void** dptr = (void**)(dnw + num);
-    std::vector<void*> ptr(B, nullptr), uptr(num);
+    // staged planes first, then the (8-byte) arrays on a 256-byte boundary: the
+    // streams' offsets and word counts, the staged planes, every plane
+    const uint64_t plane_bytes = Workspace::align((uint64_t)num * (maxw + 1) * sizeof(T));
+    std::vector<uint64_t> tab(3 * num + B, 0);
+    Scratch tmp(st);
+    PRODM_CUDA(tmp.alloc(plane_bytes + tab.size() * 8));
+    uint8_t* planes = tmp.get();
+    uint64_t* dtab = (uint64_t*)(planes + plane_bytes);
     for (int i = 0; i < num; i++) {
-        uptr[i] = planes + (uint64_t)i * (maxw + 1) * sizeof(T);
-        ptr[s + i] = uptr[i];
+        tab[i] = off[i];
+        tab[num + i] = nw[i];
+        tab[2 * num + i] = tab[3 * num + s + i] = (uint64_t)(uintptr_t)(planes + (uint64_t)i * (maxw + 1) * sizeof(T));
     }
-    std::vector<uint8_t> hostbuf(2 * num * 8 + B * sizeof(void*));
-    memcpy(hostbuf.data(), off.data(), num * 8);
-    memcpy(hostbuf.data() + num * 8, nw.data(), num * 8);
-    memcpy(hostbuf.data() + 2 * num * 8, ptr.data(), B * sizeof(void*));
-    PRODM_CUDA(cudaMemcpyAsync(doff, hostbuf.data(), hostbuf.size(), cudaMemcpyHostToDevice, st));
-    void** uptr_d;
-    PRODM_CUDA(cudaMallocAsync((void**)&uptr_d, num * sizeof(void*), st));
-    PRODM_CUDA(cudaMemcpyAsync(uptr_d, uptr.data(), num * sizeof(void*), cudaMemcpyHostToDevice, st));
-    PRODM_CUDA(cudaStreamSynchronize(st));
-    if ((rc = launch_unpack_planes(blob, doff, dnw, num, ws_, uptr_d, maxw, st))) return rc;
+    PRODM_CUDA(cudaMemcpyAsync(dtab, tab.data(), tab.size() * 8, cudaMemcpyHostToDevice, st));
+    void** dptr = (void**)(dtab + 3 * num);
+    if ((rc = launch_unpack_planes(blob, dtab, dtab + num, num, ws_, (void* const*)(dtab + 2 * num), maxw, st))) return rc;
     GrSet<T> set{1, {}};
     set.seg[0].y = out;
     set.seg[0].rbs = L.rbs;
@@ -610,10 +657,9 @@ int progressive_decode_impl(prodm_decoder* h, const uint8_t* blob, const uint32_
     set.seg[0].signs = (typename Traits<T>::S*)L.signs;
     set.seg[0].n = n;
     set.seg[0].exp = exp;
-    rc = launch_gr_decode<T>(set, B, s, s + num, st);
-    cudaFreeAsync(uptr_d, st);
-    cudaFreeAsync(tmp, st);
-    return rc;
+    if ((rc = launch_gr_decode<T>(set, B, s, s + num, st))) return rc;
+    PRODM_CUDA(L.mark(st));
+    return PRODM_OK;
 }
 }  // namespace
 }  // namespace prodm
@@ -634,7 +680,10 @@ struct prodm_mdr {
     bool refactored = false;
     uint32_t* rsizes = nullptr;
     std::vector<uint8_t> ll_stop, ll_flags;        // per level; per level and plane
+    std::vector<uint32_t> ll_raw;                  // host copies of rsizes and sizes while the stage is on after a
+    std::vector<uint32_t> ll_kept;                 // refactor (empty otherwise)
     std::vector<uint8_t*> ll_cbuf;                 // loading: stored level bytes as they arrive
+    std::vector<uint64_t> ll_ccap, lcap;           // capacities of ll_cbuf and lfile
     std::vector<uint64_t> ll_cloaded, ll_rawoff;   // stored bytes loaded, raw bytes expanded, per level
     std::vector<int> ll_expanded;                  // planes expanded per level
     std::vector<uint32_t> ll_stored;               // loading: stored sizes from the metadata
@@ -1227,9 +1276,8 @@ int mdr_unpack_loaded(prodm_mdr* h, cudaStream_t st) {
             o += h->hsizes[l * B + p];
         }
         uint64_t* dv;
-        PRODM_CUDA(cudaMallocAsync((void**)&dv, hostv.size() * 8, st));
+        PRODM_CUDA(scratch_alloc((void**)&dv, hostv.size() * 8, st));
         PRODM_CUDA(cudaMemcpyAsync(dv, hostv.data(), hostv.size() * 8, cudaMemcpyHostToDevice, st));
-        PRODM_CUDA(cudaStreamSynchronize(st));
         rc = launch_unpack_planes(h->lfile[l], dv, dv + num, num, wb, (void* const*)(dv + 2 * num), maxw, st);
         cudaFreeAsync(dv, st);
         if (rc) return rc;
@@ -1239,6 +1287,20 @@ int mdr_unpack_loaded(prodm_mdr* h, cudaStream_t st) {
 }
 
 int mdr_load_level(prodm_mdr* h, int l, const void* src, uint64_t off, uint64_t bytes, int host, cudaStream_t st);
+
+// a level's buffer of loaded bytes, kept from one metadata to the next while it is large enough
+int hold_level_buffer(prodm_mdr* h, uint8_t*& p, uint64_t& cap, uint64_t need) {
+    if (p && cap >= need) return PRODM_OK;
+    if (p) {
+        h->allocs.erase(std::find(h->allocs.begin(), h->allocs.end(), (void*)p));
+        cudaFree(p);   // (waits for the device)
+        p = nullptr;
+        cap = 0;
+    }
+    const int rc = h->alloc((void**)&p, need);
+    if (!rc) cap = need;
+    return rc;
+}
 
 // lossless stage: stored level bytes as they arrive
 int mdr_ll_load(prodm_mdr* h, int l, const void* src, uint64_t off, uint64_t bytes, int host, cudaStream_t st) {
@@ -1259,10 +1321,8 @@ int mdr_ll_load(prodm_mdr* h, int l, const void* src, uint64_t off, uint64_t byt
         if (off + bytes > h->ll_cloaded[l]) h->ll_cloaded[l] = off + bytes;
         return PRODM_OK;
     }
-    if (!h->ll_cbuf[l]) {
-        int rc = h->alloc((void**)&h->ll_cbuf[l], total);
-        if (rc) return rc;
-    }
+    int rc = hold_level_buffer(h, h->ll_cbuf[l], h->ll_ccap[l], total);
+    if (rc) return rc;
     PRODM_CUDA(cudaMemcpyAsync(h->ll_cbuf[l] + off, src, bytes, host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice,
                                st));
     if (off + bytes > h->ll_cloaded[l]) h->ll_cloaded[l] = off + bytes;
@@ -1317,38 +1377,49 @@ int mdr_ll_expand_zstd(prodm_mdr* h, cudaStream_t st) {
 int mdr_ll_expand(prodm_mdr* h, cudaStream_t st) {
     const int L = h->g.L, B = h->B;
     if (h->ll_zstd) return mdr_ll_expand_zstd(h, st);
+    // every level's complete planes together: their raw sizes (one wait), then
+    // the bytes into the plane rows (negabinary) or the raw level file
+    std::vector<LlPart> parts;
+    std::vector<std::pair<int, int>> of;   // level, plane of each part
     for (int l = 0; l <= L; l++) {
         if (!h->ll_cbuf[l]) continue;
-        uint64_t off = 0, soff = 0;
-        int complete = 0;
+        uint64_t off = 0;
         for (int p = 0; p < B; p++) {
-            off += h->ll_stored[l * B + p];
-            if (off <= h->ll_cloaded[l]) complete = p + 1;
-            else break;
-        }
-        const int first = h->ll_expanded[l];
-        if (complete <= first) continue;
-        const int num = complete - first;
-        for (int p = 0; p < first; p++) soff += h->ll_stored[l * B + p];
-        const uint64_t cap = encode_bound(h->cfg.encoder, h->cfg.dtype, h->g.elems[l], B);
-        uint8_t* raw;
-        PRODM_CUDA(cudaMallocAsync((void**)&raw, cap + 256, st));
-        std::vector<uint32_t> rsz(num);
-        int rc = ll_decompress_planes(h->ll_cbuf[l] + soff, h->ll_stored.data() + l * B + first,
-                                      h->ll_flags.data() + (size_t)l * B + first, num, raw, cap, rsz.data(), st);
-        uint64_t rbytes = 0;
-        if (!rc) {
-            for (int i = 0; i < num; i++) {
-                h->hsizes[l * B + first + i] = rsz[i];
-                rbytes += rsz[i];
+            const uint32_t n = h->ll_stored[l * B + p];
+            if (off + n > h->ll_cloaded[l]) break;
+            if (p >= h->ll_expanded[l]) {
+                parts.push_back(LlPart{h->ll_cbuf[l] + off, nullptr, 0, n, h->ll_flags[(size_t)l * B + p] != 0});
+                of.push_back({l, p});
             }
-            rc = mdr_load_level(h, l, raw, h->ll_rawoff[l], rbytes, 0, st);
+            off += n;
         }
-        cudaFreeAsync(raw, st);
-        if (rc) return rc;
-        h->ll_rawoff[l] += rbytes;
-        h->ll_expanded[l] = complete;
     }
+    if (parts.empty()) return PRODM_OK;
+    int rc = ll_raw_sizes(parts, st);
+    if (rc) return rc;
+    std::vector<uint64_t> raw(h->ll_rawoff);
+    for (size_t i = 0; i < parts.size(); i++) {
+        const int l = of[i].first, p = of[i].second;
+        if (h->nb) {
+            if (parts[i].raw != h->nblocks[l] * h->es)
+                return fail(PRODM_ECORRUPT, "load: a negabinary plane of another size than its level's");
+            parts[i].dst = h->streams + h->lvl_byte_off[l] + (uint64_t)p * h->plane_cap[l] * h->es;
+        } else {
+            const uint64_t cap = encode_bound(h->cfg.encoder, h->cfg.dtype, h->g.elems[l], B);
+            if (raw[l] + parts[i].raw > cap) return fail(PRODM_ECORRUPT, "load: the level's streams exceed their bound");
+            if ((rc = hold_level_buffer(h, h->lfile[l], h->lcap[l], cap))) return rc;
+            parts[i].dst = h->lfile[l] + raw[l];
+        }
+        raw[l] += parts[i].raw;
+    }
+    if ((rc = ll_expand(parts, st))) return rc;
+    for (size_t i = 0; i < parts.size(); i++) {
+        h->hsizes[of[i].first * B + of[i].second] = (uint32_t)parts[i].raw;
+        h->ll_expanded[of[i].first] = of[i].second + 1;
+    }
+    h->ll_rawoff = raw;
+    for (int l = 0; l <= L; l++)
+        if (raw[l] > h->loaded[l]) h->loaded[l] = raw[l];
     return PRODM_OK;
 }
 
@@ -1470,11 +1541,19 @@ int mdr_load_metadata(prodm_mdr* h, const uint8_t* buf, size_t len, cudaStream_t
         h->ll_cloaded.assign(nl, 0);
         h->ll_rawoff.assign(nl, 0);
         h->ll_expanded.assign(nl, 0);
-        if (h->ll_cbuf.empty()) h->ll_cbuf.assign(nl, nullptr);
+        if (h->ll_cbuf.empty()) {
+            h->ll_cbuf.assign(nl, nullptr);
+            h->ll_ccap.assign(nl, 0);
+        }
     }
     h->ll_zstd = zstd;
     h->ll_hbuf.assign(zstd ? nl : 0, std::vector<uint8_t>());
-    if (h->lfile.empty()) h->lfile.assign(nl, nullptr);
+    h->ll_raw.clear();
+    h->ll_kept.clear();
+    if (h->lfile.empty()) {
+        h->lfile.assign(nl, nullptr);
+        h->lcap.assign(nl, 0);
+    }
     return PRODM_OK;
 }
 
@@ -1491,20 +1570,27 @@ int mdr_load_level(prodm_mdr* h, int l, const void* src, uint64_t off, uint64_t 
     cudaMemcpyKind kind = host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice;
     if (h->nb) {   // level-file bytes [off, off + bytes) -> padded plane rows
         const uint64_t row = h->nblocks[l] * h->es, pitch = h->plane_cap[l] * h->es;
-        uint64_t pos = off, done = 0;
-        while (done < bytes) {
-            const uint64_t p = pos / row, within = pos - p * row;
-            const uint64_t piece = std::min<uint64_t>(row - within, bytes - done);
-            PRODM_CUDA(cudaMemcpyAsync(h->streams + h->lvl_byte_off[l] + p * pitch + within,
-                                       (const uint8_t*)src + done, piece, kind, st));
-            pos += piece;
-            done += piece;
+        // (a tail of one row, whole rows, a head of one row)
+        uint8_t* rows = h->streams + h->lvl_byte_off[l];
+        const uint8_t* from = (const uint8_t*)src;
+        uint64_t a = off;
+        const uint64_t b = off + bytes;
+        if (a % row) {
+            const uint64_t n = std::min(b, (a / row + 1) * row) - a;
+            PRODM_CUDA(cudaMemcpyAsync(rows + (a / row) * pitch + a % row, from, n, kind, st));
+            from += n;
+            a += n;
         }
+        if (b - a >= row) {
+            const uint64_t n = (b - a) / row;
+            PRODM_CUDA(cudaMemcpy2DAsync(rows + (a / row) * pitch, pitch, from, row, row, n, kind, st));
+            from += n * row;
+            a += n * row;
+        }
+        if (a < b) PRODM_CUDA(cudaMemcpyAsync(rows + (a / row) * pitch, from, b - a, kind, st));
     } else {
-        if (!h->lfile[l]) {
-            int rc = h->alloc((void**)&h->lfile[l], total);
-            if (rc) return rc;
-        }
+        int rc = hold_level_buffer(h, h->lfile[l], h->lcap[l], total);
+        if (rc) return rc;
         PRODM_CUDA(cudaMemcpyAsync(h->lfile[l] + off, src, bytes, kind, st));
     }
     if (off + bytes > h->loaded[l]) h->loaded[l] = off + bytes;
@@ -1568,8 +1654,8 @@ int packed_pair_impl(const T* in, int ndims, const uint32_t* dims, int L, T* out
         s_b = (T*)ws.take((uint64_t)F.n[0] * F.n[1] * C.n[2] * sizeof(T));
         s_w = (T*)ws.take(F.size() * sizeof(T));
         s_u = (T*)ws.take(C.size() * sizeof(T));
+        // (a pageable source is staged before the call returns)
         PRODM_CUDA(cudaMemcpyAsync(dtab, tab.data(), tab.size() * sizeof(T), cudaMemcpyHostToDevice, st));
-        PRODM_CUDA(cudaStreamSynchronize(st));   // host table lifetime
     }
     auto tabs_of = [&](int l, const T* (&t)[3]) {
         for (int d = 0; d < 3; d++) t[d] = dtab + toff[l * 3 + d];
@@ -1623,6 +1709,16 @@ extern "C" {
 
 const char* prodm_last_error_string(void) { return prodm::g_err.c_str(); }
 int prodm_version(void) { return 100; }
+
+int prodm_trim_scratch(void) {
+    std::vector<std::pair<int, cudaMemPool_t>> pools;
+    {
+        std::lock_guard<std::mutex> lock(prodm::g_pool_mu);
+        pools = prodm::g_pools;
+    }
+    for (const auto& q : pools) PRODM_CUDA(cudaMemPoolTrimTo(q.second, 0));
+    return PRODM_OK;
+}
 
 int prodm_max_level(int ndims, const uint32_t* dims, int* out) {
     if (!dims || !out || ndims < 1 || ndims > 3) return fail(PRODM_EINVAL, "prodm_max_level: bad arguments");
@@ -1862,7 +1958,7 @@ int prodm_interpret(int interp, int est, int dtype, int ndims, int L, double s, 
     if (!d_sizes || !d_errs || !d_index || !d_rsz) return fail(PRODM_EINVAL, "prodm_interpret: NULL pointer");
     cudaStream_t st = (cudaStream_t)stream;
     int* p;
-    PRODM_CUDA(cudaMallocAsync((void**)&p, 8, st));
+    PRODM_CUDA(scratch_alloc((void**)&p, 8, st));
     int hv[2] = {ndims, L};
     PRODM_CUDA(cudaMemcpyAsync(p, hv, 8, cudaMemcpyHostToDevice, st));
     if (dtype == PRODM_F64)
@@ -1918,6 +2014,8 @@ int prodm_mdr_refactor(prodm_mdr* h, const void* field, void* stream) {
     if (h->from_files) h->ll_latter = -1;   // a loaded stage does not carry over to a new refactor
     h->from_files = false;
     h->hsz_valid = false;
+    h->ll_raw.clear();
+    h->ll_kept.clear();
     const int rc = h->cfg.dtype == PRODM_F64 ? mdr_refactor<double>(h, (const double*)field, st)
                                              : mdr_refactor<float>(h, (const float*)field, st);
     if (rc) return rc;
@@ -1989,7 +2087,7 @@ int prodm_mdr_metadata(prodm_mdr* h, uint8_t* buf, size_t cap, size_t* len, void
 static int export_raw_level(prodm_mdr* h, int level, void* dst, uint64_t cap, int dst_is_host, uint64_t* len,
                             const uint32_t* dsizes, cudaStream_t st, const uint32_t* hsizes = nullptr) {
     const int B = h->B;
-    const bool async = dst_is_host == 2;
+    const bool wait = dst_is_host == 1;   // device and pinned memory are filled in stream order
     std::vector<uint32_t> sz(B);
     if (hsizes) {
         std::memcpy(sz.data(), hsizes, B * 4);
@@ -2007,7 +2105,7 @@ static int export_raw_level(prodm_mdr* h, int level, void* dst, uint64_t cap, in
         const size_t row = (size_t)h->nblocks[level] * h->es;
         PRODM_CUDA(cudaMemcpy2DAsync(dst, row, src, (size_t)h->plane_cap[level] * h->es, row, B,
                                      dst_is_host ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice, st));
-        if (!async) PRODM_CUDA(cudaStreamSynchronize(st));
+        if (wait) PRODM_CUDA(cudaStreamSynchronize(st));
         return PRODM_OK;
     }
     if (h->pb) {   // rows -> reference streams (8-byte aligned staging where dst is not)
@@ -2015,7 +2113,7 @@ static int export_raw_level(prodm_mdr* h, int level, void* dst, uint64_t cap, in
         const uint64_t n = h->g.elems[level];
         const size_t scr = pb_pack_scratch_bytes(n, B);
         uint8_t* tmp;
-        PRODM_CUDA(cudaMallocAsync((void**)&tmp, scr + (direct ? 0 : (total + 255) / 256 * 256), st));
+        PRODM_CUDA(scratch_alloc((void**)&tmp, scr + (direct ? 0 : (total + 255) / 256 * 256), st));
         uint8_t* out = direct ? (uint8_t*)dst : tmp + scr;
         const uint32_t* rows = (const uint32_t*)src;
         int rc = launch_pb_pack(rows, h->plane_cap[level], n, B, dsizes, total,
@@ -2027,29 +2125,78 @@ static int export_raw_level(prodm_mdr* h, int level, void* dst, uint64_t cap, in
         }
         cudaFreeAsync(tmp, st);
         if (rc) return rc;
-        if (!async) PRODM_CUDA(cudaStreamSynchronize(st));
+        if (wait) PRODM_CUDA(cudaStreamSynchronize(st));
         return PRODM_OK;
     }
     uint8_t* tmp = (uint8_t*)dst;
-    if (dst_is_host) PRODM_CUDA(cudaMallocAsync((void**)&tmp, total, st));
-    int rc = launch_gr_pack((const void* const*)(h->plane_ptrs + (uint64_t)level * B), dsizes, B,
-                            h->nblocks[level], h->rbs + h->rb_off[level], (int)h->es, tmp, st);
+    if (dst_is_host) PRODM_CUDA(scratch_alloc((void**)&tmp, total, st));
+    int rc = launch_gr_pack(src, h->plane_cap[level], dsizes, B, h->nblocks[level], h->rbs + h->rb_off[level],
+                            (int)h->es, tmp, st);
     if (rc) return rc;
     if (dst_is_host) {
         PRODM_CUDA(cudaMemcpyAsync(dst, tmp, total, cudaMemcpyDeviceToHost, st));
         cudaFreeAsync(tmp, st);
     }
-    if (!async) PRODM_CUDA(cudaStreamSynchronize(st));
+    if (wait) PRODM_CUDA(cudaStreamSynchronize(st));
     return PRODM_OK;
 }
 
-// lossless stage on: the encoders' (raw) sizes -> rsizes; per level the raw
-// level file is built in scratch, each stream's ZCB size counted and the
-// adaptive rule applied; the stored sizes -> sizes (the interpreter's cost
-// model, as the reference's metadata carries them)
+// The raw streams of levels [from, to] on the device (h_raw: raw plane sizes,
+// nl * B): negabinary planes and grouped planes 1.. lie in the handle's rows;
+// grouped stream 0 (its header in front) and the per-bit streams are built in
+// `mem`
+static int raw_streams(prodm_mdr* h, int from, int to, const uint32_t* h_raw, Scratch& mem, std::vector<LlPart>& parts,
+                       cudaStream_t st) {
+    const int B = h->B;
+    uint64_t need = 0;
+    auto align = [](uint64_t x) { return (x + 255) / 256 * 256; };
+    for (int l = from; l <= to; l++) {
+        uint64_t t = 0;
+        for (int p = 0; p < B; p++) t += h_raw[l * B + p];
+        if (h->pb) need += align(t) + pb_pack_scratch_bytes(h->g.elems[l], B);
+        else if (!h->nb) need += align(h_raw[l * B]);
+    }
+    if (need) PRODM_CUDA(mem.alloc(need));
+    uint8_t* at = mem.get();
+    for (int l = from; l <= to; l++) {
+        const uint8_t* rows = h->streams + h->lvl_byte_off[l];
+        const uint32_t* dsizes = h->rsizes + (uint64_t)l * B;
+        const uint64_t cap = h->plane_cap[l] * h->es;
+        int rc = PRODM_OK;
+        if (h->pb) {
+            uint64_t total = 0;
+            for (int p = 0; p < B; p++) total += h_raw[l * B + p];
+            rc = launch_pb_pack((const uint32_t*)rows, h->plane_cap[l], h->g.elems[l], B, dsizes, total, at,
+                                at + align(total), st);
+            uint64_t o = 0;
+            for (int p = 0; p < B; p++) {
+                parts.push_back(LlPart{at + o, nullptr, h_raw[l * B + p], 0, true});
+                o += h_raw[l * B + p];
+            }
+            at += align(total) + pb_pack_scratch_bytes(h->g.elems[l], B);
+        } else {
+            if (!h->nb) {
+                rc = launch_gr_pack(rows, h->plane_cap[l], dsizes, 1, h->nblocks[l], h->rbs + h->rb_off[l], (int)h->es, at,
+                                    st);
+                parts.push_back(LlPart{at, nullptr, h_raw[l * B], 0, true});
+                at += align(h_raw[l * B]);
+            }
+            for (int p = h->nb ? 0 : 1; p < B; p++)
+                parts.push_back(LlPart{rows + p * cap, nullptr, h_raw[l * B + p], 0, true});
+        }
+        if (rc) return rc;
+    }
+    return PRODM_OK;
+}
+
+// lossless stage on: the encoders' (raw) sizes -> rsizes; each stream's ZCB
+// size counted and the adaptive rule applied; the stored sizes -> sizes (the
+// interpreter's cost model, as the reference's metadata carries them)
 static int mdr_lossless_sizes(prodm_mdr* h, cudaStream_t st) {
     const int nl = h->g.L + 1, B = h->B;
-    std::vector<uint32_t> raw(nl * B), stored(nl * B);
+    std::vector<uint32_t> raw(nl * B), stored(nl * B), comp(nl * B);
+    h->ll_raw.clear();
+    h->ll_kept.clear();
     if (h->nb) {   // fixed raw sizes (the refactor does not rewrite them)
         for (int l = 0; l < nl; l++)
             for (int p = 0; p < B; p++) raw[l * B + p] = (uint32_t)(h->nblocks[l] * h->es);
@@ -2057,32 +2204,22 @@ static int mdr_lossless_sizes(prodm_mdr* h, cudaStream_t st) {
     } else {
         PRODM_CUDA(cudaMemcpyAsync(h->rsizes, h->sizes, nl * B * 4, cudaMemcpyDeviceToDevice, st));
         PRODM_CUDA(cudaMemcpyAsync(raw.data(), h->sizes, nl * B * 4, cudaMemcpyDeviceToHost, st));
+        PRODM_CUDA(cudaStreamSynchronize(st));
     }
-    PRODM_CUDA(cudaStreamSynchronize(st));
     h->ll_stop.assign(nl, 0);
     h->ll_flags.assign((size_t)nl * B, 0);
-    uint64_t maxraw = 0;
+    Scratch mem(st);
+    std::vector<LlPart> parts;
+    int rc = raw_streams(h, 0, nl - 1, raw.data(), mem, parts, st);
+    if (rc || (rc = ll_sizes(parts, comp.data(), st))) return rc;
     for (int l = 0; l < nl; l++) {
-        uint64_t t = 0;
-        for (int p = 0; p < B; p++) t += raw[l * B + p];
-        maxraw = t > maxraw ? t : maxraw;
-    }
-    uint8_t* tmp;
-    PRODM_CUDA(cudaMallocAsync((void**)&tmp, maxraw + 256, st));
-    int rc = PRODM_OK;
-    std::vector<uint32_t> comp(B);
-    for (int l = 0; l < nl && !rc; l++) {
-        rc = export_raw_level(h, l, tmp, maxraw, 0, nullptr, h->rsizes + (uint64_t)l * B, st);
-        if (!rc) rc = ll_stream_sizes(tmp, raw.data() + l * B, B, comp.data(), st);
-        if (rc) break;
-        h->ll_stop[l] = (uint8_t)adaptive_stopping(raw.data() + l * B, comp.data(), B, h->ll_latter,
+        h->ll_stop[l] = (uint8_t)adaptive_stopping(raw.data() + l * B, comp.data() + l * B, B, h->ll_latter,
                                                     h->ll_flags.data() + (size_t)l * B);
-        for (int p = 0; p < B; p++) stored[l * B + p] = h->ll_flags[(size_t)l * B + p] ? comp[p] : raw[l * B + p];
+        for (int p = 0; p < B; p++) stored[l * B + p] = h->ll_flags[(size_t)l * B + p] ? comp[l * B + p] : raw[l * B + p];
     }
-    cudaFreeAsync(tmp, st);
-    if (rc) return rc;
     PRODM_CUDA(cudaMemcpyAsync(h->sizes, stored.data(), nl * B * 4, cudaMemcpyHostToDevice, st));
-    PRODM_CUDA(cudaStreamSynchronize(st));
+    h->ll_raw = raw;
+    h->ll_kept = stored;
     return PRODM_OK;
 }
 
@@ -2104,33 +2241,37 @@ int prodm_mdr_export_level(prodm_mdr* h, int level, void* dst, uint64_t cap, int
         return export_raw_level(h, level, dst, cap, dst_is_host, len, h->sizes + (uint64_t)level * B, st,
                                 h->hsz.data() + (size_t)level * B);
     }
-    // lossless stage: the raw level into scratch, then its stored streams
-    std::vector<uint32_t> raw(B), stored(B);
-    PRODM_CUDA(cudaMemcpyAsync(raw.data(), h->rsizes + (uint64_t)level * B, B * 4, cudaMemcpyDeviceToHost, st));
-    PRODM_CUDA(cudaMemcpyAsync(stored.data(), h->sizes + (uint64_t)level * B, B * 4, cudaMemcpyDeviceToHost, st));
-    PRODM_CUDA(cudaStreamSynchronize(st));
-    uint64_t rtotal = 0, total = 0;
-    for (int p = 0; p < B; p++) { rtotal += raw[p]; total += stored[p]; }
+    // lossless stage: the level's stored streams, compressed straight into
+    // their places; device memory and pinned memory in stream order
+    const uint32_t* stored = (h->from_files ? h->ll_stored : h->ll_kept).data() + (size_t)level * B;
+    uint64_t total = 0;
+    for (int p = 0; p < B; p++) total += stored[p];
     if (len) *len = total;
     if (!dst) return PRODM_OK;
     if (cap < total) return fail(PRODM_EINVAL, "export buffer too small");
-    uint8_t* tmp;
-    const uint64_t rpad = (rtotal + 255) / 256 * 256;
-    PRODM_CUDA(cudaMallocAsync((void**)&tmp, rpad + (dst_is_host ? total + 256 : 256), st));
-    int rc = export_raw_level(h, level, tmp, rtotal, 0, nullptr, h->rsizes + (uint64_t)level * B, st);
-    uint8_t* out = dst_is_host ? tmp + rpad : (uint8_t*)dst;
-    std::vector<uint32_t> osz(B);
-    int stop = 0;
-    if (!rc)
-        rc = ll_compress_level(tmp, raw.data(), B, h->ll_latter, out, total, osz.data(), &stop,
-                               h->ll_flags.data() + (size_t)level * B, st);
-    if (!rc && dst_is_host) {
-        cudaError_t e = cudaMemcpyAsync(dst, out, total, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        if (e != cudaSuccess) rc = cuda_status(e, "export copy");
+    if (h->from_files && (h->ll_zstd || h->ll_expanded[level] < B || (!h->nb && (int)h->unpacked[level] < B)))
+        return fail(PRODM_EINVAL, "export_level: the level's planes are not all loaded and expanded");
+    const std::vector<uint32_t>& raw = h->from_files ? h->hsizes : h->ll_raw;
+    if (h->from_files)
+        PRODM_CUDA(cudaMemcpyAsync(h->rsizes, raw.data(), (L + 1) * B * 4, cudaMemcpyHostToDevice, st));
+    Scratch mem(st), host(st);
+    std::vector<LlPart> parts;
+    int rc = raw_streams(h, level, level, raw.data(), mem, parts, st);
+    if (rc) return rc;
+    if (dst_is_host) PRODM_CUDA(host.alloc(total));
+    uint8_t* out = dst_is_host ? host.get() : (uint8_t*)dst;
+    for (int p = 0; p < B; p++) {
+        parts[p].packed = h->ll_flags[(size_t)level * B + p] != 0;
+        parts[p].stored = stored[p];
+        parts[p].dst = out;
+        out += stored[p];
     }
-    cudaFreeAsync(tmp, st);
-    return rc;
+    if ((rc = ll_store(parts, st))) return rc;
+    if (dst_is_host) {
+        PRODM_CUDA(cudaMemcpyAsync(dst, host.get(), total, cudaMemcpyDeviceToHost, st));
+        if (dst_is_host == 1) PRODM_CUDA(cudaStreamSynchronize(st));
+    }
+    return PRODM_OK;
 }
 
 int prodm_mdr_export_level_range(prodm_mdr* h, int level, uint64_t offset, uint64_t bytes, void* dst,
@@ -2167,7 +2308,7 @@ int prodm_mdr_export_level_range(prodm_mdr* h, int level, uint64_t offset, uint6
         if (a < b) PRODM_CUDA(cudaMemcpyAsync(out, src + (a / row) * pitch, b - a, kind, st));
     } else {   // the whole file into device scratch, then the range
         uint8_t* tmp;
-        PRODM_CUDA(cudaMallocAsync((void**)&tmp, total, st));
+        PRODM_CUDA(scratch_alloc((void**)&tmp, total, st));
         uint64_t len = 0;
         rc = prodm_mdr_export_level(h, level, tmp, total, 0, &len, stream);
         if (!rc) {

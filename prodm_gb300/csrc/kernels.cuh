@@ -261,16 +261,18 @@ int launch_zcb_write(const ZStream* d_ss, int ns, uint64_t total_chunks, const u
                      cudaStream_t st);
 int launch_zcb_read(const ZStream* d_ss, int ns, uint64_t total_chunks, int* status, cudaStream_t st);
 int adaptive_stopping(const uint32_t* raw, const uint32_t* comp, int B, int latter, uint8_t* compressed);
-// one level's streams (device, concatenated, raw sizes h_sizes) -> stored
-// streams (compressed where flags say, else raw) concatenated into d_out
-int ll_compress_level(const uint8_t* d_raw, const uint32_t* h_sizes, int B, int latter, uint8_t* d_out,
-                      uint64_t cap, uint32_t* h_out_sizes, int* h_stop, const uint8_t* h_flags, cudaStream_t st);
-// compressed sizes of every stream (the ZCB size; no output written)
-int ll_stream_sizes(const uint8_t* d_raw, const uint32_t* h_sizes, int B, uint32_t* h_comp, cudaStream_t st);
-// stored streams of `num` planes (sizes h_sizes, flags) -> raw streams
-// concatenated into d_out (capacity cap); h_raw_sizes: their raw sizes
-int ll_decompress_planes(const uint8_t* d_in, const uint32_t* h_sizes, const uint8_t* h_flags, int num, uint8_t* d_out,
-                         uint64_t cap, uint32_t* h_raw_sizes, cudaStream_t st);
+// One stream of the stage: raw bytes src and stored bytes dst (store), or
+// stored src and raw dst (expand); packed: the stored bytes are compressed
+struct LlPart {
+    const uint8_t* src;
+    uint8_t* dst;
+    uint64_t raw, stored;
+    bool packed;
+};
+int ll_sizes(const std::vector<LlPart>& parts, uint32_t* h_comp, cudaStream_t st);   // every stream's compressed size
+int ll_store(const std::vector<LlPart>& parts, cudaStream_t st);                     // stream ordered
+int ll_raw_sizes(std::vector<LlPart>& parts, cudaStream_t st);                       // raw sizes of stored streams
+int ll_expand(const std::vector<LlPart>& parts, cudaStream_t st);                    // waits: a malformed chunk is an error
 
 // fileio.cu: byte ranges of a file into the handle's loader (sink(src,
 // offset within the range, bytes, src_is_host)); *mode: 1 cuFile, 0 pinned
@@ -282,7 +284,7 @@ int read_file_range(FileStaging*& fs, const char* path, uint64_t file_off, uint6
                     int* mode);
 
 // pack.cu
-int launch_gr_pack(const void* const* planes, const uint32_t* sizes, int B, uint64_t nblocks, const uint8_t* rbs,
+int launch_gr_pack(const void* planes, uint64_t cap, const uint32_t* sizes, int B, uint64_t nblocks, const uint8_t* rbs,
                    int word_bytes, uint8_t* dst, cudaStream_t st);
 int launch_unpack_planes(const uint8_t* src, const uint64_t* src_off, const uint64_t* nwords, int nplanes,
                          int word_bytes, void* const* dst, uint64_t max_words, cudaStream_t st);

@@ -109,7 +109,13 @@ __global__ void k_zcb_scan(const ZStream* __restrict__ ss, const uint32_t* __res
         if (c < nch) coff[s.chunk0 + c] = run + inc - v;
         run += __shfl_sync(FULL, inc, 31);
     }
-    if (lane == 0) out_size[blockIdx.x] = (uint32_t)(12 + 4 * nch + run);
+    if (lane == 0) {
+        out_size[blockIdx.x] = (uint32_t)(12 + 4 * nch + run);
+        if (nch == 0 && s.dst) {   // an empty stream is its header (the writer works by chunks)
+            uint32_t* out = (uint32_t*)s.dst;
+            out[0] = out[1] = out[2] = 0;
+        }
+    }
 }
 
 // dst of each stream: 4-byte aligned, its compressed size long
@@ -245,6 +251,30 @@ __global__ void __launch_bounds__(32 * ZW) k_zcb_read(const ZStream* __restrict_
     }
 }
 
+// plain copies: stream i's len bytes from src to dst, any alignment
+// (blockIdx.y = stream)
+__global__ void __launch_bounds__(256) k_ll_copy(const ZStream* __restrict__ ss) {
+    const ZStream s = ss[blockIdx.y];
+    const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, ts = (uint64_t)gridDim.x * blockDim.x;
+    const uintptr_t both = (uintptr_t)s.src | (uintptr_t)s.dst;
+    uint64_t done = 0;
+    if ((both & 15) == 0) {
+        const uint64_t n = s.len / 16;
+        for (uint64_t i = t0; i < n; i += ts) ((uint4*)s.dst)[i] = __ldcs((const uint4*)s.src + i);
+        done = n * 16;
+    } else if ((both & 3) == 0) {
+        const uint64_t n = s.len / 4;
+        for (uint64_t i = t0; i < n; i += ts) ((uint32_t*)s.dst)[i] = __ldcs((const uint32_t*)s.src + i);
+        done = n * 4;
+    }
+    for (uint64_t i = done + t0; i < s.len; i += ts) s.dst[i] = s.src[i];
+}
+// the first 12 bytes of compressed streams (raw length, chunk count)
+__global__ void k_zcb_headers(const ZStream* __restrict__ ss, int ns, uint8_t* __restrict__ out) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 12 * ns; i += gridDim.x * blockDim.x)
+        out[i] = ss[i / 12].src[i % 12];
+}
+
 unsigned zgrid(uint64_t chunks) {
     uint64_t g = (chunks + ZW - 1) / ZW;
     const uint64_t cap = (uint64_t)device_sms() * 8;
@@ -311,156 +341,238 @@ namespace prodm {
 namespace {
 uint64_t align256(uint64_t x) { return (x + 255) / 256 * 256; }
 
-// device descriptors + per-chunk scratch for `ss`; returns total chunks
+// descriptors on the device with per-chunk scratch and `extra` bytes
 struct ZJob {
-    ZStream* d_ss = nullptr;
+    Scratch mem;
+    const ZStream* ss = nullptr;
     uint32_t* csize = nullptr;
     uint32_t* coff = nullptr;
     uint32_t* outsz = nullptr;
     int* status = nullptr;
-    uint8_t* base = nullptr;
+    uint8_t* extra = nullptr;
     uint64_t chunks = 0;
-    cudaStream_t st = nullptr;
-    int setup(std::vector<ZStream>& ss, uint64_t extra, uint8_t** extra_out, cudaStream_t s) {
-        st = s;
-        chunks = 0;
-        for (auto& z : ss) {
-            z.chunk0 = chunks;
-            chunks += (z.len + 4095) / 4096;
-        }
-        const uint64_t a = align256(ss.size() * sizeof(ZStream)), b = align256(chunks * 4 + 4),
-                       c = align256(ss.size() * 4 + 4);
-        PRODM_CUDA(cudaMallocAsync((void**)&base, a + 2 * b + c + 256 + extra, st));
-        d_ss = (ZStream*)base;
+    cudaStream_t st;
+    explicit ZJob(cudaStream_t s) : mem(s), st(s) {}
+    // room for n streams of `chunks` chunks in all
+    int reserve(size_t n, uint64_t nchunks, uint64_t extra_bytes) {
+        chunks = nchunks;
+        const uint64_t a = align256(n * sizeof(ZStream)), b = align256(chunks * 4 + 4), c = align256(n * 4 + 4);
+        PRODM_CUDA(mem.alloc(a + 2 * b + c + 256 + extra_bytes));
+        uint8_t* base = mem.get();
+        ss = (const ZStream*)base;
         csize = (uint32_t*)(base + a);
         coff = (uint32_t*)(base + a + b);
         outsz = (uint32_t*)(base + a + 2 * b);
         status = (int*)(base + a + 2 * b + c);
-        if (extra_out) *extra_out = base + a + 2 * b + c + 256;
-        PRODM_CUDA(cudaMemcpyAsync(d_ss, ss.data(), ss.size() * sizeof(ZStream), cudaMemcpyHostToDevice, st));
-        PRODM_CUDA(cudaMemsetAsync(status, 0, 4, st));
+        extra = base + a + 2 * b + c + 256;
         return PRODM_OK;
     }
-    ~ZJob() {
-        if (base) cudaFreeAsync(base, st);
+    int upload(const std::vector<ZStream>& h) {   // (staged before the call returns)
+        PRODM_CUDA(cudaMemcpyAsync(mem.get(), h.data(), h.size() * sizeof(ZStream), cudaMemcpyHostToDevice, st));
+        return PRODM_OK;
     }
 };
+// the streams' first chunks in the flattened index; returns all chunks
+uint64_t number_chunks(std::vector<ZStream>& ss, size_t n) {
+    uint64_t c = 0;
+    for (size_t i = 0; i < n; i++) {
+        ss[i].chunk0 = c;
+        c += (ss[i].len + 4095) / 4096;
+    }
+    return c;
+}
+int launch_copies(const ZStream* d, const ZStream* h, size_t n, cudaStream_t st) {
+    uint64_t most = 0;
+    for (size_t i = 0; i < n; i++) most = h[i].len > most ? h[i].len : most;
+    for (size_t at = 0; at < n; at += 32768) {   // (a grid's y extent)
+        const unsigned ny = (unsigned)(n - at < 32768 ? n - at : 32768);
+        k_ll_copy<<<dim3(grid_for(most / 16 + 1, 256, n > 16 ? 1 : 4), ny), 256, 0, st>>>(d + at);
+        PRODM_CHECK_LAUNCH("k_ll_copy");
+    }
+    return PRODM_OK;
+}
 }  // namespace
 
-int ll_stream_sizes(const uint8_t* d_raw, const uint32_t* h_sizes, int B, uint32_t* h_comp, cudaStream_t st) {
-    std::vector<ZStream> ss(B);
-    uint64_t o = 0;
-    for (int p = 0; p < B; p++) {
-        ss[p] = ZStream{d_raw + o, nullptr, h_sizes[p], 0, 0};
-        o += h_sizes[p];
-    }
-    ZJob j;
-    int rc = j.setup(ss, 0, nullptr, st);
-    if (rc) return rc;
-    if ((rc = launch_zcb_count(j.d_ss, B, j.chunks, j.csize, j.coff, j.outsz, st))) return rc;
-    PRODM_CUDA(cudaMemcpyAsync(h_comp, j.outsz, B * 4, cudaMemcpyDeviceToHost, st));
-    PRODM_CUDA(cudaStreamSynchronize(st));
-    return PRODM_OK;
-}
-
-int ll_compress_level(const uint8_t* d_raw, const uint32_t* h_sizes, int B, int latter, uint8_t* d_out, uint64_t cap,
-                      uint32_t* h_out_sizes, int* h_stop, const uint8_t* h_flags, cudaStream_t st) {
-    std::vector<ZStream> ss(B);
-    std::vector<uint64_t> doff(B);
-    uint64_t o = 0, scr = 0;
-    for (int p = 0; p < B; p++) {
-        ss[p] = ZStream{d_raw + o, nullptr, h_sizes[p], 0, 0};
-        doff[p] = scr;
-        scr += align256(zcb_bound(h_sizes[p]));
-        o += h_sizes[p];
-    }
-    ZJob j;
-    uint8_t* area = nullptr;
-    int rc = j.setup(ss, scr, &area, st);
-    if (rc) return rc;
-    for (int p = 0; p < B; p++) ss[p].dst = area + doff[p];
-    PRODM_CUDA(cudaMemcpyAsync(j.d_ss, ss.data(), ss.size() * sizeof(ZStream), cudaMemcpyHostToDevice, st));
-    if ((rc = launch_zcb_count(j.d_ss, B, j.chunks, j.csize, j.coff, j.outsz, st))) return rc;
-    std::vector<uint32_t> comp(B);
-    PRODM_CUDA(cudaMemcpyAsync(comp.data(), j.outsz, B * 4, cudaMemcpyDeviceToHost, st));
-    PRODM_CUDA(cudaStreamSynchronize(st));
-    std::vector<uint8_t> flags(B);
-    const int stop = adaptive_stopping(h_sizes, comp.data(), B, latter, flags.data());
-    if (h_flags)
-        for (int p = 0; p < B; p++) flags[p] = h_flags[p];
-    uint64_t total = 0;
-    for (int p = 0; p < B; p++) total += flags[p] ? comp[p] : h_sizes[p];
-    if (total > cap) return fail(PRODM_EINVAL, "lossless: output capacity below the level's stored size");
-    if ((rc = launch_zcb_write(j.d_ss, B, j.chunks, j.csize, j.coff, st))) return rc;
-    o = 0;
-    uint64_t r = 0;
-    for (int p = 0; p < B; p++) {
-        const uint64_t n = flags[p] ? comp[p] : h_sizes[p];
-        if (n) PRODM_CUDA(cudaMemcpyAsync(d_out + o, flags[p] ? area + doff[p] : d_raw + r, n, cudaMemcpyDeviceToDevice, st));
-        h_out_sizes[p] = (uint32_t)n;
-        o += n;
-        r += h_sizes[p];
-    }
-    if (h_stop) *h_stop = stop;
-    PRODM_CUDA(cudaStreamSynchronize(st));
-    return PRODM_OK;
-}
-
-int ll_decompress_planes(const uint8_t* d_in, const uint32_t* h_sizes, const uint8_t* h_flags, int num, uint8_t* d_out,
-                         uint64_t cap, uint32_t* h_raw_sizes, cudaStream_t st) {
-    // compressed streams -> 4-byte aligned staging; their headers to the host
-    std::vector<uint64_t> soff(num), stage(num);
-    uint64_t o = 0, scr = 0;
-    for (int i = 0; i < num; i++) {
-        soff[i] = o;
-        o += h_sizes[i];
-        stage[i] = scr;
-        if (h_flags[i]) {
-            if (h_sizes[i] < 12) return fail(PRODM_ECORRUPT, "lossless: compressed stream shorter than its header");
-            scr += align256(h_sizes[i]);
-        }
-    }
-    uint8_t* area = nullptr;
-    if (scr) PRODM_CUDA(cudaMallocAsync((void**)&area, scr, st));
-    struct Guard {
-        uint8_t* p;
-        cudaStream_t s;
-        ~Guard() { if (p) cudaFreeAsync(p, s); }
-    } guard{area, st};
-    std::vector<uint8_t> hdr(12 * (size_t)num, 0);
-    for (int i = 0; i < num; i++)
-        if (h_flags[i]) {
-            PRODM_CUDA(cudaMemcpyAsync(area + stage[i], d_in + soff[i], h_sizes[i], cudaMemcpyDeviceToDevice, st));
-            PRODM_CUDA(cudaMemcpyAsync(hdr.data() + 12 * i, d_in + soff[i], 12, cudaMemcpyDeviceToHost, st));
-        }
-    PRODM_CUDA(cudaStreamSynchronize(st));
+// One call takes all the streams there are (every level of a handle): one
+// upload of descriptors and one launch per pass, where a level at a time
+// synchronised three times and a plane at a time copied once or twice
+// (257^3 fp32 files through the stage: 7.8 ms a pass of which the kernels
+// took 0.9; 0.87 ms now).
+int ll_sizes(const std::vector<LlPart>& parts, uint32_t* h_comp, cudaStream_t st) {
     std::vector<ZStream> ss;
-    uint64_t r = 0;
-    for (int i = 0; i < num; i++) {
-        uint64_t len = h_sizes[i];
-        if (h_flags[i]) {
-            uint32_t nch;
-            std::memcpy(&len, hdr.data() + 12 * i, 8);
-            std::memcpy(&nch, hdr.data() + 12 * i + 8, 4);
-            if (nch != (len + 4095) / 4096 || h_sizes[i] < 12 + 4 * (uint64_t)nch || len > 0xffffffffull)
-                return fail(PRODM_ECORRUPT, "lossless: malformed compressed stream header");
-        }
-        if (r + len > cap) return fail(PRODM_EINVAL, "lossless: output capacity below the raw size");
-        if (h_flags[i]) ss.push_back(ZStream{area + stage[i], d_out + r, len, h_sizes[i], 0});
-        else if (len) PRODM_CUDA(cudaMemcpyAsync(d_out + r, d_in + soff[i], len, cudaMemcpyDeviceToDevice, st));
-        h_raw_sizes[i] = (uint32_t)len;
-        r += len;
-    }
+    for (const LlPart& p : parts) ss.push_back(ZStream{p.src, nullptr, p.raw, 0, 0});
     if (ss.empty()) return PRODM_OK;
-    ZJob j;
-    int rc = j.setup(ss, 0, nullptr, st);
+    ZJob j(st);
+    int rc = j.reserve(ss.size(), number_chunks(ss, ss.size()), 0);
+    if (rc || (rc = j.upload(ss))) return rc;
+    if ((rc = launch_zcb_count(j.ss, (int)ss.size(), j.chunks, j.csize, j.coff, j.outsz, st))) return rc;
+    PRODM_CUDA(cudaMemcpyAsync(h_comp, j.outsz, ss.size() * 4, cudaMemcpyDeviceToHost, st));
+    PRODM_CUDA(cudaStreamSynchronize(st));
+    return PRODM_OK;
+}
+
+int ll_store(const std::vector<LlPart>& parts, cudaStream_t st) {
+    // compressed streams first; those whose place is not 4-byte aligned go
+    // through scratch; then the copies
+    std::vector<ZStream> ss, copies;
+    std::vector<uint64_t> at;   // scratch offset of a stream, or ~0
+    uint64_t scr = 0;
+    for (const LlPart& p : parts) {
+        if (!p.packed) {
+            if (p.raw) copies.push_back(ZStream{p.src, p.dst, p.raw, 0, 0});
+            continue;
+        }
+        ss.push_back(ZStream{p.src, p.dst, p.raw, p.stored, 0});
+        const bool direct = (uintptr_t)p.dst % 4 == 0;
+        at.push_back(direct ? ~0ull : scr);
+        if (!direct) scr += align256(p.stored);
+    }
+    const size_t nz = ss.size();
+    const uint64_t chunks = number_chunks(ss, nz);
+    size_t ncopy = copies.size();
+    for (uint64_t a : at) ncopy += a != ~0ull;
+    if (nz + ncopy == 0) return PRODM_OK;
+    ZJob j(st);
+    int rc = j.reserve(nz + ncopy, chunks, scr);
     if (rc) return rc;
-    if ((rc = launch_zcb_read(j.d_ss, (int)ss.size(), j.chunks, j.status, st))) return rc;
+    for (size_t i = 0; i < nz; i++)
+        if (at[i] != ~0ull) {
+            copies.push_back(ZStream{j.extra + at[i], ss[i].dst, ss[i].clen, 0, 0});
+            ss[i].dst = j.extra + at[i];
+        }
+    ss.insert(ss.end(), copies.begin(), copies.end());
+    if ((rc = j.upload(ss))) return rc;
+    if (nz) {
+        if ((rc = launch_zcb_count(j.ss, (int)nz, chunks, j.csize, j.coff, j.outsz, st))) return rc;
+        if ((rc = launch_zcb_write(j.ss, (int)nz, chunks, j.csize, j.coff, st))) return rc;
+    }
+    return ncopy ? launch_copies(j.ss + nz, ss.data() + nz, ncopy, st) : PRODM_OK;
+}
+
+int ll_raw_sizes(std::vector<LlPart>& parts, cudaStream_t st) {
+    std::vector<ZStream> ss;
+    for (const LlPart& p : parts)
+        if (p.packed) {
+            if (p.stored < 12) return fail(PRODM_ECORRUPT, "lossless: compressed stream shorter than its header");
+            ss.push_back(ZStream{p.src, nullptr, 0, p.stored, 0});
+        }
+    std::vector<uint8_t> hdr(12 * ss.size());
+    if (!ss.empty()) {
+        ZJob j(st);
+        int rc = j.reserve(ss.size(), 0, hdr.size());
+        if (rc || (rc = j.upload(ss))) return rc;
+        k_zcb_headers<<<grid_for(hdr.size(), 256), 256, 0, st>>>(j.ss, (int)ss.size(), j.extra);
+        PRODM_CHECK_LAUNCH("k_zcb_headers");
+        PRODM_CUDA(cudaMemcpyAsync(hdr.data(), j.extra, hdr.size(), cudaMemcpyDeviceToHost, st));
+        PRODM_CUDA(cudaStreamSynchronize(st));
+    }
+    size_t k = 0;
+    for (LlPart& p : parts) {
+        if (!p.packed) {
+            p.raw = p.stored;
+            continue;
+        }
+        uint64_t len;
+        uint32_t nch;
+        std::memcpy(&len, hdr.data() + 12 * k, 8);
+        std::memcpy(&nch, hdr.data() + 12 * k + 8, 4);
+        k++;
+        if (len > 0xffffffffull || nch != (len + 4095) / 4096 || p.stored < 12 + 4 * (uint64_t)nch)
+            return fail(PRODM_ECORRUPT, "lossless: malformed compressed stream header");
+        p.raw = len;
+    }
+    return PRODM_OK;
+}
+
+int ll_expand(const std::vector<LlPart>& parts, cudaStream_t st) {
+    // copies first: the uncompressed streams, and compressed ones that are not
+    // 4-byte aligned into scratch
+    std::vector<ZStream> ss, copies;
+    std::vector<uint64_t> at;
+    uint64_t scr = 0;
+    for (const LlPart& p : parts) {
+        if (!p.packed) {
+            if (p.raw) copies.push_back(ZStream{p.src, p.dst, p.raw, 0, 0});
+            continue;
+        }
+        ss.push_back(ZStream{p.src, p.dst, p.raw, p.stored, 0});
+        const bool direct = (uintptr_t)p.src % 4 == 0;
+        at.push_back(direct ? ~0ull : scr);
+        if (!direct) scr += align256(p.stored);
+    }
+    const size_t nz = ss.size();
+    const uint64_t chunks = number_chunks(ss, nz);
+    size_t ncopy = copies.size();
+    for (uint64_t a : at) ncopy += a != ~0ull;
+    if (nz + ncopy == 0) return PRODM_OK;
+    ZJob j(st);
+    int rc = j.reserve(nz + ncopy, 0, scr);
+    if (rc) return rc;
+    for (size_t i = 0; i < nz; i++)
+        if (at[i] != ~0ull) {
+            copies.push_back(ZStream{ss[i].src, j.extra + at[i], ss[i].clen, 0, 0});
+            ss[i].src = j.extra + at[i];
+        }
+    ss.insert(ss.end(), copies.begin(), copies.end());
+    if ((rc = j.upload(ss))) return rc;
+    if (ncopy && (rc = launch_copies(j.ss + nz, ss.data() + nz, ncopy, st))) return rc;
+    if (!nz) return PRODM_OK;
+    PRODM_CUDA(cudaMemsetAsync(j.status, 0, 4, st));
+    if ((rc = launch_zcb_read(j.ss, (int)nz, chunks, j.status, st))) return rc;
     int hstat = 0;
     PRODM_CUDA(cudaMemcpyAsync(&hstat, j.status, 4, cudaMemcpyDeviceToHost, st));
     PRODM_CUDA(cudaStreamSynchronize(st));
     if (hstat) return fail(PRODM_ECORRUPT, "lossless: malformed compressed chunk");
     return PRODM_OK;
+}
+
+// one level's streams (device, concatenated, raw sizes h_sizes) -> stored
+// streams (compressed where the rule says, else raw) concatenated into d_out
+static int ll_compress_level(const uint8_t* d_raw, const uint32_t* h_sizes, int B, int latter, uint8_t* d_out,
+                             uint64_t cap, uint32_t* h_out_sizes, int* h_stop, cudaStream_t st) {
+    std::vector<LlPart> parts(B);
+    uint64_t o = 0, total = 0;
+    for (int p = 0; p < B; p++) {
+        parts[p] = LlPart{d_raw + o, nullptr, h_sizes[p], 0, true};
+        o += h_sizes[p];
+    }
+    std::vector<uint32_t> comp(B);
+    int rc = ll_sizes(parts, comp.data(), st);
+    if (rc) return rc;
+    std::vector<uint8_t> flags(B);
+    *h_stop = adaptive_stopping(h_sizes, comp.data(), B, latter, flags.data());
+    for (int p = 0; p < B; p++) {
+        parts[p].packed = flags[p] != 0;
+        parts[p].stored = flags[p] ? comp[p] : h_sizes[p];
+        parts[p].dst = d_out + total;
+        h_out_sizes[p] = (uint32_t)parts[p].stored;
+        total += parts[p].stored;
+    }
+    if (total > cap) return fail(PRODM_EINVAL, "lossless: output capacity below the level's stored size");
+    if ((rc = ll_store(parts, st))) return rc;
+    PRODM_CUDA(cudaStreamSynchronize(st));
+    return PRODM_OK;
+}
+
+// stored streams of `num` planes (sizes h_sizes, flags) -> raw streams
+// concatenated into d_out (capacity cap); h_raw_sizes: their raw sizes
+static int ll_decompress_planes(const uint8_t* d_in, const uint32_t* h_sizes, const uint8_t* h_flags, int num,
+                                uint8_t* d_out, uint64_t cap, uint32_t* h_raw_sizes, cudaStream_t st) {
+    std::vector<LlPart> parts(num);
+    uint64_t o = 0, r = 0;
+    for (int i = 0; i < num; i++) {
+        parts[i] = LlPart{d_in + o, nullptr, 0, h_sizes[i], h_flags[i] != 0};
+        o += h_sizes[i];
+    }
+    int rc = ll_raw_sizes(parts, st);
+    if (rc) return rc;
+    for (int i = 0; i < num; i++) {
+        if (r + parts[i].raw > cap) return fail(PRODM_EINVAL, "lossless: output capacity below the raw size");
+        parts[i].dst = d_out + r;
+        h_raw_sizes[i] = (uint32_t)parts[i].raw;
+        r += parts[i].raw;
+    }
+    return ll_expand(parts, st);
 }
 
 }  // namespace prodm
@@ -484,7 +596,7 @@ int prodm_lossless_compress_level(const void* d_blob, const uint32_t* h_sizes, i
         latter_index < 0)
         return fail(PRODM_EINVAL, "prodm_lossless_compress_level: bad arguments");
     return ll_compress_level((const uint8_t*)d_blob, h_sizes, num_bitplanes, latter_index, (uint8_t*)d_out, capacity,
-                             h_out_sizes, h_stopping_index, nullptr, (cudaStream_t)stream);
+                             h_out_sizes, h_stopping_index, (cudaStream_t)stream);
 }
 
 int prodm_lossless_decompress_level(const void* d_blob, const uint32_t* h_sizes, int starting_bitplane,

@@ -30,9 +30,9 @@ __device__ __forceinline__ W load_bytes(const uint8_t* src) {
     return w;
 }
 
-// one CTA row of threads per plane (blockIdx.y = plane)
+// one CTA row of threads per plane (blockIdx.y = plane); plane p at planes + p * cap
 template <class W>
-__global__ void k_gr_pack(const W* const* __restrict__ planes, const uint32_t* __restrict__ sizes, int B,
+__global__ void k_gr_pack(const W* __restrict__ planes, uint64_t cap, const uint32_t* __restrict__ sizes,
                           uint64_t nblocks, const uint8_t* __restrict__ rbs, uint8_t* __restrict__ dst) {
     const int p = blockIdx.y;
     uint64_t off = 0;
@@ -51,7 +51,7 @@ __global__ void k_gr_pack(const W* const* __restrict__ planes, const uint32_t* _
         bytes -= hdr;
     }
     const uint64_t nw = bytes / sizeof(W);
-    const W* src = planes[p];
+    const W* src = planes + (uint64_t)p * cap;
     for (uint64_t w = t0; w < nw; w += ts) store_bytes<W>(dst + off + w * sizeof(W), src[w]);
 }
 
@@ -101,11 +101,11 @@ __global__ void k_fill_u32(uint32_t* dst, uint64_t n, uint32_t v) {
 
 }  // namespace
 
-int launch_gr_pack(const void* const* planes, const uint32_t* sizes, int B, uint64_t nblocks, const uint8_t* rbs,
+int launch_gr_pack(const void* planes, uint64_t cap, const uint32_t* sizes, int B, uint64_t nblocks, const uint8_t* rbs,
                    int word_bytes, uint8_t* dst, cudaStream_t st) {
-    dim3 grid(device_sms(), B);
-    if (word_bytes == 4) k_gr_pack<uint32_t><<<grid, 256, 0, st>>>((const uint32_t* const*)planes, sizes, B, nblocks, rbs, dst);
-    else k_gr_pack<uint64_t><<<grid, 256, 0, st>>>((const uint64_t* const*)planes, sizes, B, nblocks, rbs, dst);
+    dim3 grid(grid_for(2 * nblocks, 256, 1), B);
+    if (word_bytes == 4) k_gr_pack<uint32_t><<<grid, 256, 0, st>>>((const uint32_t*)planes, cap, sizes, nblocks, rbs, dst);
+    else k_gr_pack<uint64_t><<<grid, 256, 0, st>>>((const uint64_t*)planes, cap, sizes, nblocks, rbs, dst);
     PRODM_CHECK_LAUNCH("k_gr_pack");
     return PRODM_OK;
 }

@@ -889,7 +889,7 @@ int launch_pb_parse(const std::vector<PbParseJob>& jobs, cudaStream_t st) {
         for (uint64_t w : j.nwords) hv.push_back(w);
     }
     uint8_t* scratch;
-    PRODM_CUDA(cudaMallocAsync((void**)&scratch, head + fl + planes * PZ_R * PZ_E * 4, st));
+    PRODM_CUDA(scratch_alloc((void**)&scratch, head + fl + planes * PZ_R * PZ_E * 4, st));
     cudaError_t e = cudaMemcpyAsync(scratch, hv.data(), hv.size() * 8, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(scratch + head, 0, fl, st);
     const unsigned resident = resident_ctas((const void*)k_pb_parse, PZ_T, sizeof(PzShared));
