@@ -306,206 +306,343 @@ __global__ void k_reordered_to_natural(const T* __restrict__ rin, Box F, Box C, 
 // c-2 .. c+2. For double data an interior node takes the same sum regrouped as
 // one 5-point stencil, 5/6 s[c] + 1/2 (s[c-1] + s[c+1]) + 1/12 (s[c-2] + s[c+2]),
 // a third of the FP64 operations; float keeps the term order above.
-template <class W>
+template <class W, bool INTERIOR = false>   // INTERIOR: the caller knows that c is an even position in [2, nf - 3]
 __device__ __forceinline__ W l2_rhs(W sm2, W sm1, W s0, W s1, W s2, uint32_t c, uint32_t nf) {
-    if (sizeof(W) == 8 && c >= 2 && c + 3 <= nf && (c & 1u) == 0)
-        return (W)(5.0 / 6.0) * s0 + (W)0.5 * (sm1 + s1) + (W)(1.0 / 12.0) * (sm2 + s2);
+    // fused multiply-adds are written out: which product of a sum the compiler
+    // fuses depends on the code around it
+    if (sizeof(W) == 8 && (INTERIOR || (c >= 2 && c + 3 <= nf && (c & 1u) == 0)))
+        return fma((W)(1.0 / 12.0), sm2 + s2, fma((W)(5.0 / 6.0), s0, (W)0.5 * (sm1 + s1)));
     auto mf = [&](W l, W x, W r, uint32_t pos) {
-        const W dg = (pos == 0 || pos == nf - 1) ? (W)1 / 3 : (W)2 / 3;
-        return dg * x + (l + r) / 6;
+        const W dg = (!INTERIOR && (pos == 0 || pos == nf - 1)) ? (W)1 / 3 : (W)2 / 3;
+        return fma(dg, x, (l + r) / 6);
     };
     W b = mf(sm1, s0, s1, c);
-    if (c > 0 && !is_coarse(c - 1, nf)) b += (W)0.5 * mf(sm2, sm1, s0, c - 1);
-    if (c + 1 < nf && !is_coarse(c + 1, nf)) b += (W)0.5 * mf(s0, s1, s2, c + 1);
+    if (INTERIOR || (c > 0 && !is_coarse(c - 1, nf))) b = fma((W)0.5, mf(sm2, sm1, s0, c - 1), b);
+    if (INTERIOR || (c + 1 < nf && !is_coarse(c + 1, nf))) b = fma((W)0.5, mf(s0, s1, s2, c + 1), b);
     return b;
 }
 
 // One dim of the L2 projection: dst = M_c^-1 P^T M_f src along dim d.
 // Thread per line (consecutive threads on consecutive lines of the two
 // faster dims, so every access is coalesced across a warp); the fine values
-// stream through a 5-value window (two loads per coarse node, issued one
-// node ahead), the forward sweep stores d'_m in dst, the backward sweep
-// substitutes in place. cp / lo_w / inv_den: Thomas factors of the coarse
-// mass matrix (length nc, in W).
+// stream through a 5-value window, the forward sweep stores d'_m in dst, the
+// backward sweep substitutes in place. cp / lo_w / inv_den: Thomas factors of
+// the coarse mass matrix (length nc, in W). A line is a chain of dependent
+// FP64 operations (64 cycles each) whose loads are known in advance, so they
+// are issued kLineAhead nodes ahead in both sweeps: with one node ahead, and
+// none in the backward sweep, the dim-1 and dim-0 passes of 513 x 513 x 257
+// took 414 and 260 us, with four and eight and the right-hand sides of four
+// nodes ahead of their chain 325 and 168 us (FP64 floor 216 and 108 us).
+constexpr int kLineAhead = 4, kLineBack = 8;
 template <class T, class W>
-__global__ void k_l2_line(const T* __restrict__ src, Box S, int d, T* __restrict__ dst, Box D, const W* __restrict__ cp,
-                          const W* __restrict__ lo_w, const W* __restrict__ inv_den) {
+__global__ void __launch_bounds__(128) k_l2_line(const T* __restrict__ src, Box S, int d, T* dst, Box D,
+                                                 const W* __restrict__ cp, const W* __restrict__ lo_w,
+                                                 const W* __restrict__ inv_den) {
+    pdl_wait();
+    pdl_release();
     const uint32_t nf = S.n[d], nc = D.n[d];
     const int o1 = d == 0 ? 1 : 0, o2 = d == 2 ? 1 : 2;
-    const uint64_t ss[3] = {(uint64_t)S.n[1] * S.n[2], S.n[2], 1};
-    const uint64_t ds[3] = {(uint64_t)D.n[1] * D.n[2], D.n[2], 1};
+    const auto stride = [](const Box& B, int k) { return k == 2 ? 1ull : k == 1 ? B.n[2] : (uint64_t)B.n[1] * B.n[2]; };
+    const uint64_t st = stride(S, d), dt = stride(D, d);
     const uint64_t lines = (uint64_t)S.n[o1] * S.n[o2];
     for (uint64_t li = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; li < lines;
          li += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t q = (uint32_t)(li % S.n[o2]);
         uint32_t p = (uint32_t)(li / S.n[o2]);
-        const T* sl = src + p * ss[o1] + q * ss[o2];
-        T* dl = dst + p * ds[o1] + q * ds[o2];
-        const uint64_t st = ss[d], dt = ds[d];
+        const T* sl = src + p * stride(S, o1) + q * stride(S, o2);
+        T* dl = dst + p * stride(D, o1) + q * stride(D, o2);
         if (nf == nc) {
             for (uint32_t x = 0; x < nf; x++) dl[x * dt] = sl[x * st];
             continue;
         }
-        auto at = [&](int64_t x) -> W { return (x >= 0 && x < (int64_t)nf) ? (W)sl[x * st] : (W)0; };
+        auto at = [&](int64_t x) -> W { return (x >= 0 && x < (int64_t)nf) ? (W)__ldg(sl + x * st) : (W)0; };
         // regular coarse nodes sit at c = 2m; with an even nf the last one is nf - 1
         const uint32_t nreg = (nf & 1u) ? nc : nc - 1;
-        W sm2 = 0, sm1 = 0, s0 = at(0), s1 = at(1), s2 = at(2);
-        W prev = 0;
-        for (uint32_t m = 0; m < nreg; m++) {
-            const uint32_t c = 2 * m;
-            const W n3 = at((int64_t)c + 3), n4 = at((int64_t)c + 4);   // the next node's new values
-            const W b = l2_rhs<W>(sm2, sm1, s0, s1, s2, c, nf);
-            const W dp = (m == 0) ? b * inv_den[0] : (b - lo_w[m] * prev) * inv_den[m];
-            dl[m * dt] = (T)dp;
-            prev = dp;
-            sm2 = s0; sm1 = s1; s0 = s2; s1 = n3; s2 = n4;
+        W sm2 = 0, sm1 = 0, s0 = at(0), prev = 0;
+        W nx[2 * kLineAhead];   // the fine values behind the next node
+#pragma unroll
+        for (int u = 0; u < 2 * kLineAhead; u++) nx[u] = at(1 + u);
+        for (uint32_t m0 = 0; m0 < nreg; m0 += kLineAhead) {
+            W w[2 * kLineAhead + 3] = {sm2, sm1, s0};   // the values 2 m0 - 2 .. 2 (m0 + kLineAhead)
+#pragma unroll
+            for (int u = 0; u < 2 * kLineAhead; u++) {
+                w[3 + u] = nx[u];
+                nx[u] = at(2 * (int64_t)(m0 + kLineAhead) + 1 + u);
+            }
+            if (m0 && 2 * (m0 + kLineAhead - 1) + 3 <= nf) {
+                W b[kLineAhead], lo[kLineAhead], inv[kLineAhead];
+#pragma unroll
+                for (int u = 0; u < kLineAhead; u++) {
+                    lo[u] = lo_w[m0 + u];
+                    inv[u] = inv_den[m0 + u];
+                    b[u] = l2_rhs<W, true>(w[2 * u], w[2 * u + 1], w[2 * u + 2], w[2 * u + 3], w[2 * u + 4], 2 * (m0 + u), nf);
+                }
+#pragma unroll
+                for (int u = 0; u < kLineAhead; u++) {
+                    prev = fma(-lo[u], prev, b[u]) * inv[u];
+                    dl[(m0 + u) * dt] = (T)prev;
+                }
+            } else {
+#pragma unroll
+                for (int u = 0; u < kLineAhead; u++) {
+                    const uint32_t m = m0 + u;
+                    if (m < nreg) {
+                        const W b = l2_rhs<W>(w[2 * u], w[2 * u + 1], w[2 * u + 2], w[2 * u + 3], w[2 * u + 4], 2 * m, nf);
+                        prev = (m == 0) ? b * inv_den[0] : fma(-lo_w[m], prev, b) * inv_den[m];
+                        dl[m * dt] = (T)prev;
+                    }
+                }
+            }
+            sm2 = w[2 * kLineAhead];
+            sm1 = w[2 * kLineAhead + 1];
+            s0 = w[2 * kLineAhead + 2];
         }
         if (nreg < nc) {   // even nf: the last coarse node is the last fine node
             const uint32_t c = nf - 1, m = nc - 1;
             const W b = l2_rhs<W>(at((int64_t)c - 2), at((int64_t)c - 1), at(c), (W)0, (W)0, c, nf);
-            const W dp = (b - lo_w[m] * prev) * inv_den[m];
-            dl[m * dt] = (T)dp;
+            prev = fma(-lo_w[m], prev, b) * inv_den[m];
+            dl[m * dt] = (T)prev;
         }
-        W z = (W)dl[(nc - 1) * dt];
-        for (uint32_t m = nc - 1; m-- > 0;) {
-            z = (W)dl[m * dt] - cp[m] * z;
-            dl[m * dt] = (T)z;
+        W z = (W)(T)prev;   // d' of the last node
+        W r[kLineBack];     // d' of the nodes m0, m0 - 1, ..
+#pragma unroll
+        for (int u = 0; u < kLineBack; u++) r[u] = (int)nc - 2 - u >= 0 ? (W)dl[(uint64_t)(nc - 2 - u) * dt] : (W)0;
+        for (int m0 = (int)nc - 2; m0 >= 0; m0 -= kLineBack) {
+            W f[kLineBack], v[kLineBack];
+#pragma unroll
+            for (int u = 0; u < kLineBack; u++) {
+                v[u] = r[u];
+                f[u] = cp[max(m0 - u, 0)];
+                r[u] = m0 - u >= kLineBack ? (W)dl[(uint64_t)(m0 - u - kLineBack) * dt] : (W)0;
+            }
+#pragma unroll
+            for (int u = 0; u < kLineBack; u++)
+                if (m0 - u >= 0) {
+                    z = fma(-f[u], z, v[u]);
+                    dl[(uint64_t)(m0 - u) * dt] = (T)z;
+                }
         }
     }
 }
 
-// The dim-2 (contiguous) pass of the L2 projection with shared-memory staging:
-// one warp per 32 lines (fine rows (x0, x1) of F). Forward sweep: tiles of 16
-// fine columns plus two halo columns each side are staged with coalesced
-// loads (the 32 x 20 values as one flat loop); lane r then sweeps row r's
-// coarse nodes of the tile (right-hand side from the 5-point neighbourhood,
-// Thomas forward step) into an output tile stored with coalesced writes.
-// Backward sweep: the stored values come back from the end in 16-node chunks
-// (in the input tile, free by then), lane r substitutes back along its row,
-// and they are stored again. About 8 KB of shared memory per warp, so about
-// 28 warps share an SM (with 32-column tiles, 14 KB and 15 warps, the
-// passes took 9 % longer at 513 x 513 x 257 fp64). PACKED: the rows are read straight from the level's
-// packed coefficients (a natural row is an even/odd split of one contiguous
-// run of interleaved ranks; coarse nodes of rows inside the coarse box are
-// zero), so no natural-order copy is needed; else from a natural field.
-constexpr int L2_TILE = 16;                 // fine columns per tile
-constexpr int L2_STAGE = L2_TILE + 4;       // staged columns: 2 + 16 + 2
-constexpr int L2_IN_LD = L2_STAGE + 1;      // odd stride (no bank conflicts); also holds 16-node chunks
-constexpr int L2_OUT_LD = 9;                // up to 9 coarse nodes per tile, odd stride
+// The dim-2 (contiguous) pass of the L2 projection, one warp per 32 rows of F
+// and lane r on row r. The FP64 pipe bounds it (eight operations a node, 431 us
+// at 513 x 513 x 257), as long as the loads do not hold its warps up: a ring of
+// four tiles of 8 coarse nodes (of a row in packed coefficients the even and
+// the odd values are two contiguous runs, of a natural row one) is filled by
+// cp.async while earlier tiles are swept. A tile's values and Thomas factors
+// are read first, then its eight right-hand sides, which do not depend on each
+// other, then the chain of the forward step. d' leaves through the tile's slot
+// in runs of 8 and comes back the same way, from the end, for the backward
+// sweep (17 KB a warp), or stays in shared memory (KEPT: 17 KB and the 32
+// rows), and the rows leave as one run. 513 x 513 x 257 fp64: 609 us; 955 us
+// with 16-column tiles loaded, swept and stored in turn.
+// PACKED: the rows are read straight from the level's packed coefficients
+// (coarse nodes of rows inside the coarse box are zero), so no natural-order
+// copy is needed; else from a natural field.
+constexpr int kRowsRing = 4, kRowsTile = 8, kRowsLd = 2 * kRowsTile + 1;
+template <class T>
+inline size_t l2_rows_smem(uint32_t nc, bool kept) {
+    return ((size_t)(kept ? 32 * (nc | 1u) : 0) + (size_t)kRowsRing * 32 * kRowsLd) * sizeof(T);
+}
+template <class T>
+__device__ __forceinline__ void cp_async_value(T* dst, const T* src, bool on) {   // zero when off
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    const int n = on ? (int)sizeof(T) : 0;
+    if constexpr (sizeof(T) == 8)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_async_close() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_left() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-template <class T, class W, bool PACKED>
-__global__ void __launch_bounds__(32) k_l2_rows(const T* __restrict__ src, Box F, Box C, T* __restrict__ dst,
-                                                const W* __restrict__ cp, const W* __restrict__ lo_w,
-                                                const W* __restrict__ inv_den) {
-    __shared__ W sin_[32 * L2_IN_LD];
-    __shared__ W sout[32 * L2_OUT_LD];
-    const int lane = threadIdx.x;
-    const uint32_t nf = F.n[2], nc = coarse_len(nf);
-    const uint64_t lines = (uint64_t)F.n[0] * F.n[1];
-    const uint32_t c2n = C.n[2];
-    const uint64_t l0 = (uint64_t)blockIdx.x * 32;
-    if (l0 >= lines) return;
+template <class T, bool PACKED, bool KEPT>
+__global__ void __launch_bounds__(32) k_l2_rows(const T* __restrict__ src, Box F, Box C, T* dst,
+                                                const T* __restrict__ cp, const T* __restrict__ lo_w,
+                                                const T* __restrict__ inv_den) {
+    extern __shared__ __align__(16) unsigned char l2_smem[];
+    const int lane = threadIdx.x, col = lane & 7;
+    const uint32_t nf = F.n[2], nc = coarse_len(nf), P = nf - nc;
+    const uint32_t ld = nc | 1u;
+    T* ring = reinterpret_cast<T*>(l2_smem);     // [kRowsRing][32][kRowsLd]
+    T* rows = ring + kRowsRing * 32 * kRowsLd;   // KEPT: [32][ld]
+    const uint64_t lines = (uint64_t)F.n[0] * F.n[1], l0 = (uint64_t)blockIdx.x * 32;
     const int nl = (int)min((uint64_t)32, lines - l0);
-    // each row's source (base offset, inside the coarse box or not), computed
-    // once by its lane
-    __shared__ uint64_t s_base[32];
-    __shared__ int s_cc[32];
+    T* out = dst + l0 * nc;   // the warp's rows are consecutive in dst
+    pdl_wait();
+    pdl_release();
+    // this lane's row: where its even and odd values start (of a row inside
+    // the coarse box only the odd ones are there, the even ones are zero)
+    uint64_t ebase = 0, obase = 0;
+    bool cc = false;
     if (lane < nl) {
         const uint64_t li = l0 + lane;
-        const uint32_t x0 = (uint32_t)(li / F.n[1]), x1 = (uint32_t)(li - (uint64_t)x0 * F.n[1]);
         if (PACKED) {
+            const uint32_t x0 = (uint32_t)(li / F.n[1]), x1 = (uint32_t)(li - (uint64_t)x0 * F.n[1]);
             const uint32_t r0 = reord(x0, F.n[0], C.n[0]), r1 = reord(x1, F.n[1], C.n[1]);
-            const bool cc = r0 < C.n[0] && r1 < C.n[1];
-            s_cc[lane] = cc;
-            s_base[lane] = level_rank(r0, r1, cc ? c2n : 0u, F, C);
+            cc = r0 < C.n[0] && r1 < C.n[1];
+            ebase = level_rank(r0, r1, cc ? C.n[2] : 0u, F, C);
+            obase = cc ? ebase : ebase + nc;
         } else {
-            s_cc[lane] = 0;
-            s_base[lane] = li * nf;
+            ebase = obase = li * nf;
         }
     }
-    __syncwarp();
-    auto fine_at = [&](int r, int64_t x) -> W {   // natural column x of row r, 0 outside
-        if (x < 0 || x >= (int64_t)nf) return (W)0;
-        const uint64_t base = s_base[r];
-        if (!PACKED) return (W)src[base + x];
-        const uint32_t xx = (uint32_t)x;
-        const uint32_t r2 = reord(xx, nf, c2n);
-        if (s_cc[r]) return is_coarse(xx, nf) ? (W)0 : (W)src[base + (r2 - c2n)];
-        return (W)src[base + r2];
-    };
-    T* drow = dst + l0 * nc;                       // the warp's rows are consecutive in dst
     if (nc == nf) {   // no coarse subset along this dim: the projection is the identity
-        for (int r = 0; r < nl; r++)
-            for (uint32_t j = lane; j < nf; j += 32) drow[(uint64_t)r * nc + j] = (T)fine_at(r, j);
+        if (lane < nl)
+            for (uint32_t j = 0; j < nf; j++) out[(uint64_t)lane * nc + j] = cc ? (T)0 : src[ebase + j];
         return;
     }
-    const uint32_t ntiles = (nf + L2_TILE - 1) / L2_TILE;
-    W prev = 0;
-    uint32_t m = 0;                                    // next coarse node of the tile
-    for (uint32_t t = 0; t < ntiles; t++) {
-        const int64_t x0 = (int64_t)t * L2_TILE - 2;   // first staged column
-        for (int i = lane; i < nl * L2_STAGE; i += 32) {
-            const int r = i / L2_STAGE, j = i - r * L2_STAGE;
-            sin_[r * L2_IN_LD + j] = fine_at(r, x0 + j);
+    // tile t: the even and, behind them, the odd values of the nodes 8 t .. 8 t + 7
+    auto fetch = [&](uint32_t t) {
+        const uint32_t m = t * kRowsTile + col;
+        T* tile = ring + (t % kRowsRing) * 32 * kRowsLd;
+        if (t * kRowsTile < nc + 1) {
+#pragma unroll
+            for (int r0 = 0; r0 < 32; r0 += 4) {   // four rows per turn, eight lanes a run
+                const int r = r0 + (lane >> 3);
+                const uint64_t eb = __shfl_sync(0xffffffffu, ebase, r), ob = __shfl_sync(0xffffffffu, obase, r);
+                const bool zero = __shfl_sync(0xffffffffu, (int)cc, r), on = r < nl;
+                const bool e = on && m < nc && !zero, o = on && m < P;
+                const uint64_t ei = eb + (PACKED ? m : min(2 * m, nf - 1)), oi = ob + (PACKED ? m : 2 * m + 1);
+                cp_async_value(tile + r * kRowsLd + col, e ? src + ei : src, e);
+                cp_async_value(tile + r * kRowsLd + kRowsTile + col, o ? src + oi : src, o);
+            }
         }
+        cp_async_close();
+    };
+#pragma unroll
+    for (int t = 0; t < kRowsRing - 1; t++) fetch(t);
+    T* own = rows + lane * ld;
+    // Node m needs the even value of node m + 1, which may lie in the next
+    // tile, so tile t brings the nodes 8 t - 1 .. 8 t + 6. Carried over: the
+    // last two even values and the last three odd ones.
+    T em1 = 0, e0 = 0, om2 = 0, om1 = 0, o0 = 0, prev = 0;
+    for (uint32_t t = 0; t * kRowsTile < nc + 1; t++) {
+        fetch(t + kRowsRing - 1);
+        cp_async_left<kRowsRing - 1>();
         __syncwarp();
-        // coarse nodes whose fine position falls in [32t, 32t + 32): the same
-        // range for every row
-        const uint32_t xe = min((uint32_t)(t + 1) * L2_TILE, nf);
-        const uint32_t mt0 = m;
-        uint32_t mt1 = mt0;
-        while (mt1 < nc && fine_of_coarse(mt1, nf, nc) < xe) mt1++;
-        m = mt1;
-        if (lane < nl) {
-            const W* s = sin_ + lane * L2_IN_LD;
-            for (uint32_t mm = mt0; mm < mt1; mm++) {
-                const uint32_t c = fine_of_coarse(mm, nf, nc);
-                const W* w = s + ((int64_t)c - x0);   // staged columns c-2 .. c+2
-                const W b = l2_rhs<W>(w[-2], w[-1], w[0], w[1], w[2], c, nf);
-                const W dp = (mm == 0) ? b * inv_den[0] : (b - lo_w[mm] * prev) * inv_den[mm];
-                sout[lane * L2_OUT_LD + (mm - mt0)] = dp;
-                prev = dp;
+        T* tile = ring + (t % kRowsRing) * 32 * kRowsLd + lane * kRowsLd;
+        T ev[kRowsTile + 2] = {em1, e0}, od[kRowsTile + 3] = {om2, om1, o0}, dp[kRowsTile];
+#pragma unroll
+        for (int u = 0; u < kRowsTile; u++) {
+            ev[2 + u] = tile[u];
+            od[3 + u] = tile[kRowsTile + u];
+        }
+        const int j0 = (int)(t * kRowsTile) - 1;
+        if (t && 2 * (uint32_t)(j0 + kRowsTile - 1) + 3 <= nf) {
+            T lo[kRowsTile], inv[kRowsTile];
+#pragma unroll
+            for (int u = 0; u < kRowsTile; u++) {
+                lo[u] = lo_w[j0 + u];
+                inv[u] = inv_den[j0 + u];
+                dp[u] = l2_rhs<T, true>(ev[u], od[1 + u], ev[1 + u], od[2 + u], ev[2 + u], 2 * (j0 + u), nf);
+            }
+#pragma unroll
+            for (int u = 0; u < kRowsTile; u++) dp[u] = prev = fma(-lo[u], prev, dp[u]) * inv[u];
+        } else {
+#pragma unroll
+            for (int u = 0; u < kRowsTile; u++) {
+                const int j = j0 + u;
+                if (j >= 0 && j < (int)nc) {
+                    const bool lastone = j == (int)nc - 1;
+                    T sm2 = ev[u], sm1 = od[1 + u], s1 = od[2 + u], s2 = ev[2 + u];
+                    if (lastone) s1 = s2 = 0;
+                    if (!(nf & 1u)) {   // the last two nodes sit side by side
+                        if (lastone) { sm2 = od[u]; sm1 = ev[u]; }
+                        else if (j == (int)nc - 2) { s1 = ev[2 + u]; s2 = 0; }
+                    }
+                    const T b = l2_rhs<T>(sm2, sm1, ev[1 + u], s1, s2, lastone ? nf - 1 : 2 * j, nf);
+                    prev = j == 0 ? b * inv_den[0] : fma(-lo_w[j], prev, b) * inv_den[j];
+                }
+                dp[u] = prev;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kRowsTile; u++) {
+            if constexpr (KEPT) {
+                if (j0 + u >= 0 && j0 + u < (int)nc) own[j0 + u] = dp[u];
+            } else {
+                tile[u] = dp[u];   // (its own row, read above)
             }
         }
         __syncwarp();
-        const int cnt = (int)(mt1 - mt0);
-        for (int i = lane; i < nl * cnt; i += 32) {
-            const int r = i / cnt, j = i - r * cnt;
-            drow[(uint64_t)r * nc + mt0 + j] = (T)sout[r * L2_OUT_LD + j];
+        if constexpr (!KEPT) {
+            const int j = j0 + col;
+            const T* all = ring + (t % kRowsRing) * 32 * kRowsLd;
+#pragma unroll
+            for (int r0 = 0; r0 < 32; r0 += 4) {
+                const int r = r0 + (lane >> 3);
+                if (r < nl && j >= 0 && j < (int)nc) out[(uint64_t)r * nc + j] = all[r * kRowsLd + col];
+            }
+            __syncwarp();   // the slot is free for the fetch after next
         }
-        __syncwarp();
+        em1 = ev[kRowsTile];
+        e0 = ev[kRowsTile + 1];
+        om2 = od[kRowsTile];
+        om1 = od[kRowsTile + 1];
+        o0 = od[kRowsTile + 2];
     }
-    // backward substitution, 32-node chunks from the end, in the input tile
-    W z = 0;
-    uint32_t mhi = nc;
-    while (mhi > 0) {
-        const uint32_t mlo = mhi > L2_TILE ? mhi - L2_TILE : 0;
-        const int cnt = (int)(mhi - mlo);
-        for (int i = lane; i < nl * cnt; i += 32) {
-            const int r = i / cnt, j = i - r * cnt;
-            sin_[r * L2_IN_LD + j] = (W)drow[(uint64_t)r * nc + mlo + j];
+    // backward substitution, eight nodes at a time from the end
+    T z = prev;
+    auto back = [&](T* v, int m0) {   // the nodes m0 .. m0 + 7 in v[0 .. 7]
+        T x[kRowsTile], f[kRowsTile];
+#pragma unroll
+        for (int u = 0; u < kRowsTile; u++) {
+            x[u] = m0 + u < (int)nc ? v[u] : (T)0;
+            f[u] = cp[min(m0 + u, (int)nc - 1)];
         }
+#pragma unroll
+        for (int u = kRowsTile - 1; u >= 0; u--)
+            if (m0 + u < (int)nc - 1) v[u] = z = fma(-f[u], z, x[u]);
+    };
+    const int top = ((int)nc - 1) & ~(kRowsTile - 1);
+    if constexpr (KEPT) {
+        for (int m0 = top; m0 >= 0; m0 -= kRowsTile) back(own + m0, m0);
         __syncwarp();
-        if (lane < nl) {
-            W* o = sin_ + lane * L2_IN_LD;
-            for (uint32_t mm = mhi; mm-- > mlo;) {
-                z = (mm == nc - 1) ? o[mm - mlo] : o[mm - mlo] - cp[mm] * z;
-                o[mm - mlo] = z;
+        for (uint32_t j = lane; j < nc; j += 32)
+#pragma unroll 8
+            for (int r = 0; r < nl; r++) out[(uint64_t)r * nc + j] = rows[r * ld + j];
+    } else {
+        auto fetch_back = [&](int i) {   // the i-th tile from the end
+            const int m = top - i * kRowsTile + col;
+            T* tile = ring + (i % kRowsRing) * 32 * kRowsLd;
+            if (top - i * kRowsTile >= 0) {
+#pragma unroll
+                for (int r0 = 0; r0 < 32; r0 += 4) {
+                    const int r = r0 + (lane >> 3);
+                    const bool on = r < nl && m < (int)nc;
+                    cp_async_value(tile + r * kRowsLd + col, on ? out + (uint64_t)r * nc + m : out, on);
+                }
             }
+            cp_async_close();
+        };
+#pragma unroll
+        for (int i = 0; i < kRowsRing - 1; i++) fetch_back(i);
+        for (int i = 0; i * kRowsTile <= top; i++) {
+            fetch_back(i + kRowsRing - 1);
+            cp_async_left<kRowsRing - 1>();
+            __syncwarp();
+            T* all = ring + (i % kRowsRing) * 32 * kRowsLd;
+            const int m0 = top - i * kRowsTile;
+            back(all + lane * kRowsLd, m0);
+            __syncwarp();
+#pragma unroll
+            for (int r0 = 0; r0 < 32; r0 += 4) {
+                const int r = r0 + (lane >> 3);
+                if (r < nl && m0 + col < (int)nc) out[(uint64_t)r * nc + m0 + col] = all[r * kRowsLd + col];
+            }
+            __syncwarp();
         }
-        __syncwarp();
-        for (int i = lane; i < nl * cnt; i += 32) {
-            const int r = i / cnt, j = i - r * cnt;
-            drow[(uint64_t)r * nc + mlo + j] = (T)sin_[r * L2_IN_LD + j];
-        }
-        __syncwarp();
-        mhi = mlo;
     }
 }
 
 // dst[i] += sign * z[i] over a compact box written into a strided box
 template <class T>
 __global__ void k_add_box(T* __restrict__ dst, uint64_t b0, uint64_t b1, const T* __restrict__ z, Box B, T sign) {
+    pdl_wait();
+    pdl_release();
     const uint64_t total = B.size();
     for (uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
          idx += (uint64_t)gridDim.x * blockDim.x) {
@@ -673,10 +810,28 @@ int launch_l2_correction(const T* fnat, const Box& F, T* t1, T* t2, T* z, const 
         const uint32_t nc = coarse_len(F.n[2]);
         const T* tab = tabs[2];
         const uint64_t lines = (uint64_t)F.n[0] * F.n[1];
-        const unsigned grid = (unsigned)((lines + 31) / 32);
-        if (coef) k_l2_rows<T, T, true><<<grid, 32, 0, st>>>(coef, F, *C, t1, tab, tab + nc, tab + 2 * nc);
-        else k_l2_rows<T, T, false><<<grid, 32, 0, st>>>(fnat, F, F, t1, tab, tab + nc, tab + 2 * nc);
-        PRODM_CHECK_LAUNCH("k_l2_rows");
+        const dim3 grid((unsigned)((lines + 31) / 32));
+        // Keep d' on chip while that leaves six warps an SM (36 KB; 257 x 257 x 129
+        // fp64 at 34 KB: level 332 us against 360), or where all warps are
+        // resident at once anyway (129 x 129 x 257: 179 against 271); at 50 KB and
+        // 54 warps an SM (513 x 513 x 257) it is 2030 against 1797.
+        const size_t keep = l2_rows_smem<T>(nc, true);
+        const bool kept = keep <= 36 * 1024 ||
+                          (keep <= 200 * 1024 && (uint64_t)(227 * 1024 / (keep + 1024)) * kSMs >= grid.x);
+        const size_t smem = l2_rows_smem<T>(nc, kept);
+        const auto kernel = coef ? (kept ? k_l2_rows<T, true, true> : k_l2_rows<T, true, false>)
+                                 : (kept ? k_l2_rows<T, false, true> : k_l2_rows<T, false, false>);
+        cudaError_t e;
+        if (smem > 48 * 1024 &&
+            (e = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
+                cudaSuccess)
+            return cuda_status(e, "cudaFuncSetAttribute");
+        count_launch();
+        // not launched ahead: its one-warp blocks would gather on the SMs that
+        // the kernel before leaves room on (65 x 65 x 2049: level 1178 us, 587 so)
+        e = launch_chain(false, kernel, grid, dim3(32), smem, st, coef ? coef : fnat, F, coef ? *C : F, t1, tab, tab + nc,
+                         tab + 2 * nc);
+        if (e != cudaSuccess) return cuda_status(e, "k_l2_rows");
         a.n[2] = nc;
     }
     const T* src = t1;
@@ -686,8 +841,10 @@ int launch_l2_correction(const T* fnat, const Box& F, T* t1, T* t2, T* z, const 
         uint64_t lines = a.size() / a.n[d];
         uint32_t nc = b.n[d];
         const T* tab = tabs[d];
-        k_l2_line<T, T><<<grid_for(lines, th, 16), th, 0, st>>>(src, a, d, bufs[k], b, tab, tab + nc, tab + 2 * nc);
-        PRODM_CHECK_LAUNCH("k_l2_line");
+        count_launch();
+        const cudaError_t e = launch_chain(true, k_l2_line<T, T>, dim3(grid_for(lines, th, 16)), dim3(th), 0, st, src, a, d,
+                                           bufs[k], b, tab, tab + nc, tab + 2 * nc);
+        if (e != cudaSuccess) return cuda_status(e, "k_l2_line");
         src = bufs[k];
         a = b;
     }
@@ -697,8 +854,10 @@ int launch_l2_correction(const T* fnat, const Box& F, T* t1, T* t2, T* z, const 
 template <class T>
 int launch_add_box(T* dst, uint64_t b0, uint64_t b1, const T* z, const Box& B, T sign, cudaStream_t st) {
     const int th = 256;
-    k_add_box<T><<<grid_for(B.size(), th), th, 0, st>>>(dst, b0, b1, z, B, sign);
-    PRODM_CHECK_LAUNCH("k_add_box");
+    count_launch();
+    const cudaError_t e = launch_chain(true, k_add_box<T>, dim3(grid_for(B.size(), th)), dim3(th), 0, st, dst, b0, b1, z, B,
+                                       sign);
+    if (e != cudaSuccess) return cuda_status(e, "k_add_box");
     return PRODM_OK;
 }
 
