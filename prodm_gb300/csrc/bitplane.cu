@@ -806,29 +806,66 @@ __device__ __forceinline__ int gr_warp_offsets(const uint8_t* __restrict__ rbs, 
     return rv;
 }
 
-// fp64 writer
-__global__ void __launch_bounds__(256, 4) k_gr_write64(const __grid_constant__ GrSet<double> set, int B) {
+// Plane words leave through shared memory, SB blocks of a warp at a time: row
+// i holds the words of one plane (one per block that reaches it and the sign
+// words of the blocks that start there, so at most 2 SB), and SB lanes write
+// them as one run. A lane per plane and one word per block instead, every word
+// is a store to a sector of its own.
+template <class S, int SB>
+struct GrStage {
+    static constexpr int LD = 2 * SB + 1;
+    // the runs of 32 rows: row i (below rows) has c_i words (lane i's c) and goes to out + i * step + off_i
+    static __device__ __forceinline__ void flush(S* out, int64_t step, int rows, const S* stage, uint32_t off, uint32_t c,
+                                                 int lane) {
+        const int k = lane & (SB - 1);
+#pragma unroll 4
+        for (int i0 = 0; i0 < rows; i0 += 32 / SB) {
+            const int i = i0 + lane / SB;
+            const uint32_t o = __shfl_sync(FULL, off, i & 31);
+            const int ci = (int)__shfl_sync(FULL, c, i & 31), m = i < rows ? ci : 0;
+            S* dst = out + i * step + o;
+            if (k < m) dst[k] = stage[i * LD + k];
+            if (k + SB < m) dst[k + SB] = stage[i * LD + k + SB];
+        }
+    }
+};
+
+// fp64 writer. 513 x 513 x 257, 60 planes: 326 us; 1050 us with a store per
+// word and two blocks loaded at a time (DRAM floor 164 us).
+constexpr int GR_SB64 = 8;
+constexpr size_t kGrStage64 = (size_t)GR_WARPS * 64 * GrStage<uint64_t, GR_SB64>::LD * sizeof(uint64_t);
+__global__ void __launch_bounds__(256, 3) k_gr_write64(const __grid_constant__ GrSet<double> set, int B) {
     using S = uint64_t;
-    constexpr int U = 2;   // blocks loaded ahead
+    using Stage = GrStage<S, GR_SB64>;
+    constexpr int U = 4;   // blocks loaded ahead
+    extern __shared__ __align__(16) unsigned char smem[];
     uint32_t chunk;
     const GrSeg<double>& q = gr_seg(set, chunk);
     const double* __restrict__ x = q.x;
     const uint64_t n = q.n, cap = q.cap;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t nblocks = (n + 63) / 64;
+    S* stage = (S*)smem + warp * 64 * Stage::LD;
     pdl_wait();
     pdl_release();
-    const int exp = level_exp<double>(q.key, q.exp);
-    uint32_t off0, off1;
-    const int rv = gr_warp_offsets(q.rbs, nblocks, chunk, q.co, B, off0, off1);
     const uint64_t b0 = (uint64_t)chunk * GR_CHUNK + (uint64_t)warp * GR_BPW;
-    for (int j0 = 0; j0 < GR_BPW && b0 + j0 < nblocks; j0 += U) {
-        double v[2 * U];
+    double nx[2 * U];
+    auto load = [&](int j0) {
 #pragma unroll
         for (int t = 0; t < 2 * U; t++) {
             const uint64_t i = (b0 + j0) * 64 + t * 32 + lane;
-            v[t] = i < n ? __ldcs(x + i) : 0.0;
+            nx[t] = j0 < GR_BPW && i < n ? __ldcs(x + i) : 0.0;
         }
+    };
+    load(0);
+    const int exp = level_exp<double>(q.key, q.exp);
+    uint32_t off0, off1, c0 = 0, c1 = 0;
+    const int rv = gr_warp_offsets(q.rbs, nblocks, chunk, q.co, B, off0, off1);
+    for (int j0 = 0; j0 < GR_BPW && b0 + j0 < nblocks; j0 += U) {
+        double v[2 * U];
+#pragma unroll
+        for (int t = 0; t < 2 * U; t++) v[t] = nx[t];
+        load(j0 + U);
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int r = __shfl_sync(FULL, rv, j0 + u);
@@ -852,27 +889,37 @@ __global__ void __launch_bounds__(256, 4) k_gr_write64(const __grid_constant__ G
             for (int t = 0; t < 2; t++) {   // plane lane + 32 t (a valid plane for the shuffles' sake)
                 const int p = lane + 32 * t < B ? lane + 32 * t : 0;
                 const int k = B - 1 - p, src = k & 31;
-                const uint32_t a0 = __shfl_sync(FULL, lo0, src), c0 = __shfl_sync(FULL, hi0, src);
-                const uint32_t a1 = __shfl_sync(FULL, lo1, src), c1 = __shfl_sync(FULL, hi1, src);
-                w[t] = k >= 32 ? ((S)c1 << 32 | c0) : ((S)a1 << 32 | a0);
+                const uint32_t a0 = __shfl_sync(FULL, lo0, src), d0 = __shfl_sync(FULL, hi0, src);
+                const uint32_t a1 = __shfl_sync(FULL, lo1, src), d1 = __shfl_sync(FULL, hi1, src);
+                w[t] = k >= 32 ? ((S)d1 << 32 | d0) : ((S)a1 << 32 | a0);
             }
-            if (lane < B && lane >= r) {
-                S* dst = q.out + (uint64_t)lane * cap + off0;
-                if (lane == r) { dst[0] = sign; dst[1] = w[0]; }
-                else dst[0] = w[0];
+            if (lane >= r) {
+                S* dst = stage + lane * Stage::LD + c0;
+                if (lane == r) *dst++ = sign;
+                *dst = w[0];
             }
-            if (lane + 32 < B && lane + 32 >= r) {
-                S* dst = q.out + (uint64_t)(lane + 32) * cap + off1;
-                if (lane + 32 == r) { dst[0] = sign; dst[1] = w[1]; }
-                else dst[0] = w[1];
+            if (lane + 32 >= r) {
+                S* dst = stage + (lane + 32) * Stage::LD + c1;
+                if (lane + 32 == r) *dst++ = sign;
+                *dst = w[1];
             }
-            off0 += gr_words(r, lane);
-            off1 += gr_words(r, lane + 32);
+            c0 += gr_words(r, lane);
+            c1 += gr_words(r, lane + 32);
+        }
+        if ((j0 + U) % GR_SB64 == 0 || b0 + j0 + U >= nblocks) {
+            __syncwarp();
+            Stage::flush(q.out, (int64_t)cap, min(B, 32), stage, off0, c0, lane);
+            Stage::flush(q.out + 32 * cap, (int64_t)cap, B - 32, stage + 32 * Stage::LD, off1, c1, lane);
+            __syncwarp();
+            off0 += c0;
+            off1 += c1;
+            c0 = c1 = 0;
         }
     }
 }
 
-// fp32 grouped writer: one transpose per block instead of B ballots. With
+// fp32 grouped writer: one transpose per block instead of B ballots (150 x 257
+// x 301, 32 planes: 41 us, 88 us with a store per word). With
 // ERR, the exact squared-error tables (errtab.cuh, GroupedBPEncoder.hpp:76-145
 // with collect_level_errors :324-335) of the CTA's chunk go to its record
 // recs + blockIdx.x (one level per launch): four blocks per step, t =
@@ -889,16 +936,29 @@ __global__ void __launch_bounds__(256) k_gr_write32(const __grid_constant__ GrSe
     const uint64_t n = q.n, cap = q.cap;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t nblocks = (n + 31) / 32;
+    constexpr int SB = ERR ? 8 : 16, U = 4;   // blocks staged; blocks loaded ahead
+    using Stage = GrStage<uint32_t, SB>;
+    __shared__ uint32_t stages[GR_WARPS][32 * Stage::LD];
+    uint32_t* stage = stages[warp];
     pdl_wait();
     pdl_release();
+    const uint64_t b0 = (uint64_t)chunk * GR_CHUNK + (uint64_t)warp * GR_BPW;
+    float nx[U];
+    auto load = [&](int j0) {
+#pragma unroll
+        for (int g = 0; g < U; g++) {
+            const uint64_t i = (b0 + j0 + g) * 32 + lane;
+            nx[g] = j0 < GR_BPW && i < n ? __ldcs(x + i) : 0.f;
+        }
+    };
+    load(0);
     const int exp = level_exp<float>(q.key, q.exp);
     uint32_t off0, off1;
     const int rv = gr_warp_offsets(q.rbs, nblocks, chunk, q.co, B, off0, off1);
-    const int plane = B - 1 - lane;                    // lane k owns bit k
-    uint32_t off = __shfl_sync(FULL, off0, plane & 31);
+    const int plane = B - 1 - lane;                    // lane k owns bit k, row k of the stage
+    uint32_t off = __shfl_sync(FULL, off0, plane & 31), c = 0;
     const bool fast = pow2_normal(B - exp);
     const float sc = fast ? pow2f(B - exp) : 1.f;
-    const uint64_t b0 = (uint64_t)chunk * GR_CHUNK + (uint64_t)warp * GR_BPW;
     errtab::WarpQ* wq = (errtab::WarpQ*)smem;
     unsigned long long* red = (unsigned long long*)(wq + 8);
     errtab::Lane acc;
@@ -908,18 +968,19 @@ __global__ void __launch_bounds__(256) k_gr_write32(const __grid_constant__ GrSe
         acc.zero();
         errtab::zero_q(wq[warp], lane);
     }
-    for (int j0 = 0; j0 < GR_BPW && (ERR || b0 + j0 < nblocks); j0 += 4) {
-        float sh[4], mag[4];
-        uint32_t m[4], sign[4];
-        bool small[4];
+    for (int j0 = 0; j0 < GR_BPW && (ERR || b0 + j0 < nblocks); j0 += U) {
+        float v[U], sh[U], mag[U];
+        uint32_t m[U], sign[U];
+        bool small[U];
 #pragma unroll
-        for (int g = 0; g < 4; g++) {
-            const uint64_t i = (b0 + j0 + g) * 32 + lane;
-            const bool ok = i < n;
-            const float v = ok ? __ldcs(x + i) : 0.f;
-            sh[g] = scale2(v, B - exp, fast, sc);
+        for (int g = 0; g < U; g++) v[g] = nx[g];
+        load(j0 + U);
+#pragma unroll
+        for (int g = 0; g < U; g++) {
+            const bool ok = (b0 + j0 + g) * 32 + lane < n;
+            sh[g] = scale2(v[g], B - exp, fast, sc);
             const int64_t fix = (int64_t)sh[g];
-            const bool neg = v < 0.f;
+            const bool neg = v[g] < 0.f;
             m[g] = (uint32_t)(neg ? -fix : fix);
             sign[g] = __ballot_sync(FULL, neg);
             if (ERR) {
@@ -935,16 +996,23 @@ __global__ void __launch_bounds__(256) k_gr_write32(const __grid_constant__ GrSe
             acc.add4(m[0], m[1], m[2], m[3]);
         }
 #pragma unroll
-        for (int g = 0; g < 4; g++) {
+        for (int g = 0; g < U; g++) {
             const uint32_t w = transpose32(m[g], lane);
             if (ERR) acc.pc += __popc(w);
             const int r = __shfl_sync(FULL, rv, j0 + g);
-            if (lane < B && plane >= r) {
-                uint32_t* dst = q.out + (uint64_t)plane * cap + off;
-                if (plane == r) { dst[0] = sign[g]; dst[1] = w; }
-                else dst[0] = w;
+            if (plane >= r) {
+                uint32_t* dst = stage + lane * Stage::LD + c;
+                if (plane == r) *dst++ = sign[g];
+                *dst = w;
             }
-            off += gr_words(r, plane);
+            c += gr_words(r, plane);
+        }
+        if ((j0 + U) % SB == 0 || (!ERR && b0 + j0 + U >= nblocks)) {
+            __syncwarp();
+            Stage::flush(q.out + (B - 1) * (int64_t)cap, -(int64_t)cap, B, stage, off, c, lane);
+            __syncwarp();
+            off += c;
+            c = 0;
         }
     }
     if (ERR) {
@@ -962,9 +1030,37 @@ __global__ void __launch_bounds__(256) k_gr_write32(const __grid_constant__ GrSe
 // GroupedBPEncoder::progressive_decode -- :210-297 (planes [s, e)); plane p's
 // words at planes[p] (absolute plane index). signs: per-block sign words kept
 // between calls (nullable when s == 0). A device count (dnum[0]) overrides e.
-// fp32: lane p loads plane p's word of the block.
+// Lane p loads plane p's word of a block (planes p and p + 32 in 64 bits),
+// GR_DU blocks ahead of the ones in work. The sign words of a warp's 32 blocks
+// are fetched together before them, lane j block j's: gr_signs.
+// 513 x 513 x 257 fp64, most of 60 planes: 284 us; 419 us with four blocks
+// loaded, decoded and stored in turn and the sign words among them.
+template <class S>
+__device__ __forceinline__ S gr_signs(const S* const* __restrict__ planes, S* signs, uint64_t b, int rv, uint32_t off0,
+                                      uint32_t off1, int s, int e, int lane) {
+    uint32_t at = 0;   // where block lane's sign word stands in its plane
+#pragma unroll 8
+    for (int j = 0; j < GR_BPW; j++) {
+        const int r = __shfl_sync(FULL, rv, j);
+        uint32_t o = __shfl_sync(FULL, off0, r & 31);
+        if (sizeof(S) == 8) {
+            const uint32_t o1 = __shfl_sync(FULL, off1, r & 31);
+            o = r < 32 ? o : o1;
+            off1 += gr_words(r, lane + 32);
+        }
+        off0 += gr_words(r, lane);
+        if (lane == j) at = o;
+    }
+    if (rv >= e) return 0;                 // nothing of the block is there yet (or there is no block)
+    if (rv < s) return signs[b + lane];    // kept by an earlier call
+    const S sign = __ldcs(planes[rv] + at);
+    if (signs) signs[b + lane] = sign;
+    return sign;
+}
+constexpr int GR_DU = 4;
+
 __global__ void __launch_bounds__(256) k_gr_decode32(const __grid_constant__ GrSet<float> set, int B, int s, int e) {
-    constexpr int U = 8;   // blocks loaded ahead
+    constexpr int U = 2 * GR_DU;
     uint32_t chunk;
     const GrSeg<float>& q = gr_seg(set, chunk);
     const uint64_t n = q.n;
@@ -980,27 +1076,28 @@ __global__ void __launch_bounds__(256) k_gr_decode32(const __grid_constant__ GrS
     const bool fast = pow2_normal(exp - e);
     const float sc = fast ? pow2f(exp - e) : 1.f;
     const uint64_t b0 = (uint64_t)chunk * GR_CHUNK + (uint64_t)warp * GR_BPW;
-    for (int j0 = 0; j0 < GR_BPW && b0 + j0 < nblocks; j0 += U) {
-        uint32_t w[U], sg[U];
+    const uint32_t signs = gr_signs(q.planes, q.signs, b0, rv, off, 0u, s, e, lane);
+    uint32_t nx[U];
+    auto load = [&](int j0) {
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            const int r = __shfl_sync(FULL, rv, j0 + u);
-            w[u] = sg[u] = 0;
-            if (src && lane >= r) {
-                const bool head = lane == r;
-                w[u] = __ldcs(src + off + (head ? 1 : 0));
-                if (head) sg[u] = __ldcs(src + off);
-            }
-            if (r < s && lane == 0) sg[u] = q.signs[b0 + j0 + u];   // kept by an earlier call
+            const int r = j0 < GR_BPW ? __shfl_sync(FULL, rv, j0 + u) : 255;
+            nx[u] = src && lane >= r ? __ldcs(src + off + (lane == r ? 1 : 0)) : 0;
             off += gr_words(r, lane);
         }
+    };
+    load(0);
+    for (int j0 = 0; j0 < GR_BPW && b0 + j0 < nblocks; j0 += U) {
+        uint32_t w[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) w[u] = nx[u];
+        load(j0 + U);
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int r = __shfl_sync(FULL, rv, j0 + u);
-            const uint64_t b = b0 + j0 + u, i = b * 32 + lane;
+            const uint32_t sign = __shfl_sync(FULL, signs, j0 + u);
+            const uint64_t i = (b0 + j0 + u) * 32 + lane;
             if (r < e) {
-                const uint32_t sign = __shfl_sync(FULL, sg[u], r >= s ? r : 0);
-                if (r >= s && q.signs && lane == 0) q.signs[b] = sign;
                 const uint32_t col = transpose32(w[u], lane);
                 const uint32_t acc = __brev(col) >> (32 - e);
                 const float v = scale2((float)acc, exp - e, fast, sc);
@@ -1015,7 +1112,7 @@ __global__ void __launch_bounds__(256) k_gr_decode32(const __grid_constant__ GrS
 // fp64
 __global__ void __launch_bounds__(256) k_gr_decode64(const __grid_constant__ GrSet<double> set, int B, int s, int e) {
     using S = uint64_t;
-    constexpr int U = 4;   // blocks loaded ahead
+    constexpr int U = GR_DU;
     uint32_t chunk;
     const GrSeg<double>& q = gr_seg(set, chunk);
     const uint64_t n = q.n;
@@ -1030,31 +1127,33 @@ __global__ void __launch_bounds__(256) k_gr_decode64(const __grid_constant__ GrS
     const S* src0 = (lane >= s && lane < e) ? q.planes[lane] : nullptr;
     const S* src1 = (lane + 32 >= s && lane + 32 < e) ? q.planes[lane + 32] : nullptr;
     const uint64_t b0 = (uint64_t)chunk * GR_CHUNK + (uint64_t)warp * GR_BPW;
-    for (int j0 = 0; j0 < GR_BPW && b0 + j0 < nblocks; j0 += U) {
-        S w0[U], w1[U], sg[U];
+    const S signs = gr_signs(q.planes, q.signs, b0, rv, off0, off1, s, e, lane);
+    S n0[U], n1[U];
+    auto load = [&](int j0) {
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            const int r = __shfl_sync(FULL, rv, j0 + u);
-            w0[u] = w1[u] = sg[u] = 0;
-            if (src0 && lane >= r) {
-                w0[u] = __ldcs(src0 + off0 + (lane == r ? 1 : 0));
-                if (lane == r) sg[u] = __ldcs(src0 + off0);
-            }
-            if (src1 && lane + 32 >= r) {
-                w1[u] = __ldcs(src1 + off1 + (lane + 32 == r ? 1 : 0));
-                if (lane + 32 == r) sg[u] = __ldcs(src1 + off1);
-            }
-            if (r < s && lane == 0) sg[u] = q.signs[b0 + j0 + u];   // kept by an earlier call
+            const int r = j0 < GR_BPW ? __shfl_sync(FULL, rv, j0 + u) : 255;
+            n0[u] = src0 && lane >= r ? __ldcs(src0 + off0 + (lane == r ? 1 : 0)) : 0;
+            n1[u] = src1 && lane + 32 >= r ? __ldcs(src1 + off1 + (lane + 32 == r ? 1 : 0)) : 0;
             off0 += gr_words(r, lane);
             off1 += gr_words(r, lane + 32);
         }
+    };
+    load(0);
+    for (int j0 = 0; j0 < GR_BPW && b0 + j0 < nblocks; j0 += U) {
+        S w0[U], w1[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            w0[u] = n0[u];
+            w1[u] = n1[u];
+        }
+        load(j0 + U);
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const int r = __shfl_sync(FULL, rv, j0 + u);
-            const uint64_t b = b0 + j0 + u, i = b * 64 + lane;
+            const S sign = __shfl_sync(FULL, signs, j0 + u);
+            const uint64_t i = (b0 + j0 + u) * 64 + lane;
             if (r < e) {
-                const S sign = __shfl_sync(FULL, sg[u], r >= s ? r & 31 : 0);
-                if (r >= s && q.signs && lane == 0) q.signs[b] = sign;
                 // decode_block :359-368 by four warp bit transposes: lane p holds
                 // planes p and p + 32 (zero where not read); after the
                 // transposes lane v holds, per half h of the block, a word whose
@@ -1342,6 +1441,10 @@ int launch_gr_encode(GrSet<T> set, int B, double* partial, double* errs_out, cud
     if constexpr (f32) {
         unsigned long long* recs = (unsigned long long*)partial;
         if (errs_out) {
+            // (with the static stages above the 48 KB that need no leave)
+            const cudaError_t e = cudaFuncSetAttribute((const void*)k_gr_write32<true>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kErrSmemGR);
+            if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute");
             PRODM_CHAIN("k_gr_write32", k_gr_write32<true>, grid, block, kErrSmemGR, st, set, B, recs);
             ChunkSeg one = {};
             one.n = set.seg[0].n;
@@ -1352,7 +1455,10 @@ int launch_gr_encode(GrSet<T> set, int B, double* partial, double* errs_out, cud
             PRODM_CHAIN("k_gr_write32", k_gr_write32<false>, grid, block, 0, st, set, B, (unsigned long long*)nullptr);
         }
     } else {
-        PRODM_CHAIN("k_gr_write64", k_gr_write64, grid, block, 0, st, set, B);
+        const cudaError_t e = cudaFuncSetAttribute((const void*)k_gr_write64, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)kGrStage64);
+        if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute");
+        PRODM_CHAIN("k_gr_write64", k_gr_write64, grid, block, kGrStage64, st, set, B);
     }
     return PRODM_OK;
 }
