@@ -8,10 +8,16 @@
 // Estimates (qoi_utils.hpp:18-98): |V_TOT~ - V_TOT| <= sqrt-rule(V^2,
 // sum_f square-rule(V_f, eb_f)) as halving_Vtot.cpp:38-45 forms it, and
 // |T~ - T| <= division-rule(P, D, eb_P, eb_D) / R (0 where the rule gives no
-// bound, as the reference does). One thread per point, streaming; the
+// bound, as the reference does). The FP64 pipe bounds both kernels, and three
+// quarters of its work were four divisions and four roots a point (values; two
+// and two for the estimates): they are made of integer operations (exact64.cuh)
+// with the same bits, comparisons too. 257^3 points: values 2574 -> 704 us
+// (FP64 floor of the 18 operations left 523, DRAM 224), estimates 1951 -> 929
+// us. One thread per point, streaming; the
 // maxima over the field are reduced with 64-bit atomicMax on the (non-
 // negative) doubles' bit patterns.
 #include "common.cuh"
+#include "exact64.cuh"
 #include "kernels.cuh"
 
 namespace prodm {
@@ -21,20 +27,21 @@ struct Ge {
     static constexpr double R = 287.1, gamma = 1.4, mu_r = 1.716e-5, T_r = 273.15, S = 110.4;
 };
 
-// uncontracted, operation by operation as the host evaluates the rules
-__device__ __forceinline__ double bx2(double x, double eb) {
-    return __dadd_rn(__dmul_rn(__dmul_rn(2.0, fabs(x)), eb), __dmul_rn(eb, eb));
+// uncontracted, operation by operation as the host evaluates the rules; eb2 = eb * eb
+__device__ __forceinline__ double bx2(double x, double eb, double eb2) {
+    return __dadd_rn(__dmul_rn(twice_abs(x), eb), eb2);
 }
-__device__ __forceinline__ double bsqrt(double x, double eb) {
-    if (x == 0) return sqrt(eb);
-    if (x > eb) return eb / __dadd_rn(sqrt(__dsub_rn(x, eb)), sqrt(x));
-    return eb / sqrt(x);
+__device__ __forceinline__ double bsqrt(double x, double eb) {   // x, eb >= +0 or NaN
+    const bool zero = bits64(x) == 0;
+    double r = sqrt_exact(zero ? eb : x);
+    if (zero) return r;
+    if (above(x, eb)) r = __dadd_rn(sqrt_exact(__dsub_rn(x, eb)), r);
+    return div_exact(eb, r);
 }
-__device__ __forceinline__ double bdiv(double x, double y, double ebx, double eby) {
-    if (eby < fabs(y)) {
-        const double e = __dadd_rn(__dmul_rn(fabs(x), eby), __dmul_rn(fabs(y), ebx));
-        return y > 0 ? e / __dmul_rn(y, __dsub_rn(y, eby)) : e / __dmul_rn(y, __dadd_rn(y, eby));
-    }
+__device__ __forceinline__ double bdiv(double x, double y, double ebx, double eby) {   // eby >= +0 or NaN
+    const double ay = fabs(y);
+    if (above(ay, eby))   // (y (y - eby), or for y < 0 y (y + eby))
+        return div_exact(__dadd_rn(__dmul_rn(fabs(x), eby), __dmul_rn(ay, ebx)), __dmul_rn(ay, __dsub_rn(ay, eby)));
     return 0;
 }
 
@@ -45,18 +52,18 @@ __global__ void k_qoi_values(const double* __restrict__ vx, const double* __rest
                              double* __restrict__ pt, double* __restrict__ mu) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const double v2 = __dadd_rn(__dadd_rn(__dmul_rn(vx[i], vx[i]), __dmul_rn(vy[i], vy[i])), __dmul_rn(vz[i], vz[i]));
-        const double v = sqrt(v2);
-        const double t = p[i] / __dmul_rn(d[i], Ge::R);
-        const double c = sqrt(__dmul_rn(__dmul_rn(Ge::gamma, Ge::R), t));
-        const double m = v / c;
+        const double v = sqrt_exact(v2);
+        const double t = div_exact(p[i], __dmul_rn(d[i], Ge::R));
+        const double c = sqrt_exact(__dmul_rn(__dmul_rn(Ge::gamma, Ge::R), t));
+        const double m = div_exact(v, c);
         const double mt = __dadd_rn(1.0, __dmul_rn(__dmul_rn((Ge::gamma - 1) / 2, m), m));
         // x^7 and x^3 by multiplication chains instead of pow (GB300's FP64
         // pipe is slow; the chains stay within a few units in the last place)
         const double mt2 = __dmul_rn(mt, mt), mt4 = __dmul_rn(mt2, mt2);
-        const double ptv = __dmul_rn(p[i], sqrt(__dmul_rn(__dmul_rn(mt4, mt2), mt)));
-        const double trs = (Ge::T_r + Ge::S) / __dadd_rn(t, Ge::S);
-        const double tr = t / Ge::T_r;
-        const double tt3 = sqrt(__dmul_rn(__dmul_rn(tr, tr), tr));
+        const double ptv = __dmul_rn(p[i], sqrt_exact(__dmul_rn(__dmul_rn(mt4, mt2), mt)));
+        const double trs = div_exact(Ge::T_r + Ge::S, __dadd_rn(t, Ge::S));
+        const double tr = div_exact(t, Ge::T_r);
+        const double tt3 = sqrt_exact(__dmul_rn(__dmul_rn(tr, tr), tr));
         vtot[i] = v;
         temp[i] = t;
         cs[i] = c;
@@ -75,26 +82,29 @@ __global__ void k_qoi_bounds(const double* __restrict__ vx, const double* __rest
                              const double* __restrict__ d, uint64_t n, double ebx, double eby, double ebz, double ebp,
                              double ebd, double* __restrict__ bv, double* __restrict__ bt, double* __restrict__ mx) {
     double mv = 0, mt = 0;
+    ebd += 0.0;   // (-0 to +0)
+    const double ebx2 = __dmul_rn(ebx, ebx), eby2 = __dmul_rn(eby, eby), ebz2 = __dmul_rn(ebz, ebz);
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         if (vx) {
-            const double e2 = __dadd_rn(__dadd_rn(bx2(vx[i], ebx), bx2(vy[i], eby)), bx2(vz[i], ebz));
-            const double v2 =
-                __dadd_rn(__dadd_rn(__dmul_rn(vx[i], vx[i]), __dmul_rn(vy[i], vy[i])), __dmul_rn(vz[i], vz[i]));
+            const double x = vx[i], y = vy[i], z = vz[i];
+            const double e2 = __dadd_rn(__dadd_rn(bx2(x, ebx, ebx2), bx2(y, eby, eby2)), bx2(z, ebz, ebz2));
+            const double v2 = __dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z));
             const double e = bsqrt(v2, e2);
             if (bv) bv[i] = e;
-            mv = e > mv ? e : mv;
+            mv = above(e, mv) ? e : mv;
         }
         if (p) {
             const double e = __dmul_rn(1.0 / Ge::R, bdiv(p[i], d[i], ebp, ebd));
             if (bt) bt[i] = e;
-            mt = e > mt ? e : mt;
+            mt = above(e, mt) ? e : mt;
         }
     }
     if (mx) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
-            mv = fmax(mv, __shfl_xor_sync(0xffffffffu, mv, o));
-            mt = fmax(mt, __shfl_xor_sync(0xffffffffu, mt, o));
+            const double ov = __shfl_xor_sync(0xffffffffu, mv, o), ot = __shfl_xor_sync(0xffffffffu, mt, o);
+            mv = above(ov, mv) ? ov : mv;
+            mt = above(ot, mt) ? ot : mt;
         }
         if ((threadIdx.x & 31) == 0) {
             atomic_max_nonneg(mx, mv);
