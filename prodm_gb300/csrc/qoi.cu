@@ -11,9 +11,12 @@
 // bound, as the reference does). The FP64 pipe bounds both kernels, and three
 // quarters of its work were four divisions and four roots a point (values; two
 // and two for the estimates): they are made of integer operations (exact64.cuh)
-// with the same bits, comparisons too. 257^3 points: values 2574 -> 704 us
-// (FP64 floor of the 18 operations left 523, DRAM 224), estimates 1951 -> 929
-// us. One thread per point, streaming; the
+// with the same bits, comparisons too, and so are as many products as balance
+// the two kinds of pipe: three of the values' fourteen, six of the estimates'
+// ten. 257^3 points: values 2574 -> 704 us, 633 with the products (three more
+// 681, six more 740), estimates 1951 -> 840, 656 with them (none of them 840,
+// three 747, nine 649); DRAM floor 224 and 143 us. One thread per point,
+// streaming; the
 // maxima over the field are reduced with 64-bit atomicMax on the (non-
 // negative) doubles' bit patterns.
 #include "common.cuh"
@@ -29,7 +32,7 @@ struct Ge {
 
 // uncontracted, operation by operation as the host evaluates the rules; eb2 = eb * eb
 __device__ __forceinline__ double bx2(double x, double eb, double eb2) {
-    return __dadd_rn(__dmul_rn(twice_abs(x), eb), eb2);
+    return __dadd_rn(mul_exact(twice_abs(x), eb), eb2);
 }
 __device__ __forceinline__ double bsqrt(double x, double eb) {   // x, eb >= +0 or NaN
     const bool zero = bits64(x) == 0;
@@ -53,14 +56,14 @@ __global__ void k_qoi_values(const double* __restrict__ vx, const double* __rest
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const double v2 = __dadd_rn(__dadd_rn(__dmul_rn(vx[i], vx[i]), __dmul_rn(vy[i], vy[i])), __dmul_rn(vz[i], vz[i]));
         const double v = sqrt_exact(v2);
-        const double t = div_exact(p[i], __dmul_rn(d[i], Ge::R));
-        const double c = sqrt_exact(__dmul_rn(__dmul_rn(Ge::gamma, Ge::R), t));
+        const double t = div_exact(p[i], mul_exact(d[i], Ge::R));
+        const double c = sqrt_exact(mul_exact(__dmul_rn(Ge::gamma, Ge::R), t));
         const double m = div_exact(v, c);
         const double mt = __dadd_rn(1.0, __dmul_rn(__dmul_rn((Ge::gamma - 1) / 2, m), m));
         // x^7 and x^3 by multiplication chains instead of pow (GB300's FP64
         // pipe is slow; the chains stay within a few units in the last place)
         const double mt2 = __dmul_rn(mt, mt), mt4 = __dmul_rn(mt2, mt2);
-        const double ptv = __dmul_rn(p[i], sqrt_exact(__dmul_rn(__dmul_rn(mt4, mt2), mt)));
+        const double ptv = mul_exact(p[i], sqrt_exact(__dmul_rn(__dmul_rn(mt4, mt2), mt)));
         const double trs = div_exact(Ge::T_r + Ge::S, __dadd_rn(t, Ge::S));
         const double tr = div_exact(t, Ge::T_r);
         const double tt3 = sqrt_exact(__dmul_rn(__dmul_rn(tr, tr), tr));
@@ -88,7 +91,7 @@ __global__ void k_qoi_bounds(const double* __restrict__ vx, const double* __rest
         if (vx) {
             const double x = vx[i], y = vy[i], z = vz[i];
             const double e2 = __dadd_rn(__dadd_rn(bx2(x, ebx, ebx2), bx2(y, eby, eby2)), bx2(z, ebz, ebz2));
-            const double v2 = __dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z));
+            const double v2 = __dadd_rn(__dadd_rn(mul_exact(x, x), mul_exact(y, y)), mul_exact(z, z));
             const double e = bsqrt(v2, e2);
             if (bv) bv[i] = e;
             mv = above(e, mv) ? e : mv;
