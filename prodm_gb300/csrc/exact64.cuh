@@ -135,4 +135,12 @@ __device__ __forceinline__ double twice_abs(double x) {
     return mul_fp64(2.0, __longlong_as_double((long long)u));
 }
 
+// x / 2
+__device__ __forceinline__ double half_of(double x) {
+    const uint64_t u = bits64(x);
+    if (((uint32_t)(u >> 52) & 0x7ff) - 2 < 2045u) return __longlong_as_double((long long)(u - (1ull << 52)));
+    return (u << 1) == 0 ? x : mul_fp64(0.5, x);
+}
+__device__ __forceinline__ float half_of(float x) { return 0.5f * x; }
+
 }  // namespace prodm

@@ -21,6 +21,7 @@
 #include <cstdlib>
 
 #include "common.cuh"
+#include "exact64.cuh"
 #include "kernels.cuh"
 #include "rows.cuh"
 
@@ -306,12 +307,14 @@ __global__ void k_reordered_to_natural(const T* __restrict__ rin, Box F, Box C, 
 // c-2 .. c+2. For double data an interior node takes the same sum regrouped as
 // one 5-point stencil, 5/6 s[c] + 1/2 (s[c-1] + s[c+1]) + 1/12 (s[c-2] + s[c+2]),
 // a third of the FP64 operations; float keeps the term order above.
-template <class W, bool INTERIOR = false>   // INTERIOR: the caller knows that c is an even position in [2, nf - 3]
+// INTERIOR: the caller knows that c is an even position in [2, nf - 3]. HALVE:
+// halve by the exponent instead of an FP64 operation.
+template <class W, bool INTERIOR = false, bool HALVE = false>
 __device__ __forceinline__ W l2_rhs(W sm2, W sm1, W s0, W s1, W s2, uint32_t c, uint32_t nf) {
     // fused multiply-adds are written out: which product of a sum the compiler
     // fuses depends on the code around it
     if (sizeof(W) == 8 && (INTERIOR || (c >= 2 && c + 3 <= nf && (c & 1u) == 0)))
-        return fma((W)(1.0 / 12.0), sm2 + s2, fma((W)(5.0 / 6.0), s0, (W)0.5 * (sm1 + s1)));
+        return fma((W)(1.0 / 12.0), sm2 + s2, fma((W)(5.0 / 6.0), s0, HALVE ? half_of(sm1 + s1) : (W)0.5 * (sm1 + s1)));
     auto mf = [&](W l, W x, W r, uint32_t pos) {
         const W dg = (!INTERIOR && (pos == 0 || pos == nf - 1)) ? (W)1 / 3 : (W)2 / 3;
         return fma(dg, x, (l + r) / 6);
@@ -332,7 +335,8 @@ __device__ __forceinline__ W l2_rhs(W sm2, W sm1, W s0, W s1, W s2, uint32_t c, 
 // are issued kLineAhead nodes ahead in both sweeps: with one node ahead, and
 // none in the backward sweep, the dim-1 and dim-0 passes of 513 x 513 x 257
 // took 414 and 260 us, with four and eight and the right-hand sides of four
-// nodes ahead of their chain 325 and 168 us (FP64 floor 216 and 108 us).
+// nodes ahead of their chain 325 and 168 us, 272 and 150 with the halving of
+// the right-hand side done on the exponent (FP64 floor 216 and 108 us).
 constexpr int kLineAhead = 4, kLineBack = 8;
 template <class T, class W>
 __global__ void __launch_bounds__(128) k_l2_line(const T* __restrict__ src, Box S, int d, T* dst, Box D,
@@ -375,7 +379,7 @@ __global__ void __launch_bounds__(128) k_l2_line(const T* __restrict__ src, Box 
                 for (int u = 0; u < kLineAhead; u++) {
                     lo[u] = lo_w[m0 + u];
                     inv[u] = inv_den[m0 + u];
-                    b[u] = l2_rhs<W, true>(w[2 * u], w[2 * u + 1], w[2 * u + 2], w[2 * u + 3], w[2 * u + 4], 2 * (m0 + u), nf);
+                    b[u] = l2_rhs<W, true, true>(w[2 * u], w[2 * u + 1], w[2 * u + 2], w[2 * u + 3], w[2 * u + 4], 2 * (m0 + u), nf);
                 }
 #pragma unroll
                 for (int u = 0; u < kLineAhead; u++) {
@@ -428,22 +432,25 @@ __global__ void __launch_bounds__(128) k_l2_line(const T* __restrict__ src, Box 
 // The dim-2 (contiguous) pass of the L2 projection, one warp per 32 rows of F
 // and lane r on row r. The FP64 pipe bounds it (eight operations a node, 431 us
 // at 513 x 513 x 257), as long as the loads do not hold its warps up: a ring of
-// four tiles of 8 coarse nodes (of a row in packed coefficients the even and
+// tiles of 8 coarse nodes (of a row in packed coefficients the even and
 // the odd values are two contiguous runs, of a natural row one) is filled by
 // cp.async while earlier tiles are swept. A tile's values and Thomas factors
 // are read first, then its eight right-hand sides, which do not depend on each
 // other, then the chain of the forward step. d' leaves through the tile's slot
 // in runs of 8 and comes back the same way, from the end, for the backward
-// sweep (17 KB a warp), or stays in shared memory (KEPT: 17 KB and the 32
-// rows), and the rows leave as one run. 513 x 513 x 257 fp64: 609 us; 955 us
-// with 16-column tiles loaded, swept and stored in turn.
+// sweep, or stays in shared memory (KEPT), and the rows leave as one run. More
+// warps an SM count for more than a deeper ring (4.4 KB a tile): 513 x 513 x 257
+// fp64 585 us with two tiles, 601 with three, 612 with four (955 us with
+// 16-column tiles loaded, swept and stored in turn); KEPT 257 x 257 x 129 95 us
+// with three, 103 with two, 115 with four.
 // PACKED: the rows are read straight from the level's packed coefficients
 // (coarse nodes of rows inside the coarse box are zero), so no natural-order
 // copy is needed; else from a natural field.
-constexpr int kRowsRing = 4, kRowsTile = 8, kRowsLd = 2 * kRowsTile + 1;
+constexpr int kRowsTile = 8, kRowsLd = 2 * kRowsTile + 1;
+constexpr int l2_ring(bool kept) { return kept ? 3 : 2; }   // tiles
 template <class T>
 inline size_t l2_rows_smem(uint32_t nc, bool kept) {
-    return ((size_t)(kept ? 32 * (nc | 1u) : 0) + (size_t)kRowsRing * 32 * kRowsLd) * sizeof(T);
+    return ((size_t)(kept ? 32 * (nc | 1u) : 0) + (size_t)l2_ring(kept) * 32 * kRowsLd) * sizeof(T);
 }
 template <class T>
 __device__ __forceinline__ void cp_async_value(T* dst, const T* src, bool on) {   // zero when off
@@ -463,6 +470,7 @@ __global__ void __launch_bounds__(32) k_l2_rows(const T* __restrict__ src, Box F
                                                 const T* __restrict__ cp, const T* __restrict__ lo_w,
                                                 const T* __restrict__ inv_den) {
     extern __shared__ __align__(16) unsigned char l2_smem[];
+    constexpr int kRowsRing = l2_ring(KEPT);
     const int lane = threadIdx.x, col = lane & 7;
     const uint32_t nf = F.n[2], nc = coarse_len(nf), P = nf - nc;
     const uint32_t ld = nc | 1u;
