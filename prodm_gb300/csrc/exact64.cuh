@@ -124,7 +124,7 @@ __device__ __forceinline__ double mul_exact(double a, double b) {
 }
 
 constexpr uint64_t kInfBits = 0x7ff0000000000000ull;
-__device__ __forceinline__ uint64_t bits64(double x) { return (uint64_t)__double_as_longlong(x); }
+__device__ __forceinline__ unsigned long long bits64(double x) { return (unsigned long long)__double_as_longlong(x); }
 // a > b for a, b that are +0, positive or NaN (a comparison of doubles is an
 // FP64 operation too)
 __device__ __forceinline__ bool above(double a, double b) { return bits64(a) > bits64(b) && bits64(a) <= kInfBits; }
@@ -134,13 +134,5 @@ __device__ __forceinline__ double twice_abs(double x) {
     if ((uint32_t)(u >> 52) - 1 < 2045u) return __longlong_as_double((long long)(u + (1ull << 52)));
     return mul_fp64(2.0, __longlong_as_double((long long)u));
 }
-
-// x / 2
-__device__ __forceinline__ double half_of(double x) {
-    const uint64_t u = bits64(x);
-    if (((uint32_t)(u >> 52) & 0x7ff) - 2 < 2045u) return __longlong_as_double((long long)(u - (1ull << 52)));
-    return (u << 1) == 0 ? x : mul_fp64(0.5, x);
-}
-__device__ __forceinline__ float half_of(float x) { return 0.5f * x; }
 
 }  // namespace prodm

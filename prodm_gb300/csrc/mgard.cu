@@ -21,7 +21,6 @@
 #include <cstdlib>
 
 #include "common.cuh"
-#include "exact64.cuh"
 #include "kernels.cuh"
 #include "rows.cuh"
 
@@ -55,7 +54,7 @@ __device__ __forceinline__ K warp_max(K v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         K w = __shfl_xor_sync(0xffffffffu, v, o);
-        v = w > v ? w : v;
+        v = max_key(w, v);
     }
     return v;
 }
@@ -89,7 +88,7 @@ __global__ void k_decompose_level(const T* __restrict__ in, uint64_t s0, uint64_
             else coef[r0 * o0 + r1 * o1 + r2] = v;
             if (fnat) fnat[idx] = (T)0;
             K k = abs_key(v);
-            mc = k > mc ? k : mc;
+            mc = max_key(k, mc);
         } else {
             auto at = [&](int d0, int d1, int d2) -> T { return __ldg(p + (int64_t)d0 * (int64_t)s0 + (int64_t)d1 * (int64_t)s1 + d2); };
             T c = sub_rn(v, interp<T>(mask, at));
@@ -97,7 +96,7 @@ __global__ void k_decompose_level(const T* __restrict__ in, uint64_t s0, uint64_
             else coef[r0 * o0 + r1 * o1 + r2] = c;
             if (fnat) fnat[idx] = c;
             K k = abs_key(c);
-            mk = k > mk ? k : mk;
+            mk = max_key(k, mk);
         }
     }
     if (maxkey_level) {
@@ -314,7 +313,7 @@ __device__ __forceinline__ W l2_rhs(W sm2, W sm1, W s0, W s1, W s2, uint32_t c, 
     // fused multiply-adds are written out: which product of a sum the compiler
     // fuses depends on the code around it
     if (sizeof(W) == 8 && (INTERIOR || (c >= 2 && c + 3 <= nf && (c & 1u) == 0)))
-        return fma((W)(1.0 / 12.0), sm2 + s2, fma((W)(5.0 / 6.0), s0, HALVE ? half_of(sm1 + s1) : (W)0.5 * (sm1 + s1)));
+        return fma((W)(1.0 / 12.0), sm2 + s2, fma((W)(5.0 / 6.0), s0, HALVE ? (W)half_rn(sm1 + s1) : (W)0.5 * (sm1 + s1)));
     auto mf = [&](W l, W x, W r, uint32_t pos) {
         const W dg = (!INTERIOR && (pos == 0 || pos == nf - 1)) ? (W)1 / 3 : (W)2 / 3;
         return fma(dg, x, (l + r) / 6);

@@ -72,12 +72,12 @@ __global__ void k_maxabs(const T* __restrict__ x, uint64_t n, typename KeyOf<T>:
     K m = 0;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         K k = abs_key(x[i]);
-        m = k > m ? k : m;
+        m = max_key(k, m);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         K w = __shfl_xor_sync(0xffffffffu, m, o);
-        m = w > m ? w : m;
+        m = max_key(w, m);
     }
     if ((threadIdx.x & 31) == 0 && m) atomicMax(key, m);
 }

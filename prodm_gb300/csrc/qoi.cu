@@ -80,6 +80,11 @@ __device__ __forceinline__ void atomic_max_nonneg(double* addr, double v) {
     atomicMax(reinterpret_cast<unsigned long long*>(addr), (unsigned long long)__double_as_longlong(v));
 }
 
+// the larger of e and m, m where e is NaN; both >= +0 otherwise
+__device__ __forceinline__ double max_of(double e, double m) {
+    return bits64(e) <= kInfBits ? __longlong_as_double((long long)max_key(bits64(e), bits64(m))) : m;
+}
+
 __global__ void k_qoi_bounds(const double* __restrict__ vx, const double* __restrict__ vy,
                              const double* __restrict__ vz, const double* __restrict__ p,
                              const double* __restrict__ d, uint64_t n, double ebx, double eby, double ebz, double ebp,
@@ -94,20 +99,20 @@ __global__ void k_qoi_bounds(const double* __restrict__ vx, const double* __rest
             const double v2 = __dadd_rn(__dadd_rn(mul_exact(x, x), mul_exact(y, y)), mul_exact(z, z));
             const double e = bsqrt(v2, e2);
             if (bv) bv[i] = e;
-            mv = above(e, mv) ? e : mv;
+            mv = max_of(e, mv);
         }
         if (p) {
             const double e = __dmul_rn(1.0 / Ge::R, bdiv(p[i], d[i], ebp, ebd));
             if (bt) bt[i] = e;
-            mt = above(e, mt) ? e : mt;
+            mt = max_of(e, mt);
         }
     }
     if (mx) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             const double ov = __shfl_xor_sync(0xffffffffu, mv, o), ot = __shfl_xor_sync(0xffffffffu, mt, o);
-            mv = above(ov, mv) ? ov : mv;
-            mt = above(ot, mt) ? ot : mt;
+            mv = max_of(ov, mv);
+            mt = max_of(ot, mt);
         }
         if ((threadIdx.x & 31) == 0) {
             atomic_max_nonneg(mx, mv);

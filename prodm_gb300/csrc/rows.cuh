@@ -11,7 +11,7 @@ __device__ __forceinline__ K warp_max_key(K v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         K w = __shfl_xor_sync(0xffffffffu, v, o);
-        v = w > v ? w : v;
+        v = max_key(w, v);
     }
     return v;
 }
@@ -87,20 +87,20 @@ __device__ __forceinline__ void decompose_row(const T* __restrict__ p, uint64_t 
                     crow[c2] = g.ve;
                     if (frow) frow[xe] = (T)0;
                     K kk = abs_key(g.ve);
-                    mc = kk > mc ? kk : mc;
+                    mc = max_key(kk, mc);
                 } else {
                     T c = sub_rn(g.ve, corner_tree(M01, g.q));
                     coef[rb_even + c2] = c;
                     if (frow) frow[xe] = c;
                     K kk = abs_key(c);
-                    mk = kk > mk ? kk : mk;
+                    mk = max_key(kk, mk);
                 }
                 if (c2 < P) {
                     T c = sub_rn(g.vo, corner_tree_mid(M01, g.q, qn));
                     coef[rb_odd + c2] = c;
                     if (frow) frow[xe + 1] = c;
                     K kk = abs_key(c);
-                    mk = kk > mk ? kk : mk;
+                    mk = max_key(kk, mk);
                 }
             }
             load(k + D, ring[d]);
@@ -185,7 +185,7 @@ __device__ __forceinline__ void decompose_patch_item(const T* __restrict__ in, u
     auto x1_of = [&](uint32_t b) { return (uint64_t)min(2 * b, F.n[1] - 1); };
     const uint32_t b0 = u * kPatchSteps, b1 = min(b0 + kPatchSteps, C1);
     const T* base = in + (uint64_t)min(2 * i, F.n[0] - 1) * s0;
-    auto kmax = [](K& m, T v) { const K k = abs_key(v); m = k > m ? k : m; };
+    auto kmax = [](K& m, T v) { m = max_key(abs_key(v), m); };
     // the loads of one step, issued a step ahead of their use: the four
     // rows' node pairs, the corner values of rows 2b + 2 at column c and (lane
     // 31) at column c + 1, and the last node's even values
