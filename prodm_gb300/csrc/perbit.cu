@@ -234,12 +234,20 @@ __global__ void __launch_bounds__(256) k_pb_decode(const __grid_constant__ PbSet
 
 // ---------------------------------------------------------------------------
 // export: rows -> reference streams (BitEncoder layout), three passes
-//   count: bits of every (plane, 256-group chunk)
+//   count: bits of every (plane, 256-group chunk), and before each of its warps
 //   scan:  chunk bit offsets within each plane
 //   write: each group's segment of each plane (<= 64 bits) OR-ed into the
 //          zeroed destination
+// A thread walks the planes of its group (an element's sign follows its first 1
+// bit). The planes' words do not depend on each other, so PK_U are loaded at a
+// time and the next ones while these are worked on, and a warp knows its place
+// in every plane beforehand, so the warps of a chunk do not wait for one
+// another. 2^20 values, 60 planes: count 40 us and write 90 us with a load and
+// two barriers a plane, 13 and 40 us so.
 // ---------------------------------------------------------------------------
 constexpr int PK_T = 256;   // groups (threads) per chunk
+constexpr int PK_W = PK_T / 32;
+constexpr int PK_U = 10;    // planes loaded ahead
 
 __device__ __forceinline__ int pk_nvalid(uint64_t g, uint64_t ng, uint64_t n) {
     if (g >= ng) return 0;
@@ -247,36 +255,63 @@ __device__ __forceinline__ int pk_nvalid(uint64_t g, uint64_t ng, uint64_t n) {
     return r < 32 ? (int)r : 32;
 }
 
+// body(p, M) for the planes p in order, M the valid elements' bits
+template <class Body>
+__device__ __forceinline__ void pk_planes(const uint32_t* __restrict__ rows, uint64_t stride, uint64_t g, uint32_t vm, int B,
+                                          Body body) {
+    uint32_t nx[PK_U];
+    auto load = [&](int p0) {
+#pragma unroll
+        for (int u = 0; u < PK_U; u++) nx[u] = vm && p0 + u < B ? __ldg(rows + (uint64_t)(p0 + u) * stride + g) & vm : 0u;
+    };
+    load(0);
+    for (int p0 = 0; p0 < B; p0 += PK_U) {
+        uint32_t m[PK_U];
+#pragma unroll
+        for (int u = 0; u < PK_U; u++) m[u] = nx[u];
+        load(p0 + PK_U);
+#pragma unroll
+        for (int u = 0; u < PK_U; u++)
+            if (p0 + u < B) body(p0 + u, m[u]);
+    }
+}
+
+// warp_bits: the bits of a chunk's warps before each of them, [plane][chunk][PK_W]
 __global__ void __launch_bounds__(PK_T) k_pb_pack_count(const uint32_t* __restrict__ rows, uint64_t stride, uint64_t n,
-                                                        int B, uint32_t* __restrict__ chunk_bits, uint64_t nch) {
-    __shared__ uint32_t red[64];
-    const int lane = threadIdx.x & 31;
-    for (int k = threadIdx.x; k < 64; k += blockDim.x) red[k] = 0;
-    __syncthreads();
+                                                        int B, uint32_t* __restrict__ chunk_bits, uint64_t nch,
+                                                        uint16_t* __restrict__ warp_bits) {
+    __shared__ uint32_t cnt[PK_W][64];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t ng = (n + 31) / 32;
     const uint64_t g = (uint64_t)blockIdx.x * PK_T + threadIdx.x;
     const int nvalid = pk_nvalid(g, ng, n);
-    const uint32_t vm = valid_mask(nvalid);
     uint32_t seen = 0;
-    for (int p = 0; p < B; p++) {
-        const uint32_t M = nvalid ? rows[(uint64_t)p * stride + g] & vm : 0u;
-        const uint32_t F = M & ~seen;
+    pk_planes(rows, stride, g, valid_mask(nvalid), B, [&](int p, uint32_t M) {
+        const uint32_t bits = __reduce_add_sync(FULL, (uint32_t)(nvalid + __popc(M & ~seen)));
         seen |= M;
-        uint32_t bits = nvalid + __popc(F);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) bits += __shfl_xor_sync(FULL, bits, o);
-        if (lane == 0 && bits) atomicAdd(&red[p], bits);
-    }
+        if (lane == 0) cnt[warp][p] = bits;
+    });
     __syncthreads();
-    for (int p = threadIdx.x; p < B; p += blockDim.x) chunk_bits[(uint64_t)p * nch + blockIdx.x] = red[p];
+    for (int p = threadIdx.x; p < B; p += blockDim.x) {
+        const uint64_t at = (uint64_t)p * nch + blockIdx.x;
+        uint32_t run = 0;
+        for (int w = 0; w < PK_W; w++) {
+            warp_bits[at * PK_W + w] = (uint16_t)run;   // at most 7 x 32 x 64
+            run += cnt[w][p];
+        }
+        chunk_bits[at] = run;
+    }
 }
 
-__global__ void k_pb_pack_scan(const uint32_t* __restrict__ chunk_bits, uint64_t nch, uint64_t* __restrict__ chunk_off) {
-    const int lane = threadIdx.x;
+// exclusive scan of one plane's (blockIdx.x) chunk bits
+__global__ void __launch_bounds__(256) k_pb_pack_scan(const uint32_t* __restrict__ chunk_bits, uint64_t nch,
+                                                      uint64_t* __restrict__ chunk_off) {
+    __shared__ uint64_t wsum[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t base = (uint64_t)blockIdx.x * nch;
     uint64_t run = 0;
-    for (uint64_t c0 = 0; c0 < nch; c0 += 32) {
-        const uint64_t c = c0 + lane;
+    for (uint64_t c0 = 0; c0 < nch; c0 += 256) {
+        const uint64_t c = c0 + threadIdx.x;
         const uint64_t v = c < nch ? chunk_bits[base + c] : 0;
         uint64_t inc = v;
 #pragma unroll
@@ -284,8 +319,16 @@ __global__ void k_pb_pack_scan(const uint32_t* __restrict__ chunk_bits, uint64_t
             const uint64_t t = __shfl_up_sync(FULL, inc, o);
             if (lane >= o) inc += t;
         }
+        if (lane == 31) wsum[warp] = inc;
+        __syncthreads();
+        uint64_t all = 0;
+        for (int w = 0; w < 8; w++) {
+            if (w == warp) inc += all;
+            all += wsum[w];
+        }
         if (c < nch) chunk_off[base + c] = run + inc - v;
-        run += __shfl_sync(FULL, inc, 31);
+        run += all;
+        __syncthreads();
     }
 }
 
@@ -307,47 +350,56 @@ __device__ __forceinline__ uint64_t pb_segment(uint32_t M, uint32_t F, uint32_t 
 __global__ void __launch_bounds__(PK_T) k_pb_pack_write(const uint32_t* __restrict__ rows, uint64_t stride, uint64_t n,
                                                         int B, const uint32_t* __restrict__ srow,
                                                         const uint64_t* __restrict__ chunk_off, uint64_t nch,
+                                                        const uint16_t* __restrict__ warp_bits,
                                                         const uint32_t* __restrict__ sizes,
                                                         unsigned long long* __restrict__ dst) {
-    __shared__ uint64_t base[64];
-    __shared__ uint32_t wsum[PK_T / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) {
-        uint64_t a = 0;
-        for (int p = 0; p < B; p++) { base[p] = a * 8; a += sizes[p]; }
-    }
-    __syncthreads();
     const uint64_t ng = (n + 31) / 32;
     const uint64_t g = (uint64_t)blockIdx.x * PK_T + threadIdx.x;
     const int nvalid = pk_nvalid(g, ng, n);
-    const uint32_t vm = valid_mask(nvalid);
     const uint32_t S = nvalid ? srow[g] : 0u;
+    // lane p: the warp's first bit in planes p and p + 32
+    uint64_t off[2];
+    {
+        uint64_t run = 0;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int p = lane + 32 * h;
+            const uint64_t bits = p < B ? (uint64_t)sizes[p] * 8 : 0, at = (uint64_t)p * nch + blockIdx.x;
+            uint64_t inc = bits;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint64_t t = __shfl_up_sync(FULL, inc, o);
+                if (lane >= o) inc += t;
+            }
+            off[h] = p < B ? run + inc - bits + chunk_off[at] + warp_bits[at * PK_W + warp] : 0;
+            run += __shfl_sync(FULL, inc, 31);
+        }
+    }
     uint32_t seen = 0;
-    for (int p = 0; p < B; p++) {
-        const uint32_t M = nvalid ? rows[(uint64_t)p * stride + g] & vm : 0u;
+    pk_planes(rows, stride, g, valid_mask(nvalid), B, [&](int p, uint32_t M) {
         const uint32_t F = M & ~seen;
         seen |= M;
         const uint32_t len = nvalid + __popc(F);
         uint32_t inc = len;
+        if (__all_sync(FULL, len == 32)) {   // no signs in the warp
+            inc = 32 * (lane + 1);
+        } else {
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(FULL, inc, o);
-            if (lane >= o) inc += t;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(FULL, inc, o);
+                if (lane >= o) inc += t;
+            }
         }
-        if (lane == 31) wsum[warp] = inc;
-        __syncthreads();
-        uint32_t woff = 0;
-        for (int w = 0; w < warp; w++) woff += wsum[w];
-        __syncthreads();
+        const uint64_t at = __shfl_sync(FULL, p < 32 ? off[0] : off[1], p & 31) + inc - len;
         if (len) {
             const uint64_t seg = pb_segment(M, F, S);
-            const uint64_t off = base[p] + chunk_off[(uint64_t)p * nch + blockIdx.x] + woff + inc - len;
-            const uint64_t w = off >> 6;
-            const int sh = (int)(off & 63);
+            const uint64_t w = at >> 6;
+            const int sh = (int)(at & 63);
             atomicOr(dst + w, (unsigned long long)(seg << sh));
             if (sh && sh + (int)len > 64) atomicOr(dst + w + 1, (unsigned long long)(seg >> (64 - sh)));
         }
-    }
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -843,7 +895,7 @@ int launch_pb_decode(PbSet<T> set, int B, int s, int e, cudaStream_t st) {
 
 size_t pb_pack_scratch_bytes(uint64_t n, int B) {
     const uint64_t nch = (pb_groups(n) + PK_T - 1) / PK_T;
-    return ((size_t)B * nch * (4 + 8) + 511) / 256 * 256;   // a multiple of 256 bytes
+    return ((size_t)B * nch * (8 + 4 + 2 * PK_W) + 511) / 256 * 256;   // a multiple of 256 bytes
 }
 
 int launch_pb_pack(const uint32_t* rows, uint64_t stride, uint64_t n, int B, const uint32_t* sizes, uint64_t total,
@@ -852,14 +904,15 @@ int launch_pb_pack(const uint32_t* rows, uint64_t stride, uint64_t n, int B, con
     const uint64_t nch = (pb_groups(n) + PK_T - 1) / PK_T;
     uint64_t* chunk_off = (uint64_t*)scratch;
     uint32_t* chunk_bits = (uint32_t*)(chunk_off + (uint64_t)B * nch);
+    uint16_t* warp_bits = (uint16_t*)(chunk_bits + (uint64_t)B * nch);
     PRODM_CUDA(cudaMemsetAsync(dst, 0, total, st));
     if (nch == 0) return PRODM_OK;
-    k_pb_pack_count<<<(unsigned)nch, PK_T, 0, st>>>(rows, stride, n, B, chunk_bits, nch);
+    k_pb_pack_count<<<(unsigned)nch, PK_T, 0, st>>>(rows, stride, n, B, chunk_bits, nch, warp_bits);
     PRODM_CHECK_LAUNCH("k_pb_pack_count");
-    k_pb_pack_scan<<<B, 32, 0, st>>>(chunk_bits, nch, chunk_off);
+    k_pb_pack_scan<<<B, 256, 0, st>>>(chunk_bits, nch, chunk_off);
     PRODM_CHECK_LAUNCH("k_pb_pack_scan");
     k_pb_pack_write<<<(unsigned)nch, PK_T, 0, st>>>(rows, stride, n, B, rows + (uint64_t)B * stride, chunk_off, nch,
-                                                    sizes, (unsigned long long*)dst);
+                                                    warp_bits, sizes, (unsigned long long*)dst);
     PRODM_CHECK_LAUNCH("k_pb_pack_write");
     return PRODM_OK;
 }
