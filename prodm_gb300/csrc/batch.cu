@@ -113,20 +113,6 @@ __global__ void __launch_bounds__(256) k_recompose_multi(const RowSeg* __restric
     }
 }
 
-__global__ void __launch_bounds__(256) k_nb_encode_multi(const ChunkSeg* __restrict__ segs, int nseg, uint64_t total,
-                                                        int B) {
-    __shared__ uint32_t tile[32 * NB_TILE_LD];
-    for (uint64_t c = blockIdx.x; c < total; c += gridDim.x) {
-        const int s = find_seg(segs, nseg, c, &ChunkSeg::chunk_begin);
-        const ChunkSeg& q = segs[s];
-        const int exp = frexp_exp(__uint_as_float(*q.key)) + 2;     // NegaBinaryBPEncoder.hpp:21
-        const int se = B - exp;
-        const bool fast = pow2_normal(se);
-        nb_encode32_chunk(q.x, q.n, q.nblocks, B, se, fast, fast ? pow2f(se) : 1.f, q.words, q.stride,
-                          c - q.chunk_begin, tile);
-    }
-}
-
 // per (field, level) slot: bound = 4 |max| (negabinary) and the max-error
 // table (MaxErrorCollector.hpp:14-25)
 __global__ void k_bounds_tables_multi(const uint32_t* __restrict__ keys, const int* __restrict__ levels, int nf, int B,
@@ -418,8 +404,11 @@ int batch_refactor(prodm_batch* h, cudaStream_t st) {
                                                                                                  h->drows[d]);
         PRODM_CHECK_LAUNCH("k_decompose_multi");
     }
-    k_nb_encode_multi<<<persistent_grid(h, 1, h->echunks, 1), 256, 0, st>>>(h->eseg, h->en, h->echunks, h->B);
-    PRODM_CHECK_LAUNCH("k_nb_encode_multi");
+    // (no more CTAs than run at once: each walks its share of the chunks)
+    int rc = launch_nb_encode_segments(h->eseg, h->en, h->echunks, h->B,
+                                       std::min(persistent_grid(h, 1, h->echunks, 1), (unsigned)nb_encode_levels_grid(0)), st,
+                                       false);
+    if (rc) return rc;
     k_bounds_tables_multi<<<(h->nf * kMaxL + 127) / 128, 128, 0, st>>>(h->keys, h->levels_d, h->nf, h->B, h->bounds,
                                                                         h->maxerr);
     PRODM_CHECK_LAUNCH("k_bounds_tables_multi");

@@ -97,45 +97,52 @@ __device__ __forceinline__ void gr_errors(double (&acc)[NACC], double a, int B) 
 template <class T> struct Acc { using type = double; static constexpr int N = 33; };
 template <> struct Acc<double> { using type = double; static constexpr int N = 65; };
 
-// fp32 negabinary encoder without tables: grid-stride over NB_CHUNK-block chunks
-__global__ void __launch_bounds__(256) k_nb_encode32(const float* __restrict__ x, uint64_t n,
-                                                    const uint32_t* __restrict__ maxkey, int exp_arg, int B,
-                                                    uint32_t* __restrict__ out, uint64_t stride) {
-    __shared__ uint32_t tile[32 * NB_TILE_LD];
-    const int exp = (maxkey ? frexp_exp(__uint_as_float(*maxkey)) : exp_arg) + 2;   // NegaBinaryBPEncoder.hpp:21
-    const uint64_t nblocks = (n + 31) / 32;
-    const uint64_t nchunks = (nblocks + NB_CHUNK - 1) / NB_CHUNK;
-    const int se = B - exp;
-    const bool fast = pow2_normal(se);
-    const float scale = fast ? pow2f(se) : 1.f;
-    for (uint64_t c = blockIdx.x; c < nchunks; c += gridDim.x)
-        nb_encode32_chunk(x, n, nblocks, B, se, fast, scale, out, stride, c, tile);
+// fp32 negabinary encoder without tables
+__global__ void __launch_bounds__(256, 3) k_nb_encode32(const float* __restrict__ x, uint64_t n,
+                                                       const uint32_t* __restrict__ maxkey, int exp_arg, int B,
+                                                       uint32_t* __restrict__ out, uint64_t stride) {
+    __shared__ __align__(16) uint32_t stage[NB_STAGE];
+    NbSrc q;
+    q.x = x;
+    q.words = out;
+    q.n = n;
+    q.nblocks = (n + 31) / 32;
+    q.stride = stride;
+    q.se = B - ((maxkey ? frexp_exp(__uint_as_float(*maxkey)) : exp_arg) + 2);   // NegaBinaryBPEncoder.hpp:21
+    q.fast = pow2_normal(q.se);
+    q.scale = q.fast ? pow2f(q.se) : 1.f;
+    nb_encode32_chunks((q.nblocks + NB_CHUNK - 1) / NB_CHUNK, B, stage, [&](uint64_t c) {
+        q.chunk = c;
+        return q;
+    });
 }
 
-// Every level of one fp32 field in one launch, without tables: segments are
-// the levels in chunk order.
+// Every level of one fp32 field (or of many) in one launch, without tables:
+// segments are the levels in chunk order.
 __global__ void __launch_bounds__(256, 3) k_nb_encode32_levels(const ChunkSeg* __restrict__ segs, int nseg,
                                                                uint64_t total, int B) {
-    __shared__ uint32_t tile[32 * NB_TILE_LD];
+    __shared__ __align__(16) uint32_t stage[NB_STAGE];
     pdl_wait();
     pdl_release();
-    int cur = -1, se = 0;
-    bool fast = true;
-    float scale = 1.f;
-    for (uint64_t c = blockIdx.x; c < total; c += gridDim.x) {
+    int cur = -1;
+    NbSrc q;
+    nb_encode32_chunks(total, B, stage, [&](uint64_t c) {
         const int s = find_seg(segs, nseg, c, &ChunkSeg::chunk_begin);
-        const ChunkSeg& q = segs[s];
+        const ChunkSeg& g = segs[s];
         if (s != cur) {
             cur = s;
-            se = B - (frexp_exp(__uint_as_float(*q.key)) + 2);     // NegaBinaryBPEncoder.hpp:21
-            fast = pow2_normal(se);
-            scale = fast ? pow2f(se) : 1.f;
+            q.x = g.x;
+            q.words = g.words;
+            q.n = g.n;
+            q.nblocks = g.nblocks;
+            q.stride = g.stride;
+            q.se = B - (frexp_exp(__uint_as_float(*g.key)) + 2);     // NegaBinaryBPEncoder.hpp:21
+            q.fast = pow2_normal(q.se);
+            q.scale = q.fast ? pow2f(q.se) : 1.f;
         }
-        if (B == 32)
-            nb_encode32_chunk<true>(q.x, q.n, q.nblocks, B, se, fast, scale, q.words, q.stride, c - q.chunk_begin, tile);
-        else
-            nb_encode32_chunk(q.x, q.n, q.nblocks, B, se, fast, scale, q.words, q.stride, c - q.chunk_begin, tile);
-    }
+        q.chunk = c - g.chunk_begin;
+        return q;
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -1373,9 +1380,13 @@ int launch_nb_encode_levels(const ChunkSeg* segs, int nseg, uint64_t total_chunk
                             const uint32_t* keys, double* errs_out, cudaStream_t st) {
     (void)keys;   // each segment carries its level's key
     if (errs_out) return nb_err_launch(segs, ChunkSeg{}, nseg, total_chunks, B, 0, partial, errs_out, st);
-    const unsigned grid = (unsigned)nb_encode_levels_grid(0);
+    return launch_nb_encode_segments(segs, nseg, total_chunks, B, (unsigned)nb_encode_levels_grid(0), st, true);
+}
+
+int launch_nb_encode_segments(const ChunkSeg* segs, int nseg, uint64_t total_chunks, int B, unsigned grid, cudaStream_t st,
+                              bool pdl) {
     count_launch();
-    const cudaError_t e = launch_chain(true, k_nb_encode32_levels, dim3(grid), dim3(256), 0, st, segs, nseg, total_chunks, B);
+    const cudaError_t e = launch_chain(pdl, k_nb_encode32_levels, dim3(grid), dim3(256), 0, st, segs, nseg, total_chunks, B);
     if (e != cudaSuccess) return cuda_status(e, "k_nb_encode32_levels");
     return PRODM_OK;
 }

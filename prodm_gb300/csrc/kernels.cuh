@@ -126,6 +126,9 @@ int launch_nb_decode_levels(const ChunkSeg* segs, int nseg, uint64_t total_chunk
 // errs_out, per-level squared-error tables (partial: nseg * nb_encode_levels_grid(1)
 // records of kErrRecWords words)
 int nb_encode_levels_grid(int with_errors);
+// the launch itself without error tables, over the segments of any number of fields
+int launch_nb_encode_segments(const ChunkSeg* segs, int nseg, uint64_t total_chunks, int B, unsigned grid, cudaStream_t st,
+                              bool pdl);
 int launch_nb_encode_levels(const ChunkSeg* segs, int nseg, uint64_t total_chunks, int B, double* partial,
                             const uint32_t* keys, double* errs_out, cudaStream_t st);
 

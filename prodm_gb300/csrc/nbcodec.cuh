@@ -80,48 +80,129 @@ __device__ __forceinline__ void transpose32_half(const uint32_t (&R)[32], int ha
     transpose32_half_tail(a);
 }
 
-constexpr int NB_G = 8;              // blocks per warp iteration
 constexpr int NB_CHUNK = 256;        // blocks per CTA chunk
 constexpr int NB_TILE_LD = NB_CHUNK + 1;   // padded tile row: conflict-free column writes
 
-// Encode chunk c (NB_CHUNK consecutive 32-value blocks) of a level: each warp
-// transposes 32 blocks into the shared [plane][block] tile, then the CTA
-// writes every plane's words of the chunk as one contiguous run
-// (NegaBinaryBPEncoder.hpp:18-62). The error-table variant is in bitplane.cu.
-// FULLB: B == 32, so every digit has a plane and no per-digit guard is needed
-template <bool FULLB = false>
-__device__ __forceinline__ void nb_encode32_chunk(const float* __restrict__ x, uint64_t n, uint64_t nblocks, int B,
-                                                  int se, bool fast, float scale, uint32_t* __restrict__ out,
-                                                  uint64_t stride, uint64_t c, uint32_t* tile) {
+// 32 x 32 bit transpose of one lane's words: bit v of a[k] becomes bit k of
+// a[v] (halves and bytes by byte selection, then 4, 2 and 1 bits)
+__device__ __forceinline__ void transpose32_lane(uint32_t (&a)[32]) {
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+        const uint32_t x = a[i], y = a[i + 16];
+        a[i] = __byte_perm(x, y, 0x5410u);
+        a[i + 16] = __byte_perm(x, y, 0x7632u);
+    }
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+        const int k = (i & 7) + 2 * (i & 8);
+        const uint32_t x = a[k], y = a[k + 8];
+        a[k] = __byte_perm(x, y, 0x6240u);
+        a[k + 8] = __byte_perm(x, y, 0x7351u);
+    }
+#pragma unroll
+    for (int s = 0; s < 3; s++) {
+        const int j = 4 >> s;
+        const uint32_t m = s == 0 ? 0x0f0f0f0fu : s == 1 ? 0x33333333u : 0x55555555u;
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            const int k = (i / j) * 2 * j + (i % j);
+            const uint32_t x = a[k], y = a[k + j];
+            a[k] = (x & m) | ((y << j) & ~m);
+            a[k + j] = ((x >> j) & m) | (y & ~m);
+        }
+    }
+}
+
+// Encode the chunks blockIdx.x, blockIdx.x + gridDim.x, .. of total chunks of
+// NB_CHUNK 32-value blocks (NegaBinaryBPEncoder.hpp:18-62): src_of(chunk)
+// gives the level that holds a chunk and the chunk's number in it. A warp
+// takes 32 blocks: their values go to shared memory by cp.async, each lane
+// reads the 32 values of its own block back, transposes their digits in
+// registers, and the 32 lanes' words of a plane are one 128-byte store. The
+// next 32 blocks are on their way while these are transposed. 100 x 500 x 500:
+// 55 us with a warp transpose by shuffles per block and a tile of the words in
+// shared memory (integer pipe 63 % busy, shared memory and shuffles 48 %), 38 us
+// so (DRAM floor 30); 64 fields of 173 M values 414 and 301 us (floor 208).
+// The error-table variant is in bitplane.cu.
+struct NbSrc {
+    const float* x;
+    uint32_t* words;
+    uint64_t n, nblocks, stride, chunk;
+    float scale;
+    int se;
+    bool fast;
+};
+constexpr int NB_ROW = 36;   // a block's values in shared memory, 16-byte rows without bank conflicts
+constexpr int NB_STAGE = (NB_CHUNK / 32) * 32 * NB_ROW;   // words of a CTA
+
+template <class SrcOf>
+__device__ __forceinline__ void nb_encode32_chunks(uint64_t total, int B, uint32_t* stage, SrcOf src_of) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int plane = B - 1 - lane;      // lane k owns bit k = plane B-1-k
-    const uint64_t cb0 = c * NB_CHUNK;
-    const uint64_t wb0 = cb0 + (uint64_t)warp * 32;
-#pragma unroll 1
-    for (int j0 = 0; j0 < 32; j0 += NB_G) {
-        float v[NB_G];
+    uint32_t* buf = stage + warp * 32 * NB_ROW;
+    uint64_t c = blockIdx.x;
+    if (c >= total) return;
+    auto fetch = [&](const NbSrc& q) {
+        const uint64_t b = q.chunk * NB_CHUNK + (uint64_t)warp * 32;
+        if (b < q.nblocks) {
+            const uint64_t left = q.n - b * 32;
+            const int have = left < 1024 ? (int)left : 1024;
+            const float* src = q.x + b * 32;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(buf + lane);
 #pragma unroll
-        for (int g = 0; g < NB_G; g++) {
-            const uint64_t i = (wb0 + j0 + g) * 32 + lane;
-            v[g] = i < n ? __ldcs(x + i) : 0.f;
+            for (int g = 0; g < 32; g++) {
+                const int i = 32 * g + lane;
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + g * NB_ROW * 4),
+                             "l"(src + (i < have ? i : 0)), "r"(i < have ? 4 : 0)
+                             : "memory");
+            }
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    NbSrc q = src_of(c);
+    fetch(q);
+    for (;;) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();
+        uint32_t a[32];
 #pragma unroll
-        for (int g = 0; g < NB_G; g++) {
-            // NegaBinaryBPEncoder.hpp:42; the scaling is chosen once per chunk
-            // (an exact multiplication whenever 2^se is a normal float)
-            const float sh = fast ? v[g] * scale : ldexpf(v[g], se);
-            const uint32_t w = transpose32(nb_from_bin((int32_t)sh), lane);
-            if (FULLB || lane < B) tile[plane * NB_TILE_LD + warp * 32 + j0 + g] = w;
+        for (int i = 0; i < 8; i++) {
+            const uint4 v = *reinterpret_cast<const uint4*>(buf + lane * NB_ROW + 4 * i);
+            a[4 * i] = v.x;
+            a[4 * i + 1] = v.y;
+            a[4 * i + 2] = v.z;
+            a[4 * i + 3] = v.w;
         }
+        __syncwarp();
+        const NbSrc h = q;
+        c += gridDim.x;
+        if (c < total) {
+            q = src_of(c);
+            fetch(q);
+        }
+        const uint64_t b = h.chunk * NB_CHUNK + (uint64_t)warp * 32;
+        if (b < h.nblocks) {
+            // NegaBinaryBPEncoder.hpp:42; the scaling is an exact
+            // multiplication whenever 2^se is a normal float
+            if (h.fast) {
+#pragma unroll
+                for (int i = 0; i < 32; i++) a[i] = nb_from_bin((int32_t)(__uint_as_float(a[i]) * h.scale));
+            } else {
+#pragma unroll
+                for (int i = 0; i < 32; i++) a[i] = nb_from_bin((int32_t)ldexpf(__uint_as_float(a[i]), h.se));
+            }
+            transpose32_lane(a);   // a[k]: digit k of the block's values
+            if (b + lane < h.nblocks) {
+                uint32_t* dst = h.words + (uint64_t)(B - 1) * h.stride + b + lane;
+#pragma unroll
+                for (int k = 0; k < 32; k++)
+                    if (k < B) {
+                        *dst = a[k];
+                        dst -= h.stride;
+                    }
+            }
+        }
+        if (c >= total) break;
     }
-    __syncthreads();
-    const int nvalid = (int)((nblocks - cb0) < (uint64_t)NB_CHUNK ? (nblocks - cb0) : NB_CHUNK);
-    for (int p = warp; p < B; p += 8) {
-        uint32_t* dst = out + (uint64_t)p * stride + cb0;
-        const uint32_t* row = tile + p * NB_TILE_LD;
-        for (int j = lane; j < nvalid; j += 32) dst[j] = row[j];
-    }
-    __syncthreads();
 }
 
 // Decode chunk c of planes [s, s+num) (plane s+i at base + i * stride):
