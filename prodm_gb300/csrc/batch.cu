@@ -90,8 +90,10 @@ __global__ void __launch_bounds__(256, 3) k_decompose_multi(const RowSeg* __rest
         const int s = find_row_seg(s_begin, nseg, g);
         if (s != cur) { flush(); cur = s; }
         const RowSeg& q = segs[s];
-        if (q.patch)
-            decompose_patch_item<float>(q.in, q.s0, q.s1, q.F, q.C, q.coef, q.out, g - q.row_begin, lane, mk, mc);
+        if (q.patch && q.F.n[0] == 1)
+            decompose_patch_item<float, 1>(q.in, q.s0, q.s1, q.F, q.C, q.coef, q.out, g - q.row_begin, lane, mk, mc);
+        else if (q.patch)
+            decompose_patch_item<float, 0>(q.in, q.s0, q.s1, q.F, q.C, q.coef, q.out, g - q.row_begin, lane, mk, mc);
         else
             decompose_row_any<float>(q.in, q.s0, q.s1, q.F, q.C, q.coef, q.out, nullptr, g - q.row_begin, lane, mk,
                                      mc);
@@ -106,8 +108,10 @@ __global__ void __launch_bounds__(256) k_recompose_multi(const RowSeg* __restric
     for (uint32_t g = blockIdx.x * wpb + (threadIdx.x >> 5); g < total; g += gridDim.x * wpb) {
         const int s = find_row_seg(s_begin, nseg, g);
         const RowSeg& q = segs[s];
-        if (q.patch)
-            recompose_patch_item<float>(q.in, q.coef, q.F, q.C, q.out, q.s0, q.s1, g - q.row_begin, lane);
+        if (q.patch && q.F.n[0] == 1)
+            recompose_patch_item<float, 1>(q.in, q.coef, q.F, q.C, q.out, q.s0, q.s1, g - q.row_begin, lane);
+        else if (q.patch)
+            recompose_patch_item<float, 0>(q.in, q.coef, q.F, q.C, q.out, q.s0, q.s1, g - q.row_begin, lane);
         else
             recompose_row_any<float>(q.in, q.coef, q.F, q.C, q.out, q.s0, q.s1, g - q.row_begin, lane);
     }

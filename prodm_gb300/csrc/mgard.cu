@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(256) k_decompose_rows(const T* __restrict__ in
 // patch form (no natural-order copy): one
 // warp item = coarse columns 32g .. 32g + 31 of a 2 x 2 kPatchSteps strip of
 // fine rows (decompose_patch_item)
-template <class T>
+template <class T, int PLANE>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_decompose_patch(const T* __restrict__ in, uint64_t s0, uint64_t s1, Box F,
                                                          Box C, T* __restrict__ coef, T* __restrict__ coarse,
                                                          typename KeyOf<T>::type* maxkey_level,
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_decompose_patch
     const uint64_t items = patch_items(F, C);
     const uint32_t lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
     for (uint64_t w = (uint64_t)blockIdx.x * wpb + (threadIdx.x >> 5); w < items; w += (uint64_t)gridDim.x * wpb)
-        decompose_patch_item<T>(in, s0, s1, F, C, coef, coarse, w, lane, mk, mc);
+        decompose_patch_item<T, PLANE>(in, s0, s1, F, C, coef, coarse, w, lane, mk, mc);
     if (maxkey_level) {
         mk = warp_max_key(mk);
         if (lane == 0 && mk) atomicMax(maxkey_level, mk);
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_decompose_patch
 }
 
 // patch form of the recomposition (recompose_patch_item), same items as k_decompose_patch
-template <class T>
+template <class T, int PLANE>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_recompose_patch(const T* __restrict__ coarse,
                                                                                   const T* __restrict__ coef, Box F,
                                                                                   Box C, T* __restrict__ out,
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) k_recompose_patch
     const uint64_t items = patch_items(F, C);
     const uint32_t lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
     for (uint64_t w = (uint64_t)blockIdx.x * wpb + (threadIdx.x >> 5); w < items; w += (uint64_t)gridDim.x * wpb)
-        recompose_patch_item<T>(coarse, coef, F, C, out, s0, s1, w, lane);
+        recompose_patch_item<T, PLANE>(coarse, coef, F, C, out, s0, s1, w, lane);
 }
 
 template <class T>
@@ -706,7 +706,8 @@ int launch_decompose_level_packed(const T* in, uint64_t s0, uint64_t s1, const B
     const unsigned th = row_threads(F.n[2]);
     count_launch();
     if (!fnat && patch_level(F, C) && decompose_patch_enabled()) {
-        const cudaError_t e = launch_chain(true, k_decompose_patch<T>, dim3(row_grid(patch_items(F, C), th)), dim3(th), 0,
+        const auto kernel = F.n[0] == 1 ? k_decompose_patch<T, kPlaneAhead> : k_decompose_patch<T, 0>;
+        const cudaError_t e = launch_chain(true, kernel, dim3(row_grid(patch_items(F, C), th)), dim3(th), 0,
                                            st, in, s0, s1, F, C, coef, coarse, (K*)maxkey_level, (K*)maxkey_coarse);
         if (e != cudaSuccess) return cuda_status(e, "k_decompose_patch");
         return PRODM_OK;
@@ -733,7 +734,8 @@ int launch_recompose_level_packed(const T* coarse, const T* coef, const Box& F, 
     const unsigned th = row_threads(F.n[2]);
     count_launch();
     if (patch_level(F, C) && decompose_patch_enabled()) {
-        const cudaError_t e = launch_chain(pdl, k_recompose_patch<T>, dim3(row_grid(patch_items(F, C), th)), dim3(th), 0,
+        const auto kernel = F.n[0] == 1 ? k_recompose_patch<T, kPlaneAhead> : k_recompose_patch<T, 0>;
+        const cudaError_t e = launch_chain(pdl, kernel, dim3(row_grid(patch_items(F, C), th)), dim3(th), 0,
                                            st, coarse, coef, F, C, out, s0, s1);
         if (e != cudaSuccess) return cuda_status(e, "k_recompose_patch");
         return PRODM_OK;

@@ -131,6 +131,12 @@ __device__ __forceinline__ void decompose_row(const T* __restrict__ p, uint64_t 
 // P = C2 - 2 on, by the lanes that hold them.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kPatchSteps = 8;
+// PLANE > 0: 1-D and 2-D fields (one slab). Half the rows of a step and a third
+// of its loads are not there, so the registers hold PLANE steps in flight
+// instead of one. 1800 x 3600 fp32: decomposition 24.8 -> 14.3 us, recomposition
+// 10.6 -> 7.1 us with two (three: 14 % slower and 6 % faster, four spill). The
+// batched kernels hold both forms and keep to one (with two, 23 % slower).
+constexpr int kPlaneAhead = 2;
 
 // column groups of a patch row
 __host__ __device__ inline uint32_t patch_groups(uint32_t n2, uint32_t c2) {
@@ -160,7 +166,7 @@ inline bool patch_level(const Box& F, const Box& C) {
     return items >= patch_min_items() || items >= (uint64_t)F.n[0] * F.n[1];
 }
 
-template <class T>
+template <class T, int PLANE>
 __device__ __forceinline__ void decompose_patch_item(const T* __restrict__ in, uint64_t s0, uint64_t s1,
                                                      const Box& F, const Box& C, T* __restrict__ coef,
                                                      T* __restrict__ coarse, uint64_t item, uint32_t lane,
@@ -175,45 +181,57 @@ __device__ __forceinline__ void decompose_patch_item(const T* __restrict__ in, u
     const uint32_t c = 32 * g + lane;
     const bool act = c < P;                        // a column pair (2c, 2c+1)
     const bool ld = c < C2;                        // holds coarse column c
-    const bool two = i < F.n[0] - C0;              // fine row 2i + 1 exists
+    const bool two = !PLANE && i < F.n[0] - C0;    // fine row 2i + 1 exists
     // a lone column: the lane's own, or (odd rows, P a multiple of 32) lane 31's neighbour
     const bool even = !(F.n[2] & 1u);
     const bool last = even ? ld && !act : (g == npg - 1) && ((P & 31) ? (lane == (P & 31)) : (lane == 31));
     const bool own = c >= P;
     const uint32_t lc = even ? c : P;              // its coarse column
     const uint32_t xc = min(2 * c, F.n[2] - 1);    // the node of coarse column c
-    auto x1_of = [&](uint32_t b) { return (uint64_t)min(2 * b, F.n[1] - 1); };
     const uint32_t b0 = u * kPatchSteps, b1 = min(b0 + kPatchSteps, C1);
-    const T* base = in + (uint64_t)min(2 * i, F.n[0] - 1) * s0;
+    // Everything a step touches lies a fixed distance behind the step before
+    // (the last row of an even dim 1 but half of it), so pointers advance and no
+    // rank is computed per step: with four ranks of 64-bit products a step the
+    // kernels issued on 57 % of the cycles (finest level of 513^3 221 us, 204
+    // without; of 100 x 500 x 500 49 and 41 us).
+    const T* next_row = in + (uint64_t)min(2 * i, F.n[0] - 1) * s0 + (uint64_t)min(2 * b0, F.n[1] - 1) * s1 + xc;
+    T* k00 = coef + level_rank(i, b0, C2, F, C) + c;               // even-even row: odd nodes only
+    T* k01 = coef + level_rank(i, C1 + b0, 0, F, C) + c;
+    T* k10 = coef + level_rank(C0 + i, b0, 0, F, C) + c;
+    const uint64_t to11 = (uint64_t)C1 * F.n[2];                   // row (C0 + i, C1 + b) from (C0 + i, b)
+    T* crow = coarse + ((uint64_t)i * C1 + b0) * C2 + c;
+    const int lone = (int)lc - (int)c;                             // the lone column from the lane's own
     auto kmax = [](K& m, T v) { m = max_key(abs_key(v), m); };
-    // the loads of one step, issued a step ahead of their use: the four
+    // the loads of one step, issued D steps ahead of their use: the four
     // rows' node pairs, the corner values of rows 2b + 2 at column c and (lane
     // 31) at column c + 1, and the last node's even values
+    constexpr int D = PLANE ? PLANE : 1;
     struct Step {
         T a00, e01, o01, e10, o10, e11, o11, q02, q22, n02, n22, l01, l10, l11;
     };
-    auto load_step = [&](uint32_t b, Step& S) {
+    auto load_step = [&](uint32_t b, Step& S) {   // called for b0, b0 + 1, ..
         const bool odd = b < O1, more = b + 1 < C1;
-        const T* r00 = base + x1_of(b) * s1;
+        const T* r00 = next_row;
         const T* r01 = r00 + s1;
         const T* r10 = r00 + s0;
         const T* r11 = r10 + s1;
-        const T* r02 = base + x1_of(b + 1) * s1;
-        const uint32_t x = xc, xl = min(2 * lc, F.n[2] - 1);
-        S.a00 = act ? r00[x + 1] : (T)0;
-        S.e01 = act && odd ? r01[x] : (T)0;
-        S.o01 = act && odd ? r01[x + 1] : (T)0;
-        S.e10 = act && two ? r10[x] : (T)0;
-        S.o10 = act && two ? r10[x + 1] : (T)0;
-        S.e11 = act && two && odd ? r11[x] : (T)0;
-        S.o11 = act && two && odd ? r11[x + 1] : (T)0;
-        S.q02 = ld && more ? r02[x] : (T)0;
-        S.q22 = ld && more && two ? r02[2 * s0 + x] : (T)0;
-        S.n02 = lane == 31 && act && more ? r02[x + 2] : (T)0;
-        S.n22 = lane == 31 && act && more && two ? r02[2 * s0 + x + 2] : (T)0;
+        const T* r02 = r00 + (2 * b + 2 < F.n[1] ? 2 * s1 : s1);
+        const int xl = (int)min(2 * lc, F.n[2] - 1) - (int)xc;
+        S.a00 = act ? r00[1] : (T)0;
+        S.e01 = act && odd ? r01[0] : (T)0;
+        S.o01 = act && odd ? r01[1] : (T)0;
+        S.e10 = act && two ? r10[0] : (T)0;
+        S.o10 = act && two ? r10[1] : (T)0;
+        S.e11 = act && two && odd ? r11[0] : (T)0;
+        S.o11 = act && two && odd ? r11[1] : (T)0;
+        S.q02 = ld && more ? r02[0] : (T)0;
+        S.q22 = ld && more && two ? r02[2 * s0] : (T)0;
+        S.n02 = lane == 31 && act && more ? r02[2] : (T)0;
+        S.n22 = lane == 31 && act && more && two ? r02[2 * s0 + 2] : (T)0;
         S.l01 = last && odd ? r01[xl] : (T)0;
         S.l10 = last && two ? r10[xl] : (T)0;
         S.l11 = last && two && odd ? r11[xl] : (T)0;
+        next_row = r02;
     };
     // corner values at column c + 1: the next lane's, lane 31's own load
     auto next_col = [&](T q, T own_next) {
@@ -222,61 +240,56 @@ __device__ __forceinline__ void decompose_patch_item(const T* __restrict__ in, u
     };
     T q00, q20 = 0;
     {
-        const T* r = base + x1_of(b0) * s1;
-        const uint32_t x = xc;
-        q00 = ld ? r[x] : (T)0;
-        T n00 = lane == 31 && act ? r[x + 2] : (T)0, n20 = 0;
+        const T* r = next_row;
+        q00 = ld ? r[0] : (T)0;
+        T n00 = lane == 31 && act ? r[2] : (T)0, n20 = 0;
         if (two) {
-            q20 = ld ? r[2 * s0 + x] : (T)0;
-            n20 = lane == 31 && act ? r[2 * s0 + x + 2] : (T)0;
+            q20 = ld ? r[2 * s0] : (T)0;
+            n20 = lane == 31 && act ? r[2 * s0 + 2] : (T)0;
         }
         n00 = next_col(q00, n00);
         n20 = next_col(q20, n20);
-        Step S;
-        load_step(b0, S);
+        Step next[D];
+#pragma unroll
+        for (int s = 0; s < D; s++)
+            if (b0 + s < b1) load_step(b0 + s, next[s]);
         T qn00 = n00, qn20 = n20;
         T h00 = avg_rn(q00, qn00), h20 = avg_rn(q20, qn20);
-        for (uint32_t b = b0; b < b1; b++) {
-            Step Sn = S;
-            if (b + 1 < b1) load_step(b + 1, Sn);
+        auto step = [&](uint32_t b, const Step& S) {
             const bool odd = b < O1;
             const T qn02 = next_col(S.q02, S.n02), qn22 = next_col(S.q22, S.n22);
             const T q02 = S.q02, q22 = S.q22;
             const T h02 = avg_rn(q02, qn02), h22 = avg_rn(q22, qn22);
-            const uint64_t rb00 = level_rank(i, b, C2, F, C);              // even-even row: odd nodes only
-            const uint64_t rb01 = level_rank(i, C1 + b, 0, F, C);
-            const uint64_t rb10 = level_rank(C0 + i, b, 0, F, C);
-            const uint64_t rb11 = level_rank(C0 + i, C1 + b, 0, F, C);
-            T* crow = coarse + ((uint64_t)i * C1 + b) * C2;
+            T* k11 = k10 + to11;
             const T v0 = avg_rn(q00, q02), hv0 = avg_rn(h00, h02);
             const T v2 = avg_rn(q20, q22), hv2 = avg_rn(h20, h22);
             if (act) {
-                crow[c] = q00;
+                crow[0] = q00;
                 kmax(mc, q00);
                 T d = sub_rn(S.a00, h00);
-                coef[rb00 + c] = d;
+                k00[0] = d;
                 kmax(mk, d);
                 if (odd) {
                     d = sub_rn(S.e01, v0);
-                    coef[rb01 + c] = d;
+                    k01[0] = d;
                     kmax(mk, d);
                     d = sub_rn(S.o01, hv0);
-                    coef[rb01 + C2 + c] = d;
+                    k01[C2] = d;
                     kmax(mk, d);
                 }
                 if (two) {
                     d = sub_rn(S.e10, avg_rn(q00, q20));
-                    coef[rb10 + c] = d;
+                    k10[0] = d;
                     kmax(mk, d);
                     d = sub_rn(S.o10, avg_rn(h00, h20));
-                    coef[rb10 + C2 + c] = d;
+                    k10[C2] = d;
                     kmax(mk, d);
                     if (odd) {
                         d = sub_rn(S.e11, avg_rn(v0, v2));
-                        coef[rb11 + c] = d;
+                        k11[0] = d;
                         kmax(mk, d);
                         d = sub_rn(S.o11, avg_rn(hv0, hv2));
-                        coef[rb11 + C2 + c] = d;
+                        k11[C2] = d;
                         kmax(mk, d);
                     }
                 }
@@ -284,32 +297,46 @@ __device__ __forceinline__ void decompose_patch_item(const T* __restrict__ in, u
             if (last) {   // a lone column: even nodes only
                 const T p00 = own ? q00 : qn00, p02 = own ? q02 : qn02;
                 const T p20 = own ? q20 : qn20, p22 = own ? q22 : qn22;
-                crow[lc] = p00;
+                crow[lone] = p00;
                 kmax(mc, p00);
                 const T w0 = avg_rn(p00, p02);
                 if (odd) {
                     const T d = sub_rn(S.l01, w0);
-                    coef[rb01 + lc] = d;
+                    k01[lone] = d;
                     kmax(mk, d);
                 }
                 if (two) {
                     T d = sub_rn(S.l10, avg_rn(p00, p20));
-                    coef[rb10 + lc] = d;
+                    k10[lone] = d;
                     kmax(mk, d);
                     if (odd) {
                         d = sub_rn(S.l11, avg_rn(w0, avg_rn(p20, p22)));
-                        coef[rb11 + lc] = d;
+                        k11[lone] = d;
                         kmax(mk, d);
                     }
                 }
             }
+            k00 += P;
+            k01 += F.n[2];
+            k10 += F.n[2];
+            crow += C2;
             q00 = q02;
             qn00 = qn02;
             h00 = h02;
             q20 = q22;
             qn20 = qn22;
             h20 = h22;
-            S = Sn;
+        };
+        for (uint32_t b = b0; b < b1; b += D) {
+            Step now[D];
+#pragma unroll
+            for (int s = 0; s < D; s++) {
+                now[s] = next[s];
+                if (b + D + s < b1) load_step(b + D + s, next[s]);
+            }
+#pragma unroll
+            for (int s = 0; s < D; s++)
+                if (b + s < b1) step(b + s, now[s]);
         }
     }
 }
@@ -321,7 +348,7 @@ __device__ __forceinline__ void decompose_patch_item(const T* __restrict__ in, u
 // are the coefficient plus the interpolation of decompose_patch_item (the
 // row kernels' corner trees, so the output is bit-identical to theirs). Each
 // step's loads are issued a step ahead of their use.
-template <class T>
+template <class T, int PLANE>
 __device__ __forceinline__ void recompose_patch_item(const T* __restrict__ coarse, const T* __restrict__ coef,
                                                      const Box& F, const Box& C, T* __restrict__ out, uint64_t s0,
                                                      uint64_t s1, uint64_t item, uint32_t lane) {
@@ -334,85 +361,90 @@ __device__ __forceinline__ void recompose_patch_item(const T* __restrict__ coars
     const uint32_t c = 32 * g + lane;
     const bool act = c < P;
     const bool ld = c < C2;
-    const bool two = i < F.n[0] - C0;
+    const bool two = !PLANE && i < F.n[0] - C0;
     const bool even = !(F.n[2] & 1u);
     const bool last = even ? ld && !act : (g == npg - 1) && ((P & 31) ? (lane == (P & 31)) : (lane == 31));
     const bool own = c >= P;
     const uint32_t lc = even ? c : P;
     const uint32_t b0 = u * kPatchSteps, b1 = min(b0 + kPatchSteps, C1);
     const uint64_t cs0 = (uint64_t)C1 * C2;
-    const T* slab0 = coarse + (uint64_t)i * cs0;         // coarse rows (i, b)
-    const T* slab1 = slab0 + cs0;                         // (i + 1, b)
+    // (pointers advance from step to step, as in decompose_patch_item)
+    const T* next_q = coarse + (uint64_t)i * cs0 + (uint64_t)b0 * C2 + c;   // coarse row (i, b), (i + 1, b) cs0 behind
+    const T* k00 = coef + level_rank(i, b0, C2, F, C) + c;
+    const T* k01 = coef + level_rank(i, C1 + b0, 0, F, C) + c;
+    const T* k10 = coef + level_rank(C0 + i, b0, 0, F, C) + c;
+    const uint64_t to11 = (uint64_t)C1 * F.n[2];
+    const int lone = (int)lc - (int)c;
+    T* o00 = out + (uint64_t)min(2 * i, F.n[0] - 1) * s0 + (uint64_t)min(2 * b0, F.n[1] - 1) * s1 + 2 * (uint64_t)c;
+    constexpr int D = PLANE ? PLANE : 1;
     struct Step {
         T q02, q22, n02, n22, ca, cbe, cbo, cce, cco, cde, cdo, lb, lc, ld_;
     };
-    auto load_step = [&](uint32_t b, Step& S) {
+    auto load_step = [&](uint32_t b, Step& S) {   // called for b0, b0 + 1, ..
         const bool odd = b < O1, more = b + 1 < C1;
-        const uint64_t rb00 = level_rank(i, b, C2, F, C);
-        const uint64_t rb01 = level_rank(i, C1 + b, 0, F, C);
-        const uint64_t rb10 = level_rank(C0 + i, b, 0, F, C);
-        const uint64_t rb11 = level_rank(C0 + i, C1 + b, 0, F, C);
-        const T* q0 = slab0 + (uint64_t)(b + 1) * C2;
-        const T* q1 = slab1 + (uint64_t)(b + 1) * C2;
-        S.q02 = ld && more ? __ldg(q0 + c) : (T)0;
-        S.q22 = ld && more && two ? __ldg(q1 + c) : (T)0;
-        S.n02 = lane == 31 && act && more ? __ldg(q0 + c + 1) : (T)0;
-        S.n22 = lane == 31 && act && more && two ? __ldg(q1 + c + 1) : (T)0;
-        S.ca = act ? __ldg(coef + rb00 + c) : (T)0;
-        S.cbe = act && odd ? __ldg(coef + rb01 + c) : (T)0;
-        S.cbo = act && odd ? __ldg(coef + rb01 + C2 + c) : (T)0;
-        S.cce = act && two ? __ldg(coef + rb10 + c) : (T)0;
-        S.cco = act && two ? __ldg(coef + rb10 + C2 + c) : (T)0;
-        S.cde = act && two && odd ? __ldg(coef + rb11 + c) : (T)0;
-        S.cdo = act && two && odd ? __ldg(coef + rb11 + C2 + c) : (T)0;
-        S.lb = last && odd ? __ldg(coef + rb01 + lc) : (T)0;
-        S.lc = last && two ? __ldg(coef + rb10 + lc) : (T)0;
-        S.ld_ = last && two && odd ? __ldg(coef + rb11 + lc) : (T)0;
+        const T* q0 = next_q + C2;
+        const T* q1 = q0 + cs0;
+        const T* k11 = k10 + to11;
+        S.q02 = ld && more ? __ldg(q0) : (T)0;
+        S.q22 = ld && more && two ? __ldg(q1) : (T)0;
+        S.n02 = lane == 31 && act && more ? __ldg(q0 + 1) : (T)0;
+        S.n22 = lane == 31 && act && more && two ? __ldg(q1 + 1) : (T)0;
+        S.ca = act ? __ldg(k00) : (T)0;
+        S.cbe = act && odd ? __ldg(k01) : (T)0;
+        S.cbo = act && odd ? __ldg(k01 + C2) : (T)0;
+        S.cce = act && two ? __ldg(k10) : (T)0;
+        S.cco = act && two ? __ldg(k10 + C2) : (T)0;
+        S.cde = act && two && odd ? __ldg(k11) : (T)0;
+        S.cdo = act && two && odd ? __ldg(k11 + C2) : (T)0;
+        S.lb = last && odd ? __ldg(k01 + lone) : (T)0;
+        S.lc = last && two ? __ldg(k10 + lone) : (T)0;
+        S.ld_ = last && two && odd ? __ldg(k11 + lone) : (T)0;
+        next_q = q0;
+        k00 += P;
+        k01 += F.n[2];
+        k10 += F.n[2];
     };
     auto next_col = [&](T q, T own_next) {
         const T n = __shfl_down_sync(0xffffffffu, q, 1);
         return lane == 31 ? own_next : n;
     };
-    const T* q0 = slab0 + (uint64_t)b0 * C2;
-    const T* q1 = slab1 + (uint64_t)b0 * C2;
-    T q00 = ld ? __ldg(q0 + c) : (T)0, q20 = ld && two ? __ldg(q1 + c) : (T)0;
-    T qn00 = next_col(q00, lane == 31 && act ? __ldg(q0 + c + 1) : (T)0);
-    T qn20 = next_col(q20, lane == 31 && act && two ? __ldg(q1 + c + 1) : (T)0);
+    const T* q1 = next_q + cs0;
+    T q00 = ld ? __ldg(next_q) : (T)0, q20 = ld && two ? __ldg(q1) : (T)0;
+    T qn00 = next_col(q00, lane == 31 && act ? __ldg(next_q + 1) : (T)0);
+    T qn20 = next_col(q20, lane == 31 && act && two ? __ldg(q1 + 1) : (T)0);
     T h00 = avg_rn(q00, qn00), h20 = avg_rn(q20, qn20);
-    Step S;
-    load_step(b0, S);
-    for (uint32_t b = b0; b < b1; b++) {
-        Step Sn = S;
-        if (b + 1 < b1) load_step(b + 1, Sn);
+    Step next[D];
+#pragma unroll
+    for (int s = 0; s < D; s++)
+        if (b0 + s < b1) load_step(b0 + s, next[s]);
+    auto step = [&](uint32_t b, const Step& S) {
         const bool odd = b < O1;
         const T q02 = S.q02, q22 = S.q22;
         const T qn02 = next_col(q02, S.n02), qn22 = next_col(q22, S.n22);
         const T h02 = avg_rn(q02, qn02), h22 = avg_rn(q22, qn22);
         const T v0 = avg_rn(q00, q02), hv0 = avg_rn(h00, h02);
         const T v2 = avg_rn(q20, q22), hv2 = avg_rn(h20, h22);
-        T* o00 = out + (uint64_t)min(2 * i, F.n[0] - 1) * s0 + (uint64_t)min(2 * b, F.n[1] - 1) * s1;
         T* o01 = o00 + s1;
         T* o10 = o00 + s0;
         T* o11 = o10 + s1;
         if (act) {
-            const uint64_t x = 2 * (uint64_t)c;
-            o00[x] = q00;
-            o00[x + 1] = add_rn(S.ca, h00);
+            o00[0] = q00;
+            o00[1] = add_rn(S.ca, h00);
             if (odd) {
-                o01[x] = add_rn(S.cbe, v0);
-                o01[x + 1] = add_rn(S.cbo, hv0);
+                o01[0] = add_rn(S.cbe, v0);
+                o01[1] = add_rn(S.cbo, hv0);
             }
             if (two) {
-                o10[x] = add_rn(S.cce, avg_rn(q00, q20));
-                o10[x + 1] = add_rn(S.cco, avg_rn(h00, h20));
+                o10[0] = add_rn(S.cce, avg_rn(q00, q20));
+                o10[1] = add_rn(S.cco, avg_rn(h00, h20));
                 if (odd) {
-                    o11[x] = add_rn(S.cde, avg_rn(v0, v2));
-                    o11[x + 1] = add_rn(S.cdo, avg_rn(hv0, hv2));
+                    o11[0] = add_rn(S.cde, avg_rn(v0, v2));
+                    o11[1] = add_rn(S.cdo, avg_rn(hv0, hv2));
                 }
             }
         }
         if (last) {   // a lone column: even nodes only
-            const uint32_t x = min(2 * lc, F.n[2] - 1);
+            const int x = (int)min(2 * lc, F.n[2] - 1) - 2 * (int)c;
             const T p00 = own ? q00 : qn00, p02 = own ? q02 : qn02;
             const T p20 = own ? q20 : qn20, p22 = own ? q22 : qn22;
             o00[x] = p00;
@@ -423,13 +455,24 @@ __device__ __forceinline__ void recompose_patch_item(const T* __restrict__ coars
                 if (odd) o11[x] = add_rn(S.ld_, avg_rn(w0, avg_rn(p20, p22)));
             }
         }
+        o00 += 2 * b + 2 < F.n[1] ? 2 * s1 : s1;
         q00 = q02;
         qn00 = qn02;
         h00 = h02;
         q20 = q22;
         qn20 = qn22;
         h20 = h22;
-        S = Sn;
+    };
+    for (uint32_t b = b0; b < b1; b += D) {
+        Step now[D];
+#pragma unroll
+        for (int s = 0; s < D; s++) {
+            now[s] = next[s];
+            if (b + D + s < b1) load_step(b + D + s, next[s]);
+        }
+#pragma unroll
+        for (int s = 0; s < D; s++)
+            if (b + s < b1) step(b + s, now[s]);
     }
 }
 
