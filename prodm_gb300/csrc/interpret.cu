@@ -342,16 +342,15 @@ __device__ __forceinline__ uint64_t mag_units80(__int128 v) {
     return (uint64_t)(a >> 80) + 1;
 }
 
-constexpr int kFixK = 5;   // positions per thread in the fixed-point pass (256 threads cover 17 x 64)
-
 __device__ __forceinline__ __int128 shfl_up128(__int128 x, int o) {
     const unsigned long long lo = __shfl_up_sync(0xffffffffu, (unsigned long long)x, o);
     const unsigned long long hi = __shfl_up_sync(0xffffffffu, (unsigned long long)((unsigned __int128)x >> 64), o);
     return (__int128)(((unsigned __int128)hi << 64) | lo);
 }
 // exclusive prefix over the CTA's threads (in thread order) of one value per
-// thread: warp scans by shuffles, then the warp totals; tot: one slot per warp
-__device__ __int128 cta_exclusive_scan(__int128 v, __int128* tot) {
+// thread, and the sum of all: warp scans by shuffles, then the warp totals;
+// tot: one slot per warp
+__device__ __noinline__ __int128 cta_exclusive_scan(__int128 v, __int128* tot, __int128& sum) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     __int128 x = v;
 #pragma unroll
@@ -372,6 +371,7 @@ __device__ __int128 cta_exclusive_scan(__int128 v, __int128* tot) {
     }
     __syncthreads();
     const __int128 off = wid > 0 ? tot[wid - 1] : (__int128)0;
+    sum = tot[nw - 1];
     __syncthreads();   // the slots may be reused right after
     return off + x - v;
 }
@@ -402,15 +402,27 @@ __device__ bool interpret_blocks(int kind, int nl, int B, const uint32_t* __rest
                                  BlockWalkSmem& w) {
     const int tid = threadIdx.x, nth = blockDim.x;
     // initial estimate, the sign-exclude first planes, heap membership
+    if (kind != 1 && tid < nl) {
+        w.start[tid] = index[tid];
+        w.rs[tid] = 0;
+        w.in_heap[tid] = index[tid] != B;
+    }
     if (tid == 0) {
         double acc = 0;
-        for (int i = 0; i < nl; i++) acc += ev[i * 65 + index[i]];
+        for (int i0 = 0; i0 < nl; i0 += 4) {   // the adds depend on each other, the loads do not
+            double e[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) e[u] = i0 + u < nl ? ev[(i0 + u) * 65 + index[i0 + u]] : 0.0;
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (i0 + u < nl) acc += e[u];
+        }
         bool met = false;
         w.fail = 0;
-        for (int i = 0; i < nl; i++) {
+        for (int i = 0; kind == 1 && i < nl; i++) {
             w.start[i] = index[i];
             w.rs[i] = 0;
-            w.in_heap[i] = kind != 1 && index[i] != B;
+            w.in_heap[i] = 0;
         }
         if (kind == 1) {
             if (acc < tol) {
@@ -443,35 +455,79 @@ __device__ bool interpret_blocks(int kind, int nl, int B, const uint32_t* __rest
         w.npos = 0;
     }
     __syncthreads();
-    // each level's chain and blocks (one thread per level), the blocks into
-    // one shared list
-    uint8_t* lfirst = reinterpret_cast<uint8_t*>(w.order);   // [kMaxLevels][64]: first entry of each block
-    if (tid < nl) {
-        const int l = tid;
-        int cnt = 0, nb = 0;
-        if (w.in_heap[l]) {
-            long long runmin = 0;
-            for (int j = w.start[l]; j < B; j += en[l * 64 + j]) {
-                const long long k = ekey[l * 64 + j];
-                if (enan[l * 64 + j]) w.fail = 1;
-                if (cnt == 0 || k < runmin) {
-                    lfirst[l * 64 + nb++] = (uint8_t)cnt;
-                    runmin = k;
+    // each level's chain and blocks, the blocks into one shared list: a warp a
+    // level, lane j on the entries j and j + 32. An entry starts a block when
+    // its key is below every earlier entry's of the chain: a prefix minimum,
+    // taken as the prefix maximum of the complements.
+    {
+        const int lane = tid & 31;
+        for (int l = tid >> 5; l < nl; l += nth >> 5) {
+            const int first = w.in_heap[l] ? w.start[l] : B;
+            const unsigned long long from = first < 64 ? ~0ull << first : 0ull, upto = B < 64 ? (1ull << B) - 1 : ~0ull;
+            unsigned long long mem = from & upto;   // the chain's entries
+            int step[2] = {1, 1};
+#pragma unroll
+            for (int h = 0; h < 2; h++)
+                if (mem >> (lane + 32 * h) & 1) step[h] = en[l * 64 + lane + 32 * h];
+            if (__any_sync(0xffffffffu, step[0] != 1 || step[1] != 1)) {   // some entries take several planes
+                mem = 0;
+                for (int j = first; j < B;) {
+                    mem |= 1ull << j;
+                    j += __shfl_sync(0xffffffffu, j < 32 ? step[0] : step[1], j & 31);
                 }
-                w.ch_j[l][cnt++] = (uint8_t)j;
             }
-        }
-        w.n_ent[l] = (uint8_t)cnt;
-        w.lnb[l] = nb;
-        w.lat[l] = 0;
-        if (nb) {   // the level's blocks into the shared list: key (its first entry's) and info
-            atomicAdd(&w.npos, cnt);
-            const int at = atomicAdd(&w.nblk, nb);
-            w.lat[l] = at;
-            for (int b = 0; b < nb; b++) {
-                const int f0 = lfirst[l * 64 + b], f1 = b + 1 < nb ? lfirst[l * 64 + b + 1] : cnt;
-                blk_key[at + b] = ekey[l * 64 + w.ch_j[l][f0]];
-                w.binfo[at + b] = (uint32_t)l | (uint32_t)(f1 - f0) << 16 | (uint32_t)f0 << 24;
+            unsigned long long v[2], before[2];   // ~key in unsigned order, 0 where no entry
+            bool bad = false;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int j = lane + 32 * h;
+                v[h] = 0;
+                if (mem >> j & 1) {
+                    v[h] = ~((unsigned long long)ekey[l * 64 + j] ^ 0x8000000000000000ull);
+                    bad |= enan[l * 64 + j] != 0;
+                }
+            }
+            if (bad) w.fail = 1;
+            unsigned long long run = 0;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                unsigned long long x = v[h];
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
+                    if (lane >= o) x = max_key(x, y);
+                }
+                const unsigned long long e = __shfl_up_sync(0xffffffffu, x, 1);
+                before[h] = max_key(run, lane ? e : 0ull);
+                run = max_key(run, __shfl_sync(0xffffffffu, x, 31));
+            }
+            const unsigned s0 = __ballot_sync(0xffffffffu, v[0] > before[0]), s1 = __ballot_sync(0xffffffffu, v[1] > before[1]);
+            const unsigned long long starts = (unsigned long long)s1 << 32 | s0;
+            const int cnt = __popcll(mem), nb = __popcll(starts);
+            int at = 0;
+            if (lane == 0) {
+                w.n_ent[l] = (uint8_t)cnt;
+                w.lnb[l] = nb;
+                if (nb) {
+                    atomicAdd(&w.npos, cnt);
+                    at = atomicAdd(&w.nblk, nb);
+                }
+                w.lat[l] = at;
+            }
+            at = __shfl_sync(0xffffffffu, at, 0);
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int j = lane + 32 * h;
+                const unsigned long long below = (1ull << j) - 1;
+                const int pos = __popcll(mem & below);
+                if (mem >> j & 1) w.ch_j[l][pos] = (uint8_t)j;
+                if (starts >> j & 1) {
+                    const unsigned long long later = starts & ~below & ~(1ull << j);
+                    const int end = later ? __popcll(mem & ((later & (0 - later)) - 1)) : cnt;
+                    const int b = at + __popcll(starts & below);
+                    blk_key[b] = ekey[l * 64 + j];
+                    w.binfo[b] = (uint32_t)l | (uint32_t)(end - pos) << 16 | (uint32_t)pos << 24;
+                }
             }
         }
     }
@@ -490,23 +546,32 @@ __device__ bool interpret_blocks(int kind, int nl, int B, const uint32_t* __rest
         int rank = (int)(bi >> 24);
         bool tie = false;
         int behind = 0;   // the group's entries at higher levels
-        for (int l2 = 0; l2 < nl; l2++) {
-            const int nb2 = w.lnb[l2];
-            if (l2 == l || nb2 == 0) continue;
-            const int base = w.lat[l2];
-            int lo = 0, hi = nb2;
-            while (lo < hi) {
-                const int mid = (lo + hi) >> 1;
-                if (blk_key[base + mid] > k) lo = mid + 1;
-                else hi = mid;
+        for (int l0 = 0; l0 < nl; l0 += 4) {   // four levels' searches at a time
+            int lo[4], nb2[4], base[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const int l2 = min(l0 + u, nl - 1);
+                nb2[u] = l0 + u < nl && l2 != l ? w.lnb[l2] : 0;
+                base[u] = w.lat[l2];
+                lo[u] = 0;
             }
-            int first = lo;
-            if (lo < nb2 && blk_key[base + lo] == k) {
-                tie = true;
-                if (l2 < l) first = lo + 1;   // the lower level's tied block goes first
-                else behind += (int)((w.binfo[base + lo] >> 16) & 255);
+#pragma unroll 1
+            for (int s = 64; s; s >>= 1)   // (unrolled as a whole it is slower: the code runs once, from a cold cache)
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (lo[u] + s <= nb2[u] && blk_key[base[u] + lo[u] + s - 1] > k) lo[u] += s;
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                if (nb2[u] == 0) continue;
+                const int l2 = l0 + u;
+                int first = lo[u];
+                if (first < nb2[u] && blk_key[base[u] + first] == k) {
+                    tie = true;
+                    if (l2 < l) first++;   // the lower level's tied block goes first
+                    else behind += (int)((w.binfo[base[u] + first] >> 16) & 255);
+                }
+                rank += first < nb2[u] ? (int)(w.binfo[base[u] + first] >> 24) : (int)w.n_ent[l2];
             }
-            rank += first < nb2 ? (int)(w.binfo[base + first] >> 24) : (int)w.n_ent[l2];
         }
         const int f0 = bi >> 24, n = (bi >> 16) & 255;
         for (int e = 0; e < n; e++) {
@@ -550,66 +615,42 @@ __device__ bool interpret_blocks(int kind, int nl, int B, const uint32_t* __rest
     __syncthreads();
     for (int p = tid; p < np; p += nth) {
         const uint32_t tq = terms[p];
-        atomicMax(&w.maxev, max(exp_field(ev[tq & 0xffffu]), exp_field(ev[tq >> 16])));
+        const double sub = ev[tq & 0xffffu], add = ev[tq >> 16];
+        atomicMax(&w.maxev, max(exp_field(sub), exp_field(add)));
+        if (!(add <= sub && add >= 0.0)) w.ties_fall = 0;   // a pop that raises the estimate, or a negative term
     }
     __syncthreads();
     if (w.fixed_ok && w.maxev < 0x7ff) {
         const int elsb = (w.maxev - 1022 + 1) + 12 - 125;   // all |values| < 2^(maxev - 1022 + 1); 2^11 pops of headroom
-        const int p0 = tid * kFixK;
-        __int128 rr[kFixK], rp[kFixK];
-        __int128 dsum = 0;
-#pragma unroll
-        for (int u = 0; u < kFixK; u++) {
-            rr[u] = rp[u] = 0;
-            if (p0 + u < np) {
-                const uint32_t tq = terms[p0 + u];
-                const __int128 a = fixed_units(ev[tq & 0xffffu], elsb), b = fixed_units(ev[tq >> 16], elsb);
-                rp[u] = -a;   // R'_p - R_{p-1} for now
-                rr[u] = b - a;
-                dsum += b - a;
-            }
-        }
-        const __int128 afix = fixed_units(w.acc0, elsb);
-        __int128 run = afix + cta_exclusive_scan(dsum, w.tot);   // R_{p0 - 1}
-        uint64_t usum = 0, uu[kFixK];
+        const __int128 afix = fixed_units(w.acc0, elsb), tfix = fixed_units(tol, elsb);
         const uint64_t u_tied = 4 * mag_units80(afix);
-        int fell = 1;   // no pop raises the estimate or has a negative term
-#pragma unroll
-        for (int u = 0; u < kFixK; u++) {
-            uu[u] = 0;
-            if (p0 + u < np) {
-                const bool tied = w.tie[p0 + u] != 0;
-                if (rr[u] > 0 || rr[u] < rp[u]) fell = 0;   // add > sub, or add < 0
-                rp[u] += run;    // R'_p
-                run += rr[u];    // R_p
-                rr[u] = run;
-                uu[u] = tied ? u_tied : mag_units80(rp[u]) + mag_units80(rr[u]);
-                usum += uu[u];
+        __int128 run = afix, urun = 0;   // R and the bound's sum before the round's positions
+        for (int q = 0; q < np; q += nth) {   // a position per thread and round
+            const int p = q + tid;
+            __int128 sub = 0, d = 0, sum;
+            if (p < np) {
+                const uint32_t tq = terms[p];
+                sub = fixed_units(ev[tq & 0xffffu], elsb);
+                d = fixed_units(ev[tq >> 16], elsb) - sub;
+            }
+            const __int128 before = run + cta_exclusive_scan(d, w.tot, sum), r = before + d;   // R_{p-1}, R_p
+            run += sum;
+            const int tie = p < np ? w.tie[p] : 0;
+            const uint64_t u = p >= np ? 0 : tie ? u_tied : mag_units80(before - sub) + mag_units80(r);
+            const __int128 ubefore = urun + cta_exclusive_scan((__int128)u, w.tot, sum);
+            urun += sum;
+            if (p < np) {
+                const __int128 e = ((ubefore + u) << 28) + 2 * p + 4;   // in units; 2^-52 * 2^80 = 2^28
+                const bool clear = r - e >= tfix + 1;   // certainly not met
+                if (tie) {
+                    if (!(w.ties_fall && (tie == 1 || clear))) atomicMin(&w.first_tie, p);
+                } else if (r + e < tfix) {
+                    atomicMin(&w.first_met, p);
+                } else if (!clear) {
+                    atomicMin(&w.first_amb, p);
+                }
             }
         }
-        if (!fell) w.ties_fall = 0;
-        uint64_t srun = (uint64_t)cta_exclusive_scan((__int128)usum, w.tot);
-        const __int128 tfix = fixed_units(tol, elsb);
-        int fm = np, fa = np, ft = np;
-#pragma unroll
-        for (int u = 0; u < kFixK; u++) {
-            const int p = p0 + u;
-            if (p >= np) break;
-            srun += uu[u];
-            const __int128 e = ((__int128)srun << 28) + 2 * p + 4;   // in units; 2^-52 * 2^80 = 2^28
-            const int tie = w.tie[p];
-            const bool clear = rr[u] - e >= tfix + 1;   // certainly not met
-            if (tie) {
-                if (!(w.ties_fall && (tie == 1 || clear)) && ft == np) ft = p;
-            } else if (rr[u] + e < tfix) {
-                if (fm == np) fm = p;
-            } else if (!clear) {
-                if (fa == np) fa = p;
-            }
-        }
-        if (fm < np) atomicMin(&w.first_met, fm);
-        if (fa < np) atomicMin(&w.first_amb, fa);
-        if (ft < np) atomicMin(&w.first_tie, ft);
     } else if (tid == 0) {
         w.fixed_ok = 0;
     }
@@ -690,10 +731,10 @@ __global__ void __launch_bounds__(256, 1) k_interpret(int nfields, int kind, int
                                                    uint8_t* __restrict__ index, uint64_t idx_stride,
                                                    uint32_t* __restrict__ rsz, bool early) {
     // The kernel writes the plane counts that the previous retrieval's kernels
-    // read, so it waits for them before the walk. With `early` (the host knows
+    // read, so it waits for them before it does. With `early` (the host knows
     // that only this handle's reconstruction kernels, which write none of the
-    // tables, ran since they were last written) the tables are read and
-    // tabulated before that wait; otherwise everything waits.
+    // tables and counts, ran since they were last written) everything else, the
+    // walk as well, comes before that wait; otherwise all of it waits.
     if (!early) {
         pdl_wait();
         pdl_release();
@@ -746,18 +787,19 @@ __global__ void __launch_bounds__(256, 1) k_interpret(int nfields, int kind, int
         s_en[l * 64 + j] = (int8_t)num;
     }
     __syncthreads();
-    if (early) {
-        pdl_wait();
-        pdl_release();
-    }
     __shared__ uint32_t s_rs[kMaxLevels];
     __shared__ int s_ok;
     uint32_t* gr = rsz + f * idx_stride;
     const double tol = tols ? tols[f] : tol0;
     {   // the block-ordered walk; s_errs is free after the tabulation and holds its block keys
         __shared__ BlockWalkSmem s_bw;
-        if (interpret_blocks(kind, nl, B, s_sizes, s_ev, s_key, s_nan, s_en, tol, s_idx, s_rs,
-                             reinterpret_cast<long long*>(s_errs), s_bw)) {
+        const bool done = interpret_blocks(kind, nl, B, s_sizes, s_ev, s_key, s_nan, s_en, tol, s_idx, s_rs,
+                                           reinterpret_cast<long long*>(s_errs), s_bw);
+        if (early) {
+            pdl_wait();
+            pdl_release();
+        }
+        if (done) {
             if (threadIdx.x < nl) {
                 gi[threadIdx.x] = s_idx[threadIdx.x];
                 gr[threadIdx.x] = s_rs[threadIdx.x];
