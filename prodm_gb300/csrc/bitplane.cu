@@ -787,18 +787,20 @@ __global__ void k_gr_scan(const __grid_constant__ GrSet<T> set, int B) {
 // A warp's blocks: its first one's word index in planes lane and lane + 32,
 // and the recording planes (lane j: block j; 255, which no plane reaches,
 // where there is no block)
+template <int NW = GR_WARPS>
 __device__ __forceinline__ int gr_warp_offsets(const uint8_t* __restrict__ rbs, uint64_t nblocks, uint64_t chunk,
                                                const uint32_t* __restrict__ chunk_off, int B, uint32_t& off0,
                                                uint32_t& off1) {
-    __shared__ uint32_t cnt[GR_WARPS][64];
+    constexpr int BPW = GR_CHUNK / NW;
+    __shared__ uint32_t cnt[NW][64];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t b = chunk * GR_CHUNK + (uint64_t)warp * GR_BPW + lane;
-    const int rv = b < nblocks ? rbs[b] : 255;
+    const uint64_t b = chunk * GR_CHUNK + (uint64_t)warp * BPW + lane;
+    const int rv = lane < BPW && b < nblocks ? rbs[b] : 255;
     off0 = lane < B ? chunk_off[chunk * B + lane] : 0;
     off1 = lane + 32 < B ? chunk_off[chunk * B + lane + 32] : 0;
     uint32_t c0 = 0, c1 = 0;
 #pragma unroll 8
-    for (int j = 0; j < GR_BPW; j++) {
+    for (int j = 0; j < BPW; j++) {
         const int r = __shfl_sync(FULL, rv, j);
         c0 += gr_words(r, lane);
         c1 += gr_words(r, lane + 32);
@@ -1042,12 +1044,12 @@ __global__ void __launch_bounds__(256) k_gr_write32(const __grid_constant__ GrSe
 // are fetched together before them, lane j block j's: gr_signs.
 // 513 x 513 x 257 fp64, most of 60 planes: 284 us; 419 us with four blocks
 // loaded, decoded and stored in turn and the sign words among them.
-template <class S>
+template <int BPW, class S>
 __device__ __forceinline__ S gr_signs(const S* const* __restrict__ planes, S* signs, uint64_t b, int rv, uint32_t off0,
                                       uint32_t off1, int s, int e, int lane) {
     uint32_t at = 0;   // where block lane's sign word stands in its plane
 #pragma unroll 8
-    for (int j = 0; j < GR_BPW; j++) {
+    for (int j = 0; j < BPW; j++) {
         const int r = __shfl_sync(FULL, rv, j);
         uint32_t o = __shfl_sync(FULL, off0, r & 31);
         if (sizeof(S) == 8) {
@@ -1065,9 +1067,17 @@ __device__ __forceinline__ S gr_signs(const S* const* __restrict__ planes, S* si
     return sign;
 }
 constexpr int GR_DU = 4;
+// Warps a chunk is decoded by. A warp's blocks come one after the other, so 32
+// warps with 8 blocks each instead of 8 with 32: fp32 65^3 13.2 -> 8.1 us, 129^3
+// 18.9 -> 16.0, 257^3 76.1 -> 75.2. An fp64 warp needs twice the registers, and
+// past a chunk an SM 8 warps are faster (257 x 257 x 129 52.3 us, 56.5 with 32;
+// 65^3 24.9 us, 17.9 with 32).
+constexpr int GR_WIDE = 32;
+inline bool gr_decode_wide64(unsigned chunks) { return chunks <= (unsigned)(kSMs); }
 
-__global__ void __launch_bounds__(256) k_gr_decode32(const __grid_constant__ GrSet<float> set, int B, int s, int e) {
-    constexpr int U = 2 * GR_DU;
+template <int NW>
+__global__ void __launch_bounds__(NW * 32) k_gr_decode32(const __grid_constant__ GrSet<float> set, int B, int s, int e) {
+    constexpr int BPW = GR_CHUNK / NW, U = 2 * GR_DU;
     uint32_t chunk;
     const GrSeg<float>& q = gr_seg(set, chunk);
     const uint64_t n = q.n;
@@ -1078,23 +1088,23 @@ __global__ void __launch_bounds__(256) k_gr_decode32(const __grid_constant__ GrS
     if (q.dnum) e = q.dnum[0];
     const int exp = level_exp<float>(q.key, q.exp);
     uint32_t off, unused;
-    const int rv = gr_warp_offsets(q.rbs, nblocks, chunk, q.co, B, off, unused);
+    const int rv = gr_warp_offsets<NW>(q.rbs, nblocks, chunk, q.co, B, off, unused);
     const uint32_t* src = (lane < B && lane >= s && lane < e) ? q.planes[lane] : nullptr;
     const bool fast = pow2_normal(exp - e);
     const float sc = fast ? pow2f(exp - e) : 1.f;
-    const uint64_t b0 = (uint64_t)chunk * GR_CHUNK + (uint64_t)warp * GR_BPW;
-    const uint32_t signs = gr_signs(q.planes, q.signs, b0, rv, off, 0u, s, e, lane);
+    const uint64_t b0 = (uint64_t)chunk * GR_CHUNK + (uint64_t)warp * BPW;
+    const uint32_t signs = gr_signs<BPW>(q.planes, q.signs, b0, rv, off, 0u, s, e, lane);
     uint32_t nx[U];
     auto load = [&](int j0) {
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            const int r = j0 < GR_BPW ? __shfl_sync(FULL, rv, j0 + u) : 255;
+            const int r = j0 < BPW ? __shfl_sync(FULL, rv, j0 + u) : 255;
             nx[u] = src && lane >= r ? __ldcs(src + off + (lane == r ? 1 : 0)) : 0;
             off += gr_words(r, lane);
         }
     };
     load(0);
-    for (int j0 = 0; j0 < GR_BPW && b0 + j0 < nblocks; j0 += U) {
+    for (int j0 = 0; j0 < BPW && b0 + j0 < nblocks; j0 += U) {
         uint32_t w[U];
 #pragma unroll
         for (int u = 0; u < U; u++) w[u] = nx[u];
@@ -1117,9 +1127,10 @@ __global__ void __launch_bounds__(256) k_gr_decode32(const __grid_constant__ GrS
 }
 
 // fp64
-__global__ void __launch_bounds__(256) k_gr_decode64(const __grid_constant__ GrSet<double> set, int B, int s, int e) {
+template <int NW>
+__global__ void __launch_bounds__(NW * 32) k_gr_decode64(const __grid_constant__ GrSet<double> set, int B, int s, int e) {
     using S = uint64_t;
-    constexpr int U = GR_DU;
+    constexpr int BPW = GR_CHUNK / NW, U = GR_DU;
     uint32_t chunk;
     const GrSeg<double>& q = gr_seg(set, chunk);
     const uint64_t n = q.n;
@@ -1130,16 +1141,16 @@ __global__ void __launch_bounds__(256) k_gr_decode64(const __grid_constant__ GrS
     if (q.dnum) e = q.dnum[0];
     const int exp = level_exp<double>(q.key, q.exp);
     uint32_t off0, off1;
-    const int rv = gr_warp_offsets(q.rbs, nblocks, chunk, q.co, B, off0, off1);
+    const int rv = gr_warp_offsets<NW>(q.rbs, nblocks, chunk, q.co, B, off0, off1);
     const S* src0 = (lane >= s && lane < e) ? q.planes[lane] : nullptr;
     const S* src1 = (lane + 32 >= s && lane + 32 < e) ? q.planes[lane + 32] : nullptr;
-    const uint64_t b0 = (uint64_t)chunk * GR_CHUNK + (uint64_t)warp * GR_BPW;
-    const S signs = gr_signs(q.planes, q.signs, b0, rv, off0, off1, s, e, lane);
+    const uint64_t b0 = (uint64_t)chunk * GR_CHUNK + (uint64_t)warp * BPW;
+    const S signs = gr_signs<BPW>(q.planes, q.signs, b0, rv, off0, off1, s, e, lane);
     S n0[U], n1[U];
     auto load = [&](int j0) {
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            const int r = j0 < GR_BPW ? __shfl_sync(FULL, rv, j0 + u) : 255;
+            const int r = j0 < BPW ? __shfl_sync(FULL, rv, j0 + u) : 255;
             n0[u] = src0 && lane >= r ? __ldcs(src0 + off0 + (lane == r ? 1 : 0)) : 0;
             n1[u] = src1 && lane + 32 >= r ? __ldcs(src1 + off1 + (lane + 32 == r ? 1 : 0)) : 0;
             off0 += gr_words(r, lane);
@@ -1147,7 +1158,7 @@ __global__ void __launch_bounds__(256) k_gr_decode64(const __grid_constant__ GrS
         }
     };
     load(0);
-    for (int j0 = 0; j0 < GR_BPW && b0 + j0 < nblocks; j0 += U) {
+    for (int j0 = 0; j0 < BPW && b0 + j0 < nblocks; j0 += U) {
         S w0[U], w1[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
@@ -1488,12 +1499,15 @@ int launch_gr_offsets(GrSet<T> set, int B, cudaStream_t st) {
 
 template <class T>
 int launch_gr_decode(GrSet<T> set, int B, int s, int e, cudaStream_t st) {
-    const dim3 grid(gr_number(set)), block(GR_WARPS * 32);
+    const dim3 grid(gr_number(set));
     if (!grid.x) return PRODM_OK;
-    if constexpr (std::is_same<T, float>::value)
-        PRODM_CHAIN("k_gr_decode32", k_gr_decode32, grid, block, 0, st, set, B, s, e);
-    else
-        PRODM_CHAIN("k_gr_decode64", k_gr_decode64, grid, block, 0, st, set, B, s, e);
+    if constexpr (std::is_same<T, float>::value) {
+        PRODM_CHAIN("k_gr_decode32", k_gr_decode32<GR_WIDE>, grid, dim3(GR_WIDE * 32), 0, st, set, B, s, e);
+    } else {
+        const int warps = gr_decode_wide64(grid.x) ? GR_WIDE : GR_WARPS;
+        PRODM_CHAIN("k_gr_decode64", (warps == GR_WIDE ? k_gr_decode64<GR_WIDE> : k_gr_decode64<GR_WARPS>), grid,
+                    dim3(warps * 32), 0, st, set, B, s, e);
+    }
     return PRODM_OK;
 }
 
