@@ -611,6 +611,15 @@ __global__ void __launch_bounds__(256) k_nb_decode(const typename Traits<T>::S* 
 constexpr int GR_WARPS = 8;
 constexpr int GR_BPW = 32;                       // blocks per warp
 constexpr int GR_CHUNK = GR_WARPS * GR_BPW;      // blocks per CTA
+// The decoders and the first pass have 32 warps with 8 blocks each: a warp's
+// blocks come one after the other, and 8 warps with 32 were fp32 13.2 us for 8.1
+// (decode 65^3), 18.9 for 16.0 (129^3), 76.1 for 75.2 (257^3); first pass 9.2 for
+// 6.7, 9.5 for 8.2 and 35.6 for 35.6. An fp64 warp needs twice the registers, so
+// past a chunk an SM it is 8 warps there (decode 257 x 257 x 129 52.3 us for
+// 56.5, first pass 257^3 39.5 for 43.8; before, 65^3 24.9 for 17.9 and 129^3 16.6
+// for 9.5).
+constexpr int GR_WIDE = 32;
+inline bool gr_wide64(unsigned chunks) { return chunks <= (unsigned)kSMs; }
 
 // |trunc(ldexp(v, B - exp))| and the sign (GroupedBPEncoder.hpp:41-42). For
 // doubles whose scaled value is not needed (SH false: no error tables) the
@@ -661,12 +670,12 @@ __device__ __forceinline__ const GrSeg<T>& gr_seg(const GrSet<T>& set, uint32_t&
 }
 
 // first pass: each block's recording bitplane and the chunk's word counts
-template <class T, bool ERR>
-__global__ void __launch_bounds__(256) k_gr_rb(const __grid_constant__ GrSet<T> set, int B,
+template <class T, bool ERR, int NW>
+__global__ void __launch_bounds__(NW * 32) k_gr_rb(const __grid_constant__ GrSet<T> set, int B,
                                                double* __restrict__ partial) {
     using FP = typename Traits<T>::FP;
     using A = typename Acc<T>::type;
-    constexpr int BS = Traits<T>::kBlock, H = BS / 32;
+    constexpr int BS = Traits<T>::kBlock, H = BS / 32, BPW = GR_CHUNK / NW;
     constexpr int U = ERR ? 1 : 8 / H;   // blocks loaded ahead
     uint32_t chunk;
     const GrSeg<T>& q = gr_seg(set, chunk);
@@ -674,7 +683,7 @@ __global__ void __launch_bounds__(256) k_gr_rb(const __grid_constant__ GrSet<T> 
     const uint64_t n = q.n;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t nblocks = (n + BS - 1) / BS;
-    __shared__ uint32_t cnt[GR_WARPS][64];
+    __shared__ uint32_t cnt[NW][64];
     uint32_t c0 = 0, c1 = 0;
     A acc[Acc<T>::N];
     if (ERR) {
@@ -686,9 +695,9 @@ __global__ void __launch_bounds__(256) k_gr_rb(const __grid_constant__ GrSet<T> 
     const int exp = level_exp<T>(q.key, q.exp);
     const bool fast = pow2_normal(B - exp);
     const float sc = fast ? pow2f(B - exp) : 1.f;
-    const uint64_t b0 = (uint64_t)chunk * GR_CHUNK + (uint64_t)warp * GR_BPW;
+    const uint64_t b0 = (uint64_t)chunk * GR_CHUNK + (uint64_t)warp * BPW;
     int rv = B;   // lane j: block j's recording plane
-    for (int j0 = 0; j0 < GR_BPW && b0 + j0 < nblocks; j0 += U) {
+    for (int j0 = 0; j0 < BPW && b0 + j0 < nblocks; j0 += U) {
         T v[U * H];
 #pragma unroll
         for (int t = 0; t < U * H; t++) {
@@ -726,13 +735,13 @@ __global__ void __launch_bounds__(256) k_gr_rb(const __grid_constant__ GrSet<T> 
             }
         }
     }
-    if (b0 + lane < nblocks) q.rbs[b0 + lane] = (uint8_t)rv;
+    if (lane < BPW && b0 + lane < nblocks) q.rbs[b0 + lane] = (uint8_t)rv;
     cnt[warp][lane] = c0;
     cnt[warp][lane + 32] = c1;
     __syncthreads();
     if (threadIdx.x < 64 && (int)threadIdx.x < B) {
         uint32_t t = 0;
-        for (int w = 0; w < GR_WARPS; w++) t += cnt[w][threadIdx.x];
+        for (int w = 0; w < NW; w++) t += cnt[w][threadIdx.x];
         q.cw[(uint64_t)chunk * B + threadIdx.x] = t;
     }
     if (ERR) flush_errors(acc, B, partial);
@@ -1067,13 +1076,6 @@ __device__ __forceinline__ S gr_signs(const S* const* __restrict__ planes, S* si
     return sign;
 }
 constexpr int GR_DU = 4;
-// Warps a chunk is decoded by. A warp's blocks come one after the other, so 32
-// warps with 8 blocks each instead of 8 with 32: fp32 65^3 13.2 -> 8.1 us, 129^3
-// 18.9 -> 16.0, 257^3 76.1 -> 75.2. An fp64 warp needs twice the registers, and
-// past a chunk an SM 8 warps are faster (257 x 257 x 129 52.3 us, 56.5 with 32;
-// 65^3 24.9 us, 17.9 with 32).
-constexpr int GR_WIDE = 32;
-inline bool gr_decode_wide64(unsigned chunks) { return chunks <= (unsigned)(kSMs); }
 
 template <int NW>
 __global__ void __launch_bounds__(NW * 32) k_gr_decode32(const __grid_constant__ GrSet<float> set, int B, int s, int e) {
@@ -1451,13 +1453,15 @@ int launch_gr_encode(GrSet<T> set, int B, double* partial, double* errs_out, cud
     if (!grid.x) return PRODM_OK;
     if (!f32 && errs_out) {
         if constexpr (!f32) {
-            PRODM_CHAIN("k_gr_rb", k_gr_rb<T, true>, grid, block, 0, st, set, B, partial);
+            PRODM_CHAIN("k_gr_rb", (k_gr_rb<T, true, GR_WARPS>), grid, block, 0, st, set, B, partial);
             k_reduce_partials<T><<<(B + 8) / 8, 256, 0, st>>>(partial, (int)grid.x, B, set.seg[0].key, set.seg[0].exp, 0,
                                                              1, errs_out);
             PRODM_CHECK_LAUNCH("k_reduce_partials");
         }
     } else {
-        PRODM_CHAIN("k_gr_rb", k_gr_rb<T, false>, grid, block, 0, st, set, B, (double*)nullptr);
+        const int warps = f32 || gr_wide64(grid.x) ? GR_WIDE : GR_WARPS;
+        PRODM_CHAIN("k_gr_rb", (warps == GR_WIDE ? k_gr_rb<T, false, GR_WIDE> : k_gr_rb<T, false, GR_WARPS>), grid,
+                    dim3(warps * 32), 0, st, set, B, (double*)nullptr);
     }
     PRODM_CHAIN("k_gr_scan", k_gr_scan<T>, dim3(B, set.n), dim3(1024), 0, st, set, B);
     if constexpr (f32) {
@@ -1504,7 +1508,7 @@ int launch_gr_decode(GrSet<T> set, int B, int s, int e, cudaStream_t st) {
     if constexpr (std::is_same<T, float>::value) {
         PRODM_CHAIN("k_gr_decode32", k_gr_decode32<GR_WIDE>, grid, dim3(GR_WIDE * 32), 0, st, set, B, s, e);
     } else {
-        const int warps = gr_decode_wide64(grid.x) ? GR_WIDE : GR_WARPS;
+        const int warps = gr_wide64(grid.x) ? GR_WIDE : GR_WARPS;
         PRODM_CHAIN("k_gr_decode64", (warps == GR_WIDE ? k_gr_decode64<GR_WIDE> : k_gr_decode64<GR_WARPS>), grid,
                     dim3(warps * 32), 0, st, set, B, s, e);
     }
