@@ -34,7 +34,6 @@ __device__ __forceinline__ int level_exp(const typename KeyOf<T>::type* maxkey, 
 }
 
 // quantisation shared by the encoders
-__device__ __forceinline__ int32_t trunc_fps(float v) { return (int32_t)v; }
 __device__ __forceinline__ int64_t trunc_fps(double v) { return (int64_t)v; }
 
 // ---------------------------------------------------------------------------
@@ -515,96 +514,6 @@ __global__ void __launch_bounds__(256) k_nb_decode32(const uint32_t* __restrict_
 }
 
 // ---------------------------------------------------------------------------
-// NegaBinary encoder -- NegaBinaryBPEncoder.hpp:18-62 (+ :65-125 errors)
-// ---------------------------------------------------------------------------
-template <class T, bool ERR>
-__global__ void __launch_bounds__(256) k_nb_encode(const T* __restrict__ x, uint64_t n,
-                                                   const typename KeyOf<T>::type* __restrict__ maxkey, int exp_arg,
-                                                   int B, typename Traits<T>::S* __restrict__ out, uint64_t stride,
-                                                   double* __restrict__ partial) {
-    using S = typename Traits<T>::S;
-    using FPS = typename Traits<T>::FPS;
-    using FP = typename Traits<T>::FP;
-    using A = typename Acc<T>::type;
-    constexpr int BS = Traits<T>::kBlock;
-    const int exp = level_exp<T>(maxkey, exp_arg) + 2;   // :21
-    const int lane = threadIdx.x & 31;
-    const uint64_t nblocks = (n + BS - 1) / BS;
-    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-    A acc[Acc<T>::N];
-    if (ERR) {
-#pragma unroll
-        for (int k = 0; k < Acc<T>::N; k++) acc[k] = 0;
-    }
-    for (uint64_t b = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); b < nblocks; b += warps) {
-        FP nb[BS / 32];
-#pragma unroll
-        for (int h = 0; h < BS / 32; h++) {
-            uint64_t i = b * BS + h * 32 + lane;
-            nb[h] = 0;
-            if (i < n) {
-                T shifted = ldexp_t(x[i], B - exp);          // :42
-                FPS q = trunc_fps(shifted);
-                nb[h] = nb_from_bin(q);
-                if (ERR) nb_errors(acc, nb[h], (A)shifted, (A)(shifted - (T)q), B);
-            }
-        }
-        S mine0 = 0, mine1 = 0;
-        for (int p = 0; p < B; p++) {                        // encode_block :240-250
-            const int k = B - 1 - p;
-            S w = (S)__ballot_sync(FULL, (nb[0] >> k) & 1u);
-            if (BS == 64) w |= (S)__ballot_sync(FULL, (nb[BS / 32 - 1] >> k) & 1u) << (BS == 64 ? 32 : 0);
-            if ((p & 31) == lane) {
-                if (p < 32) mine0 = w; else mine1 = w;
-            }
-        }
-        if (lane < B) out[(uint64_t)lane * stride + b] = mine0;
-        if (lane + 32 < B) out[(uint64_t)(lane + 32) * stride + b] = mine1;
-    }
-    if (ERR) flush_errors(acc, B, partial);
-}
-
-// NegaBinaryBPEncoder::progressive_decode -- :132-192. planes [s, s+num)
-// with plane (s+i) at base[i * stride]; a device count (dnum[0]) overrides num.
-template <class T>
-__global__ void __launch_bounds__(256) k_nb_decode(const typename Traits<T>::S* __restrict__ base, uint64_t stride,
-                                                   uint64_t n, const typename KeyOf<T>::type* __restrict__ maxkey,
-                                                   int exp_arg, int s, int num, const uint8_t* __restrict__ dnum,
-                                                   T* __restrict__ out) {
-    using S = typename Traits<T>::S;
-    using FP = typename Traits<T>::FP;
-    constexpr int BS = Traits<T>::kBlock;
-    if (dnum) num = dnum[0] - s;
-    const int exp = level_exp<T>(maxkey, exp_arg) + 2;
-    const int e = s + num;
-    const int lane = threadIdx.x & 31;
-    const uint64_t nblocks = (n + BS - 1) / BS;
-    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-    for (uint64_t b = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); b < nblocks; b += warps) {
-        S w0 = 0, w1 = 0;
-        if (lane < num) w0 = __ldg(base + (uint64_t)lane * stride + b);
-        if (lane + 32 < num) w1 = __ldg(base + (uint64_t)(lane + 32) * stride + b);
-        FP acc[BS / 32];
-#pragma unroll
-        for (int h = 0; h < BS / 32; h++) acc[h] = 0;
-        for (int i = 0; i < num; i++) {                       // decode_block :251-260
-            S w = __shfl_sync(FULL, i < 32 ? w0 : w1, i & 31);
-            const int k = num - 1 - i;
-#pragma unroll
-            for (int h = 0; h < BS / 32; h++) acc[h] |= (FP)((w >> (h * 32 + lane)) & 1u) << k;
-        }
-#pragma unroll
-        for (int h = 0; h < BS / 32; h++) {
-            uint64_t i = b * BS + h * 32 + lane;
-            if (i < n) {
-                T v = num == 0 ? (T)0 : ldexp_t((T)nb_to_bin(acc[h]), -e + exp);
-                out[i] = (num != 0 && (e & 1)) ? -v : v;       // :153, :177
-            }
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
 // Grouped encoder -- GroupedBPEncoder.hpp:18-73 (+ :76-145 errors)
 // Chunk = 8 warps x 32 blocks per CTA.
 // ---------------------------------------------------------------------------
@@ -649,6 +558,168 @@ __device__ __forceinline__ T gr_value(typename Traits<T>::FP acc, int s, bool ne
     }
     const T v = ldexp_t((T)acc, s);
     return neg ? -v : v;
+}
+
+// ---------------------------------------------------------------------------
+// fp64 negabinary encoder -- NegaBinaryBPEncoder.hpp:18-62 (+ :65-125 errors)
+// and decoder
+// ---------------------------------------------------------------------------
+// fp64 encoder with the error tables (NegaBinaryBPEncoder.hpp:65-125), a warp a
+// block
+__global__ void __launch_bounds__(256) k_nb_encode64_err(const double* __restrict__ x, uint64_t n,
+                                                         const unsigned long long* __restrict__ maxkey, int exp_arg, int B,
+                                                         uint64_t* __restrict__ out, uint64_t stride,
+                                                         double* __restrict__ partial) {
+    const int exp = level_exp<double>(maxkey, exp_arg) + 2;   // :21
+    const int lane = threadIdx.x & 31;
+    const uint64_t nblocks = (n + 63) / 64;
+    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+    double acc[Acc<double>::N];
+#pragma unroll
+    for (int k = 0; k < Acc<double>::N; k++) acc[k] = 0;
+    for (uint64_t b = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); b < nblocks; b += warps) {
+        uint64_t nb[2];
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const uint64_t i = b * 64 + h * 32 + lane;
+            nb[h] = 0;
+            if (i < n) {
+                const double shifted = ldexp(x[i], B - exp);          // :42
+                const int64_t q = trunc_fps(shifted);
+                nb[h] = nb_from_bin(q);
+                nb_errors(acc, nb[h], shifted, shifted - (double)q, B);
+            }
+        }
+        uint64_t mine0 = 0, mine1 = 0;
+        for (int p = 0; p < B; p++) {                        // encode_block :240-250
+            const int k = B - 1 - p;
+            const uint64_t w = (uint64_t)__ballot_sync(FULL, (nb[0] >> k) & 1u) |
+                               (uint64_t)__ballot_sync(FULL, (nb[1] >> k) & 1u) << 32;
+            if ((p & 31) == lane) {
+                if (p < 32) mine0 = w; else mine1 = w;
+            }
+        }
+        if (lane < B) out[(uint64_t)lane * stride + b] = mine0;
+        if (lane + 32 < B) out[(uint64_t)(lane + 32) * stride + b] = mine1;
+    }
+    flush_errors(acc, B, partial);
+}
+
+// (int64_t)ldexp(v, k) by integer operations while |v| 2^k < 2^63
+__device__ __forceinline__ int64_t nb_fix64(double v, int k) {
+    const int ev = (int)(((uint64_t)__double_as_longlong(v) >> 52) & 0x7ff);
+    if (ev == 0x7ff || ev - 1075 + k > 10) return trunc_fps(ldexp(v, k));
+    const int64_t m = (int64_t)fixed_mag(v, k);
+    return __double_as_longlong(v) < 0 ? -m : m;
+}
+
+// fp64 without tables. A warp takes eight blocks, four 32 x 32 bit transposes
+// each, the second four's values on their way while the first are transposed,
+// and their words leave through shared memory, eight lanes a plane: a store per
+// word is one to a sector of its own, and a ballot per plane 120 of them a block.
+// 513 x 513 x 257, 60 planes: 1499 us that way, 261 so (DRAM floor 164; with 32
+// blocks a warp 279, and 33^3 twice as slow).
+constexpr int NB64_BLOCKS = 8, NB64_LD = NB64_BLOCKS + 1;
+__global__ void __launch_bounds__(256, 3) k_nb_encode64(const double* __restrict__ x, uint64_t n,
+                                                        const unsigned long long* __restrict__ maxkey, int exp_arg, int B,
+                                                        uint64_t* __restrict__ out, uint64_t stride) {
+    constexpr int U = 4;   // blocks loaded ahead
+    __shared__ uint64_t stages[8][64 * NB64_LD];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint64_t* stage = stages[warp];
+    const uint64_t nblocks = (n + 63) / 64, step = (uint64_t)gridDim.x * 8 * NB64_BLOCKS;
+    pdl_wait();
+    pdl_release();
+    const int k = B - (level_exp<double>(maxkey, exp_arg) + 2);   // :21
+    for (uint64_t b0 = ((uint64_t)blockIdx.x * 8 + warp) * NB64_BLOCKS; b0 < nblocks; b0 += step) {
+        double nx[2 * U];
+        auto load = [&](int j0) {
+#pragma unroll
+            for (int t = 0; t < 2 * U; t++) {
+                const uint64_t i = (b0 + j0) * 64 + t * 32 + lane;
+                nx[t] = i < n ? __ldcs(x + i) : 0.0;
+            }
+        };
+        load(0);
+#pragma unroll
+        for (int j0 = 0; j0 < NB64_BLOCKS; j0 += U) {
+            double v[2 * U];
+#pragma unroll
+            for (int t = 0; t < 2 * U; t++) v[t] = nx[t];
+            if (j0 + U < NB64_BLOCKS) load(j0 + U);
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const uint64_t m0 = nb_from_bin(nb_fix64(v[2 * u], k)), m1 = nb_from_bin(nb_fix64(v[2 * u + 1], k));
+                // lane i: digit i (low halves) and 32 + i of values 0..31 and 32..63
+                const uint32_t lo0 = transpose32((uint32_t)m0, lane), hi0 = transpose32((uint32_t)(m0 >> 32), lane);
+                const uint32_t lo1 = transpose32((uint32_t)m1, lane), hi1 = transpose32((uint32_t)(m1 >> 32), lane);
+                stage[lane * NB64_LD + j0 + u] = (uint64_t)lo1 << 32 | lo0;   // row: digit
+                stage[(lane + 32) * NB64_LD + j0 + u] = (uint64_t)hi1 << 32 | hi0;
+            }
+        }
+        __syncwarp();
+        const uint64_t b = b0 + (lane & 7);
+        for (int d = lane >> 3; d < B; d += 4)   // digit d is plane B - 1 - d
+            if (b < nblocks) out[(uint64_t)(B - 1 - d) * stride + b] = stage[d * NB64_LD + (lane & 7)];
+        __syncwarp();
+    }
+}
+
+// fp64 NegaBinaryBPEncoder::progressive_decode -- :132-192. planes [s, s+num)
+// with plane (s+i) at base[i * stride]; a device count (dnum[0]) overrides num.
+// A warp takes eight blocks: their words of four planes come in one load and
+// are turned to a plane per lane in shared memory. 513 x 513 x 257, two
+// retrievals: 780 us a decode with a load per block and plane and a shuffle per
+// plane, 252 so (DRAM floor, with 14 and 36 planes, about 130).
+__global__ void __launch_bounds__(256, 2) k_nb_decode64(const uint64_t* __restrict__ base, uint64_t stride, uint64_t n,
+                                                        const unsigned long long* __restrict__ maxkey, int exp_arg, int s,
+                                                        int num, const uint8_t* __restrict__ dnum,
+                                                        double* __restrict__ out) {
+    __shared__ uint64_t stages[8][64 * NB64_LD];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint64_t* stage = stages[warp];
+    pdl_wait();
+    pdl_release();
+    if (dnum) num = dnum[0] - s;
+    const int exp = level_exp<double>(maxkey, exp_arg) + 2, e = s + num;
+    const uint64_t nblocks = (n + 63) / 64, step = (uint64_t)gridDim.x * 8 * NB64_BLOCKS;
+    if (num == 0) {
+        for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+            out[i] = 0.0;
+        return;
+    }
+    for (uint64_t b0 = ((uint64_t)blockIdx.x * 8 + warp) * NB64_BLOCKS; b0 < nblocks; b0 += step) {
+        uint64_t w[16];   // planes lane / 8 + 4 t of block lane % 8
+#pragma unroll
+        for (int t = 0; t < 16; t++) {
+            const int p = (lane >> 3) + 4 * t;
+            w[t] = p < num && b0 + (lane & 7) < nblocks ? __ldcs(base + (uint64_t)p * stride + b0 + (lane & 7)) : 0;
+        }
+#pragma unroll
+        for (int t = 0; t < 16; t++) stage[((lane >> 3) + 4 * t) * NB64_LD + (lane & 7)] = w[t];
+        __syncwarp();
+#pragma unroll 2
+        for (int j = 0; j < NB64_BLOCKS && b0 + j < nblocks; j++) {
+            const uint64_t w0 = stage[lane * NB64_LD + j];
+            const uint32_t pl0 = transpose32((uint32_t)w0, lane), ph0 = transpose32((uint32_t)(w0 >> 32), lane);
+            uint32_t pl1 = 0, ph1 = 0;
+            if (num > 32) {
+                const uint64_t w1 = stage[(lane + 32) * NB64_LD + j];
+                pl1 = transpose32((uint32_t)w1, lane);
+                ph1 = transpose32((uint32_t)(w1 >> 32), lane);
+            }
+            const uint64_t i = (b0 + j) * 64 + lane;
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                // plane p at bit 63 - p, then digit num - 1 - p
+                const uint64_t a = h ? (uint64_t)__brev(ph0) << 32 | __brev(ph1) : (uint64_t)__brev(pl0) << 32 | __brev(pl1);
+                const int64_t q = (int64_t)nb_to_bin(a >> (64 - num));
+                const uint64_t mag = (uint64_t)(q < 0 ? -q : q);
+                if (i + 32 * h < n) out[i + 32 * h] = gr_value<double>(mag, exp - e, (q < 0) != (bool)(e & 1));   // :153, :177
+            }
+        }
+        __syncwarp();
+    }
 }
 
 // word counts contributed by a block with recording plane r to plane p
@@ -1360,18 +1431,21 @@ int launch_nb_encode(const T* x, uint64_t n, const void* maxkey, int exp, int B,
         PRODM_CHECK_LAUNCH("k_nb_encode32");
         return PRODM_OK;
     }
-    const unsigned grid = errs_out ? persistent_grid_for((const void*)k_nb_encode<T, true>, th, 0, nblocks, kPartialSlots)
-                                   : grid_for(nblocks * 32, th, 8);
-    if (errs_out) {
-        k_nb_encode<T, true><<<grid, th, 0, st>>>(x, n, (const K*)maxkey, exp, B, (typename Traits<T>::S*)out, stride,
-                                                  partial);
-        PRODM_CHECK_LAUNCH("k_nb_encode");
-        k_reduce_partials<T><<<(B + 8) / 8, 256, 0, st>>>(partial, (int)grid, B, (const K*)maxkey, exp, 2, 1, errs_out);
-        PRODM_CHECK_LAUNCH("k_reduce_partials");
-    } else {
-        k_nb_encode<T, false><<<grid, th, 0, st>>>(x, n, (const K*)maxkey, exp, B, (typename Traits<T>::S*)out, stride,
-                                                   nullptr);
-        PRODM_CHECK_LAUNCH("k_nb_encode");
+    if constexpr (std::is_same<T, double>::value) {
+        if (errs_out) {
+            const unsigned grid = persistent_grid_for((const void*)k_nb_encode64_err, th, 0, nblocks, kPartialSlots);
+            k_nb_encode64_err<<<grid, th, 0, st>>>(x, n, (const K*)maxkey, exp, B, (uint64_t*)out, stride, partial);
+            PRODM_CHECK_LAUNCH("k_nb_encode64_err");
+            k_reduce_partials<T><<<(B + 8) / 8, 256, 0, st>>>(partial, (int)grid, B, (const K*)maxkey, exp, 2, 1, errs_out);
+            PRODM_CHECK_LAUNCH("k_reduce_partials");
+        } else {
+            const uint64_t nch = (nblocks + 8 * NB64_BLOCKS - 1) / (8 * NB64_BLOCKS);
+            const unsigned grid = persistent_grid_for((const void*)k_nb_encode64, th, 0, nch, nch);
+            count_launch();
+            const cudaError_t e = launch_chain(true, k_nb_encode64, dim3(grid), dim3(th), 0, st, x, n, (const K*)maxkey, exp, B,
+                                               (uint64_t*)out, stride);
+            if (e != cudaSuccess) return cuda_status(e, "k_nb_encode64");
+        }
     }
     return PRODM_OK;
 }
@@ -1419,9 +1493,14 @@ int launch_nb_decode(const void* base, uint64_t stride, uint64_t n, const void* 
         PRODM_CHECK_LAUNCH("k_nb_decode32");
         return PRODM_OK;
     }
-    k_nb_decode<T><<<grid_for(nblocks * 32, th, 8), th, 0, st>>>((const typename Traits<T>::S*)base, stride, n,
-                                                                 (const K*)maxkey, exp, s, num, dnum, out);
-    PRODM_CHECK_LAUNCH("k_nb_decode");
+    if constexpr (std::is_same<T, double>::value) {
+        const uint64_t nch = (nblocks + 8 * NB64_BLOCKS - 1) / (8 * NB64_BLOCKS);
+        const unsigned grid = persistent_grid_for((const void*)k_nb_decode64, th, 0, nch, nch);
+        count_launch();
+        const cudaError_t e = launch_chain(true, k_nb_decode64, dim3(grid), dim3(th), 0, st, (const uint64_t*)base, stride, n,
+                                           (const K*)maxkey, exp, s, num, dnum, out);
+        if (e != cudaSuccess) return cuda_status(e, "k_nb_decode64");
+    }
     return PRODM_OK;
 }
 

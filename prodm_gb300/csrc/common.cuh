@@ -319,9 +319,9 @@ __device__ __forceinline__ unsigned long long abs_key(double v) {
 __device__ __forceinline__ uint32_t max_key(uint32_t a, uint32_t b) { return a > b ? a : b; }
 __device__ __forceinline__ unsigned long long max_key(unsigned long long a, unsigned long long b) {
     const uint32_t al = (uint32_t)a, ah = (uint32_t)(a >> 32), bl = (uint32_t)b, bh = (uint32_t)(b >> 32);
-    uint32_t t, less;   // less: all ones where a < b
-    asm("sub.cc.u32 %0, %2, %4;\n\tsubc.cc.u32 %0, %3, %5;\n\tsubc.u32 %1, 0, 0;"
-        : "=&r"(t), "=&r"(less) : "r"(al), "r"(ah), "r"(bl), "r"(bh));
+    uint32_t less;   // all ones where a < b
+    asm("{\n\t.reg .u32 t;\n\tsub.cc.u32 t, %1, %3;\n\tsubc.cc.u32 t, %2, %4;\n\tsubc.u32 %0, 0, 0;\n\t}"
+        : "=r"(less) : "r"(al), "r"(ah), "r"(bl), "r"(bh));
     return (unsigned long long)((bh & less) | (ah & ~less)) << 32 | ((bl & less) | (al & ~less));
 }
 __device__ __forceinline__ float key_to_val(uint32_t k, float) { return __uint_as_float(k); }
