@@ -522,13 +522,16 @@ constexpr int GR_BPW = 32;                       // blocks per warp
 constexpr int GR_CHUNK = GR_WARPS * GR_BPW;      // blocks per CTA
 // The decoders and the first pass have 32 warps with 8 blocks each: a warp's
 // blocks come one after the other, and 8 warps with 32 were fp32 13.2 us for 8.1
-// (decode 65^3), 18.9 for 16.0 (129^3), 76.1 for 75.2 (257^3); first pass 9.2 for
-// 6.7, 9.5 for 8.2 and 35.6 for 35.6. An fp64 warp needs twice the registers, so
+// (decode 65^3), 18.9 for 16.0 (129^3), 42.9 for 40.5 (257 x 257 x 129, 1040
+// chunks); first pass 9.2 for 6.7, 9.5 for 8.2 and (257^3) 35.6 for 35.6. With
+// many chunks the decoder's 8 warps, which load a group of blocks ahead, are
+// faster when all planes are there (150 x 257 x 301: 51 us for 56). An fp64 warp needs twice the registers, so
 // past a chunk an SM it is 8 warps there (decode 257 x 257 x 129 52.3 us for
 // 56.5, first pass 257^3 39.5 for 43.8; before, 65^3 24.9 for 17.9 and 129^3 16.6
 // for 9.5).
 constexpr int GR_WIDE = 32;
 inline bool gr_wide64(unsigned chunks) { return chunks <= (unsigned)kSMs; }
+inline bool gr_wide_decode32(unsigned chunks) { return chunks <= 8u * kSMs; }
 
 // |trunc(ldexp(v, B - exp))| and the sign (GroupedBPEncoder.hpp:41-42). For
 // doubles whose scaled value is not needed (SH false: no error tables) the
@@ -1585,7 +1588,9 @@ int launch_gr_decode(GrSet<T> set, int B, int s, int e, cudaStream_t st) {
     const dim3 grid(gr_number(set));
     if (!grid.x) return PRODM_OK;
     if constexpr (std::is_same<T, float>::value) {
-        PRODM_CHAIN("k_gr_decode32", k_gr_decode32<GR_WIDE>, grid, dim3(GR_WIDE * 32), 0, st, set, B, s, e);
+        const int warps = gr_wide_decode32(grid.x) ? GR_WIDE : GR_WARPS;
+        PRODM_CHAIN("k_gr_decode32", (warps == GR_WIDE ? k_gr_decode32<GR_WIDE> : k_gr_decode32<GR_WARPS>), grid,
+                    dim3(warps * 32), 0, st, set, B, s, e);
     } else {
         const int warps = gr_wide64(grid.x) ? GR_WIDE : GR_WARPS;
         PRODM_CHAIN("k_gr_decode64", (warps == GR_WIDE ? k_gr_decode64<GR_WIDE> : k_gr_decode64<GR_WARPS>), grid,

@@ -134,6 +134,24 @@ __host__ __device__ inline uint32_t fine_of_coarse(uint32_t m, uint32_t n, uint3
     return m == nc - 1 ? n - 1 : 2 * m;
 }
 
+// Coordinates of element idx of a box. A 64-bit division is a hundred
+// instructions, four times a 32-bit one, and two of them per element bounded the
+// kernels that walk a box by elements (copy of 150 x 257 x 301 fp32 44 us, with
+// 32-bit ones 39).
+__device__ __forceinline__ void split3(uint64_t idx, const Box& B, uint32_t& x0, uint32_t& x1, uint32_t& x2) {
+    if ((idx >> 32) == 0) {
+        const uint32_t i = (uint32_t)idx, t = i / B.n[2];
+        x2 = i - t * B.n[2];
+        x0 = t / B.n[1];
+        x1 = t - x0 * B.n[1];
+    } else {
+        const uint64_t t = idx / B.n[2];
+        x2 = (uint32_t)(idx - t * B.n[2]);
+        x0 = (uint32_t)(t / B.n[1]);
+        x1 = (uint32_t)(t - (uint64_t)x0 * B.n[1]);
+    }
+}
+
 // Position of reordered coordinate r in the interleaved order of the level
 // box(F) \ box(C) (row-major walk that skips the coarse box,
 // DirectInterleaver.hpp:23-31).

@@ -166,11 +166,14 @@ inline bool patch_level(const Box& F, const Box& C) {
     return items >= patch_min_items() || items >= (uint64_t)F.n[0] * F.n[1];
 }
 
-template <class T, int PLANE>
+// INPLACE: coef is the reordered box itself (strides o0, o1), where the coarse
+// values are its corner.
+template <class T, int PLANE, bool INPLACE = false>
 __device__ __forceinline__ void decompose_patch_item(const T* __restrict__ in, uint64_t s0, uint64_t s1,
                                                      const Box& F, const Box& C, T* __restrict__ coef,
                                                      T* __restrict__ coarse, uint64_t item, uint32_t lane,
-                                                     typename KeyOf<T>::type& mk, typename KeyOf<T>::type& mc) {
+                                                     typename KeyOf<T>::type& mk, typename KeyOf<T>::type& mc,
+                                                     uint64_t o0 = 0, uint64_t o1 = 0) {
     using K = typename KeyOf<T>::type;
     const uint32_t C0 = C.n[0], C1 = C.n[1], C2 = C.n[2];
     const uint32_t O1 = F.n[1] - C1, P = F.n[2] - C2;   // odd nodes of dims 1 and 2
@@ -195,11 +198,14 @@ __device__ __forceinline__ void decompose_patch_item(const T* __restrict__ in, u
     // kernels issued on 57 % of the cycles (finest level of 513^3 221 us, 204
     // without; of 100 x 500 x 500 49 and 41 us).
     const T* next_row = in + (uint64_t)min(2 * i, F.n[0] - 1) * s0 + (uint64_t)min(2 * b0, F.n[1] - 1) * s1 + xc;
-    T* k00 = coef + level_rank(i, b0, C2, F, C) + c;               // even-even row: odd nodes only
-    T* k01 = coef + level_rank(i, C1 + b0, 0, F, C) + c;
-    T* k10 = coef + level_rank(C0 + i, b0, 0, F, C) + c;
-    const uint64_t to11 = (uint64_t)C1 * F.n[2];                   // row (C0 + i, C1 + b) from (C0 + i, b)
-    T* crow = coarse + ((uint64_t)i * C1 + b0) * C2 + c;
+    auto at = [&](uint32_t r0, uint32_t r1, uint32_t r2) {
+        return coef + (INPLACE ? r0 * o0 + r1 * o1 + r2 : level_rank(r0, r1, r2, F, C)) + c;
+    };
+    T* k00 = at(i, b0, C2);                                        // even-even row: odd nodes only
+    T* k01 = at(i, C1 + b0, 0);
+    T* k10 = at(C0 + i, b0, 0);
+    const uint64_t to11 = C1 * (INPLACE ? o1 : (uint64_t)F.n[2]);  // row (C0 + i, C1 + b) from (C0 + i, b)
+    T* crow = INPLACE ? at(i, b0, 0) : coarse + ((uint64_t)i * C1 + b0) * C2 + c;
     const int lone = (int)lc - (int)c;                             // the lone column from the lane's own
     auto kmax = [](K& m, T v) { m = max_key(abs_key(v), m); };
     // the loads of one step, issued D steps ahead of their use: the four
@@ -316,10 +322,10 @@ __device__ __forceinline__ void decompose_patch_item(const T* __restrict__ in, u
                     }
                 }
             }
-            k00 += P;
-            k01 += F.n[2];
-            k10 += F.n[2];
-            crow += C2;
+            k00 += INPLACE ? o1 : P;
+            k01 += INPLACE ? o1 : F.n[2];
+            k10 += INPLACE ? o1 : F.n[2];
+            crow += INPLACE ? o1 : C2;
             q00 = q02;
             qn00 = qn02;
             h00 = h02;
@@ -348,7 +354,7 @@ __device__ __forceinline__ void decompose_patch_item(const T* __restrict__ in, u
 // are the coefficient plus the interpolation of decompose_patch_item (the
 // row kernels' corner trees, so the output is bit-identical to theirs). Each
 // step's loads are issued a step ahead of their use.
-template <class T, int PLANE>
+template <class T, int PLANE, bool INPLACE = false>   // INPLACE: coef (and coarse) is the compact reordered box
 __device__ __forceinline__ void recompose_patch_item(const T* __restrict__ coarse, const T* __restrict__ coef,
                                                      const Box& F, const Box& C, T* __restrict__ out, uint64_t s0,
                                                      uint64_t s1, uint64_t item, uint32_t lane) {
@@ -367,12 +373,15 @@ __device__ __forceinline__ void recompose_patch_item(const T* __restrict__ coars
     const bool own = c >= P;
     const uint32_t lc = even ? c : P;
     const uint32_t b0 = u * kPatchSteps, b1 = min(b0 + kPatchSteps, C1);
-    const uint64_t cs0 = (uint64_t)C1 * C2;
+    const uint64_t cs1 = INPLACE ? F.n[2] : C2, cs0 = (INPLACE ? F.n[1] : C1) * cs1;
     // (pointers advance from step to step, as in decompose_patch_item)
-    const T* next_q = coarse + (uint64_t)i * cs0 + (uint64_t)b0 * C2 + c;   // coarse row (i, b), (i + 1, b) cs0 behind
-    const T* k00 = coef + level_rank(i, b0, C2, F, C) + c;
-    const T* k01 = coef + level_rank(i, C1 + b0, 0, F, C) + c;
-    const T* k10 = coef + level_rank(C0 + i, b0, 0, F, C) + c;
+    const T* next_q = coarse + (uint64_t)i * cs0 + (uint64_t)b0 * cs1 + c;   // coarse row (i, b), (i + 1, b) cs0 behind
+    auto at = [&](uint32_t r0, uint32_t r1, uint32_t r2) {
+        return coef + (INPLACE ? r0 * cs0 + r1 * cs1 + r2 : level_rank(r0, r1, r2, F, C)) + c;
+    };
+    const T* k00 = at(i, b0, C2);
+    const T* k01 = at(i, C1 + b0, 0);
+    const T* k10 = at(C0 + i, b0, 0);
     const uint64_t to11 = (uint64_t)C1 * F.n[2];
     const int lone = (int)lc - (int)c;
     T* o00 = out + (uint64_t)min(2 * i, F.n[0] - 1) * s0 + (uint64_t)min(2 * b0, F.n[1] - 1) * s1 + 2 * (uint64_t)c;
@@ -382,7 +391,7 @@ __device__ __forceinline__ void recompose_patch_item(const T* __restrict__ coars
     };
     auto load_step = [&](uint32_t b, Step& S) {   // called for b0, b0 + 1, ..
         const bool odd = b < O1, more = b + 1 < C1;
-        const T* q0 = next_q + C2;
+        const T* q0 = next_q + cs1;
         const T* q1 = q0 + cs0;
         const T* k11 = k10 + to11;
         S.q02 = ld && more ? __ldg(q0) : (T)0;
@@ -400,7 +409,7 @@ __device__ __forceinline__ void recompose_patch_item(const T* __restrict__ coars
         S.lc = last && two ? __ldg(k10 + lone) : (T)0;
         S.ld_ = last && two && odd ? __ldg(k11 + lone) : (T)0;
         next_q = q0;
-        k00 += P;
+        k00 += INPLACE ? F.n[2] : P;
         k01 += F.n[2];
         k10 += F.n[2];
     };
