@@ -741,21 +741,22 @@ def run_perbit(shape=(513, 513, 513), levels=7, planes=60, rels=(1e-3, 1e-5, 1e-
     ms = e0.elapsed_time(e1) / steps
     err = float((out - x).abs().max())
 
-    # kernel stages (finest level): algorithmic bytes / event time
+    # kernel stages (all levels in one launch each): algorithmic bytes / event time
     m.set_timing(True)
     step()
     torch.cuda.synchronize()
     st = m.stage_times()
     m.set_timing(False)
-    lel = api.level_dims(shape, levels)[1]
-    n_f = int(lel[levels])
+    lel = [int(n) for n in api.level_dims(shape, levels)[1]]
+    n_f = lel[levels]
     peak, peak_src = measured_peak()
     stage_ms = {}
     for (kind, _), (t, _) in st.items():
         stage_ms[kind] = stage_ms.get(kind, 0.0) + t
     enc_ms = st[("encode", levels)][0]
-    enc_bytes = n_f * 8 + n_f * (planes + 1) // 8
-    dec_ms, dec_bytes = st[("decode", levels)][0], sum(n_f * (int(ix[levels]) + 1) // 8 + n_f * 8 for ix in idxs)
+    enc_bytes = sum(n * 8 + n * (planes + 1) // 8 for n in lel)
+    dec_ms = st[("decode", levels)][0]
+    dec_bytes = sum(n * (int(ix[l]) + 1) // 8 + n * 8 for ix in idxs for l, n in enumerate(lel))
 
     # export: rows -> reference streams on the host
     t0 = time.time()

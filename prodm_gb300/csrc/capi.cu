@@ -1104,8 +1104,8 @@ int mdr_decode_recompose(prodm_mdr* h, T* out, cudaStream_t st) {
         Stage sg(h, 3, 0, st);
         if ((rc = launch_nb_decode_levels(h->dseg, h->dseg_n, h->dseg_chunks, st, true))) return rc;
     }
-    if (!h->nb) {   // every level in one launch (timed as level 0)
-        Stage sg(h, 3, 0, st);
+    if (!h->nb) {
+        Stage sg(h, 3, L, st);   // every level in one launch (timed as the finest level, as in the encoder)
         rc = h->pb ? launch_pb_decode<T>(mdr_pb_set<T>(h), B, 0, 0, st)
                    : launch_gr_decode<T>(mdr_gr_set<T>(h, 0, L), B, 0, 0, st);
         if (rc) return rc;
