@@ -371,10 +371,12 @@ __device__ __forceinline__ W l2_rhs(W sm2, W sm1, W s0, W s1, W s2, uint32_t c, 
 // none in the backward sweep, the dim-1 and dim-0 passes of 513 x 513 x 257
 // took 414 and 260 us, with four and eight and the right-hand sides of four
 // nodes ahead of their chain 325 and 168 us, 272 and 150 with the halving of
-// the right-hand side done on the exponent (FP64 floor 216 and 108 us).
-constexpr int kLineAhead = 4, kLineBack = 8;
+// the right-hand side done on the exponent, and 248 and 131 in one-warp blocks
+// with twelve nodes back (eight 252 and 135; blocks of two warps 255 and 148;
+// FP64 floor 189 and 95).
+constexpr int kLineAhead = 4, kLineBack = 12;
 template <class T, class W>
-__global__ void __launch_bounds__(128) k_l2_line(const T* __restrict__ src, Box S, int d, T* dst, Box D,
+__global__ void __launch_bounds__(32, 16) k_l2_line(const T* __restrict__ src, Box S, int d, T* dst, Box D,
                                                  const W* __restrict__ cp, const W* __restrict__ lo_w,
                                                  const W* __restrict__ inv_den) {
     pdl_wait();
@@ -879,7 +881,7 @@ template void mass_factors<double>(uint32_t, double*);
 template <class T>
 int launch_l2_correction(const T* fnat, const Box& F, T* t1, T* t2, T* z, const T* const tabs[3], cudaStream_t st,
                          const T* coef, const Box* C) {
-    const int th = 128;
+    const int th = 32;
     Box a = F;
     T* bufs[3] = {t1, t2, z};
     {
