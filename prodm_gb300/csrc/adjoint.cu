@@ -159,8 +159,9 @@ __device__ __forceinline__ void adj_lone_item(const T* __restrict__ g, const Box
     }
 }
 
+// (one-warp blocks: 257^3 fp32 31.9 us for the finest level, 33.8 in blocks of eight)
 template <class T, bool COEF>
-__global__ void __launch_bounds__(256, 2) k_adj_level(const T* __restrict__ g, Box F, Box C, T* __restrict__ gcoef,
+__global__ void __launch_bounds__(32, 16) k_adj_level(const T* __restrict__ g, Box F, Box C, T* __restrict__ gcoef,
                                                       T* __restrict__ gc) {
     pdl_wait();   // the gradient comes from the previous launch
     pdl_release();
@@ -176,10 +177,10 @@ __global__ void __launch_bounds__(256, 2) k_adj_level(const T* __restrict__ g, B
 template <class T, bool COEF>
 int launch_adj_level(const T* g, const Box& F, const Box& C, T* gcoef, T* gc, cudaStream_t st) {
     uint64_t body;
-    const uint64_t need = (adj_items(F, C, body) + 7) / 8;
-    const unsigned grid = persistent_grid_for((const void*)k_adj_level<T, COEF>, 256, 0, need, need);
+    const uint64_t need = adj_items(F, C, body);
+    const unsigned grid = persistent_grid_for((const void*)k_adj_level<T, COEF>, 32, 0, need, need);
     count_launch();
-    const cudaError_t e = launch_chain(true, k_adj_level<T, COEF>, dim3(grid), dim3(256), 0, st, g, F, C, gcoef, gc);
+    const cudaError_t e = launch_chain(true, k_adj_level<T, COEF>, dim3(grid), dim3(32), 0, st, g, F, C, gcoef, gc);
     if (e != cudaSuccess) return cuda_status(e, "k_adj_level");
     return PRODM_OK;
 }
