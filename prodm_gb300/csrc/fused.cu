@@ -863,6 +863,13 @@ static int ws_decode_warps() {
     return n == 6 ? 6 : (n == 8 ? 8 : 5);
 }
 
+// The attribute belongs to the kernel, not to the call: set to one figure that
+// covers every call, so that threads with different row lengths do not lower it
+// for each other between this and their launch.
+static cudaError_t allow_smem(const void* kern, size_t smem) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max((int)smem, 220 * 1024));
+}
+
 template <int RS, int ND>
 static int launch_fused_ws(const CUtensorMap& map, uint32_t bw, const void* maxkey, const uint8_t* dnum,
                            const float* coarse, const Box& F, const Box& C, float* out, uint64_t s0, uint64_t s1,
@@ -870,7 +877,7 @@ static int launch_fused_ws(const CUtensorMap& map, uint32_t bw, const void* maxk
     const uint32_t tld = ws_tile_blocks(F, ND), nr = ws_unit_rows(ND);
     const size_t smem = (size_t)2 * 32 * RS * 4 + (size_t)2 * tld * CB_LD * 4;
     const void* kern = (const void*)k_decode_recompose_nb32_ws<RS, ND>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute");
     const uint64_t need = ((uint64_t)F.n[0] * F.n[1] + nr - 1) / nr;
     const unsigned grid = persistent_grid_for(kern, 512, smem, need, need);
@@ -892,7 +899,7 @@ static int launch_fused_tma(const CUtensorMap& map, uint32_t bw, const void* max
     const size_t smem = (size_t)32 * RS * 4 + (size_t)fused_unit_blocks_rows(F, nr) * CB_LD * 4;
     const auto kernel = nr == 8 ? k_decode_recompose_nb32_tma<RS, false> : k_decode_recompose_nb32_tma<RS, true>;
     const void* kern = (const void*)kernel;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute");
     const uint64_t rows = (uint64_t)F.n[0] * F.n[1];
     const uint64_t need = (rows + nr - 1) / nr;
@@ -988,7 +995,7 @@ static int launch_tma_multi(const FusedSeg* segs, int nseg, uint64_t total_units
                             int* status, cudaStream_t st) {
     const size_t smem = (size_t)32 * RS * 4 + (size_t)tld * CB_LD * 4;
     const void* kern = (const void*)k_decode_recompose_nb32_tma_multi<RS>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute");
     uint64_t cap = persistent_grid_for(kern, 256, smem, total_units, total_units);
     if (ctas_per_sm) cap = std::min<uint64_t>(cap, (uint64_t)device_sms() * ctas_per_sm);
@@ -1014,7 +1021,7 @@ int launch_decode_recompose_nb32_ws_multi(const FusedSeg* segs, int nseg, uint64
     constexpr int RS = kWsMultiStride;
     const size_t smem = (size_t)2 * 32 * RS * 4 + (size_t)2 * tld * CB_LD * 4;
     const void* kern = (const void*)k_decode_recompose_nb32_ws_multi<RS, 5>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute");
     const unsigned grid = persistent_grid_for(kern, 512, smem, total_units, total_units);
     k_decode_recompose_nb32_ws_multi<RS, 5><<<grid, 512, smem, st>>>(segs, nseg, total_units, tld, status,

@@ -492,6 +492,7 @@ __global__ void __launch_bounds__(32, 16) k_l2_line(const T* __restrict__ src, B
 // (coarse nodes of rows inside the coarse box are zero), so no natural-order
 // copy is needed; else from a natural field.
 constexpr int kRowsTile = 8, kRowsLd = 2 * kRowsTile + 1;
+constexpr int kL2RowsKeep = 200 * 1024;   // shared memory that rows may stay in
 constexpr int l2_ring(bool kept) { return kept ? 3 : 2; }   // tiles
 template <class T>
 inline size_t l2_rows_smem(uint32_t nc, bool kept) {
@@ -903,14 +904,14 @@ int launch_l2_correction(const T* fnat, const Box& F, T* t1, T* t2, T* z, const 
         // 54 warps an SM (513 x 513 x 257) it is 2030 against 1797.
         const size_t keep = l2_rows_smem<T>(nc, true);
         const bool kept = keep <= 36 * 1024 ||
-                          (keep <= 200 * 1024 && (uint64_t)(227 * 1024 / (keep + 1024)) * kSMs >= grid.x);
+                          (keep <= (size_t)kL2RowsKeep && (uint64_t)(227 * 1024 / (keep + 1024)) * kSMs >= grid.x);
         const size_t smem = l2_rows_smem<T>(nc, kept);
         const auto kernel = coef ? (kept ? k_l2_rows<T, true, true> : k_l2_rows<T, true, false>)
                                  : (kept ? k_l2_rows<T, false, true> : k_l2_rows<T, false, false>);
         cudaError_t e;
-        if (smem > 48 * 1024 &&
-            (e = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
-                cudaSuccess)
+        // (the most any call needs, not this call's: another thread may launch the kernel in between)
+        if (smem > 48 * 1024 && (e = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                          kL2RowsKeep)) != cudaSuccess)
             return cuda_status(e, "cudaFuncSetAttribute");
         count_launch();
         // not launched ahead: its one-warp blocks would gather on the SMs that
