@@ -741,8 +741,10 @@ __global__ void __launch_bounds__(256) k_interleave_rows(T* __restrict__ data, u
 // ---------------------------------------------------------------------------
 // host launchers
 // ---------------------------------------------------------------------------
-// one warp per row, 8 warps per CTA; enough CTAs for full occupancy
-unsigned row_threads(uint32_t) { return 256; }
+// one warp per row, four warps per CTA (f64 recompositions of 513 x 257 x 257's
+// small levels 86 us, with eight 90 and with one 92; fp32 1 % from eight, with
+// two 10 % slower); enough CTAs for full occupancy
+unsigned row_threads(uint32_t) { return 128; }
 // PRODM_DECOMPOSE_PATCH=0 keeps every level on the row kernels (decomposition and
 // recomposition; read per launch)
 bool decompose_patch_enabled() {
