@@ -2038,6 +2038,15 @@ int prodm_mdr_level_info(prodm_mdr* h, uint32_t* hs, double* hb, double* he, voi
     return PRODM_OK;
 }
 
+// the lossless stage's stored plane sizes, nl * B, on the host: the loaded
+// metadata's or those of the last refactor. NULL where there are none: the
+// stage was switched on before the first refactor, or a refactor failed in it.
+static const uint32_t* ll_stored_sizes(const prodm_mdr* h) {
+    const std::vector<uint32_t>& s = h->from_files ? h->ll_stored : h->ll_kept;
+    return s.size() == (size_t)(h->g.L + 1) * h->B ? s.data() : nullptr;
+}
+static int ll_no_sizes() { return fail(PRODM_EINVAL, "the lossless stage has no stored sizes: refactor first"); }
+
 int prodm_mdr_metadata(prodm_mdr* h, uint8_t* buf, size_t cap, size_t* len, void* stream) {
     if (!h || !len) return fail(PRODM_EINVAL, "NULL pointer");
     const int L = h->g.L, B = h->B, nl = L + 1, nd = h->g.ndims;
@@ -2047,6 +2056,7 @@ int prodm_mdr_metadata(prodm_mdr* h, uint8_t* buf, size_t cap, size_t* len, void
     *len = need;
     if (!buf) return PRODM_OK;
     if (cap < need) return fail(PRODM_EINVAL, "metadata buffer too small");
+    if (h->ll_latter >= 0 && !ll_stored_sizes(h)) return ll_no_sizes();
     std::vector<uint32_t> sz(nl * B);
     std::vector<uint8_t> bd(nl * h->es);
     std::vector<double> er(nl * (B + 1));
@@ -2243,7 +2253,9 @@ int prodm_mdr_export_level(prodm_mdr* h, int level, void* dst, uint64_t cap, int
     }
     // lossless stage: the level's stored streams, compressed straight into
     // their places; device memory and pinned memory in stream order
-    const uint32_t* stored = (h->from_files ? h->ll_stored : h->ll_kept).data() + (size_t)level * B;
+    const uint32_t* stored = ll_stored_sizes(h);
+    if (!stored) return ll_no_sizes();
+    stored += (size_t)level * B;
     uint64_t total = 0;
     for (int p = 0; p < B; p++) total += stored[p];
     if (len) *len = total;
