@@ -66,6 +66,14 @@ int prodm_version(void);
  * a pool of this library, which keeps up to 1 GiB per device between calls;
  * this gives back what is not in use. */
 int prodm_trim_scratch(void);
+/* Stream capture: kernels and copies of a captured call run at each replay,
+ * what the call noted on the host happens once. Refused with
+ * PRODM_EUNSUPPORTED on a capturing stream, before anything is queued:
+ * decomposition, recomposition and packed recomposition (and its adjoint) in
+ * the orthogonal basis, progressive decoding of grouped and per-bit streams,
+ * a retrieval that still has loaded planes to unpack (one before the capture
+ * unpacks them), and the export of a level with the lossless stage. Calls that
+ * wait for the stream fail in a capture with PRODM_ECUDA. */
 
 /* ---------------------------------------------------------------------------
  * Level geometry

@@ -69,6 +69,14 @@ cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
     return cudaMallocFromPoolAsync(p, bytes, pool, st);
 }
 
+int refuse_capture(cudaStream_t st, const char* call) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    const cudaError_t e = cudaStreamIsCapturing(st, &cs);
+    if (e != cudaSuccess) return cuda_status(e, call);
+    if (cs == cudaStreamCaptureStatusNone) return PRODM_OK;
+    return fail(PRODM_EUNSUPPORTED, std::string(call) + ": not during a stream capture");
+}
+
 int device_sms() {
     static std::mutex mu;
     static std::vector<std::pair<int, int>> cache;
@@ -265,6 +273,7 @@ int decompose_impl(T* data, int ndims, const uint32_t* dims, int L, const uint32
     if ((rc = view_strides(ndims, dims, strides, s0, s1))) return rc;
     if (L == 0) return PRODM_OK;
     const bool orth = basis == PRODM_BASIS_ORTHOGONAL;
+    if (orth && (rc = refuse_capture(st, "decomposition in the orthogonal basis"))) return rc;
     const Box& top = g.box[L];
     Workspace ws(wsp, wsb, st);
     ws.reserve(top.size() * sizeof(T));
@@ -281,8 +290,7 @@ int decompose_impl(T* data, int ndims, const uint32_t* dims, int L, const uint32
         os = orth_take(ws, top, sizeof(T));
         std::vector<T> tab = build_tabs<T>(g, toff);
         dtab = (T*)ws.take(tab.size() * sizeof(T));
-        // (a pageable source is staged before the call returns)
-        PRODM_CUDA(cudaMemcpyAsync(dtab, tab.data(), tab.size() * sizeof(T), cudaMemcpyHostToDevice, st));
+        if ((rc = launch_put(dtab, tab.data(), tab.size() * sizeof(T), st))) return rc;
     }
     for (int step = 0; step < L; step++) {
         const int l = inverse ? step + 1 : L - step;
@@ -571,9 +579,11 @@ int progressive_decode_impl(prodm_decoder* h, const uint8_t* blob, const uint32_
     }
     if (n == 0) return fail(PRODM_EINVAL, "decode: n must be >= 1");
     if (s < 0 || num < 0 || s + num > B) return fail(PRODM_EINVAL, "decode: planes outside [0, total_bitplanes)");
+    int rc;
+    // grouped and per-bit levels carry state from call to call
+    if (h->enc != PRODM_ENC_NEGABINARY && (rc = refuse_capture(st, "progressive decode"))) return rc;
     if (h->enc == PRODM_ENC_PERBIT) return pb_progressive_decode<T>(h, blob, hs, n, exp, s, num, level, B, out, st);
     const uint64_t nb = nblocks_of(dtype, n);
-    int rc;
     if (h->enc == PRODM_ENC_NEGABINARY) {
         for (int i = 0; i < num; i++)
             if (hs[i] != nb * sizeof(T)) return fail(PRODM_ECORRUPT, "decode: negabinary stream size mismatch");
@@ -590,7 +600,6 @@ int progressive_decode_impl(prodm_decoder* h, const uint8_t* blob, const uint32_
     if ((int)h->levels.size() <= level) h->levels.resize(level + 1);
     auto& L = h->levels[level];
     const uint64_t nch = gr_nchunks(nb);
-    uint64_t hdr = 0;
     if (!L.have) {
         if (s != 0) return fail(PRODM_EINVAL, "decode: the first call for a level must start at plane 0");
         if (hs[0] < 4 + nb) return fail(PRODM_ECORRUPT, "decode: stream 0 shorter than its header");
@@ -617,38 +626,28 @@ int progressive_decode_impl(prodm_decoder* h, const uint8_t* blob, const uint32_
         L.have = true;
         L.n = n;
         L.B = B;
-        hdr = 4 + nb;
     } else if (L.n != n || L.B != B) {
         return fail(PRODM_EINVAL, "decode: level shape changed between calls");
     }
-    // unpack planes [s, s+num) into aligned scratch
-    std::vector<uint64_t> off(num), nw(num);
+    // unpack planes [s, s+num) into aligned scratch, and the table of the planes' addresses behind them
+    if (num > 64) return fail(PRODM_EINVAL, "decode: grouped streams hold at most 64 planes");
+    UnpackSet up;
+    up.n = num;
     uint64_t o = 0, maxw = 0;
     for (int i = 0; i < num; i++) {
-        uint64_t skip = (i == 0 && s == 0) ? hdr : 0;
-        if (s == 0 && i == 0 && hdr == 0) skip = 4 + nb;
+        const uint64_t skip = i == 0 && s == 0 ? 4 + nb : 0;   // stream 0's header
         if (hs[i] < skip || (hs[i] - skip) % sizeof(T)) return fail(PRODM_ECORRUPT, "decode: stream size not word aligned");
-        off[i] = o + skip;
-        nw[i] = (hs[i] - skip) / sizeof(T);
-        maxw = nw[i] > maxw ? nw[i] : maxw;
+        up.off[i] = o + skip;
+        up.words[i] = (hs[i] - skip) / sizeof(T);
+        maxw = up.words[i] > maxw ? up.words[i] : maxw;
         o += hs[i];
     }
-    // staged planes first, then the (8-byte) arrays on a 256-byte boundary: the
-    // streams' offsets and word counts, the staged planes, every plane
     const uint64_t plane_bytes = Workspace::align((uint64_t)num * (maxw + 1) * sizeof(T));
-    std::vector<uint64_t> tab(3 * num + B, 0);
     Scratch tmp(st);
-    PRODM_CUDA(tmp.alloc(plane_bytes + tab.size() * 8));
-    uint8_t* planes = tmp.get();
-    uint64_t* dtab = (uint64_t*)(planes + plane_bytes);
-    for (int i = 0; i < num; i++) {
-        tab[i] = off[i];
-        tab[num + i] = nw[i];
-        tab[2 * num + i] = tab[3 * num + s + i] = (uint64_t)(uintptr_t)(planes + (uint64_t)i * (maxw + 1) * sizeof(T));
-    }
-    PRODM_CUDA(cudaMemcpyAsync(dtab, tab.data(), tab.size() * 8, cudaMemcpyHostToDevice, st));
-    void** dptr = (void**)(dtab + 3 * num);
-    if ((rc = launch_unpack_planes(blob, dtab, dtab + num, num, ws_, (void* const*)(dtab + 2 * num), maxw, st))) return rc;
+    PRODM_CUDA(tmp.alloc(plane_bytes + B * sizeof(void*)));
+    void** dptr = (void**)(tmp.get() + plane_bytes);
+    for (int i = 0; i < num; i++) up.dst[i] = tmp.get() + (uint64_t)i * (maxw + 1) * sizeof(T);
+    if ((rc = launch_unpack_planes(blob, up, ws_, dptr + s, st))) return rc;
     GrSet<T> set{1, {}};
     set.seg[0].y = out;
     set.seg[0].rbs = L.rbs;
@@ -918,6 +917,7 @@ int mdr_alloc_all(prodm_mdr* h) {
         for (int l = 0; l <= L; l++)
             for (int p = 0; p < B; p++) sz[l * B + p] = (uint32_t)(h->nblocks[l] * es);
         PRODM_CUDA(cudaMemcpy(h->sizes, sz.data(), sz.size() * 4, cudaMemcpyHostToDevice));
+        PRODM_CUDA(cudaMemcpy(h->rsizes, sz.data(), sz.size() * 4, cudaMemcpyHostToDevice));   // (fixed)
     } else if (h->pb) {
         if ((rc = h->alloc((void**)&h->pbcounts, (L + 1) * 64 * 4))) return rc;
         if ((rc = h->alloc((void**)&h->pbstatus, (L + 1) * 4))) return rc;
@@ -1164,6 +1164,18 @@ int mdr_interpret(prodm_mdr* h, double tol, int interp, int est, double s, cudaS
                                h->index, 0, h->rsz, st, true, early, max_est ? (const T*)h->bounds : nullptr);
 }
 
+// planes of a level that lie completely inside its loaded prefix
+int planes_complete(const prodm_mdr* h, int l) {
+    uint64_t off = 0;
+    int complete = 0;
+    for (int p = 0; p < h->B; p++) {
+        off += h->hsizes[l * h->B + p];
+        if (off > h->loaded[l]) break;
+        complete = p + 1;
+    }
+    return complete;
+}
+
 // per-bit levels loaded from files: parse the planes that lie completely
 // inside the loaded prefixes and are not parsed yet into the levels' rows, the
 // finest level's CTAs first and all levels together
@@ -1180,13 +1192,7 @@ int pb_parse_loaded(prodm_mdr* h, cudaStream_t st) {
             if ((rc = launch_pb_init_unseen(rows + (uint64_t)(B + 1) * rw, rows + (uint64_t)B * rw, n, st))) return rc;
             h->header_done[l] = 1;
         }
-        uint64_t off = 0;
-        int complete = 0;
-        for (int p = 0; p < B; p++) {
-            off += h->hsizes[l * B + p];
-            if (off <= h->loaded[l]) complete = p + 1;
-            else break;
-        }
+        const int complete = planes_complete(h, l);
         const int first = (int)h->unpacked[l];
         if (complete <= first) continue;
         PbParseJob job;
@@ -1239,6 +1245,12 @@ int mdr_unpack_loaded(prodm_mdr* h, cudaStream_t st) {
     const int L = h->g.L, B = h->B;
     const int wb = (int)h->es;
     int rc;
+    // the host notes which planes are unpacked, so it happens now or not at all
+    for (int l = 0; l <= L; l++)
+        if (h->lfile[l] && planes_complete(h, l) > (int)h->unpacked[l]) {
+            if ((rc = refuse_capture(st, "unpacking of loaded level files"))) return rc;
+            break;
+        }
     if (h->pb) return pb_parse_loaded(h, st);
     for (int l = 0; l <= L; l++) {
         if (!h->lfile[l]) continue;
@@ -1252,35 +1264,22 @@ int mdr_unpack_loaded(prodm_mdr* h, cudaStream_t st) {
             h->header_done[l] = 1;
         }
         // planes fully loaded
-        uint64_t off = 0;
-        int complete = 0;
-        for (int p = 0; p < B; p++) {
-            off += h->hsizes[l * B + p];
-            if (off <= h->loaded[l]) complete = p + 1;
-            else break;
-        }
-        int first = (int)h->unpacked[l];
+        const int complete = planes_complete(h, l);
+        const int first = (int)h->unpacked[l];
         if (complete <= first) continue;
-        int num = complete - first;
-        std::vector<uint64_t> hostv(3 * num);
+        UnpackSet up;
+        up.n = complete - first;
         uint64_t o = 0;
         for (int p = 0; p < first; p++) o += h->hsizes[l * B + p];
-        uint64_t maxw = 0;
-        for (int i = 0; i < num; i++) {
-            int p = first + i;
-            uint64_t skip = p == 0 ? hdr : 0;
-            hostv[i] = o + skip;
-            hostv[num + i] = (h->hsizes[l * B + p] - skip) / h->es;
-            hostv[2 * num + i] = (uint64_t)(uintptr_t)(h->streams + h->lvl_byte_off[l] + (uint64_t)p * h->plane_cap[l] * h->es);
-            maxw = hostv[num + i] > maxw ? hostv[num + i] : maxw;
+        for (int i = 0; i < up.n; i++) {
+            const int p = first + i;
+            const uint64_t skip = p == 0 ? hdr : 0;
+            up.off[i] = o + skip;
+            up.words[i] = (h->hsizes[l * B + p] - skip) / h->es;
+            up.dst[i] = h->streams + h->lvl_byte_off[l] + (uint64_t)p * h->plane_cap[l] * h->es;
             o += h->hsizes[l * B + p];
         }
-        uint64_t* dv;
-        PRODM_CUDA(scratch_alloc((void**)&dv, hostv.size() * 8, st));
-        PRODM_CUDA(cudaMemcpyAsync(dv, hostv.data(), hostv.size() * 8, cudaMemcpyHostToDevice, st));
-        rc = launch_unpack_planes(h->lfile[l], dv, dv + num, num, wb, (void* const*)(dv + 2 * num), maxw, st);
-        cudaFreeAsync(dv, st);
-        if (rc) return rc;
+        if ((rc = launch_unpack_planes(h->lfile[l], up, wb, nullptr, st))) return rc;
         h->unpacked[l] = complete;
     }
     return PRODM_OK;
@@ -1638,6 +1637,7 @@ int packed_pair_impl(const T* in, int ndims, const uint32_t* dims, int L, T* out
         return PRODM_OK;
     }
     const bool orth = basis == PRODM_BASIS_ORTHOGONAL;
+    if (orth && (rc = refuse_capture(st, "packed recomposition in the orthogonal basis"))) return rc;
     const size_t cb = g.box[L - 1].size() * sizeof(T);
     Workspace ws(wsp, wsb, st);
     packed_pair_reserve(ws, g, basis, sizeof(T));
@@ -1654,8 +1654,7 @@ int packed_pair_impl(const T* in, int ndims, const uint32_t* dims, int L, T* out
         s_b = (T*)ws.take((uint64_t)F.n[0] * F.n[1] * C.n[2] * sizeof(T));
         s_w = (T*)ws.take(F.size() * sizeof(T));
         s_u = (T*)ws.take(C.size() * sizeof(T));
-        // (a pageable source is staged before the call returns)
-        PRODM_CUDA(cudaMemcpyAsync(dtab, tab.data(), tab.size() * sizeof(T), cudaMemcpyHostToDevice, st));
+        if ((rc = launch_put(dtab, tab.data(), tab.size() * sizeof(T), st))) return rc;
     }
     auto tabs_of = [&](int l, const T* (&t)[3]) {
         for (int d = 0; d < 3; d++) t[d] = dtab + toff[l * 3 + d];
@@ -2207,10 +2206,9 @@ static int mdr_lossless_sizes(prodm_mdr* h, cudaStream_t st) {
     std::vector<uint32_t> raw(nl * B), stored(nl * B), comp(nl * B);
     h->ll_raw.clear();
     h->ll_kept.clear();
-    if (h->nb) {   // fixed raw sizes (the refactor does not rewrite them)
+    if (h->nb) {   // fixed raw sizes, in rsizes already
         for (int l = 0; l < nl; l++)
             for (int p = 0; p < B; p++) raw[l * B + p] = (uint32_t)(h->nblocks[l] * h->es);
-        PRODM_CUDA(cudaMemcpyAsync(h->rsizes, raw.data(), nl * B * 4, cudaMemcpyHostToDevice, st));
     } else {
         PRODM_CUDA(cudaMemcpyAsync(h->rsizes, h->sizes, nl * B * 4, cudaMemcpyDeviceToDevice, st));
         PRODM_CUDA(cudaMemcpyAsync(raw.data(), h->sizes, nl * B * 4, cudaMemcpyDeviceToHost, st));
@@ -2227,7 +2225,7 @@ static int mdr_lossless_sizes(prodm_mdr* h, cudaStream_t st) {
                                                     h->ll_flags.data() + (size_t)l * B);
         for (int p = 0; p < B; p++) stored[l * B + p] = h->ll_flags[(size_t)l * B + p] ? comp[l * B + p] : raw[l * B + p];
     }
-    PRODM_CUDA(cudaMemcpyAsync(h->sizes, stored.data(), nl * B * 4, cudaMemcpyHostToDevice, st));
+    if ((rc = launch_put(h->sizes, stored.data(), nl * B * 4, st))) return rc;
     h->ll_raw = raw;
     h->ll_kept = stored;
     return PRODM_OK;
@@ -2263,12 +2261,13 @@ int prodm_mdr_export_level(prodm_mdr* h, int level, void* dst, uint64_t cap, int
     if (cap < total) return fail(PRODM_EINVAL, "export buffer too small");
     if (h->from_files && (h->ll_zstd || h->ll_expanded[level] < B || (!h->nb && (int)h->unpacked[level] < B)))
         return fail(PRODM_EINVAL, "export_level: the level's planes are not all loaded and expanded");
+    int rc = refuse_capture(st, "export of a level with the lossless stage");
+    if (rc) return rc;
     const std::vector<uint32_t>& raw = h->from_files ? h->hsizes : h->ll_raw;
-    if (h->from_files)
-        PRODM_CUDA(cudaMemcpyAsync(h->rsizes, raw.data(), (L + 1) * B * 4, cudaMemcpyHostToDevice, st));
+    if (h->from_files && !h->nb && (rc = launch_put(h->rsizes, raw.data(), (L + 1) * B * 4, st))) return rc;
     Scratch mem(st), host(st);
     std::vector<LlPart> parts;
-    int rc = raw_streams(h, level, level, raw.data(), mem, parts, st);
+    rc = raw_streams(h, level, level, raw.data(), mem, parts, st);
     if (rc) return rc;
     if (dst_is_host) PRODM_CUDA(host.alloc(total));
     uint8_t* out = dst_is_host ? host.get() : (uint8_t*)dst;

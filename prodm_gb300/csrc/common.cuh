@@ -56,6 +56,11 @@ class Scratch {   // one allocation, freed on its stream
     cudaStream_t st_;
 };
 
+// Refuses a stream that is being captured: for calls that decide on the host
+// what to queue from state which the captured work would change later, once per
+// replay, and for calls that wait.
+int refuse_capture(cudaStream_t st, const char* call);
+
 // GB300's SM count (2 dies x 76): the fallback when the device cannot be
 // queried and the basis of fixed buffer sizes (kPartialSlots); grids are
 // sized from the current device's own count (device_sms)

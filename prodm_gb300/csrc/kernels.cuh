@@ -289,8 +289,15 @@ int read_file_range(FileStaging*& fs, const char* path, uint64_t file_off, uint6
 // pack.cu
 int launch_gr_pack(const void* planes, uint64_t cap, const uint32_t* sizes, int B, uint64_t nblocks, const uint8_t* rbs,
                    int word_bytes, uint8_t* dst, cudaStream_t st);
-int launch_unpack_planes(const uint8_t* src, const uint64_t* src_off, const uint64_t* nwords, int nplanes,
-                         int word_bytes, void* const* dst, uint64_t max_words, cudaStream_t st);
+// a table of the caller's frame to device memory (both 4-byte aligned, a multiple of 4 bytes)
+int launch_put(void* dst, const void* src, size_t bytes, cudaStream_t st);
+// planes of one level's streams (byte offset and words of each behind src) to aligned rows
+struct UnpackSet {
+    int n;
+    uint64_t off[64], words[64];
+    void* dst[64];
+};
+int launch_unpack_planes(const uint8_t* src, const UnpackSet& set, int word_bytes, void** table, cudaStream_t st);
 template <class T>
 int launch_maxabs(const T* x, uint64_t n, void* maxkey, cudaStream_t st);
 template <class T>

@@ -352,7 +352,11 @@ struct ZJob {
     uint8_t* extra = nullptr;
     uint64_t chunks = 0;
     cudaStream_t st;
+    bool copying = false;
     explicit ZJob(cudaStream_t s) : mem(s), st(s) {}
+    ~ZJob() {
+        if (copying) cudaStreamSynchronize(st);
+    }
     // room for n streams of `chunks` chunks in all
     int reserve(size_t n, uint64_t nchunks, uint64_t extra_bytes) {
         chunks = nchunks;
@@ -367,8 +371,17 @@ struct ZJob {
         extra = base + a + 2 * b + c + 256;
         return PRODM_OK;
     }
-    int upload(const std::vector<ZStream>& h) {   // (staged before the call returns)
+    // the descriptors by value (the call may end before they are used), or for a
+    // call that ends in wait() by a copy, which `h` has to outlive this job for
+    int put(const std::vector<ZStream>& h) { return launch_put(mem.get(), h.data(), h.size() * sizeof(ZStream), st); }
+    int upload(const std::vector<ZStream>& h) {
+        copying = true;
         PRODM_CUDA(cudaMemcpyAsync(mem.get(), h.data(), h.size() * sizeof(ZStream), cudaMemcpyHostToDevice, st));
+        return PRODM_OK;
+    }
+    int wait() {
+        PRODM_CUDA(cudaStreamSynchronize(st));
+        copying = false;
         return PRODM_OK;
     }
 };
@@ -407,8 +420,7 @@ int ll_sizes(const std::vector<LlPart>& parts, uint32_t* h_comp, cudaStream_t st
     if (rc || (rc = j.upload(ss))) return rc;
     if ((rc = launch_zcb_count(j.ss, (int)ss.size(), j.chunks, j.csize, j.coff, j.outsz, st))) return rc;
     PRODM_CUDA(cudaMemcpyAsync(h_comp, j.outsz, ss.size() * 4, cudaMemcpyDeviceToHost, st));
-    PRODM_CUDA(cudaStreamSynchronize(st));
-    return PRODM_OK;
+    return j.wait();
 }
 
 int ll_store(const std::vector<LlPart>& parts, cudaStream_t st) {
@@ -441,7 +453,7 @@ int ll_store(const std::vector<LlPart>& parts, cudaStream_t st) {
             ss[i].dst = j.extra + at[i];
         }
     ss.insert(ss.end(), copies.begin(), copies.end());
-    if ((rc = j.upload(ss))) return rc;
+    if ((rc = j.put(ss))) return rc;
     if (nz) {
         if ((rc = launch_zcb_count(j.ss, (int)nz, chunks, j.csize, j.coff, j.outsz, st))) return rc;
         if ((rc = launch_zcb_write(j.ss, (int)nz, chunks, j.csize, j.coff, st))) return rc;
@@ -464,7 +476,7 @@ int ll_raw_sizes(std::vector<LlPart>& parts, cudaStream_t st) {
         k_zcb_headers<<<grid_for(hdr.size(), 256), 256, 0, st>>>(j.ss, (int)ss.size(), j.extra);
         PRODM_CHECK_LAUNCH("k_zcb_headers");
         PRODM_CUDA(cudaMemcpyAsync(hdr.data(), j.extra, hdr.size(), cudaMemcpyDeviceToHost, st));
-        PRODM_CUDA(cudaStreamSynchronize(st));
+        if ((rc = j.wait())) return rc;
     }
     size_t k = 0;
     for (LlPart& p : parts) {
@@ -516,12 +528,12 @@ int ll_expand(const std::vector<LlPart>& parts, cudaStream_t st) {
     ss.insert(ss.end(), copies.begin(), copies.end());
     if ((rc = j.upload(ss))) return rc;
     if (ncopy && (rc = launch_copies(j.ss + nz, ss.data() + nz, ncopy, st))) return rc;
-    if (!nz) return PRODM_OK;
+    if (!nz) return j.wait();
     PRODM_CUDA(cudaMemsetAsync(j.status, 0, 4, st));
     if ((rc = launch_zcb_read(j.ss, (int)nz, chunks, j.status, st))) return rc;
     int hstat = 0;
     PRODM_CUDA(cudaMemcpyAsync(&hstat, j.status, 4, cudaMemcpyDeviceToHost, st));
-    PRODM_CUDA(cudaStreamSynchronize(st));
+    if ((rc = j.wait())) return rc;
     if (hstat) return fail(PRODM_ECORRUPT, "lossless: malformed compressed chunk");
     return PRODM_OK;
 }

@@ -5,6 +5,8 @@
 // streams of planes 0..B-1 concatenated; for the grouped encoder stream 0 is
 // [u32 nblocks][u8 rb x nblocks][words] (GroupedBPEncoder.hpp:370-377), so
 // every later word may sit at any byte offset.
+#include <cstring>
+
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -55,13 +57,15 @@ __global__ void k_gr_pack(const W* __restrict__ planes, uint64_t cap, const uint
     for (uint64_t w = t0; w < nw; w += ts) store_bytes<W>(dst + off + w * sizeof(W), src[w]);
 }
 
+// the planes travel in the launch; table (nullable) receives their addresses
 template <class W>
-__global__ void k_unpack_planes(const uint8_t* __restrict__ src, const uint64_t* __restrict__ src_off,
-                                const uint64_t* __restrict__ nwords, W* const* __restrict__ dst) {
+__global__ void k_unpack_planes(const uint8_t* __restrict__ src, const __grid_constant__ UnpackSet set,
+                                void** __restrict__ table) {
     const int p = blockIdx.y;
-    const uint64_t nw = nwords[p];
-    const uint8_t* s = src + src_off[p];
-    W* d = dst[p];
+    const uint64_t nw = set.words[p];
+    const uint8_t* s = src + set.off[p];
+    W* d = (W*)set.dst[p];
+    if (table && blockIdx.x == 0 && threadIdx.x == 0) table[p] = d;
     for (uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < nw; w += (uint64_t)gridDim.x * blockDim.x)
         d[w] = load_bytes<W>(s + w * sizeof(W));
 }
@@ -99,7 +103,57 @@ __global__ void k_fill_u32(uint32_t* dst, uint64_t n, uint32_t v) {
         dst[i] = v;
 }
 
+// Tables made on the host for one call (factors, sizes, stream descriptors)
+// travel in launches of their own where nothing waits for the call's end. An asynchronous copy from
+// pageable memory may read its source after the call has returned: the runtime
+// promises no staging, this GPU reads pageable memory directly, and in a
+// captured graph the copy reads it at every replay. The host pays for the whole
+// parameter, so there are three sizes of it; larger tables take several launches
+// of the largest.
+template <int WORDS>
+struct PutWords {
+    uint32_t w[WORDS];
+};
+constexpr int kPutSmall = 256, kPutMiddle = 2048, kPutLarge = 8000;   // (a kernel's parameters hold 32,764 bytes)
+template <int WORDS>
+__global__ void __launch_bounds__(256) k_put(uint32_t* __restrict__ dst, uint32_t n,
+                                             const __grid_constant__ PutWords<WORDS> src) {
+    const uint32_t i = blockIdx.x * 256 + threadIdx.x;
+    if (i < n) dst[i] = src.w[i];
+}
+template <int WORDS>
+int put_words(uint32_t* dst, const uint8_t* src, uint32_t n, cudaStream_t st) {
+    PutWords<WORDS> v;
+    memcpy(v.w, src, (size_t)n * 4);
+    k_put<WORDS><<<(n + 255) / 256, 256, 0, st>>>(dst, n, v);
+    PRODM_CHECK_LAUNCH("k_put");
+    return PRODM_OK;
+}
+
 }  // namespace
+
+// Tables above eight launches (factors of dims of tens of thousands of nodes)
+// are copied, and the call waits for the copy.
+int launch_put(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+    if (bytes > 8 * (size_t)kPutLarge * 4) {
+        PRODM_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
+        PRODM_CUDA(cudaStreamSynchronize(st));
+        return PRODM_OK;
+    }
+    uint32_t* to = (uint32_t*)dst;
+    const uint8_t* from = (const uint8_t*)src;
+    int rc = PRODM_OK;
+    for (size_t n = bytes / 4; n && !rc;) {
+        const uint32_t m = (uint32_t)(n < kPutLarge ? n : kPutLarge);
+        rc = m <= kPutSmall    ? put_words<kPutSmall>(to, from, m, st)
+             : m <= kPutMiddle ? put_words<kPutMiddle>(to, from, m, st)
+                               : put_words<kPutLarge>(to, from, m, st);
+        to += m;
+        from += (size_t)m * 4;
+        n -= m;
+    }
+    return rc;
+}
 
 int launch_gr_pack(const void* planes, uint64_t cap, const uint32_t* sizes, int B, uint64_t nblocks, const uint8_t* rbs,
                    int word_bytes, uint8_t* dst, cudaStream_t st) {
@@ -110,12 +164,13 @@ int launch_gr_pack(const void* planes, uint64_t cap, const uint32_t* sizes, int 
     return PRODM_OK;
 }
 
-int launch_unpack_planes(const uint8_t* src, const uint64_t* src_off, const uint64_t* nwords, int nplanes,
-                         int word_bytes, void* const* dst, uint64_t max_words, cudaStream_t st) {
-    if (nplanes <= 0) return PRODM_OK;
-    dim3 grid(grid_for(max_words, 256, 4), nplanes);
-    if (word_bytes == 4) k_unpack_planes<uint32_t><<<grid, 256, 0, st>>>(src, src_off, nwords, (uint32_t* const*)dst);
-    else k_unpack_planes<uint64_t><<<grid, 256, 0, st>>>(src, src_off, nwords, (uint64_t* const*)dst);
+int launch_unpack_planes(const uint8_t* src, const UnpackSet& set, int word_bytes, void** table, cudaStream_t st) {
+    if (set.n <= 0) return PRODM_OK;
+    uint64_t most = 0;
+    for (int p = 0; p < set.n; p++) most = set.words[p] > most ? set.words[p] : most;
+    dim3 grid(grid_for(most, 256, 4), set.n);
+    if (word_bytes == 4) k_unpack_planes<uint32_t><<<grid, 256, 0, st>>>(src, set, table);
+    else k_unpack_planes<uint64_t><<<grid, 256, 0, st>>>(src, set, table);
     PRODM_CHECK_LAUNCH("k_unpack_planes");
     return PRODM_OK;
 }

@@ -941,10 +941,12 @@ int launch_pb_parse(const std::vector<PbParseJob>& jobs, cudaStream_t st) {
         for (const uint64_t* p : j.planes) hv.push_back((uint64_t)(uintptr_t)p);
         for (uint64_t w : j.nwords) hv.push_back(w);
     }
-    uint8_t* scratch;
-    PRODM_CUDA(scratch_alloc((void**)&scratch, head + fl + planes * PZ_R * PZ_E * 4, st));
-    cudaError_t e = cudaMemcpyAsync(scratch, hv.data(), hv.size() * 8, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(scratch + head, 0, fl, st);
+    Scratch mem(st);
+    PRODM_CUDA(mem.alloc(head + fl + planes * PZ_R * PZ_E * 4));
+    uint8_t* scratch = mem.get();
+    const int rc = launch_put(scratch, hv.data(), hv.size() * 8, st);
+    if (rc) return rc;
+    cudaError_t e = cudaMemsetAsync(scratch + head, 0, fl, st);
     const unsigned resident = resident_ctas((const void*)k_pb_parse, PZ_T, sizeof(PzShared));
     size_t at = 0, next = 0;
     while (e == cudaSuccess && next < jobs.size()) {
@@ -975,7 +977,6 @@ int launch_pb_parse(const std::vector<PbParseJob>& jobs, cudaStream_t st) {
         void* args[] = {(void*)&set};
         e = cudaLaunchCooperativeKernel((const void*)k_pb_parse, dim3(ctas), dim3(PZ_T), args, sizeof(PzShared), st);
     }
-    cudaFreeAsync(scratch, st);
     if (e != cudaSuccess) return cuda_status(e, "k_pb_parse");
     return PRODM_OK;
 }
