@@ -297,15 +297,17 @@ int prodm_mdr_level_info(prodm_mdr* h, uint32_t* h_sizes, double* h_bounds, doub
  * extension carrying the squared-error tables; *len receives the size. */
 int prodm_mdr_metadata(prodm_mdr* h, uint8_t* h_buf, size_t capacity, size_t* len, void* stream);
 /* reference level-file bytes of one level into dst: dst_is_host 0 device
- * memory filled in stream order, 1 host memory (returns when the bytes are there), 2 pinned host
- * memory filled asynchronously in stream order (synchronise the stream, or
- * wait on an event recorded after the call, before reading it). */
+ * memory, 1 host memory (either returns when the bytes are there, to be read
+ * from any stream), 2 pinned host memory filled asynchronously in stream order
+ * (synchronise the stream, or wait on an event recorded after the call, before
+ * reading it). */
 int prodm_mdr_export_level(prodm_mdr* h, int level, void* dst, uint64_t capacity, int dst_is_host, uint64_t* len,
                            void* stream);
 /* bytes [offset, offset + bytes) of the same level file into dst (dst_is_host
- * as above): a reader can start on the first planes of a level before the
- * rest of the file is out (ConcatLevelFileRetriever reads level files in
- * such consecutive pieces, FileRetriever.hpp:15-35) */
+ * as above, but device memory too is filled in stream order): a reader can
+ * start on the first planes of a level before the rest of the file is out
+ * (ConcatLevelFileRetriever reads level files in such consecutive pieces,
+ * FileRetriever.hpp:15-35) */
 int prodm_mdr_export_level_range(prodm_mdr* h, int level, uint64_t offset, uint64_t bytes, void* dst,
                                  int dst_is_host, void* stream);
 

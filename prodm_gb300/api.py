@@ -29,12 +29,6 @@ def _stream(stream=None):
     return C.c_void_p(s.cuda_stream)
 
 
-def _order_after(stream):
-    """Device results written on another stream are there for the current one."""
-    if stream is not None and stream != torch.cuda.current_stream():
-        torch.cuda.current_stream().wait_stream(stream)
-
-
 def _u32(seq):
     a = (C.c_uint32 * len(seq))(*[int(x) for x in seq])
     return a
@@ -321,7 +315,6 @@ class MDRField:
         call("prodm_mdr_export_level", self.h, level, None, 0, 0, C.byref(n), _stream(stream))
         buf = torch.empty(max(n.value, 1), dtype=torch.uint8, device="cuda")
         call("prodm_mdr_export_level", self.h, level, _ptr(buf), n.value, 0, C.byref(n), _stream(stream))
-        _order_after(stream)
         return buf[:n.value]
 
     def export_level_into(self, level, out, stream=None):
@@ -335,8 +328,6 @@ class MDRField:
         n = C.c_uint64()
         call("prodm_mdr_export_level", self.h, level, C.c_void_p(out.data_ptr()), out.numel(),
              0 if out.is_cuda else 2, C.byref(n), _stream(stream))
-        if out.is_cuda:
-            _order_after(stream)
         return n.value
 
     def export_level_range_into(self, level, offset, out, stream=None):
@@ -349,8 +340,6 @@ class MDRField:
             raise ValueError("host output must be pinned memory")
         call("prodm_mdr_export_level_range", self.h, level, int(offset), out.numel(),
              C.c_void_p(out.data_ptr()) if out.numel() else None, 0 if out.is_cuda else 2, _stream(stream))
-        if out.is_cuda:
-            _order_after(stream)
 
     def set_lossless(self, latter_index=26, stream=None):
         """Lossless stage on (latter_index >= 0, the reference's default 26) or off (None / < 0)."""

@@ -2096,7 +2096,7 @@ int prodm_mdr_metadata(prodm_mdr* h, uint8_t* buf, size_t cap, size_t* len, void
 static int export_raw_level(prodm_mdr* h, int level, void* dst, uint64_t cap, int dst_is_host, uint64_t* len,
                             const uint32_t* dsizes, cudaStream_t st, const uint32_t* hsizes = nullptr) {
     const int B = h->B;
-    const bool wait = dst_is_host == 1;   // device and pinned memory are filled in stream order
+    const bool wait = dst_is_host != 2;
     std::vector<uint32_t> sz(B);
     if (hsizes) {
         std::memcpy(sz.data(), hsizes, B * 4);
@@ -2250,7 +2250,7 @@ int prodm_mdr_export_level(prodm_mdr* h, int level, void* dst, uint64_t cap, int
                                 h->hsz.data() + (size_t)level * B);
     }
     // lossless stage: the level's stored streams, compressed straight into
-    // their places; device memory and pinned memory in stream order
+    // their places
     const uint32_t* stored = ll_stored_sizes(h);
     if (!stored) return ll_no_sizes();
     stored += (size_t)level * B;
@@ -2278,10 +2278,8 @@ int prodm_mdr_export_level(prodm_mdr* h, int level, void* dst, uint64_t cap, int
         out += stored[p];
     }
     if ((rc = ll_store(parts, st))) return rc;
-    if (dst_is_host) {
-        PRODM_CUDA(cudaMemcpyAsync(dst, host.get(), total, cudaMemcpyDeviceToHost, st));
-        if (dst_is_host == 1) PRODM_CUDA(cudaStreamSynchronize(st));
-    }
+    if (dst_is_host) PRODM_CUDA(cudaMemcpyAsync(dst, host.get(), total, cudaMemcpyDeviceToHost, st));
+    if (dst_is_host != 2) PRODM_CUDA(cudaStreamSynchronize(st));
     return PRODM_OK;
 }
 
