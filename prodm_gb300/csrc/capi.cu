@@ -438,7 +438,7 @@ struct prodm_decoder {
         uint8_t* state = nullptr;     // grouped: rbs, chunk_off, signs; per-bit: pbrows
         size_t bytes = 0;
         cudaEvent_t used = nullptr;   // behind the last call's work on the state,
-        bool open = false;            // unless that call left before it was recorded
+        bool open = false;            // unless a call is on it or could not record it
         uint8_t* rbs = nullptr;
         uint32_t* chunk_off = nullptr;
         void* signs = nullptr;
@@ -447,22 +447,25 @@ struct prodm_decoder {
         // the state comes from the scratch pool: a decoder per field and pass
         // is the reference's use, and cudaMalloc and cudaFree wait for the device
         cudaError_t hold(size_t need, cudaStream_t st) {
-            if (state && bytes >= need && !open) {
-                open = true;
-                return used ? cudaStreamWaitEvent(st, used, 0) : cudaSuccess;
-            }
+            if (state && bytes >= need) return enter(st);
             drop();
-            open = true;
             const cudaError_t e = scratch_alloc((void**)&state, need, st);
             bytes = e == cudaSuccess ? need : 0;
+            open = true;
             return e;
         }
-        cudaError_t mark(cudaStream_t st) {
+        // every call's work on the state comes behind the last call's, on
+        // whichever streams the two are
+        cudaError_t enter(cudaStream_t st) {
+            const cudaError_t e = open ? cudaDeviceSynchronize() : used ? cudaStreamWaitEvent(st, used, 0) : cudaSuccess;
+            open = true;
+            return e;
+        }
+        void leave(cudaStream_t st) {
             cudaError_t e = cudaSuccess;
             if (!used) e = cudaEventCreateWithFlags(&used, cudaEventDisableTiming);
             if (e == cudaSuccess) e = cudaEventRecord(used, st);
-            open = open && e != cudaSuccess;
-            return e;
+            open = e != cudaSuccess;
         }
         void drop() {   // behind the last use, whatever became of its stream
             if (!state) return;
@@ -470,7 +473,31 @@ struct prodm_decoder {
             else cudaEventSynchronize(used);
             cudaFree(state);
             state = nullptr;
+            open = false;
         }
+    };
+    // one call's use of a level: from hold or enter to wherever the call returns
+    class Use {
+      public:
+        Use(Level& l, cudaStream_t st) : l_(l), st_(st) {}
+        Use(const Use&) = delete;
+        Use& operator=(const Use&) = delete;
+        ~Use() {
+            if (in_) l_.leave(st_);
+        }
+        cudaError_t hold(size_t need) {
+            in_ = true;
+            return l_.hold(need, st_);
+        }
+        cudaError_t enter() {
+            in_ = true;
+            return l_.enter(st_);
+        }
+
+      private:
+        Level& l_;
+        cudaStream_t st_;
+        bool in_ = false;
     };
     std::vector<Level> levels;
     ~prodm_decoder() {
@@ -493,9 +520,10 @@ int pb_progressive_decode(prodm_decoder* h, const uint8_t* blob, const uint32_t*
     if ((int)h->levels.size() <= level) h->levels.resize(level + 1);
     auto& L = h->levels[level];
     const uint64_t rw = pb_row_words(n);
+    prodm_decoder::Use use(L, st);
     if (!L.have) {
         if (s != 0) return fail(PRODM_EINVAL, "decode: the first call for a level must start at plane 0");
-        PRODM_CUDA(L.hold((uint64_t)(B + 2) * rw * 4 + 16, st));
+        PRODM_CUDA(use.hold((uint64_t)(B + 2) * rw * 4 + 16));
         L.pbrows = (uint32_t*)L.state;
         int rc = launch_pb_init_unseen(L.pbrows + (uint64_t)(B + 1) * rw, L.pbrows + (uint64_t)B * rw, n, st);
         if (rc) return rc;
@@ -505,6 +533,8 @@ int pb_progressive_decode(prodm_decoder* h, const uint8_t* blob, const uint32_t*
         L.parsed = 0;
     } else if (L.n != n || L.B != B) {
         return fail(PRODM_EINVAL, "decode: level shape changed between calls");
+    } else {
+        PRODM_CUDA(use.enter());
     }
     if (s != L.parsed)
         return fail(PRODM_EINVAL, "decode: per-bit planes are decoded in order; this level continues at plane " +
@@ -554,7 +584,6 @@ int pb_progressive_decode(prodm_decoder* h, const uint8_t* blob, const uint32_t*
     if (!rc) {
         cudaError_t e = cudaMemcpyAsync(&hstat, status, 4, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        if (e == cudaSuccess) e = L.mark(st);
         if (e != cudaSuccess) rc = cuda_status(e, "per-bit decode");
     }
     if (tmp) cudaFreeAsync(tmp, st);
@@ -599,6 +628,7 @@ int progressive_decode_impl(prodm_decoder* h, const uint8_t* blob, const uint32_
     }
     if ((int)h->levels.size() <= level) h->levels.resize(level + 1);
     auto& L = h->levels[level];
+    prodm_decoder::Use use(L, st);
     const uint64_t nch = gr_nchunks(nb);
     if (!L.have) {
         if (s != 0) return fail(PRODM_EINVAL, "decode: the first call for a level must start at plane 0");
@@ -608,7 +638,7 @@ int progressive_decode_impl(prodm_decoder* h, const uint8_t* blob, const uint32_
         PRODM_CUDA(cudaStreamSynchronize(st));
         if (cnt != nb) return fail(PRODM_ECORRUPT, "decode: block count in stream 0 does not match n");
         const size_t a0 = Workspace::align(nb * sizeof(T)), a1 = Workspace::align(nch * B * 4);
-        PRODM_CUDA(L.hold(a0 + a1 + nb, st));
+        PRODM_CUDA(use.hold(a0 + a1 + nb));
         L.signs = L.state;
         L.chunk_off = (uint32_t*)(L.state + a0);
         L.rbs = L.state + a0 + a1;
@@ -628,6 +658,8 @@ int progressive_decode_impl(prodm_decoder* h, const uint8_t* blob, const uint32_
         L.B = B;
     } else if (L.n != n || L.B != B) {
         return fail(PRODM_EINVAL, "decode: level shape changed between calls");
+    } else {
+        PRODM_CUDA(use.enter());
     }
     // unpack planes [s, s+num) into aligned scratch, and the table of the planes' addresses behind them
     if (num > 64) return fail(PRODM_EINVAL, "decode: grouped streams hold at most 64 planes");
@@ -656,9 +688,7 @@ int progressive_decode_impl(prodm_decoder* h, const uint8_t* blob, const uint32_
     set.seg[0].signs = (typename Traits<T>::S*)L.signs;
     set.seg[0].n = n;
     set.seg[0].exp = exp;
-    if ((rc = launch_gr_decode<T>(set, B, s, s + num, st))) return rc;
-    PRODM_CUDA(L.mark(st));
-    return PRODM_OK;
+    return launch_gr_decode<T>(set, B, s, s + num, st);
 }
 }  // namespace
 }  // namespace prodm
