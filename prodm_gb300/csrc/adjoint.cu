@@ -42,6 +42,31 @@ __host__ __device__ inline uint64_t adj_items(const Box& F, const Box& C, uint64
     return body + (32 * groups < C.n[2] ? (uint64_t)C.n[0] * ((C.n[1] + 31) / 32) : 0);
 }
 
+__device__ __forceinline__ bool not_finite(float v) { return (__float_as_uint(v) & 0x7f800000u) == 0x7f800000u; }
+__device__ __forceinline__ bool not_finite(double v) { return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000; }
+
+// The sum at the coarse node *p with each of the up to 27 values weighted before
+// it is added, node by node: for where the dim-by-dim sum, whose pairs are added
+// before they are halved, is not finite. have: odd nodes before (even bits) and
+// behind (odd bits) it, dims 0, 1, 2.
+template <class T>
+__device__ __noinline__ T adj_sum_ordered(const T* __restrict__ p, int64_t s0, int64_t s1, uint32_t have) {
+    T acc = 0;
+    for (int a = 0; a < 3; a++) {
+        if (a && !(have >> (a - 1) & 1u)) continue;
+        for (int b = 0; b < 3; b++) {
+            if (b && !(have >> (b + 1) & 1u)) continue;
+            for (int c = 0; c < 3; c++) {
+                if (c && !(have >> (c + 3) & 1u)) continue;
+                const T w = (a ? (T)0.5 : (T)1) * (b ? (T)0.5 : (T)1) * (c ? (T)0.5 : (T)1);
+                const int64_t at = (a ? 2 * a - 3 : 0) * s0 + (b ? 2 * b - 3 : 0) * s1 + (c ? 2 * c - 3 : 0);
+                acc += w * p[at];
+            }
+        }
+    }
+    return acc;
+}
+
 template <class T, bool COEF>
 __device__ __forceinline__ void adj_patch_item(const T* __restrict__ g, const Box& F, const Box& C,
                                                T* __restrict__ gcoef, T* __restrict__ gc, uint64_t item, uint32_t lane) {
@@ -91,12 +116,15 @@ __device__ __forceinline__ void adj_patch_item(const T* __restrict__ g, const Bo
     }
     Step S;
     load_step(b0, S);
+    bool bad = false;
     for (uint32_t b = b0; b < b1; b++) {
         Step N = S;
         if (b + 1 < b1) load_step(b + 1, N);
         const T hm = sum(S.me), om = sum(S.mo), ha = sum(S.ae), oa = sum(S.ao), hb = sum(S.be), ob = sum(S.bo);
         const T m = hm + (T)0.5 * (lm + om), a = ha + (T)0.5 * (la + oa), d = hb + (T)0.5 * (lb + ob);
-        if (ld) gc[((uint64_t)i * C1 + b) * C2 + c] = m + (T)0.5 * (a + d);
+        const T v = m + (T)0.5 * (a + d);
+        if (ld) gc[((uint64_t)i * C1 + b) * C2 + c] = v;
+        bad |= not_finite(v);
         if (COEF) {
             const bool odd = b < O1;
             const uint64_t r00 = level_rank(i, b, C2, F, C);   // even-even row: odd nodes only
@@ -122,6 +150,14 @@ __device__ __forceinline__ void adj_patch_item(const T* __restrict__ g, const Bo
         lb = ob;
         S = N;
     }
+    if (bad && ld)
+        for (uint32_t b = b0; b < b1; b++) {
+            T* v = gc + ((uint64_t)i * C1 + b) * C2 + c;
+            if (not_finite(*v))
+                *v = adj_sum_ordered(mid + (uint64_t)min(2 * b, F.n[1] - 1) * s1 + xc, (int64_t)s0, (int64_t)s1,
+                                     (uint32_t)before | behind << 1 | (b >= 1 && b - 1 < O1) << 2 | (b < O1) << 3 |
+                                         (c >= 1 && c - 1 < P) << 4 | (uint32_t)pair << 5);
+        }
 }
 
 // the columns behind the groups (no odd node behind them): a lane per b
@@ -147,7 +183,11 @@ __device__ __forceinline__ void adj_lone_item(const T* __restrict__ g, const Box
             return row(plane, on, x1) + (T)0.5 * (row(plane, on && left, x1 - 1) + row(plane, on && odd, x1 + 1));
         };
         const T m = three(mid, true), a = three(mid - s0, before), d = three(mid + s0, behind);
-        gc[((uint64_t)i * C1 + b) * C2 + c] = m + (T)0.5 * (a + d);
+        T v = m + (T)0.5 * (a + d);
+        if (not_finite(v))
+            v = adj_sum_ordered(mid + (uint64_t)x1 * s1 + xc, (int64_t)s0, (int64_t)s1,
+                                (uint32_t)before | behind << 1 | left << 2 | odd << 3 | lo << 4);
+        gc[((uint64_t)i * C1 + b) * C2 + c] = v;
         if (COEF) {
             const T* p = mid + (uint64_t)x1 * s1 + xc;
             if (odd) gcoef[level_rank(i, C1 + b, 0, F, C) + c] = p[s1];
