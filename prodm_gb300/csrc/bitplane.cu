@@ -1467,8 +1467,7 @@ int nb_encode_levels_grid(int with_errors) {
 }
 
 int launch_nb_encode_levels(const ChunkSeg* segs, int nseg, uint64_t total_chunks, int B, double* partial,
-                            const uint32_t* keys, double* errs_out, cudaStream_t st) {
-    (void)keys;   // each segment carries its level's key
+                            double* errs_out, cudaStream_t st) {
     if (errs_out) return nb_err_launch(segs, ChunkSeg{}, nseg, total_chunks, B, 0, partial, errs_out, st);
     return launch_nb_encode_segments(segs, nseg, total_chunks, B, (unsigned)nb_encode_levels_grid(0), st, true);
 }
@@ -1598,6 +1597,8 @@ int launch_gr_decode(GrSet<T> set, int B, int s, int e, cudaStream_t st) {
     }
     return PRODM_OK;
 }
+
+#undef PRODM_CHAIN
 
 template <class T>
 int launch_sq_collect(const T* x, uint64_t n, int B, T maxv, double* partial, double* out, cudaStream_t st) {

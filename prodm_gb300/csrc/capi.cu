@@ -1093,8 +1093,7 @@ int mdr_refactor(prodm_mdr* h, const T* field, cudaStream_t st) {
     if (h->eseg && sizeof(T) == 4) {
         // fp32 negabinary: every level in one launch (timed as the finest level)
         Stage sg(h, 1, L, st);
-        return launch_nb_encode_levels(h->eseg, L + 1, h->eseg_chunks, B, h->lpartial, (const uint32_t*)keys,
-                                       h->sq ? h->sqerr : nullptr, st);
+        return launch_nb_encode_levels(h->eseg, L + 1, h->eseg_chunks, B, h->lpartial, h->sq ? h->sqerr : nullptr, st);
     }
     // every level in one go (timed as the finest level), but for the fp64
     // negabinary encoder and the error tables, which take a level per launch

@@ -317,7 +317,6 @@ __device__ __forceinline__ T corner_tree_mid(int m01, const T* q, const T* qn) {
     if (m01 != 3) return avg_rn(avg_rn(q[0], qn[0]), avg_rn(q[1], qn[1]));
     return avg_rn(avg_rn(avg_rn(q[0], qn[0]), avg_rn(q[1], qn[1])), avg_rn(avg_rn(q[2], qn[2]), avg_rn(q[3], qn[3])));
 }
-__host__ __device__ inline int corner_count(int m01) { return m01 == 0 ? 1 : (m01 == 3 ? 4 : 2); }
 
 // last segment whose first global item is <= g (segments sorted by `begin`)
 template <class Seg>

@@ -3,13 +3,15 @@
 //
 // The unfused path writes the decoded level coefficients (n_L values) and
 // reads them back in the recomposition; at the finest level that is most of
-// the field. Here one warp owns one fine row (x0, x1): the coefficients of a
-// row occupy one contiguous run of interleaved ranks, so the warp decodes the
-// 32-value blocks covering that run (one bit transpose per block) into shared
-// memory and then writes the recomposed row with coalesced stores. Decoding
-// and recomposition use exactly the arithmetic of the standalone kernels
-// (NegaBinaryBPEncoder.hpp:132-192; the multilinear interpolation of the
-// hierarchical basis), so the output is bit-identical to the unfused path.
+// the field. Here a CTA takes a unit of consecutive fine rows (x0, x1), whose
+// coefficients occupy one contiguous run of interleaved ranks: TMA brings the
+// run's plane words into shared memory, two threads a block transpose them back
+// to values there, and a warp a row (several a row where rows are long) writes
+// the recomposed rows with coalesced stores. In the warp-specialised kernels
+// some warps decode the next unit while the others recompose the last one.
+// Decoding and recomposition use exactly the arithmetic of the standalone
+// kernels (NegaBinaryBPEncoder.hpp:132-192; the multilinear interpolation of
+// the hierarchical basis), so the output is bit-identical to the unfused path.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 

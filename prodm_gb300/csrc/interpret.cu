@@ -5,9 +5,11 @@
 // estimators of MaxErrorEstimator.hpp:13-68 and SquaredErrorEstimator.hpp:
 // 12-68. The estimators compute in the data type T exactly as the reference
 // templates do, and the max-heap follows the sift order of the C++ standard
-// library's priority_queue, so ties resolve identically. One thread runs one
-// interpretation (one field); the kernel takes all inputs from device memory
-// so a whole retrieval can run without a host round trip.
+// library's priority_queue, so ties resolve identically. A CTA takes one
+// field: its threads tabulate every efficiency and order the pops by blocks of
+// entries; where the stop depends on a tie, one warp or one thread runs the
+// heap itself. All inputs come from device memory, so a whole retrieval can run
+// without a host round trip.
 #include <climits>
 
 #include "common.cuh"

@@ -130,7 +130,7 @@ int nb_encode_levels_grid(int with_errors);
 int launch_nb_encode_segments(const ChunkSeg* segs, int nseg, uint64_t total_chunks, int B, unsigned grid, cudaStream_t st,
                               bool pdl);
 int launch_nb_encode_levels(const ChunkSeg* segs, int nseg, uint64_t total_chunks, int B, double* partial,
-                            const uint32_t* keys, double* errs_out, cudaStream_t st);
+                            double* errs_out, cudaStream_t st);
 
 // fused.cu
 bool decode_recompose_nb32_ok(const Box& F);

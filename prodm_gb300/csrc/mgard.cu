@@ -49,74 +49,41 @@ __device__ __forceinline__ T interp(int mask, Get at) {
     }
 }
 
-template <class K>
-__device__ __forceinline__ K warp_max(K v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        K w = __shfl_xor_sync(0xffffffffu, v, o);
-        v = max_key(w, v);
-    }
-    return v;
-}
-
 // ---------------------------------------------------------------------------
-// forward level: in = natural-order fine box (strides s0, s1, 1)
-// PACKED:  coef[rank] and coarse[compact C box]
-// INPLACE: out[reordered position] with strides o0, o1, 1 (coef and coarse)
+// forward level by elements: in = compact natural-order fine box; out = its
+// reordered positions (strides o0, o1, 1), coarse values in the corner
 // fnat (optional): natural-order coefficient field, zero at coarse nodes
 // ---------------------------------------------------------------------------
-template <class T, bool PACKED>
-__global__ void k_decompose_level(const T* __restrict__ in, uint64_t s0, uint64_t s1, Box F, Box C,
-                                  T* __restrict__ coef, T* __restrict__ coarse, uint64_t o0, uint64_t o1,
-                                  T* __restrict__ fnat, typename KeyOf<T>::type* maxkey_level,
-                                  typename KeyOf<T>::type* maxkey_coarse) {
-    using K = typename KeyOf<T>::type;
-    K mk = 0, mc = 0;
-    const uint64_t total = F.size();
+template <class T>
+__global__ void k_decompose_level(const T* __restrict__ in, Box F, Box C, T* __restrict__ out, uint64_t o0, uint64_t o1,
+                                  T* __restrict__ fnat) {
+    const uint64_t total = F.size(), s0 = (uint64_t)F.n[1] * F.n[2], s1 = F.n[2];
     for (uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
          idx += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t x0, x1, x2;
         split3(idx, F, x0, x1, x2);
-        const T* p = in + x0 * s0 + x1 * s1 + x2;
+        const T* p = in + idx;
         T v = *p;
         int mask = (is_coarse(x0, F.n[0]) ? 0 : 1) | (is_coarse(x1, F.n[1]) ? 0 : 2) | (is_coarse(x2, F.n[2]) ? 0 : 4);
         uint32_t r0 = reord(x0, F.n[0], C.n[0]), r1 = reord(x1, F.n[1], C.n[1]), r2 = reord(x2, F.n[2], C.n[2]);
-        if (mask == 0) {
-            if (PACKED) coarse[((uint64_t)r0 * C.n[1] + r1) * C.n[2] + r2] = v;
-            else coef[r0 * o0 + r1 * o1 + r2] = v;
-            if (fnat) fnat[idx] = (T)0;
-            K k = abs_key(v);
-            mc = max_key(k, mc);
-        } else {
+        if (mask) {
             auto at = [&](int d0, int d1, int d2) -> T { return __ldg(p + (int64_t)d0 * (int64_t)s0 + (int64_t)d1 * (int64_t)s1 + d2); };
-            T c = sub_rn(v, interp<T>(mask, at));
-            if (PACKED) coef[level_rank(r0, r1, r2, F, C)] = c;
-            else coef[r0 * o0 + r1 * o1 + r2] = c;
-            if (fnat) fnat[idx] = c;
-            K k = abs_key(c);
-            mk = max_key(k, mk);
+            v = sub_rn(v, interp<T>(mask, at));
         }
-    }
-    if (maxkey_level) {
-        mk = warp_max(mk);
-        if ((threadIdx.x & 31) == 0 && mk) atomicMax(maxkey_level, mk);
-    }
-    if (maxkey_coarse) {
-        mc = warp_max(mc);
-        if ((threadIdx.x & 31) == 0 && mc) atomicMax(maxkey_coarse, mc);
+        out[r0 * o0 + r1 * o1 + r2] = v;
+        if (fnat) fnat[idx] = mask ? v : (T)0;
     }
 }
 
 // ---------------------------------------------------------------------------
-// inverse level: coarse values (already corrected back to nodal values for
-// the orthogonal basis) + coefficients -> natural-order fine box.
-// PACKED:  coarse = compact C box, coef = packed level coefficients
-// INPLACE: both read from a compact reordered copy of the level box (rin)
+// inverse level by elements: rin = compact reordered copy of the level box, its
+// coarse corner nodal values (already corrected for the orthogonal basis) ->
+// natural-order fine box
 // ---------------------------------------------------------------------------
-template <class T, bool PACKED>
-__global__ void k_recompose_level(const T* __restrict__ coarse, const T* __restrict__ coef, Box F, Box C,
-                                  T* __restrict__ out, uint64_t s0, uint64_t s1) {
-    const uint64_t total = F.size();
+template <class T>
+__global__ void k_recompose_level(const T* __restrict__ rin, Box F, Box C, T* __restrict__ out, uint64_t s0,
+                                  uint64_t s1) {
+    const uint64_t total = F.size(), fs0 = (uint64_t)F.n[1] * F.n[2], fs1 = F.n[2];
     for (uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
          idx += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t x0, x1, x2;
@@ -126,33 +93,17 @@ __global__ void k_recompose_level(const T* __restrict__ coarse, const T* __restr
         uint32_t c0 = (mask & 1) ? (x0 >> 1) : reord(x0, F.n[0], C.n[0]);
         uint32_t c1 = (mask & 2) ? (x1 >> 1) : reord(x1, F.n[1], C.n[1]);
         uint32_t c2 = (mask & 4) ? (x2 >> 1) : reord(x2, F.n[2], C.n[2]);
+        const T* cb = rin + c0 * fs0 + c1 * fs1 + c2;
         T v;
-        if (PACKED) {
-            const T* cb = coarse + ((uint64_t)c0 * C.n[1] + c1) * C.n[2] + c2;
-            const uint64_t cs0 = (uint64_t)C.n[1] * C.n[2], cs1 = C.n[2];
-            if (mask == 0) {
-                v = *cb;
-            } else {
-                // corner offsets: -1 -> low corner (0), +1 -> next coarse node (1)
-                auto at = [&](int d0, int d1, int d2) -> T {
-                    return __ldg(cb + (d0 > 0 ? cs0 : 0) + (d1 > 0 ? cs1 : 0) + (d2 > 0 ? 1 : 0));
-                };
-                uint32_t r0 = reord(x0, F.n[0], C.n[0]), r1 = reord(x1, F.n[1], C.n[1]), r2 = reord(x2, F.n[2], C.n[2]);
-                v = add_rn(coef[level_rank(r0, r1, r2, F, C)], interp<T>(mask, at));
-            }
+        if (mask == 0) {
+            v = *cb;
         } else {
-            // rin: compact reordered fine box; coarse region = [0,C)
-            const uint64_t fs0 = (uint64_t)F.n[1] * F.n[2], fs1 = F.n[2];
-            const T* cb = coarse + c0 * fs0 + c1 * fs1 + c2;
-            if (mask == 0) {
-                v = *cb;
-            } else {
-                auto at = [&](int d0, int d1, int d2) -> T {
-                    return __ldg(cb + (d0 > 0 ? fs0 : 0) + (d1 > 0 ? fs1 : 0) + (d2 > 0 ? 1 : 0));
-                };
-                uint32_t r0 = reord(x0, F.n[0], C.n[0]), r1 = reord(x1, F.n[1], C.n[1]), r2 = reord(x2, F.n[2], C.n[2]);
-                v = add_rn(coef[r0 * fs0 + r1 * fs1 + r2], interp<T>(mask, at));
-            }
+            // corner offsets: -1 -> low corner (0), +1 -> next coarse node (1)
+            auto at = [&](int d0, int d1, int d2) -> T {
+                return __ldg(cb + (d0 > 0 ? fs0 : 0) + (d1 > 0 ? fs1 : 0) + (d2 > 0 ? 1 : 0));
+            };
+            uint32_t r0 = reord(x0, F.n[0], C.n[0]), r1 = reord(x1, F.n[1], C.n[1]), r2 = reord(x2, F.n[2], C.n[2]);
+            v = add_rn(rin[r0 * fs0 + r1 * fs1 + r2], interp<T>(mask, at));
         }
         out[x0 * s0 + x1 * s1 + x2] = v;
     }
@@ -744,7 +695,7 @@ __global__ void __launch_bounds__(256) k_interleave_rows(T* __restrict__ data, u
 // one warp per row, four warps per CTA (f64 recompositions of 513 x 257 x 257's
 // small levels 86 us, with eight 90 and with one 92; fp32 1 % from eight, with
 // two 10 % slower); enough CTAs for full occupancy
-unsigned row_threads(uint32_t) { return 128; }
+constexpr unsigned kRowThreads = 128;
 // PRODM_DECOMPOSE_PATCH=0 keeps every level on the row kernels (decomposition and
 // recomposition; read per launch)
 bool decompose_patch_enabled() {
@@ -768,7 +719,7 @@ template <class T>
 int launch_decompose_level_packed(const T* in, uint64_t s0, uint64_t s1, const Box& F, const Box& C, T* coef, T* coarse,
                                   T* fnat, void* maxkey_level, void* maxkey_coarse, cudaStream_t st) {
     using K = typename KeyOf<T>::type;
-    const unsigned th = row_threads(F.n[2]);
+    const unsigned th = kRowThreads;
     count_launch();
     if (!fnat && patch_level(F, C) && decompose_patch_enabled()) {
         const auto kernel = F.n[0] == 1 ? k_decompose_patch<T, kPlaneAhead> : k_decompose_patch<T, 0>;
@@ -792,8 +743,7 @@ int launch_decompose_level_inplace(const T* in, const Box& F, const Box& C, T* o
         PRODM_CHECK_LAUNCH("k_decompose_patch_inplace");
         return PRODM_OK;
     }
-    k_decompose_level<T, false><<<grid_for(F.size(), th), th, 0, st>>>(
-        in, (uint64_t)F.n[1] * F.n[2], F.n[2], F, C, out, nullptr, o0, o1, fnat, nullptr, nullptr);
+    k_decompose_level<T><<<grid_for(F.size(), th), th, 0, st>>>(in, F, C, out, o0, o1, fnat);
     PRODM_CHECK_LAUNCH("k_decompose_level");
     return PRODM_OK;
 }
@@ -801,7 +751,7 @@ int launch_decompose_level_inplace(const T* in, const Box& F, const Box& C, T* o
 template <class T>
 int launch_recompose_level_packed(const T* coarse, const T* coef, const Box& F, const Box& C, T* out, uint64_t s0,
                                   uint64_t s1, cudaStream_t st, bool pdl) {
-    const unsigned th = row_threads(F.n[2]);
+    const unsigned th = kRowThreads;
     count_launch();
     if (patch_level(F, C) && decompose_patch_enabled()) {
         const auto kernel = F.n[0] == 1 ? k_recompose_patch<T, kPlaneAhead> : k_recompose_patch<T, 0>;
@@ -825,7 +775,7 @@ int launch_recompose_level_inplace(const T* rin, const Box& F, const Box& C, T* 
         PRODM_CHECK_LAUNCH("k_recompose_patch_inplace");
         return PRODM_OK;
     }
-    k_recompose_level<T, false><<<grid_for(F.size(), th), th, 0, st>>>(rin, rin, F, C, out, s0, s1);
+    k_recompose_level<T><<<grid_for(F.size(), th), th, 0, st>>>(rin, F, C, out, s0, s1);
     PRODM_CHECK_LAUNCH("k_recompose_level");
     return PRODM_OK;
 }

@@ -34,10 +34,6 @@ __device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) 
 __device__ __forceinline__ bool pow2_normal(int e) { return e >= -126 && e <= 127; }
 __device__ __forceinline__ float scale2(float v, int e, bool fast, float sc) { return fast ? v * sc : ldexpf(v, e); }
 
-// (-2)^i as a float (exact)
-__device__ __forceinline__ constexpr float nbw(int i) { return (i & 1) ? -(float)(1u << i) : (float)(1u << i); }
-
-
 // asynchronous 16-byte global -> shared copy (cp.async), both addresses 16-byte aligned (L2 only)
 __device__ __forceinline__ void cp_async16(uint32_t* dst, const uint32_t* src) {
     const unsigned d = (unsigned)__cvta_generic_to_shared(dst);

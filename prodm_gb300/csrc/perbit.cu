@@ -423,8 +423,9 @@ __global__ void __launch_bounds__(PK_T) k_pb_pack_write(const uint32_t* __restri
 // parsed; the widths, which grow with the root of the distance from the
 // step's first group, are laid out over the threads once per chunk); then one
 // warp follows the chain of true starts through the slots, and two others
-// parse their words while the next step's windows are tried. A true start outside its window ends the step there, and the first
-// pair of a step has its exact start, so every step goes on. The groups
+// parse their words while the next step's windows are tried. A true start
+// outside its window ends the step there, and the first pair of a step has its
+// exact start, so every step goes on. The groups
 // without unseen elements hold one bit per element at offsets known once the
 // signs before them are counted. One warp of the CTA moves the masks: it
 // fetches the next chunk's and hands on the last one's while the other warps
@@ -436,7 +437,7 @@ __global__ void __launch_bounds__(PK_T) k_pb_pack_write(const uint32_t* __restri
 // 5.0 and 5.3 ms).
 // ---------------------------------------------------------------------------
 constexpr int PZ_R = 8;                      // ring depth (chunks)
-constexpr long long kPzSpin = 1ll << 24;     // x >= 256 ns per wait
+constexpr long long kPzSpin = 1ll << 24;     // polls per wait: an acquire load from L2 and a sleep of 0 to 64 ns each
 constexpr int PZ_N = 224;                    // parsing threads: starts tried per step
 constexpr int PZ_S = PZ_N + 64;              // and the warps that keep the true starts' words
 constexpr int PZ_T = PZ_S + 32;              // and the warp that moves the masks
