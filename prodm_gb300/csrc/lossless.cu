@@ -410,7 +410,7 @@ int launch_copies(const ZStream* d, const ZStream* h, size_t n, cudaStream_t st)
 // upload of descriptors and one launch per pass, where a level at a time
 // synchronised three times and a plane at a time copied once or twice
 // (257^3 fp32 files through the stage: 7.8 ms a pass of which the kernels
-// took 0.9; 0.87 ms now).
+// took 0.9; 1.05 ms now).
 int ll_sizes(const std::vector<LlPart>& parts, uint32_t* h_comp, cudaStream_t st) {
     std::vector<ZStream> ss;
     for (const LlPart& p : parts) ss.push_back(ZStream{p.src, nullptr, p.raw, 0, 0});
