@@ -49,7 +49,7 @@ class _Lib:
         self._setup()
 
     def _fn(self, name, restype, *args):
-        f = getattr(self.lib, name)
+        f = self.lib[name]   # an object of its own: threads declare and call side by side
         f.restype = restype
         f.argtypes = list(args)
         return f
